@@ -455,11 +455,26 @@ __global__ void k_export_records(ConvArgs a) {
   }
 }
 
-// Rows per warp segment: the CTA count should fill whole waves of the
-// resident CTAs (a partial last wave idles SMs), while each segment pays two
-// extra rows of gamma solves at its ends.
+// Rows per warp segment.  Grids that give every resident CTA 24 rows or more:
+// the CTA count should fill whole waves of the resident CTAs (a partial last
+// wave idles SMs), while each segment pays two extra rows of gamma solves at
+// its ends.  Smaller grids leave SMs idle at that length and each row of a
+// segment is a serial load-solve-update chain (about 0.4 us when few warps
+// share an SM), so their segments are short: one row while the grid has no
+// more rows of CTAs than resident slots, else 3 (one pass of the unrolled
+// loop), and 6 once 3-row segments oversubscribe the slots.  Measured, us per
+// step, whole columns (the rule above with nothing to choose) -> these:
+// 256^2 87 -> 3.1 (3 rows 3.7), 512^2 165 -> 4.7 (1 row 5.4, 6 rows 5.7),
+// 1024^2 317 -> 10.0 (1 row 13.6, 12 rows 11.2), 1531 x 1021 432 -> 13.1
+// (3 rows 13.5, 12 rows 13.5); variable mobility 1531 x 1021 411 -> 17.0
+// (3 rows 18.5, 12 rows 17.9).
 int segment_rows(int Nx, int Ny, int resident) {
   const int nbx = ((Nx + kCols - 1) / kCols + kWarps - 1) / kWarps;
+  const long long load = (long long)nbx * Ny;  // CTA rows
+  if (load < 24LL * resident) {
+    const int rows = load <= resident ? 1 : (load <= 6LL * resident ? 3 : 6);
+    return rows < Ny ? rows : Ny;
+  }
   int best = Ny;
   double best_score = 0.0;
   for (int waves = 1; waves <= 256; waves++) {

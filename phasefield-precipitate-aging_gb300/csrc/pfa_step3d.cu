@@ -469,7 +469,11 @@ __global__ void k_export3d(Conv3DArgs a) {
 }
 
 // z planes per segment: fill whole waves of resident CTAs, two extra planes
-// of gamma solves per segment; tiles of tx x ty output cells per plane
+// of gamma solves per segment; tiles of tx x ty output cells per plane.
+// Segments under 16 planes only where they fit one wave: a small grid's
+// columns leave SMs idle otherwise (FP32, us per step, whole columns ->
+// one wave of short segments: 32^3 29.4 -> 3.7, 64^3 47.5 -> 7.8, 96^3
+// 64.7 -> 13.0, 200 x 100 x 60 42.5 -> 17.4).
 int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
   const long long cols = (long long)((Nx + tx - 1) / tx) * ((Ny + ty - 1) / ty);
   int best = Nz;
@@ -478,7 +482,7 @@ int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
     const long long segs = (long long)waves * resident / cols;
     if (segs < 1) continue;
     const int planes = int((Nz + segs - 1) / segs);
-    if (planes < 16 && segs > 1) break;
+    if (planes < 16 && segs > 1 && waves > 1) break;
     const long long used = cols * ((Nz + planes - 1) / planes);
     const long long slots = ((used + resident - 1) / resident) * (long long)resident;
     const double score = double(used) / double(slots) / (1.0 + 2.0 / planes);
