@@ -207,6 +207,7 @@ static Step2DArgs step_args(State* s, double alpha, double dt) {
   std::memcpy(a.mask9, s->mask9, sizeof(a.mask9));
   a.nine = !s->five_point;
   a.varmob = s->varmob;
+  model_coef64(a.m, s->mask9, &a.c);
   a.k = s->fk;
   for (int i = 0; i < 2; i++)
     for (int j = 0; j < 2; j++) a.dtD[i][j] = float(dt * s->m.D[i][j]);
@@ -630,7 +631,6 @@ static int init_core(CudaData* dev, int nx, int ny, int nm, const double* mask,
   if (!nuc_ready) {
     CK(nucleation_setup());
     CK(prepare_step2d_f32());
-    CK(prepare_step2d_f64());
     nuc_ready = true;
   }
   if (cr) {

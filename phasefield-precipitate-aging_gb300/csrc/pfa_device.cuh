@@ -166,6 +166,128 @@ __device__ __forceinline__ double dlap64(double Dl, double Dm, double Dh, double
   return ((Dh + Dm) * (ch - cm) - (Dm + Dl) * (cm - cl)) * r2;
 }
 
+// ---- FP64 step: reduced forms ----
+// A warp's FP64 instruction occupies its scheduler's FP64 path for 64 cycles
+// and an SM completes one every 19 cycles (measured), about 76 times an FP32
+// instruction's cost, so the step counts FP64 operations: factors common to
+// all cells are folded on the host (Coef64), tests are integer tests on the
+// high words, and a cell takes the cheapest form that rounds to the same
+// values:
+//   kSolveHi: |phi| < 1e-7 in both phases.  p(phi) = 10 phi^3 < 1e-20, so the
+//     general solve returns X, Y themselves (p shifts them by less than half
+//     an ulp) and is skipped;
+//   kLinearHi: |phi| < 2^-60.  p' dP, the cubic terms of the double well and
+//     the coupling are below 2^-53 of 2 omega phi, so the Allen-Cahn update
+//     is phi + kl lap phi - kw phi.
+// Compositions that are not finite (or above kBigHi, 2^64) take the general
+// forms, whose NaN propagation is the reference's.
+constexpr int kSolveHi = 0x3e7ad7f2;   // high word of 1e-7
+constexpr int kLinearHi = 0x3c300000;  // 2^-60
+constexpr int kBigHi = 0x43f00000;     // 2^64
+
+// high word without the sign: orders the magnitudes of doubles
+__device__ __forceinline__ int mag_hi(double v) { return __double2hiint(v) & 0x7fffffff; }
+
+// neither phase nor composition needs the general forms of the given bound
+__device__ __forceinline__ bool below64(double X, double Y, double phd, double phl, int bound) {
+  return max(mag_hi(phd), mag_hi(phl)) < bound && max(mag_hi(X), mag_hi(Y)) < kBigHi;
+}
+
+// x^gamma of one cell (fict_gam_Cr / fict_gam_Nb, thermo/parabola625.c:245-261)
+// with the quadratic forms nested: 56 FP64 operations, a reciprocal included,
+// against 84 over shared monomials.  All terms of the denominator are
+// non-negative on the simplex, as in the monomial form.
+__device__ __forceinline__ void gamma64(double X, double Y, double phd, double phl, double& g1,
+                                        double& g2) {
+  const double pD = p64(phd), pL = p64(phl), pG = 1.0 - pD - pL;
+  constexpr double d0 = kDen[0], d1 = kDen[1], d2 = kDen[2], d4 = kDen[4], d5 = kDen[5];
+  static_assert(kDen[3] == 1.0, "the pG^2 coefficient of the denominator");
+  const double den = fma(pD, fma(d0, pD, fma(d1, pG, d2 * pL)),
+                         fma(pG, fma(d4, pL, pG), (d5 * pL) * pL));
+  const double r = 1.0 / den;
+  {
+    constexpr FictRow c = kFict[0][0];
+    static_assert(kFict[0][0].scale == 1.0 && kFict[0][0].l[1] == 1.0 &&
+                  kFict[0][0].m[1] == 0.0 && kFict[0][0].q[3] == 0.0, "pure gamma: x^gamma = X");
+    const double l = fma(c.l[0], pD, fma(c.l[2], pL, pG));
+    const double m = fma(c.m[0], pD, c.m[2] * pL);
+    const double q = fma(pD, fma(c.q[0], pD, fma(c.q[1], pG, c.q[2] * pL)),
+                         pL * fma(c.q[4], pG, c.q[5] * pL));
+    g1 = fma(X, l, fma(Y, m, q)) * r;
+  }
+  {
+    constexpr FictRow c = kFict[0][1];
+    static_assert(kFict[0][1].scale == -1.0 && kFict[0][1].l[1] == 0.0 &&
+                  kFict[0][1].m[1] == -1.0 && kFict[0][1].q[3] == 0.0, "pure gamma: x^gamma = Y");
+    const double l = fma(c.l[0], pD, c.l[2] * pL);
+    const double m = fma(c.m[0], pD, fma(c.m[2], pL, -pG));
+    const double q = fma(pD, fma(c.q[0], pD, fma(c.q[1], pG, c.q[2] * pL)),
+                         pL * fma(c.q[4], pG, c.q[5] * pL));
+    g2 = -fma(X, l, fma(Y, m, q)) * r;
+  }
+}
+
+// Allen-Cahn update of phase I from its Laplacian (Coef64); u = x^gamma -
+// xe_gamma, e = phi_del phi_lav.  The increments are summed before they meet
+// phi, so phi' is rounded once at phi's own magnitude.
+template <int I>
+__device__ __forceinline__ double allen_cahn64(const Coef64& K, double ph, double pj, double e,
+                                               double lap, double u1, double u2) {
+  const double* c = K.P[I];
+  const double P = fma(u1, fma(c[2], u1, fma(c[3], u2, c[0])), u2 * fma(c[4], u2, c[1]));
+  const double t = fma(-ph, ph, ph);
+  const double w = fma(t, P, fma(2.0 * K.kw[I], ph, -K.kw[I]));
+  return ph + fma(t, w, fma(-K.ka[I] * pj, e, K.kl[I] * lap));
+}
+
+template <int I>
+__device__ __forceinline__ double allen_cahn_linear64(const Coef64& K, double ph, double lap) {
+  return ph + fma(K.kl[I], lap, -K.kw[I] * ph);
+}
+
+// both phases of one cell (gamma compositions g1, g2)
+__device__ __forceinline__ void phases64(const Coef64& K, double X, double Y, double g1, double g2,
+                                         double phd, double phl, double lapD, double lapL,
+                                         double& od, double& ol) {
+  if (below64(X, Y, phd, phl, kLinearHi)) {
+    od = allen_cahn_linear64<0>(K, phd, lapD);
+    ol = allen_cahn_linear64<1>(K, phl, lapL);
+  } else {
+    const double u1 = g1 - kXe[0][0], u2 = g2 - kXe[0][1], e = phd * phl;
+    od = allen_cahn64<0>(K, phd, phl, e, lapD, u1, u2);
+    ol = allen_cahn64<1>(K, phl, phd, e, lapL, u1, u2);
+  }
+}
+
+// The diffusivities of dmatrix64 times the scale in `pre` (prefactors of Nb,
+// Cr, Ni), regrouped: per column c the three weighted mobilities A = e_Nb
+// (s_c + h_Nb,c), B = e_Cr (s_c + h_Cr,c), C = e_Ni x_Ni s_c give W = X B + Y
+// A + C, D_Cr,c = X (B - W), D_Nb,c = Y (A - W): 22 operations for 60.
+__device__ __forceinline__ void dmatrix64_scaled(const double pre[3], double X, double Y,
+                                                 double& d00, double& d01, double& d10,
+                                                 double& d11) {
+  const double xni = 1.0 - X - Y;
+  const double eNb = pre[0] * exp(Y * fma(-34.982563536715503, xni, 14.437947842988088));
+  const double eCr = pre[1] * exp(X * fma(-7.1543718172640256, xni, 3.3541967644499233));
+  const double eNi = pre[2] * xni *
+                     exp(fma(X, fma(-8.5221193705645018, xni, 4.0036674816806448),
+                             -Y * fma(442.62877981749585, xni, 0.82164267100913768)));
+  {
+    const double s = fma(-kHCrCr, X, -kHCrNb * Y);
+    const double A = eNb * (s + kHCrNbAddA), B = eCr * (s + kHCrCrAdd);
+    const double W = fma(X, B, fma(Y, A, eNi * s));
+    d00 = X * (B - W);
+    d10 = Y * (A - W);
+  }
+  {
+    const double s = fma(-kHCrNb, X, -kHNbNb * Y);
+    const double A = eNb * (s + kHNbNbAdd), B = eCr * (s + kHCrNbAddB);
+    const double W = fma(X, B, fma(Y, A, eNi * s));
+    d01 = X * (B - W);
+    d11 = Y * (A - W);
+  }
+}
+
 // ---- FP32 fast forms ----
 __device__ __forceinline__ float p32(float x) {
   const float x2 = x * x;

@@ -95,6 +95,7 @@ Step3DArgs step_args(Grid3D* g) {
   a.Ny = g->Ny;
   a.Nz = g->Nz;
   a.m = g->m;
+  model_coef64(g->m, nullptr, &a.c);
   a.k = g->fk;
   const double dt = g->m.dt;
   for (int i = 0; i < 2; i++)

@@ -51,6 +51,31 @@ struct FastCoef {
 
 void model_fast_coef(FastCoef* out);
 
+// Coefficients of the FP64 step, folded on the host from ModelConst, the mask
+// and the time step (every factor that is the same for all cells, so that a
+// cell's FP64 operations are the ones that depend on its values):
+//   x' = x + D lap x^gamma,  D = dt D (times the neighbour weight when iso)
+//   phi_i' = phi_i + kl_i lap phi_i + t (t P_i(u) - kw_i (1 - 2 phi_i))
+//            - ka_i phi_i phi_j^2,   t = phi_i (1 - phi_i),
+// with P_i = 30 dt L_i dP_i: u1 (c1 + c11 u1 + c12 u2) + u2 (c2 + c22 u2) in
+// u = x^gamma - xe_gamma, the quadratic of FastCoef::dP without its constant
+// term, which is zero to rounding (1e-7 of 1e8 J/m^3).  Against the tabulated
+// paraboloids in extended precision the identity holds to 2e-19 in phi'.
+struct Coef64 {
+  double D[2][2];
+  double kl[2], kw[2], ka[2];
+  double P[2][5];  // c1 c2 c11 c12 c22
+  int iso;       // all neighbour weights equal: lap = weight (sum + iso_c centre)
+  double iso_c;
+  double vm_pre[3];  // variable mobility: prefactors (Nb, Cr, Ni) times dt / (2 dx^2)
+  double vm_qy;      // and the weight of the y faces, (1/dy^2) / (1/dx^2)
+};
+
+struct ModelConst;
+// weights: the neighbour weights (2D: mask9 row-major; 3D: nullptr, 1/d^2 of
+// m.idx2); uses m.dt and m.alpha
+void model_coef64(const ModelConst& m, const double* mask9, Coef64* out);
+
 // The FP32 form's kernels index a grid's (2D) or a plane's (3D) records with
 // 32-bit integers: rows of ceil(Nx / 32) * 32 records, Ny rows, below 2^31.
 inline bool fp32_records_fit(int Nx, int Ny) {

@@ -25,6 +25,7 @@ struct Step2DArgs {
                         // instead of packed 16-bit counts (8-byte B records)
   ModelConst m;
   double mask9[9];      // full 3x3 mask, row-major (rows y-1..y+1)
+  Coef64 c;             // FP64 form
   FastCoef k;
   float dtD[2][2];      // dt * D
   float dtL[2];         // dt * L
@@ -118,6 +119,7 @@ struct Step3DArgs {
   int Nx, Ny, Nz, pitch;
   int zrows;            // z planes per segment (set by the launcher)
   ModelConst m;         // m.idx2 = 1/dx^2, 1/dy^2, 1/dz^2
+  Coef64 c;             // FP64 form
   FastCoef k;
   float dtD[2][2], dtL[2], om2[2], alpha2, kap[2], idx2f[3];
   int* status;          // FP32 form: set to 3 when a staging wait gave up (may be null)
@@ -158,8 +160,6 @@ cudaError_t launch_evolution(const StageArgs& a, cudaStream_t s);
 // fictitious compositions), and the divergences of Cr and Nb into a.o[0], a.o[1]
 cudaError_t launch_mobility(const StageArgs& a, cudaStream_t s);
 cudaError_t launch_chem_convolution(const StageArgs& a, cudaStream_t s);
-// the fused FP64 variable-mobility step's one-time set-up (shared memory)
-cudaError_t prepare_step2d_f64();
 cudaError_t launch_dataviz(const double* cr, const double* nb, const double* pd,
                            const double* pl, double* ni, double* phi, int nx, int ny,
                            cudaStream_t s);

@@ -78,22 +78,13 @@ double model_kks_diffusivity(const double Dcr[2], const double Dnb[2]) {
   return worst;
 }
 
-void model_fast_coef(FastCoef* o) {
-  std::memset(o, 0, sizeof(*o));
-  for (int k = 0; k < 6; k++) o->den[k] = float(kDen[k]);
-  for (int c = 0; c < 2; c++) {
-    const FictRow& r = kFict[0][c];
-    for (int k = 0; k < 3; k++) {
-      o->num[c][k] = float(r.scale * r.l[k]);
-      o->num[c][3 + k] = float(r.scale * r.m[k]);
-    }
-    for (int k = 0; k < 6; k++) o->num[c][6 + k] = float(r.scale * r.q[k]);
-  }
-  // Grand-potential difference Delta P_i(u), u = x^gamma - xe_gamma.  With
-  // g = 1/2 u^T H u + e u_2 (e = B xeCr - C) and equal chemical potentials,
-  //   Delta P = u^T [1/2 (Hg S Hg - Hg)] u + [f (S Hg)_2 - Hg dxe] . u
-  //             + 1/2 f^2 S_22 - e_g dxe_2,
-  // S = H_i^-1, f = e_g - e_i, dxe = xe_gamma - xe_i.
+// Grand-potential difference Delta P_i(u), u = x^gamma - xe_gamma.  With
+// g = 1/2 u^T H u + e u_2 (e = B xeCr - C) and equal chemical potentials,
+//   Delta P = u^T [1/2 (Hg S Hg - Hg)] u + [f (S Hg)_2 - Hg dxe] . u
+//             + 1/2 f^2 S_22 - e_g dxe_2,
+// S = H_i^-1, f = e_g - e_i, dxe = xe_gamma - xe_i.  Per phase (delta,
+// laves): c0 c1 c2 c11 c12 c22.
+static void model_dP(double dP[2][6]) {
   auto H = [](int ph, double h[2][2]) {
     h[0][0] = 2 * kG[ph][0];
     h[0][1] = h[1][0] = kG[ph][1];
@@ -121,14 +112,59 @@ void model_fast_coef(FastCoef* o) {
     const double l0 = f * SH[1][0] - (Hg[0][0] * dxe[0] + Hg[0][1] * dxe[1]);
     const double l1 = f * SH[1][1] - (Hg[1][0] * dxe[0] + Hg[1][1] * dxe[1]);
     const double c0 = 0.5 * f * f * S[1][1] - eg * dxe[1];
-    float* out = o->dP[ph - 1];
-    out[0] = float(c0);
-    out[1] = float(l0);
-    out[2] = float(l1);
-    out[3] = float(Q[0][0]);
-    out[4] = float(Q[0][1] + Q[1][0]);
-    out[5] = float(Q[1][1]);
+    const double c[6] = {c0, l0, l1, Q[0][0], Q[0][1] + Q[1][0], Q[1][1]};
+    std::memcpy(dP[ph - 1], c, sizeof(c));
   }
+}
+
+void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
+  std::memset(o, 0, sizeof(*o));
+  double dP[2][6];
+  model_dP(dP);
+  // 2D: upper, left, right, lower weights; 3D: 1/dx^2, 1/dy^2, 1/dz^2
+  bool iso;
+  double w;
+  if (mask9) {
+    w = mask9[1];
+    iso = mask9[0] == 0.0 && mask9[2] == 0.0 && mask9[6] == 0.0 && mask9[8] == 0.0 &&
+          mask9[3] == w && mask9[5] == w && mask9[7] == w && w != 0.0;
+    o->iso_c = iso ? mask9[4] / w : 0.0;
+  } else {
+    w = m.idx2[0];
+    iso = m.idx2[1] == w && m.idx2[2] == w;
+    o->iso_c = -6.0;
+  }
+  o->iso = iso;
+  const double f = iso ? w : 1.0;
+  for (int i = 0; i < 2; i++) {
+    for (int j = 0; j < 2; j++) o->D[i][j] = m.dt * m.D[i][j] * f;
+    o->kl[i] = m.dt * m.L[i] * m.kappa[i] * f;
+    o->kw[i] = 2.0 * m.dt * m.L[i] * m.omega[i];
+    for (int j = 0; j < 5; j++) o->P[i][j] = 30.0 * m.dt * m.L[i] * dP[i][j + 1];
+    o->ka[i] = 2.0 * m.dt * m.L[i] * m.alpha;
+  }
+  const double r2x = 0.5 * m.dt * m.idx2[0];
+  o->vm_pre[0] = kMobPreNb * r2x;
+  o->vm_pre[1] = kMobPreCr * r2x;
+  o->vm_pre[2] = kMobPreNi * r2x;
+  o->vm_qy = m.idx2[0] > 0.0 ? m.idx2[1] / m.idx2[0] : 0.0;
+}
+
+void model_fast_coef(FastCoef* o) {
+  std::memset(o, 0, sizeof(*o));
+  for (int k = 0; k < 6; k++) o->den[k] = float(kDen[k]);
+  for (int c = 0; c < 2; c++) {
+    const FictRow& r = kFict[0][c];
+    for (int k = 0; k < 3; k++) {
+      o->num[c][k] = float(r.scale * r.l[k]);
+      o->num[c][3 + k] = float(r.scale * r.m[k]);
+    }
+    for (int k = 0; k < 6; k++) o->num[c][6 + k] = float(r.scale * r.q[k]);
+  }
+  double dP[2][6];
+  model_dP(dP);
+  for (int i = 0; i < 2; i++)
+    for (int j = 0; j < 6; j++) o->dP[i][j] = float(dP[i][j]);
   o->xe_gam[0] = float(kXe[0][0]);
   o->xe_gam[1] = float(kXe[0][1]);
   for (int ph = 0; ph < 3; ph++)

@@ -4,10 +4,17 @@
 // launches (src/main.cpp:289-305): zero-flux boundary fill, fictitious
 // gamma compositions (src/discretization.cu:50-74), 5- or 9-point mask
 // convolution (:550-603), Cahn-Hilliard (:843-886) and Allen-Cahn (:888-980).
-// Each CTA stages one tile plus its one-cell halo in shared memory, computes
-// p(phi) and x^gamma once per staged cell, then the Laplacians and both
-// updates for its interior cells.  Domain edges are handled by clamped
-// (mirrored) indexing, which is what the reference's halo fill produces.
+// Each CTA stages one tile plus its one-cell halo in shared memory with
+// x^gamma per staged cell, then forms the Laplacians and both updates of its
+// interior cells.  Domain edges are handled by clamped (mirrored) indexing,
+// which is what the reference's halo fill produces.
+//
+// The FP64 pipe bounds it (19 cycles per warp instruction and SM), so the
+// arithmetic is in the reduced forms of pfa_device.cuh: 14 FP64 operations a
+// cell where both phases are exactly zero around it, 28 in the phases' far
+// tails, about 110 inside precipitates and their interfaces (the reference's
+// expressions: about 300 everywhere).  4096^2 with 4 particles: 7.78 -> 0.56
+// ms/step; 2048^2 1.95 -> 0.16 ms; 256^2 38.8 -> 14.5 us.
 //
 // Layout: the reference's, (Ny + 2) rows of pitch elements with a one-cell
 // ghost ring, interior cell (x, y) at (y + 1) * pitch + x + 1.  The FP32
@@ -24,10 +31,7 @@ using namespace dev;
 namespace {
 
 constexpr int kTX = 32;   // tile width (one warp)
-constexpr int kTY = 16;   // tile height
-constexpr int kBY = 8;    // thread rows per CTA
 constexpr int kEX = kTX + 2;
-constexpr int kEY = kTY + 2;
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
@@ -56,230 +60,180 @@ __device__ __forceinline__ void store_with_halo(T* f, int pitch, int gx, int gy,
 }
 
 // ---------------------------------------------------------------------------
-// Plain FP64 fused step (faithful to the reference's formulas).
-// NINE: the mask has non-zero corners (9-point stencil, src/mesh.cpp:198-213).
-template <bool NINE>
-__global__ void __launch_bounds__(kTX* kBY) k_step2d_f64(Step2DArgs a) {
-  __shared__ double s_phd[kEY][kEX], s_phl[kEY][kEX], s_gcr[kEY][kEX], s_gnb[kEY][kEX];
-  __shared__ double s_pd[kEY][kEX], s_pl[kEY][kEX], s_rden[kEY][kEX];
-  const double* __restrict__ icr = static_cast<const double*>(a.in[0]);
-  const double* __restrict__ inb = static_cast<const double*>(a.in[1]);
-  const double* __restrict__ ipd = static_cast<const double*>(a.in[2]);
-  const double* __restrict__ ipl = static_cast<const double*>(a.in[3]);
-  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY;
-  const int tid = threadIdx.y * kTX + threadIdx.x;
+// Plain FP64 fused step.  MASK: the neighbour weights are all equal (kIso), the
+// general 5-point mask (kFive), or a mask with corners (kNine,
+// src/mesh.cpp:198-213).  TY: rows of the tile, one row per warp; the warps
+// past them stage the tile's halo cells, so that a cell's solve and its
+// update are never behind another cell's in the same warp.
+enum { kIso = 0, kFive = 1, kNine = 2 };
 
-  for (int e = tid; e < kEX * kEY; e += kTX * kBY) {
-    const int ex = e % kEX, ey = e / kEX;
-    const int gx = clampi(x0 + ex - 1, 0, a.Nx - 1);
-    const int gy = clampi(y0 + ey - 1, 0, a.Ny - 1);
-    const size_t i = size_t(gy + 1) * a.pitch + gx + 1;
-    const double X = icr[i], Y = inb[i], phd = ipd[i], phl = ipl[i];
-    const double pD = p64(phd), pL = p64(phl), pG = 1.0 - pD - pL;
-    Poly64 m;
-    poly64(pD, pG, pL, m);
-    s_phd[ey][ex] = phd;
-    s_phl[ey][ex] = phl;
-    s_gcr[ey][ex] = fict64<0, 0>(X, Y, m);
-    s_gnb[ey][ex] = fict64<0, 1>(X, Y, m);
-    s_pd[ey][ex] = pD;
-    s_pl[ey][ex] = pL;
-    s_rden[ey][ex] = m.rden;
+constexpr int halo_warps(int ty) { return (2 * kEX + 2 * ty + 31) / 32; }
+constexpr int tile_threads(int ty) { return 32 * (ty + halo_warps(ty)); }
+
+// this thread's cell (ex, ey) of the (TY + 2) x 34 staged tile: its own
+// output cell in the first TY warps, a halo cell in the rest (false: none)
+template <int TY>
+__device__ __forceinline__ bool tile_cell(int& ex, int& ey) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < TY) {
+    ex = lane + 1;
+    ey = w + 1;
+    return true;
   }
-  __syncthreads();
-
-  const ModelConst& M = a.m;
-  for (int r = threadIdx.y; r < kTY; r += kBY) {
-    const int gx = x0 + threadIdx.x, gy = y0 + r;
-    if (gx >= a.Nx || gy >= a.Ny) continue;
-    const int ex = threadIdx.x + 1, ey = r + 1;
-    // Mask convolution in the reference's order (rows j = y-1..y+1, columns
-    // i = x-1..x+1, value += mask * tile, contracted to FMA); zero mask
-    // entries are exact no-ops there and are skipped for the 5-point mask.
-    auto lap = [&](double (*s)[kEX]) {
-      double v;
-      if (NINE) {
-        v = a.mask9[0] * s[ey - 1][ex - 1];
-        v = fma(a.mask9[1], s[ey - 1][ex], v);
-        v = fma(a.mask9[2], s[ey - 1][ex + 1], v);
-        v = fma(a.mask9[3], s[ey][ex - 1], v);
-        v = fma(a.mask9[4], s[ey][ex], v);
-        v = fma(a.mask9[5], s[ey][ex + 1], v);
-        v = fma(a.mask9[6], s[ey + 1][ex - 1], v);
-        v = fma(a.mask9[7], s[ey + 1][ex], v);
-        v = fma(a.mask9[8], s[ey + 1][ex + 1], v);
-      } else {
-        v = M.mask[0] * s[ey - 1][ex];
-        v = fma(M.mask[1], s[ey][ex - 1], v);
-        v = fma(M.mask[2], s[ey][ex], v);
-        v = fma(M.mask[3], s[ey][ex + 1], v);
-        v = fma(M.mask[4], s[ey + 1][ex], v);
-      }
-      return v;
-    };
-    const double lapCr = lap(s_gcr), lapNb = lap(s_gnb), lapD = lap(s_phd), lapL = lap(s_phl);
-    const size_t i = size_t(gy + 1) * a.pitch + gx + 1;
-    const double X = icr[i], Y = inb[i];
-    const double phd = s_phd[ey][ex], phl = s_phl[ey][ex];
-
-    // Cahn-Hilliard, composition_kernel src/discretization.cu:843-865
-    const double ocr = X + M.dt * (M.D[0][0] * lapCr + M.D[0][1] * lapNb);
-    const double onb = Y + M.dt * (M.D[1][0] * lapCr + M.D[1][1] * lapNb);
-
-    // Allen-Cahn, src/discretization.cu:888-980
-    Poly64 m;
-    m.lin[0] = s_pd[ey][ex];
-    m.lin[2] = s_pl[ey][ex];
-    m.lin[1] = 1.0 - m.lin[0] - m.lin[2];
-    m.mono[0] = m.lin[0] * m.lin[0];
-    m.mono[1] = m.lin[0] * m.lin[1];
-    m.mono[2] = m.lin[0] * m.lin[2];
-    m.mono[3] = m.lin[1] * m.lin[1];
-    m.mono[4] = m.lin[1] * m.lin[2];
-    m.mono[5] = m.lin[2] * m.lin[2];
-    m.rden = s_rden[ey][ex];
-    const double gam_Cr = s_gcr[ey][ex], gam_Nb = s_gnb[ey][ex];
-    const double gam_nrg = g64<0>(gam_Cr, gam_Nb);
-    const double dgGdxCr = dg64<0>(gam_Cr, gam_Nb);
-    const double dgGdxNb = dg64<1>(gam_Cr, gam_Nb);
-    double od, ol;
-    {
-      const double del_Cr = fict64<1, 0>(X, Y, m), del_Nb = fict64<1, 1>(X, Y, m);
-      const double del_nrg = g64<1>(del_Cr, del_Nb);
-      const double gp = gam_nrg - del_nrg - dgGdxCr * (gam_Cr - del_Cr) - dgGdxNb * (gam_Nb - del_Nb);
-      const double dF = -pp64(phd) * gp + 2.0 * M.omega[0] * phd * (phd - 1.0) * (2.0 * phd - 1.0) +
-                        2.0 * M.alpha * phd * phl * phl - M.kappa[0] * lapD;
-      od = phd - M.dt * M.L[0] * dF;
-    }
-    {
-      const double lav_Cr = fict64<2, 0>(X, Y, m), lav_Nb = fict64<2, 1>(X, Y, m);
-      const double lav_nrg = g64<2>(lav_Cr, lav_Nb);
-      const double gp = gam_nrg - lav_nrg - dgGdxCr * (gam_Cr - lav_Cr) - dgGdxNb * (gam_Nb - lav_Nb);
-      const double dF = -pp64(phl) * gp + 2.0 * M.omega[1] * phl * (phl - 1.0) * (2.0 * phl - 1.0) +
-                        2.0 * M.alpha * phl * phd * phd - M.kappa[1] * lapL;
-      ol = phl - M.dt * M.L[1] * dF;
-    }
-    const bool h = a.write_halo;
-    store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
-    store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
-    store_with_halo(static_cast<double*>(a.out[2]), a.pitch, gx, gy, a.Nx, a.Ny, od, h);
-    store_with_halo(static_cast<double*>(a.out[3]), a.pitch, gx, gy, a.Nx, a.Ny, ol, h);
+  const int h = (w - TY) * 32 + lane;
+  if (h < 2 * kEX) {
+    ey = h < kEX ? 0 : TY + 1;
+    ex = h < kEX ? h : h - kEX;
+  } else {
+    const int k = h - 2 * kEX;
+    ey = 1 + (k < TY ? k : k - TY);
+    ex = k < TY ? 0 : kEX - 1;
   }
+  return h < 2 * kEX + 2 * TY;
+}
+
+// Laplacian (kIso: over the weight, which Coef64 folds into its factors)
+template <int MASK>
+__device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[kEX], int ex, int ey) {
+  if constexpr (MASK == kIso) {
+    return fma(a.c.iso_c, s[ey][ex],
+               (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]));
+  } else if constexpr (MASK == kFive) {
+    double v = a.m.mask[0] * s[ey - 1][ex];
+    v = fma(a.m.mask[1], s[ey][ex - 1], v);
+    v = fma(a.m.mask[2], s[ey][ex], v);
+    v = fma(a.m.mask[3], s[ey][ex + 1], v);
+    return fma(a.m.mask[4], s[ey + 1][ex], v);
+  } else {
+    double v = a.mask9[0] * s[ey - 1][ex - 1];
+    v = fma(a.mask9[1], s[ey - 1][ex], v);
+    v = fma(a.mask9[2], s[ey - 1][ex + 1], v);
+    v = fma(a.mask9[3], s[ey][ex - 1], v);
+    v = fma(a.mask9[4], s[ey][ex], v);
+    v = fma(a.mask9[5], s[ey][ex + 1], v);
+    v = fma(a.mask9[6], s[ey + 1][ex - 1], v);
+    v = fma(a.mask9[7], s[ey + 1][ex], v);
+    return fma(a.mask9[8], s[ey + 1][ex + 1], v);
+  }
+}
+
+// one staged cell: its values, x^gamma, and whether the tile must look at the
+// phases at all (an all-zero phase field stays zero: its Laplacian, p' and
+// well vanish; compositions that are not finite make 0 x NaN, see kBigHi)
+struct Cell64 {
+  double X, Y, pd, pl, g1, g2;
+  int phase;
+};
+
+__device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
+  const size_t i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
+  Cell64 c;
+  c.X = __ldg(static_cast<const double*>(a.in[0]) + i);
+  c.Y = __ldg(static_cast<const double*>(a.in[1]) + i);
+  c.pd = __ldg(static_cast<const double*>(a.in[2]) + i);
+  c.pl = __ldg(static_cast<const double*>(a.in[3]) + i);
+  c.g1 = c.X;
+  c.g2 = c.Y;
+  if (!below64(c.X, c.Y, c.pd, c.pl, kSolveHi)) gamma64(c.X, c.Y, c.pd, c.pl, c.g1, c.g2);
+  c.phase = mag_hi(c.pd) | mag_hi(c.pl) | __double2loint(c.pd) | __double2loint(c.pl) |
+            int(max(mag_hi(c.X), mag_hi(c.Y)) >= kBigHi);
+  return c;
+}
+
+template <int MASK, int TY>
+__global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_constant__ Step2DArgs a) {
+  __shared__ double s_g1[TY + 2][kEX], s_g2[TY + 2][kEX], s_pd[TY + 2][kEX], s_pl[TY + 2][kEX];
+  int ex, ey;
+  const bool staged = tile_cell<TY>(ex, ey);
+  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
+  Cell64 c;
+  c.phase = 0;
+  if (staged) {
+    c = stage64(a, gx, gy);
+    s_g1[ey][ex] = c.g1;
+    s_g2[ey][ex] = c.g2;
+    s_pd[ey][ex] = c.pd;
+    s_pl[ey][ex] = c.pl;
+  }
+  const bool phases = __syncthreads_or(c.phase);
+  if (threadIdx.x >= 32 * TY || gx >= a.Nx || gy >= a.Ny) return;
+  // Cahn-Hilliard, composition_kernel src/discretization.cu:843-865
+  const Coef64& K = a.c;
+  const double l1 = lap64<MASK>(a, s_g1, ex, ey), l2 = lap64<MASK>(a, s_g2, ex, ey);
+  const double ocr = c.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
+  const double onb = c.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
+  const bool h = a.write_halo;
+  store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
+  store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
+  // Allen-Cahn, src/discretization.cu:888-980
+  double od = 0.0, ol = 0.0;
+  if (phases)
+    phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<MASK>(a, s_pd, ex, ey),
+             lap64<MASK>(a, s_pl, ex, ey), od, ol);
+  store_with_halo(static_cast<double*>(a.out[2]), a.pitch, gx, gy, a.Nx, a.Ny, od, h);
+  store_with_halo(static_cast<double*>(a.out[3]), a.pitch, gx, gy, a.Nx, a.Ny, ol, h);
 }
 
 // ---------------------------------------------------------------------------
 // Plain FP64 step with the variable-mobility Cahn-Hilliard (5-point mask):
 // the reference's disabled mobility kernels, chemical_convolution_Cr/Nb
 // (src/discretization.cu:175-358, 618-778) and the commented update of
-// composition_kernel (:848-856), fused.  Each CTA stages its tile and halo:
-// per cell the phases, the six fictitious compositions and the 16 flux
-// coefficients (dev::mobility64, three FP64 exponentials), then forms the
-// divergences (terms 7-8 along x only, as the reference) and the Laplacians
-// of the phases, and updates its interior cells.  Staged arrays are laid out
-// one after another in dynamic shared memory (kVmArrays x kVmCells doubles).
-constexpr int kVmTY = 8;                      // tile height (one row per thread row)
-constexpr int kVmCells = kEX * (kVmTY + 2);   // staged cells (tile + halo)
-constexpr int kVmArrays = 27;                 // phd phl fict[6] mob[16] pD pL rden
-constexpr size_t kVmSmem = sizeof(double) * kVmArrays * kVmCells;
-
-__global__ void __launch_bounds__(kTX* kVmTY) k_step2d_f64_varmob(Step2DArgs a) {
-  extern __shared__ double vm[];
-  auto S = [&](int k, int ex, int ey) -> double& { return vm[k * kVmCells + ey * kEX + ex]; };
-  const double* __restrict__ icr = static_cast<const double*>(a.in[0]);
-  const double* __restrict__ inb = static_cast<const double*>(a.in[1]);
-  const double* __restrict__ ipd = static_cast<const double*>(a.in[2]);
-  const double* __restrict__ ipl = static_cast<const double*>(a.in[3]);
-  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kVmTY;
-  const int tid = threadIdx.y * kTX + threadIdx.x;
-  for (int e = tid; e < kVmCells; e += kTX * kVmTY) {
-    const int ex = e % kEX, ey = e / kEX;
-    const int gx = clampi(x0 + ex - 1, 0, a.Nx - 1);
-    const int gy = clampi(y0 + ey - 1, 0, a.Ny - 1);
-    const size_t i = size_t(gy + 1) * a.pitch + gx + 1;
-    const double X = icr[i], Y = inb[i], phd = ipd[i], phl = ipl[i];
-    const double pD = p64(phd), pL = p64(phl), pG = 1.0 - pD - pL;
-    Poly64 m;
-    poly64(pD, pG, pL, m);
-    const double xg[2] = {fict64<0, 0>(X, Y, m), fict64<0, 1>(X, Y, m)};
-    const double xd[2] = {fict64<1, 0>(X, Y, m), fict64<1, 1>(X, Y, m)};
-    const double xl[2] = {fict64<2, 0>(X, Y, m), fict64<2, 1>(X, Y, m)};
-    double mob[16];
-    mobility64(X, Y, phd, phl, pD, pG, pL, xg, xd, xl, mob);
-    S(0, ex, ey) = phd;
-    S(1, ex, ey) = phl;
-    S(2, ex, ey) = xg[0];
-    S(3, ex, ey) = xg[1];
-    S(4, ex, ey) = xd[0];
-    S(5, ex, ey) = xd[1];
-    S(6, ex, ey) = xl[0];
-    S(7, ex, ey) = xl[1];
-#pragma unroll
-    for (int k = 0; k < 16; k++) S(8 + k, ex, ey) = mob[k];
-    S(24, ex, ey) = pD;
-    S(25, ex, ey) = pL;
-    S(26, ex, ey) = m.rden;
+// composition_kernel (:848-856), in the reduced form: with paraboloid
+// energies the phases' fictitious compositions share their diffusion
+// potentials, the 16 coefficient-weighted gradients sum to D(X, Y) grad
+// x^gamma (to the 1e-14 the potentials' rounding leaves), and the flux through
+// a face is (D_n + D_c)(u_n - u_c).  Each staged cell forms D once (three
+// exponentials), each face's flux is formed once: a thread forms its east and
+// lower faces, the halo warps the west faces of the first column and the
+// upper faces of the first row.
+template <bool ISO, int TY>
+__global__ void __launch_bounds__(tile_threads(TY))
+    k_step2d_f64_varmob(const __grid_constant__ Step2DArgs a) {
+  __shared__ double s_g1[TY + 2][kEX], s_g2[TY + 2][kEX], s_pd[TY + 2][kEX], s_pl[TY + 2][kEX];
+  __shared__ double s_d[4][TY + 2][kEX];
+  __shared__ double s_fx[2][TY][kTX + 1], s_fy[2][TY + 1][kTX];
+  int ex, ey;
+  const bool staged = tile_cell<TY>(ex, ey);
+  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
+  Cell64 c;
+  c.phase = 0;
+  if (staged) {
+    c = stage64(a, gx, gy);
+    s_g1[ey][ex] = c.g1;
+    s_g2[ey][ex] = c.g2;
+    s_pd[ey][ex] = c.pd;
+    s_pl[ey][ex] = c.pl;
+    dmatrix64_scaled(a.c.vm_pre, c.X, c.Y, s_d[0][ey][ex], s_d[1][ey][ex], s_d[2][ey][ex],
+                     s_d[3][ey][ex]);
+  }
+  const bool phases = __syncthreads_or(c.phase);
+  // flux into (ex, ey) from (nx, ny): component k is (D_n + D_c)_k . (u_n - u_c)
+  auto flux = [&](int x, int y, int nx, int ny, double& f1, double& f2) {
+    const double u1 = s_g1[ny][nx] - s_g1[y][x], u2 = s_g2[ny][nx] - s_g2[y][x];
+    f1 = fma(s_d[0][ny][nx] + s_d[0][y][x], u1, (s_d[1][ny][nx] + s_d[1][y][x]) * u2);
+    f2 = fma(s_d[2][ny][nx] + s_d[2][y][x], u1, (s_d[3][ny][nx] + s_d[3][y][x]) * u2);
+  };
+  const bool own = threadIdx.x < 32 * TY;
+  if (own) {
+    flux(ex, ey, ex + 1, ey, s_fx[0][ey - 1][ex], s_fx[1][ey - 1][ex]);
+    flux(ex, ey, ex, ey + 1, s_fy[0][ey][ex - 1], s_fy[1][ey][ex - 1]);
+  } else if (staged && ex == 0 && ey >= 1 && ey <= TY) {
+    flux(0, ey, 1, ey, s_fx[0][ey - 1][0], s_fx[1][ey - 1][0]);
+  } else if (staged && ey == 0 && ex >= 1 && ex <= kTX) {
+    flux(ex, 0, ex, 1, s_fy[0][0][ex - 1], s_fy[1][0][ex - 1]);
   }
   __syncthreads();
-
-  const ModelConst& M = a.m;
-  const int gx = x0 + threadIdx.x, gy = y0 + threadIdx.y;
-  if (gx >= a.Nx || gy >= a.Ny) return;
-  const int ex = threadIdx.x + 1, ey = threadIdx.y + 1;
-  const double r2x = 0.5 * M.idx2[0], r2y = 0.5 * M.idx2[1];  // 1 / (2 d^2)
-  double div[2];
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const int mb = 8 + 8 * k;  // this component's coefficients
-    double d = 0.0;
-#pragma unroll
-    for (int t = 0; t < 6; t++) {
-      const int D = mb + t, c = 2 + t;
-      d += dlap64(S(D, ex - 1, ey), S(D, ex, ey), S(D, ex + 1, ey), S(c, ex - 1, ey), S(c, ex, ey),
-                  S(c, ex + 1, ey), r2x);
-      d += dlap64(S(D, ex, ey - 1), S(D, ex, ey), S(D, ex, ey + 1), S(c, ex, ey - 1), S(c, ex, ey),
-                  S(c, ex, ey + 1), r2y);
-    }
-    d += dlap64(S(mb + 6, ex - 1, ey), S(mb + 6, ex, ey), S(mb + 6, ex + 1, ey), S(0, ex - 1, ey),
-                S(0, ex, ey), S(0, ex + 1, ey), r2x);
-    d += dlap64(S(mb + 7, ex - 1, ey), S(mb + 7, ex, ey), S(mb + 7, ex + 1, ey), S(1, ex - 1, ey),
-                S(1, ex, ey), S(1, ex + 1, ey), r2x);
-    div[k] = d;
-  }
-  auto lap = [&](int k) {
-    double v = M.mask[0] * S(k, ex, ey - 1);
-    v = fma(M.mask[1], S(k, ex - 1, ey), v);
-    v = fma(M.mask[2], S(k, ex, ey), v);
-    v = fma(M.mask[3], S(k, ex + 1, ey), v);
-    return fma(M.mask[4], S(k, ex, ey + 1), v);
-  };
-  const double lapD = lap(0), lapL = lap(1);
-  const size_t i = size_t(gy + 1) * a.pitch + gx + 1;
-  const double X = icr[i], Y = inb[i];
-  const double phd = S(0, ex, ey), phl = S(1, ex, ey);
-  const double ocr = X + M.dt * div[0];
-  const double onb = Y + M.dt * div[1];
-  // Allen-Cahn, src/discretization.cu:888-980, as in k_step2d_f64
-  const double gam_Cr = S(2, ex, ey), gam_Nb = S(3, ex, ey);
-  const double gam_nrg = g64<0>(gam_Cr, gam_Nb);
-  const double dgGdxCr = dg64<0>(gam_Cr, gam_Nb);
-  const double dgGdxNb = dg64<1>(gam_Cr, gam_Nb);
-  double od, ol;
-  {
-    const double del_Cr = S(4, ex, ey), del_Nb = S(5, ex, ey);
-    const double del_nrg = g64<1>(del_Cr, del_Nb);
-    const double gp = gam_nrg - del_nrg - dgGdxCr * (gam_Cr - del_Cr) - dgGdxNb * (gam_Nb - del_Nb);
-    const double dF = -pp64(phd) * gp + 2.0 * M.omega[0] * phd * (phd - 1.0) * (2.0 * phd - 1.0) +
-                      2.0 * M.alpha * phd * phl * phl - M.kappa[0] * lapD;
-    od = phd - M.dt * M.L[0] * dF;
-  }
-  {
-    const double lav_Cr = S(6, ex, ey), lav_Nb = S(7, ex, ey);
-    const double lav_nrg = g64<2>(lav_Cr, lav_Nb);
-    const double gp = gam_nrg - lav_nrg - dgGdxCr * (gam_Cr - lav_Cr) - dgGdxNb * (gam_Nb - lav_Nb);
-    const double dF = -pp64(phl) * gp + 2.0 * M.omega[1] * phl * (phl - 1.0) * (2.0 * phl - 1.0) +
-                      2.0 * M.alpha * phl * phd * phd - M.kappa[1] * lapL;
-    ol = phl - M.dt * M.L[1] * dF;
-  }
+  if (!own || gx >= a.Nx || gy >= a.Ny) return;
+  const Coef64& K = a.c;
+  const int tx = ex - 1, ty = ey - 1;
+  const double ocr = c.X + fma(K.vm_qy, s_fy[0][ty + 1][tx] - s_fy[0][ty][tx],
+                               s_fx[0][ty][tx + 1] - s_fx[0][ty][tx]);
+  const double onb = c.Y + fma(K.vm_qy, s_fy[1][ty + 1][tx] - s_fy[1][ty][tx],
+                               s_fx[1][ty][tx + 1] - s_fx[1][ty][tx]);
+  double od = 0.0, ol = 0.0;
+  if (phases)
+    phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<ISO ? kIso : kFive>(a, s_pd, ex, ey),
+             lap64<ISO ? kIso : kFive>(a, s_pl, ex, ey), od, ol);
   const bool h = a.write_halo;
   store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
   store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
@@ -287,28 +241,49 @@ __global__ void __launch_bounds__(kTX* kVmTY) k_step2d_f64_varmob(Step2DArgs a) 
   store_with_halo(static_cast<double*>(a.out[3]), a.pitch, gx, gy, a.Nx, a.Ny, ol, h);
 }
 
+// Rows per tile.  The tile's halo is staged (and, next to precipitates,
+// solved) again, so tall tiles do least; but a tile inside a precipitate takes
+// its SM's FP64 pipe for microseconds, so a small grid is cut finer to spread
+// such tiles over the SMs.  Measured, us per step at 1 / 2 / 4 / 8 rows:
+// 64 x 48 5.5 / 6.3 / 7.2 / 11.0, 256^2 27.3 / 14.8 / 14.5 / 16.4, 512^2 30.6
+// / 28.5 / 28.5 / 31.1, 1024^2 76 / 66.5 / 62.6 / 62.4; variable mobility
+// (every staged cell has its exponentials) 64 x 48 9.4 / 10.9 / 13.2 / 20.5,
+// 128^2 20.0 / 15.3 / 13.2 / 20.5, 256^2 61.6 / 45.1 / 38.3 / 35.6.
+int tile_rows(int Nx, int Ny, bool varmob) {
+  const long long rows = (long long)((Nx + kTX - 1) / kTX) * Ny;  // tile rows of 32 cells
+  if (varmob) return rows < 304 ? 1 : (rows < 1216 ? 4 : 8);
+  return rows < 1216 ? 1 : (rows < 9728 ? 4 : 8);
+}
+
+template <int TY>
+cudaError_t launch_rows(const Step2DArgs& a, cudaStream_t s) {
+  const dim3 grid((a.Nx + kTX - 1) / kTX, (a.Ny + TY - 1) / TY);
+  constexpr int n = tile_threads(TY);
+  if (a.varmob) {
+    if (a.c.iso)
+      k_step2d_f64_varmob<true, TY><<<grid, n, 0, s>>>(a);
+    else
+      k_step2d_f64_varmob<false, TY><<<grid, n, 0, s>>>(a);
+  } else if (a.nine) {
+    k_step2d_f64<kNine, TY><<<grid, n, 0, s>>>(a);
+  } else if (a.c.iso) {
+    k_step2d_f64<kIso, TY><<<grid, n, 0, s>>>(a);
+  } else {
+    k_step2d_f64<kFive, TY><<<grid, n, 0, s>>>(a);
+  }
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
-cudaError_t prepare_step2d_f64() {
-  return cudaFuncSetAttribute(k_step2d_f64_varmob, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(kVmSmem));
-}
-
 cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s) {
-  if (a.varmob) {
-    if (a.nine) return cudaErrorInvalidValue;
-    dim3 grid((a.Nx + kTX - 1) / kTX, (a.Ny + kVmTY - 1) / kVmTY);
-    k_step2d_f64_varmob<<<grid, dim3(kTX, kVmTY), kVmSmem, s>>>(a);
-    return cudaGetLastError();
+  if (a.varmob && a.nine) return cudaErrorInvalidValue;  // refused by the host before
+  switch (tile_rows(a.Nx, a.Ny, a.varmob)) {
+    case 1: return launch_rows<1>(a, s);
+    case 4: return launch_rows<4>(a, s);
+    default: return launch_rows<8>(a, s);
   }
-  dim3 grid((a.Nx + kTX - 1) / kTX, (a.Ny + kTY - 1) / kTY);
-  dim3 block(kTX, kBY);
-  if (a.nine)
-    k_step2d_f64<true><<<grid, block, 0, s>>>(a);
-  else
-    k_step2d_f64<false><<<grid, block, 0, s>>>(a);
-  return cudaGetLastError();
 }
 
 }  // namespace pfa

@@ -10,7 +10,8 @@
 //        columns and rows.  x-neighbours come from shuffles, y-neighbours
 //        from planes published in shared memory, z-neighbours from a
 //        three-plane register window rotated by a 3x-unrolled loop, one
-//        barrier per plane.
+//        barrier per plane; the reduced FP64 forms of pfa_device.cuh (128^3
+//        1.45 -> 0.34 ms, 256^3 9.3 -> 1.3 ms a step).
 //   k_stream3d_f32: the precision form (FP32 arithmetic, every field
 //        Kahan-compensated, the equilibrium-referenced gamma solve) on
 //        interior-only records (pfa_step2d_f32.cu): A = float4 {x_Cr, x_Nb,
@@ -67,7 +68,8 @@ __device__ __forceinline__ void store64(double* f, const Step3DArgs& a, int x, i
         f[((long long)(zs[k] + 1) * (a.Ny + 2) + (ys[j] + 1)) * a.pitch + (xs[i] + 1)] = v;
 }
 
-// One thread's column of the FP64 kernel.
+// One thread's column of the FP64 kernel (ISO: equal spacings).
+template <bool ISO>
 struct S64 {
   const Step3DArgs& a;
   int cx, cy;  // clamped column / row of this thread
@@ -89,12 +91,11 @@ struct S64 {
     return r;
   }
 
-  // gamma solve of one cell
+  // gamma solve of one cell (skipped where it returns X, Y themselves)
   __device__ __forceinline__ Nb3<double> solve(const Raw3<double>& r) const {
-    const double pD = p64(r.pd), pL = p64(r.pl), pG = 1.0 - pD - pL;
-    Poly64 m;
-    poly64(pD, pG, pL, m);
-    return Nb3<double>{fict64<0, 0>(r.x, r.y, m), fict64<0, 1>(r.x, r.y, m), r.pd, r.pl};
+    Nb3<double> n{r.x, r.y, r.pd, r.pl};
+    if (!below64(r.x, r.y, r.pd, r.pl, kSolveHi)) gamma64(r.x, r.y, r.pd, r.pl, n.gcr, n.gnb);
+    return n;
   }
 
   // update plane z of this thread's column from the window (up, c, dn)
@@ -109,53 +110,47 @@ struct S64 {
     Nb3<double> wv, e;
     wv.gcr = __shfl_up_sync(0xffffffffu, c.gcr, 1);
     wv.gnb = __shfl_up_sync(0xffffffffu, c.gnb, 1);
-    wv.pd = __shfl_up_sync(0xffffffffu, c.pd, 1);
-    wv.pl = __shfl_up_sync(0xffffffffu, c.pl, 1);
     e.gcr = __shfl_down_sync(0xffffffffu, c.gcr, 1);
     e.gnb = __shfl_down_sync(0xffffffffu, c.gnb, 1);
-    e.pd = __shfl_down_sync(0xffffffffu, c.pd, 1);
-    e.pl = __shfl_down_sync(0xffffffffu, c.pl, 1);
+    // an all-zero phase neighbourhood stays zero (compositions that are not
+    // finite make 0 x NaN and go the general way)
+    auto bits = [](double v) { return mag_hi(v) | __double2loint(v); };
+    auto any = [&](const Nb3<double>& v) { return bits(v.pd) | bits(v.pl); };
+    const bool phases = __any_sync(0xffffffffu, (any(up) | any(c) | any(dn) | any(s) | any(n) |
+                                                 int(max(mag_hi(rc.x), mag_hi(rc.y)) >= kBigHi)) != 0);
+    if (phases) {  // the whole warp
+      wv.pd = __shfl_up_sync(0xffffffffu, c.pd, 1);
+      wv.pl = __shfl_up_sync(0xffffffffu, c.pl, 1);
+      e.pd = __shfl_down_sync(0xffffffffu, c.pd, 1);
+      e.pl = __shfl_down_sync(0xffffffffu, c.pl, 1);
+    }
     if (!out) return;
-    const ModelConst& M = a.m;
-    // 7-point mask in the order z-1, y-1, x-1, centre, x+1, y+1, z+1
-    const double mx = M.idx2[0], my = M.idx2[1], mz = M.idx2[2], mc = -2. * (mx + my + mz);
+    const Coef64& K = a.c;
+    // 7-point Laplacian (ISO: over the weight, which Coef64 folds into its factors)
+    const double mx = a.m.idx2[0], my = a.m.idx2[1], mz = a.m.idx2[2];
     auto lap = [&](double z0, double y0, double x0, double vc, double x1, double y1, double z1) {
-      double v = mz * z0;
-      v = fma(my, y0, v);
-      v = fma(mx, x0, v);
-      v = fma(mc, vc, v);
-      v = fma(mx, x1, v);
-      v = fma(my, y1, v);
-      return fma(mz, z1, v);
+      if constexpr (ISO)
+        return fma(K.iso_c, vc, ((z0 + z1) + (y0 + y1)) + (x0 + x1));
+      else
+        return fma(mz, z0 + z1, fma(my, y0 + y1, fma(mx, x0 + x1, -2. * (mx + my + mz) * vc)));
     };
-    const double lapCr = lap(up.gcr, s.gcr, wv.gcr, c.gcr, e.gcr, n.gcr, dn.gcr);
-    const double lapNb = lap(up.gnb, s.gnb, wv.gnb, c.gnb, e.gnb, n.gnb, dn.gnb);
-    const double lapD = lap(up.pd, s.pd, wv.pd, c.pd, e.pd, n.pd, dn.pd);
-    const double lapL = lap(up.pl, s.pl, wv.pl, c.pl, e.pl, n.pl, dn.pl);
-    const double X = rc.x, Y = rc.y, pd = c.pd, pl = c.pl;
-    const double ocr = X + M.dt * (M.D[0][0] * lapCr + M.D[0][1] * lapNb);
-    const double onb = Y + M.dt * (M.D[1][0] * lapCr + M.D[1][1] * lapNb);
-    const double pD = p64(pd), pL = p64(pl), pG = 1.0 - pD - pL;
-    Poly64 m;
-    poly64(pD, pG, pL, m);
-    const double gcr = c.gcr, gnb = c.gnb;
-    const double gam = g64<0>(gcr, gnb);
-    const double dgCr = dg64<0>(gcr, gnb), dgNb = dg64<1>(gcr, gnb);
-    const double dCr = fict64<1, 0>(X, Y, m), dNb = fict64<1, 1>(X, Y, m);
-    const double gpd = gam - g64<1>(dCr, dNb) - dgCr * (gcr - dCr) - dgNb * (gnb - dNb);
-    const double dFd = -pp64(pd) * gpd + 2.0 * M.omega[0] * pd * (pd - 1.0) * (2.0 * pd - 1.0) +
-                       2.0 * M.alpha * pd * pl * pl - M.kappa[0] * lapD;
-    const double lCr = fict64<2, 0>(X, Y, m), lNb = fict64<2, 1>(X, Y, m);
-    const double gpl = gam - g64<2>(lCr, lNb) - dgCr * (gcr - lCr) - dgNb * (gnb - lNb);
-    const double dFl = -pp64(pl) * gpl + 2.0 * M.omega[1] * pl * (pl - 1.0) * (2.0 * pl - 1.0) +
-                       2.0 * M.alpha * pl * pd * pd - M.kappa[1] * lapL;
-    store64(static_cast<double*>(a.out[0]), a, cx, cy, z, ocr);
-    store64(static_cast<double*>(a.out[1]), a, cx, cy, z, onb);
-    store64(static_cast<double*>(a.out[2]), a, cx, cy, z, pd - M.dt * M.L[0] * dFd);
-    store64(static_cast<double*>(a.out[3]), a, cx, cy, z, pl - M.dt * M.L[1] * dFl);
+    const double l1 = lap(up.gcr, s.gcr, wv.gcr, c.gcr, e.gcr, n.gcr, dn.gcr);
+    const double l2 = lap(up.gnb, s.gnb, wv.gnb, c.gnb, e.gnb, n.gnb, dn.gnb);
+    store64(static_cast<double*>(a.out[0]), a, cx, cy, z,
+            rc.x + fma(K.D[0][0], l1, K.D[0][1] * l2));
+    store64(static_cast<double*>(a.out[1]), a, cx, cy, z,
+            rc.y + fma(K.D[1][0], l1, K.D[1][1] * l2));
+    double od = 0.0, ol = 0.0;
+    if (phases)
+      phases64(K, rc.x, rc.y, c.gcr, c.gnb, c.pd, c.pl,
+               lap(up.pd, s.pd, wv.pd, c.pd, e.pd, n.pd, dn.pd),
+               lap(up.pl, s.pl, wv.pl, c.pl, e.pl, n.pl, dn.pl), od, ol);
+    store64(static_cast<double*>(a.out[2]), a, cx, cy, z, od);
+    store64(static_cast<double*>(a.out[3]), a, cx, cy, z, ol);
   }
 };
 
+template <bool ISO>
 __global__ void __launch_bounds__(32 * kW) k_stream3d_f64(Step3DArgs a) {
   __shared__ Nb3<double> sh[2][kW][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -163,7 +158,7 @@ __global__ void __launch_bounds__(32 * kW) k_stream3d_f64(Step3DArgs a) {
   const int y = blockIdx.y * kRowsOut - 1 + w;
   const int z0 = blockIdx.z * a.zrows;
   const int z1 = min(z0 + a.zrows, a.Nz);
-  const S64 S{a, min(max(x, 0), a.Nx - 1), min(max(y, 0), a.Ny - 1),
+  const S64<ISO> S{a, min(max(x, 0), a.Nx - 1), min(max(y, 0), a.Ny - 1),
               lane >= 1 && lane <= kCols && w >= 1 && w <= kRowsOut && x < a.Nx && y < a.Ny};
   Raw3<double> r0 = S.load(z0), r1 = S.load(z0 + 1), r2;
   Nb3<double> n0 = S.solve(S.load(z0 - 1)), n1 = S.solve(r0), n2;
@@ -494,6 +489,17 @@ int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
   return best;
 }
 
+// FP64: a column next to a precipitate costs several times one in the matrix,
+// so short segments that spread the precipitates over the SMs beat whole
+// waves of equal ones.  us per step at 3 / 12 / whole-wave planes: 128^3 336 /
+// 376 / 576, 200 x 100 x 60 213 / 284 / 513, 256^3 1371 / 1314 / 1415; 64^3
+// at 2 / 3 / 8: 117 / 123 / 151, 32^3 51 / 68 / 151.
+int segment_planes_f64(int Nx, int Ny, int Nz) {
+  const long long cols = (long long)((Nx + kCols - 1) / kCols) * ((Ny + kRowsOut - 1) / kRowsOut);
+  const int planes = cols * Nz <= 1216 ? 2 : (cols * Nz <= 12160 ? 3 : 12);
+  return std::min(planes, Nz);
+}
+
 int g_resident3[2] = {0, 0};
 
 template <bool F64>
@@ -503,7 +509,7 @@ cudaError_t query3() {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) {
     if (F64)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f64, 32 * kW, 0);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f64<true>, 32 * kW, 0);
     else
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f32<false>, 32 * kW3, kSmem3);
   }
@@ -560,10 +566,13 @@ cudaError_t encode_step3d_maps(Tma3* t, const void* A, const void* B, int Nx, in
 cudaError_t launch_step3d(Step3DArgs a, bool f64, const Tma3* t, cudaStream_t s) {
   const int resident = g_resident3[f64] > 0 ? g_resident3[f64] : 152;
   const int tx = f64 ? kCols : kCols3, ty = f64 ? kRowsOut : kRows3;
-  a.zrows = segment_planes(a.Nx, a.Ny, a.Nz, resident, tx, ty);
+  a.zrows = f64 ? segment_planes_f64(a.Nx, a.Ny, a.Nz) : segment_planes(a.Nx, a.Ny, a.Nz, resident, tx, ty);
   dim3 grid((a.Nx + tx - 1) / tx, (a.Ny + ty - 1) / ty, (a.Nz + a.zrows - 1) / a.zrows);
   if (f64) {
-    k_stream3d_f64<<<grid, 32 * kW, 0, s>>>(a);
+    if (a.c.iso)
+      k_stream3d_f64<true><<<grid, 32 * kW, 0, s>>>(a);
+    else
+      k_stream3d_f64<false><<<grid, 32 * kW, 0, s>>>(a);
   } else {
     if (!t) return cudaErrorInvalidValue;
     if (a.skip_plane >= 0)

@@ -1,0 +1,112 @@
+"""The FP64 step's cheaper forms (zero, far-tail and general phases; the
+skipped gamma solve) and its tile heights, against the oracle."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import field_err
+from pfa_gb300 import ic
+
+pytestmark = pytest.mark.gpu
+
+
+def mixed_fields(shape, seed):
+    """Compositions of the matrix with noise; phases log-uniform from 1e-40 to
+    0.3 (both sides of every threshold of the forms), zero in patches."""
+    rng = np.random.default_rng(seed)
+    f = [rng.uniform(0.28, 0.33, shape), rng.uniform(0.02, 0.17, shape)]
+    for _ in range(2):
+        a = 10.0 ** rng.uniform(-40, -0.5, shape)
+        edges = 10.0 ** rng.choice([-18.1, -18.05, -7.01, -6.99], shape)
+        a = np.where(rng.random(shape) < 0.2, edges, a)
+        zero = rng.random([max(1, n // 16) + 1 for n in shape]) < 0.4
+        for d in range(len(shape)):
+            zero = np.repeat(zero, 16, axis=d)
+        a[zero[tuple(slice(0, n) for n in shape)]] = 0.0
+        f.append(a)
+    out = []
+    for a in f:
+        h = np.empty([n + 2 for n in shape])
+        h[(slice(1, -1),) * len(shape)] = a
+        out.append(ic.mirror_halo(h))
+    return out
+
+
+def around(a):
+    """Largest magnitude in each cell's neighbourhood (itself and its faces)."""
+    m = np.abs(a)
+    r = m.copy()
+    for d in range(a.ndim):
+        for s in (-1, 1):
+            r = np.maximum(r, np.roll(m, s, axis=d))
+    return r
+
+
+def check_cells(got, want, rel):
+    """Every cell within `rel` of the largest value the step reads around it."""
+    core = (slice(1, -1),) * got[0].ndim
+    for a, b in zip(got, want):
+        scale = around(b)
+        assert np.all((np.abs(a - b) <= rel * scale)[core])
+
+
+# tiles of 1, 4 and 8 rows (up to 1215, 9727 and more tile rows of 32 cells),
+# partial tiles on both axes
+@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 405), (70, 406), (161, 1621), (191, 1622)])
+@pytest.mark.parametrize("mask", ["iso", "five", "nine"])
+def test_forms_2d(pfa, orc, nx, ny, mask):
+    f = mixed_fields((ny, nx), nx * ny)
+    p = pfa.model_params()
+    q = O.model_params()
+    dx, dy = p["dx"], p["dx"] * (1.25 if mask == "five" else 1.0)
+    m = pfa.nine_point_mask(dx, dy) if mask == "nine" else pfa.five_point_mask(dx, dy)
+    g = pfa.Grid2D(f, dict(p, dy=dy), mask=m)
+    g.run(1)
+    got = g.read()
+    g.close()
+    q.dy = dy
+    want = orc.run2d(f, q.with_mask(m) if mask == "nine" else q, 1)
+    # one step: rounding of a few dozen operations on values of one
+    # neighbourhood (the solve's cancellation inside delta: 350)
+    check_cells(got, want, 350 * 16 * 2.0 ** -53)
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 130), (40, 700)])
+def test_forms_varmob(pfa, orc, nx, ny):
+    f = mixed_fields((ny, nx), nx + ny)
+    g = pfa.Grid2D(f, pfa.model_params(), mobility="variable")
+    g.run(1)
+    got = g.read()
+    g.close()
+    check_cells(got, orc.run2d_varmob(f, O.model_params(), 1), 350 * 16 * 2.0 ** -53)
+
+
+# segments of 2, 3 and 12 planes; partial tiles on every axis
+@pytest.mark.parametrize("n", [(31, 15, 3), (64, 40, 131), (95, 61, 700)])
+def test_forms_3d(pfa, orc, n):
+    f = mixed_fields(n[::-1], sum(n))
+    g = pfa.Grid3D(f, pfa.model_params(dim=3))
+    g.run(1)
+    got = g.read()
+    g.close()
+    check_cells(got, orc.run3d(f, O.model_params(dim=3), 1), 350 * 16 * 2.0 ** -53)
+
+
+def test_not_a_number_spreads_as_in_the_plain_forms(pfa, orc):
+    """A NaN and an infinity in a composition reach the same cells of the same
+    fields as in the oracle's expressions, phases zero or not."""
+    f = ic.grid2d(70, 40, seed=3, stripe_width=9, n_particles=1, radius=4.0)
+    f[0][10, 50] = np.nan
+    f[1][30, 60] = np.inf
+    want = orc.run2d(f, O.model_params(), 3)
+    g = pfa.Grid2D(f, pfa.model_params())
+    g.run(3)
+    got = g.read()
+    g.close()
+    core = (slice(1, -1), slice(1, -1))
+    for a, b in zip(got, want):
+        assert np.array_equal(np.isfinite(a[core]), np.isfinite(b[core]))
+    ok = [np.isfinite(b) for b in want]
+    err = field_err([np.where(k, a, 0.0) for a, k in zip(got, ok)],
+                    [np.where(k, b, 0.0) for b, k in zip(want, ok)])
+    assert max(err) <= 1e-12
