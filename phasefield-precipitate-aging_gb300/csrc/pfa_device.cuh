@@ -259,6 +259,79 @@ __device__ __forceinline__ void phases64(const Coef64& K, double X, double Y, do
   }
 }
 
+// ---- FP64 step: Cahn-Hilliard increments without FP64 operations ----
+// An explicit step adds D lap x^gamma, about 1e-3 of a composition or less,
+// to it, so the increment needs fewer bits than the composition.  Its parts:
+//  * the neighbour sum in 64-bit fixed point, units of 2^-58 (fix58): exact
+//    for compositions of 2^-6 and above (smaller ones lose bits below 2^-58,
+//    which D scales to 1e-20);
+//  * the product with D in FP32 pairs (inc58): 2^-48 of the increment;
+//  * the addition as one integer added to the composition's bits (add_inc),
+//    correctly rounded up to 2^-5 ulp of the increment's own rounding.
+// 266 FP64-pipe cycles per warp become about 60 of the FP32 and integer
+// pipes.  Valid for compositions in [2^-20, 1) (in_unit) and |x^gamma| below a
+// few units (the neighbour sum must stay below 2^5); a tile with any other
+// value takes the FP64 forms.
+
+// v in [2^-20, 1)
+__device__ __forceinline__ bool in_unit(double v) {
+  return unsigned(__double2hiint(v)) - 0x3eb00000u < 0x01400000u;
+}
+
+// v 2^58 (toward zero), v in [2^-20, 1)
+__device__ __forceinline__ long long fix58(double v) {
+  const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
+  const unsigned th = __funnelshift_l(lo, hi, 11) | 0x80000000u, tl = lo << 11;  // 1.m at bit 63
+  const unsigned r = 1028u - (hi >> 20);                                       // 6 .. 25
+  return (long long)(((unsigned long long)(th >> r) << 32) | __funnelshift_r(tl, th, r));
+}
+
+// the same for any |v| < 4
+__device__ __forceinline__ long long fix58_signed(double v) {
+  const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
+  const unsigned E = (hi >> 20) & 0x7ffu;
+  if (E < 965u) return 0;  // below 2^-58
+  const unsigned long long t =
+      ((unsigned long long)(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32) | (lo << 11);
+  const long long f = (long long)(t >> (1028u - E));
+  return hi >> 31 ? -f : f;
+}
+
+// row K of D times the sums S1, S2 (2^-58): an unevaluated FP32 pair h + l
+__device__ __forceinline__ void split58(long long S, float& a, float& b) {
+  const int hi = int((S + 0x80000000ll) >> 32);
+  a = float(hi);
+  b = float(int(S));
+  if (hi > (1 << 24) || hi < -(1 << 24)) b += float(hi - int(a)) * 4294967296.0f;  // a was rounded
+}
+template <int K>
+__device__ __forceinline__ void inc58(const Coef64& c, float a1, float b1, float a2, float b2,
+                                      float& h, float& l) {
+  const float p1 = c.Dh[K][0] * a1, p2 = c.Dh[K][1] * a2;
+  float e = fmaf(c.Dh[K][0], a1, -p1) + fmaf(c.Dh[K][1], a2, -p2);
+  e = fmaf(c.Dl[K][0], a1, fmaf(c.Dl[K][1], a2, e));
+  e = fmaf(c.Dq[K][0], b1, fmaf(c.Dq[K][1], b2, e));
+  h = p1 + p2;  // the exact sum is h + (p1 - (h - t)) + (p2 - t)
+  const float t = h - p1;
+  l = e + ((p1 - (h - t)) + (p2 - t));
+}
+
+// X + (h + l), X in [2^-20, 1): the increment in units of X's last place as
+// an integer, added to X's bits.  An increment above a quarter of X, or a
+// result in another binade, goes through FP64.
+__device__ __forceinline__ double add_inc(double X, float h, float l) {
+  const int E = __double2hiint(X) >> 20;
+  const float scale = __int_as_float((1202 - E) << 23);  // 2^(1075 - E)
+  const float hs = h * scale, ls = l * scale;
+  const int ai = __float2int_rn(hs * 0x1p-20f);
+  const int bi = __float2int_rn(fmaf(float(ai), -0x1p20f, hs) + ls);
+  const long long old = __double_as_longlong(X);
+  const long long sum = old + ((long long)ai * (1 << 20) + bi);
+  if (fabsf(hs) < 0x1p50f && ((unsigned long long)(old ^ sum) >> 52) == 0)
+    return __longlong_as_double(sum);
+  return X + (double(h) + double(l));
+}
+
 // The diffusivities of dmatrix64 times the scale in `pre` (prefactors of Nb,
 // Cr, Ni), regrouped: per column c the three weighted mobilities A = e_Nb
 // (s_c + h_Nb,c), B = e_Cr (s_c + h_Cr,c), C = e_Ni x_Ni s_c give W = X B + Y

@@ -65,11 +65,21 @@ struct Coef64 {
   double D[2][2];
   double kl[2], kw[2], ka[2];
   double P[2][5];  // c1 c2 c11 c12 c22
-  int iso;       // all neighbour weights equal: lap = weight (sum + iso_c centre)
+  // neighbour weights: kMaskIso: faces equal, lap = weight (sum of the faces
+  // + iso_c centre); kMaskIso9: faces four times the corners, lap = weight (4
+  // faces + corners + iso_c centre); the weight is folded into D and kl.  Both
+  // need weights that sum to zero up to rounding.  Any other mask:
+  // kMaskFive, kMaskNine.
+  int mask;
   double iso_c;
+  // iso masks: D in FP32 parts for sums in units of 2^-58 (dev::inc58):
+  // 2^-26 D = Dh + Dl, Dq = 2^-58 D
+  float Dh[2][2], Dl[2][2], Dq[2][2];
   double vm_pre[3];  // variable mobility: prefactors (Nb, Cr, Ni) times dt / (2 dx^2)
   double vm_qy;      // and the weight of the y faces, (1/dy^2) / (1/dx^2)
 };
+
+enum { kMaskIso = 0, kMaskFive = 1, kMaskNine = 2, kMaskIso9 = 3 };
 
 struct ModelConst;
 // weights: the neighbour weights (2D: mask9 row-major; 3D: nullptr, 1/d^2 of

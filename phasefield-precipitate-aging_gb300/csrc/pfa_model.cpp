@@ -121,23 +121,39 @@ void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
   std::memset(o, 0, sizeof(*o));
   double dP[2][6];
   model_dP(dP);
-  // 2D: upper, left, right, lower weights; 3D: 1/dx^2, 1/dy^2, 1/dz^2
-  bool iso;
-  double w;
+  double f = 1.0;  // the weight folded into D and kl
   if (mask9) {
-    w = mask9[1];
-    iso = mask9[0] == 0.0 && mask9[2] == 0.0 && mask9[6] == 0.0 && mask9[8] == 0.0 &&
-          mask9[3] == w && mask9[5] == w && mask9[7] == w && w != 0.0;
-    o->iso_c = iso ? mask9[4] / w : 0.0;
+    const double corner = mask9[0], face = mask9[1];
+    double sum = 0.0;
+    for (int k = 0; k < 9; k++) sum += mask9[k];
+    const bool zero_sum = std::fabs(sum) <= 1e-15 * std::fabs(mask9[4]);
+    const bool corners = mask9[2] == corner && mask9[6] == corner && mask9[8] == corner;
+    const bool faces = mask9[3] == face && mask9[5] == face && mask9[7] == face && face != 0.0;
+    o->mask = corners && corner == 0.0 ? kMaskFive : kMaskNine;
+    if (corners && faces && zero_sum) {
+      if (corner == 0.0) {
+        o->mask = kMaskIso;
+        f = face;
+      } else if (std::fabs(face - 4.0 * corner) <= 4e-16 * std::fabs(face)) {
+        o->mask = kMaskIso9;
+        f = corner;
+      }
+      o->iso_c = mask9[4] / f;
+    }
   } else {
-    w = m.idx2[0];
-    iso = m.idx2[1] == w && m.idx2[2] == w;
+    const bool iso = m.idx2[1] == m.idx2[0] && m.idx2[2] == m.idx2[0];
+    o->mask = iso ? kMaskIso : kMaskFive;
     o->iso_c = -6.0;
+    if (iso) f = m.idx2[0];
   }
-  o->iso = iso;
-  const double f = iso ? w : 1.0;
   for (int i = 0; i < 2; i++) {
-    for (int j = 0; j < 2; j++) o->D[i][j] = m.dt * m.D[i][j] * f;
+    for (int j = 0; j < 2; j++) {
+      o->D[i][j] = m.dt * m.D[i][j] * f;
+      const double d = std::ldexp(o->D[i][j], -26);
+      o->Dh[i][j] = float(d);
+      o->Dl[i][j] = float(d - double(o->Dh[i][j]));
+      o->Dq[i][j] = float(std::ldexp(d, -32));
+    }
     o->kl[i] = m.dt * m.L[i] * m.kappa[i] * f;
     o->kw[i] = 2.0 * m.dt * m.L[i] * m.omega[i];
     for (int j = 0; j < 5; j++) o->P[i][j] = 30.0 * m.dt * m.L[i] * dP[i][j + 1];

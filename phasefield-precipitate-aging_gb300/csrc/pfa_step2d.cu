@@ -60,13 +60,9 @@ __device__ __forceinline__ void store_with_halo(T* f, int pitch, int gx, int gy,
 }
 
 // ---------------------------------------------------------------------------
-// Plain FP64 fused step.  MASK: the neighbour weights are all equal (kIso), the
-// general 5-point mask (kFive), or a mask with corners (kNine,
-// src/mesh.cpp:198-213).  TY: rows of the tile, one row per warp; the warps
+// Plain FP64 fused step.  MASK: the kind of Coef64::mask.  TY: rows of the tile, one row per warp; the warps
 // past them stage the tile's halo cells, so that a cell's solve and its
 // update are never behind another cell's in the same warp.
-enum { kIso = 0, kFive = 1, kNine = 2 };
-
 constexpr int halo_warps(int ty) { return (2 * kEX + 2 * ty + 31) / 32; }
 constexpr int tile_threads(int ty) { return 32 * (ty + halo_warps(ty)); }
 
@@ -92,18 +88,22 @@ __device__ __forceinline__ bool tile_cell(int& ex, int& ey) {
   return h < 2 * kEX + 2 * TY;
 }
 
-// Laplacian (kIso: over the weight, which Coef64 folds into its factors)
+// Laplacian (iso masks: over the weight, which Coef64 folds into its factors)
 template <int MASK>
 __device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[kEX], int ex, int ey) {
-  if constexpr (MASK == kIso) {
+  if constexpr (MASK == kMaskIso) {
     return fma(a.c.iso_c, s[ey][ex],
                (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]));
-  } else if constexpr (MASK == kFive) {
+  } else if constexpr (MASK == kMaskFive) {
     double v = a.m.mask[0] * s[ey - 1][ex];
     v = fma(a.m.mask[1], s[ey][ex - 1], v);
     v = fma(a.m.mask[2], s[ey][ex], v);
     v = fma(a.m.mask[3], s[ey][ex + 1], v);
     return fma(a.m.mask[4], s[ey + 1][ex], v);
+  } else if constexpr (MASK == kMaskIso9) {
+    const double f = (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]);
+    const double k = (s[ey - 1][ex - 1] + s[ey + 1][ex + 1]) + (s[ey - 1][ex + 1] + s[ey + 1][ex - 1]);
+    return fma(a.c.iso_c, s[ey][ex], fma(4.0, f, k));
   } else {
     double v = a.mask9[0] * s[ey - 1][ex - 1];
     v = fma(a.mask9[1], s[ey - 1][ex], v);
@@ -117,12 +117,21 @@ __device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[k
   }
 }
 
-// one staged cell: its values, x^gamma, and whether the tile must look at the
+// the same over a staged fixed-point array (iso masks; exact)
+template <int MASK>
+__device__ __forceinline__ long long sum58(const long long (*s)[kEX], int ex, int ey) {
+  const long long f = (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]);
+  if constexpr (MASK == kMaskIso) return f - 4 * s[ey][ex];
+  const long long k = (s[ey - 1][ex - 1] + s[ey + 1][ex + 1]) + (s[ey - 1][ex + 1] + s[ey + 1][ex - 1]);
+  return 4 * f + k - 20 * s[ey][ex];
+}
+
+// one staged cell: its values and x^gamma.  phase: the tile must look at the
 // phases at all (an all-zero phase field stays zero: its Laplacian, p' and
 // well vanish; compositions that are not finite make 0 x NaN, see kBigHi)
 struct Cell64 {
   double X, Y, pd, pl, g1, g2;
-  int phase;
+  bool solved, phase;
 };
 
 __device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
@@ -134,34 +143,73 @@ __device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
   c.pl = __ldg(static_cast<const double*>(a.in[3]) + i);
   c.g1 = c.X;
   c.g2 = c.Y;
-  if (!below64(c.X, c.Y, c.pd, c.pl, kSolveHi)) gamma64(c.X, c.Y, c.pd, c.pl, c.g1, c.g2);
-  c.phase = mag_hi(c.pd) | mag_hi(c.pl) | __double2loint(c.pd) | __double2loint(c.pl) |
-            int(max(mag_hi(c.X), mag_hi(c.Y)) >= kBigHi);
+  c.solved = !below64(c.X, c.Y, c.pd, c.pl, kSolveHi);
+  if (c.solved) gamma64(c.X, c.Y, c.pd, c.pl, c.g1, c.g2);
+  const int bits = mag_hi(c.pd) | mag_hi(c.pl) | __double2loint(c.pd) | __double2loint(c.pl);
+  c.phase = bits != 0 || max(mag_hi(c.X), mag_hi(c.Y)) >= kBigHi;
   return c;
 }
 
+// MASK: Coef64::mask.  Bound by the FP64 pipe next to precipitates and by
+// memory elsewhere.
 template <int MASK, int TY>
 __global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_constant__ Step2DArgs a) {
-  __shared__ double s_g1[TY + 2][kEX], s_g2[TY + 2][kEX], s_pd[TY + 2][kEX], s_pl[TY + 2][kEX];
+  constexpr bool kFixed = MASK == kMaskIso || MASK == kMaskIso9;
+  // |x^gamma| < 4 (5 points) or 1 (9 points): the neighbour sum stays below 2^5
+  constexpr int kGammaHi = MASK == kMaskIso9 ? 0x3ff00000 : 0x40100000;
+  // x^gamma as doubles, or (kFixed) in fixed point
+  __shared__ long long s_g1[TY + 2][kEX], s_g2[TY + 2][kEX];
+  __shared__ double s_pd[TY + 2][kEX], s_pl[TY + 2][kEX];
+  auto as_double = [](long long (*s)[kEX]) { return reinterpret_cast<double (*)[kEX]>(s); };
   int ex, ey;
   const bool staged = tile_cell<TY>(ex, ey);
   const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
   Cell64 c;
-  c.phase = 0;
+  c.phase = false;
+  bool wide = false;  // outside the fixed-point forms' range
   if (staged) {
     c = stage64(a, gx, gy);
-    s_g1[ey][ex] = c.g1;
-    s_g2[ey][ex] = c.g2;
+    wide = !(in_unit(c.X) && in_unit(c.Y) && max(mag_hi(c.g1), mag_hi(c.g2)) < kGammaHi);
+    if (!kFixed || wide) {
+      as_double(s_g1)[ey][ex] = c.g1;
+      as_double(s_g2)[ey][ex] = c.g2;
+    } else if (c.solved) {
+      s_g1[ey][ex] = fix58_signed(c.g1);
+      s_g2[ey][ex] = fix58_signed(c.g2);
+    } else {
+      s_g1[ey][ex] = fix58(c.X);
+      s_g2[ey][ex] = fix58(c.Y);
+    }
     s_pd[ey][ex] = c.pd;
     s_pl[ey][ex] = c.pl;
   }
   const bool phases = __syncthreads_or(c.phase);
+  const bool fixed = kFixed && !__syncthreads_or(wide);
+  if (kFixed && !fixed) {  // the whole tile in FP64
+    if (staged) {
+      as_double(s_g1)[ey][ex] = c.g1;
+      as_double(s_g2)[ey][ex] = c.g2;
+    }
+    __syncthreads();
+  }
   if (threadIdx.x >= 32 * TY || gx >= a.Nx || gy >= a.Ny) return;
   // Cahn-Hilliard, composition_kernel src/discretization.cu:843-865
   const Coef64& K = a.c;
-  const double l1 = lap64<MASK>(a, s_g1, ex, ey), l2 = lap64<MASK>(a, s_g2, ex, ey);
-  const double ocr = c.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
-  const double onb = c.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
+  double ocr, onb;
+  if (fixed) {
+    float a1, b1, a2, b2, h, l;
+    split58(sum58<MASK>(s_g1, ex, ey), a1, b1);
+    split58(sum58<MASK>(s_g2, ex, ey), a2, b2);
+    inc58<0>(K, a1, b1, a2, b2, h, l);
+    ocr = add_inc(c.X, h, l);
+    inc58<1>(K, a1, b1, a2, b2, h, l);
+    onb = add_inc(c.Y, h, l);
+  } else {
+    const double l1 = lap64<MASK>(a, as_double(s_g1), ex, ey);
+    const double l2 = lap64<MASK>(a, as_double(s_g2), ex, ey);
+    ocr = c.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
+    onb = c.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
+  }
   const bool h = a.write_halo;
   store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
   store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
@@ -196,7 +244,7 @@ __global__ void __launch_bounds__(tile_threads(TY))
   const bool staged = tile_cell<TY>(ex, ey);
   const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
   Cell64 c;
-  c.phase = 0;
+  c.phase = false;
   if (staged) {
     c = stage64(a, gx, gy);
     s_g1[ey][ex] = c.g1;
@@ -232,8 +280,8 @@ __global__ void __launch_bounds__(tile_threads(TY))
                                s_fx[1][ty][tx + 1] - s_fx[1][ty][tx]);
   double od = 0.0, ol = 0.0;
   if (phases)
-    phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<ISO ? kIso : kFive>(a, s_pd, ex, ey),
-             lap64<ISO ? kIso : kFive>(a, s_pl, ex, ey), od, ol);
+    phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<ISO ? kMaskIso : kMaskFive>(a, s_pd, ex, ey),
+             lap64<ISO ? kMaskIso : kMaskFive>(a, s_pl, ex, ey), od, ol);
   const bool h = a.write_halo;
   store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
   store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
@@ -260,16 +308,17 @@ cudaError_t launch_rows(const Step2DArgs& a, cudaStream_t s) {
   const dim3 grid((a.Nx + kTX - 1) / kTX, (a.Ny + TY - 1) / TY);
   constexpr int n = tile_threads(TY);
   if (a.varmob) {
-    if (a.c.iso)
+    if (a.c.mask == kMaskIso)
       k_step2d_f64_varmob<true, TY><<<grid, n, 0, s>>>(a);
     else
       k_step2d_f64_varmob<false, TY><<<grid, n, 0, s>>>(a);
-  } else if (a.nine) {
-    k_step2d_f64<kNine, TY><<<grid, n, 0, s>>>(a);
-  } else if (a.c.iso) {
-    k_step2d_f64<kIso, TY><<<grid, n, 0, s>>>(a);
-  } else {
-    k_step2d_f64<kFive, TY><<<grid, n, 0, s>>>(a);
+    return cudaGetLastError();
+  }
+  switch (a.c.mask) {
+    case kMaskIso: k_step2d_f64<kMaskIso, TY><<<grid, n, 0, s>>>(a); break;
+    case kMaskIso9: k_step2d_f64<kMaskIso9, TY><<<grid, n, 0, s>>>(a); break;
+    case kMaskFive: k_step2d_f64<kMaskFive, TY><<<grid, n, 0, s>>>(a); break;
+    default: k_step2d_f64<kMaskNine, TY><<<grid, n, 0, s>>>(a);
   }
   return cudaGetLastError();
 }

@@ -569,7 +569,7 @@ cudaError_t launch_step3d(Step3DArgs a, bool f64, const Tma3* t, cudaStream_t s)
   a.zrows = f64 ? segment_planes_f64(a.Nx, a.Ny, a.Nz) : segment_planes(a.Nx, a.Ny, a.Nz, resident, tx, ty);
   dim3 grid((a.Nx + tx - 1) / tx, (a.Ny + ty - 1) / ty, (a.Nz + a.zrows - 1) / a.zrows);
   if (f64) {
-    if (a.c.iso)
+    if (a.c.mask == kMaskIso)
       k_stream3d_f64<true><<<grid, 32 * kW, 0, s>>>(a);
     else
       k_stream3d_f64<false><<<grid, 32 * kW, 0, s>>>(a);
