@@ -316,6 +316,12 @@ __device__ __forceinline__ void inc58(const Coef64& c, float a1, float b1, float
   l = e + ((p1 - (h - t)) + (p2 - t));
 }
 
+// the FP64 form of add_inc (a call: inlined, its FP64 operations are issued
+// for every cell and the result selected)
+static __device__ __noinline__ double add_inc64(double X, float h, float l) {
+  return X + (double(h) + double(l));
+}
+
 // X + (h + l), X in [2^-20, 1): the increment in units of X's last place as
 // an integer, added to X's bits.  An increment above a quarter of X, or a
 // result in another binade, goes through FP64.
@@ -329,7 +335,7 @@ __device__ __forceinline__ double add_inc(double X, float h, float l) {
   const long long sum = old + ((long long)ai * (1 << 20) + bi);
   if (fabsf(hs) < 0x1p50f && ((unsigned long long)(old ^ sum) >> 52) == 0)
     return __longlong_as_double(sum);
-  return X + (double(h) + double(l));
+  return add_inc64(X, h, l);
 }
 
 // The diffusivities of dmatrix64 times the scale in `pre` (prefactors of Nb,

@@ -35,14 +35,10 @@ constexpr int kEX = kTX + 2;
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// Write a value to interior cell (gx, gy) and, for cells on the domain edge,
-// to the ghost cells that mirror it (corners take the diagonal value).
-template <class T>
-__device__ __forceinline__ void store_with_halo(T* f, int pitch, int gx, int gy, int Nx, int Ny,
-                                                T v, bool halo) {
+// The ghost cells that mirror interior cell (gx, gy) of the domain's edge
+// (corners take the diagonal value).
+__device__ __noinline__ void store_ghosts(double* f, int pitch, int gx, int gy, int Nx, int Ny, double v) {
   const size_t row = size_t(gy + 1) * pitch;
-  f[row + gx + 1] = v;
-  if (!halo) return;
   const bool l = gx == 0, r = gx == Nx - 1, b = gy == 0, t = gy == Ny - 1;
   if (l) f[row] = v;
   if (r) f[row + Nx + 1] = v;
@@ -56,6 +52,21 @@ __device__ __forceinline__ void store_with_halo(T* f, int pitch, int gx, int gy,
     f[top + gx + 1] = v;
     if (l) f[top] = v;
     if (r) f[top + Nx + 1] = v;
+  }
+}
+
+// the four new values of interior cell (gx, gy), element i of the fields
+__device__ __forceinline__ void store_cell(const Step2DArgs& a, size_t i, int gx, int gy, double cr,
+                                           double nb, double pd, double pl) {
+  static_cast<double*>(a.out[0])[i] = cr;
+  static_cast<double*>(a.out[1])[i] = nb;
+  static_cast<double*>(a.out[2])[i] = pd;
+  static_cast<double*>(a.out[3])[i] = pl;
+  if (a.write_halo && (gx == 0 || gx == a.Nx - 1 || gy == 0 || gy == a.Ny - 1)) {
+    const double v[4] = {cr, nb, pd, pl};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      store_ghosts(static_cast<double*>(a.out[k]), a.pitch, gx, gy, a.Nx, a.Ny, v[k]);
   }
 }
 
@@ -131,22 +142,26 @@ __device__ __forceinline__ long long sum58(const long long (*s)[kEX], int ex, in
 // well vanish; compositions that are not finite make 0 x NaN, see kBigHi)
 struct Cell64 {
   double X, Y, pd, pl, g1, g2;
+  size_t i;  // element of the fields
   bool solved, phase;
+  bool unit;  // both compositions in [2^-20, 1)
 };
 
 __device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
-  const size_t i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
   Cell64 c;
-  c.X = __ldg(static_cast<const double*>(a.in[0]) + i);
-  c.Y = __ldg(static_cast<const double*>(a.in[1]) + i);
-  c.pd = __ldg(static_cast<const double*>(a.in[2]) + i);
-  c.pl = __ldg(static_cast<const double*>(a.in[3]) + i);
+  c.i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
+  c.X = __ldg(static_cast<const double*>(a.in[0]) + c.i);
+  c.Y = __ldg(static_cast<const double*>(a.in[1]) + c.i);
+  c.pd = __ldg(static_cast<const double*>(a.in[2]) + c.i);
+  c.pl = __ldg(static_cast<const double*>(a.in[3]) + c.i);
   c.g1 = c.X;
   c.g2 = c.Y;
-  c.solved = !below64(c.X, c.Y, c.pd, c.pl, kSolveHi);
+  c.unit = in_unit(c.X) && in_unit(c.Y);
+  const bool big = !c.unit && max(mag_hi(c.X), mag_hi(c.Y)) >= kBigHi;
+  const int m = max(mag_hi(c.pd), mag_hi(c.pl));
+  c.phase = (m | __double2loint(c.pd) | __double2loint(c.pl)) != 0 || big;
+  c.solved = m >= kSolveHi || big;
   if (c.solved) gamma64(c.X, c.Y, c.pd, c.pl, c.g1, c.g2);
-  const int bits = mag_hi(c.pd) | mag_hi(c.pl) | __double2loint(c.pd) | __double2loint(c.pl);
-  c.phase = bits != 0 || max(mag_hi(c.X), mag_hi(c.Y)) >= kBigHi;
   return c;
 }
 
@@ -169,7 +184,7 @@ __global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_co
   bool wide = false;  // outside the fixed-point forms' range
   if (staged) {
     c = stage64(a, gx, gy);
-    wide = !(in_unit(c.X) && in_unit(c.Y) && max(mag_hi(c.g1), mag_hi(c.g2)) < kGammaHi);
+    wide = !c.unit || (c.solved && max(mag_hi(c.g1), mag_hi(c.g2)) >= kGammaHi);
     if (!kFixed || wide) {
       as_double(s_g1)[ey][ex] = c.g1;
       as_double(s_g2)[ey][ex] = c.g2;
@@ -210,16 +225,12 @@ __global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_co
     ocr = c.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
     onb = c.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
   }
-  const bool h = a.write_halo;
-  store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
-  store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
   // Allen-Cahn, src/discretization.cu:888-980
   double od = 0.0, ol = 0.0;
   if (phases)
     phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<MASK>(a, s_pd, ex, ey),
              lap64<MASK>(a, s_pl, ex, ey), od, ol);
-  store_with_halo(static_cast<double*>(a.out[2]), a.pitch, gx, gy, a.Nx, a.Ny, od, h);
-  store_with_halo(static_cast<double*>(a.out[3]), a.pitch, gx, gy, a.Nx, a.Ny, ol, h);
+  store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
 // ---------------------------------------------------------------------------
@@ -282,11 +293,7 @@ __global__ void __launch_bounds__(tile_threads(TY))
   if (phases)
     phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<ISO ? kMaskIso : kMaskFive>(a, s_pd, ex, ey),
              lap64<ISO ? kMaskIso : kMaskFive>(a, s_pl, ex, ey), od, ol);
-  const bool h = a.write_halo;
-  store_with_halo(static_cast<double*>(a.out[0]), a.pitch, gx, gy, a.Nx, a.Ny, ocr, h);
-  store_with_halo(static_cast<double*>(a.out[1]), a.pitch, gx, gy, a.Nx, a.Ny, onb, h);
-  store_with_halo(static_cast<double*>(a.out[2]), a.pitch, gx, gy, a.Nx, a.Ny, od, h);
-  store_with_halo(static_cast<double*>(a.out[3]), a.pitch, gx, gy, a.Nx, a.Ny, ol, h);
+  store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
 // Rows per tile.  The tile's halo is staged (and, next to precipitates,
