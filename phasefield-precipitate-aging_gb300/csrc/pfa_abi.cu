@@ -61,7 +61,7 @@ static int fail(int code, const char* what) {
 
 // ---------------------------------------------------------------------------
 struct GraphEntry {
-  int precision, len, nuc_first, cur;
+  int precision, len, nuc_first, cur, cur_end;
   const void* ptrs[8];
   double dt, alpha;
   cudaGraphExec_t exec;
@@ -237,9 +237,13 @@ static Step2DArgs step_args(State* s, double alpha, double dt) {
   return a;
 }
 
-// One fused step: FP64 old -> new, or FP32 cur -> 1 - cur.
-static int fused_step(CudaData* dev, State* s, double alpha, double dt) {
+// One fused step: FP64 old -> new, or FP32 cur -> 1 - cur (*steps in: the most
+// steps it may take, out: the steps taken -- two in one pass where that is
+// the faster way).
+static int fused_step(CudaData* dev, State* s, double alpha, double dt, int* steps = nullptr) {
   Step2DArgs a = step_args(s, alpha, dt);
+  const int most = steps ? *steps : 1;
+  if (steps) *steps = 1;
   if (s->precision == PFA_FP64) {
     a.in[0] = dev->conc_Cr_old;
     a.in[1] = dev->conc_Nb_old;
@@ -267,7 +271,9 @@ static int fused_step(CudaData* dev, State* s, double alpha, double dt) {
   // the 5-point FP32 kernel takes the centre weight as -2 (left + upper);
   // a mask whose weights do not sum to zero goes through the general form
   a.nine = !s->five_point || !s->zero_sum;
-  CK(launch_step2d_f32(a, s->st));
+  const bool two = most >= 2 && two_steps_f32(a);
+  if (two) *steps = 2;
+  CK(launch_step2d_f32(a, two, s->st));
   s->cur = n;
   return 0;
 }
@@ -333,8 +339,9 @@ static int swap_ptrs(CudaData* dev) {
 // latest fields in *_old (FP64) or f32[cur] (FP32), as the caller-side
 // swaps of src/main.cpp:318-321 would.
 static int launch_chunk(CudaData* dev, State* s, int len, bool nuc_first, double alpha, double dt) {
-  for (int k = 0; k < len; k++) {
-    if (int r = fused_step(dev, s, alpha, dt)) return r;
+  for (int k = 0, n; k < len; k += n) {
+    n = k == 0 && nuc_first ? 1 : len - k;
+    if (int r = fused_step(dev, s, alpha, dt, &n)) return r;
     if (k == 0 && nuc_first)
       if (int r = nucleate(dev, s, s->nuc_sigma[0], s->nuc_sigma[1], s->nuc_unit_a, s->nuc_d[0],
                            s->nuc_d[1], s->nuc_d[2], s->nuc_dt))
@@ -363,7 +370,7 @@ static int run_chunk(CudaData* dev, State* s, int len, bool nuc_first, double al
     if (g.precision == key.precision && g.len == len && g.nuc_first == key.nuc_first &&
         g.cur == key.cur && !std::memcmp(g.ptrs, key.ptrs, sizeof(p)) && g.dt == dt &&
         g.alpha == alpha)
-      exec = g.exec;
+      exec = g.exec, key.cur_end = g.cur_end;
   const int cur0 = s->cur;
   const uint64_t calls0 = s->calls;
   if (!exec) {
@@ -378,6 +385,7 @@ static int run_chunk(CudaData* dev, State* s, int len, bool nuc_first, double al
                          &dev->conc_Nb_new, &dev->phi_del_old, &dev->phi_del_new,
                          &dev->phi_lav_old, &dev->phi_lav_new};
     for (int k = 0; k < 8; k++) *slots[k] = const_cast<double*>(static_cast<const double*>(p[k]));
+    key.cur_end = s->cur;
     s->cur = cur0;
     s->calls = calls0;
     if (r || e != cudaSuccess) {
@@ -392,7 +400,9 @@ static int run_chunk(CudaData* dev, State* s, int len, bool nuc_first, double al
     s->graphs.push_back(key);
   }
   CK(cudaGraphLaunch(exec, s->st));
-  // an even number of steps returns every ping-pong pointer to its place
+  // an even number of steps returns every FP64 ping-pong pointer to its
+  // place; the FP32 records may end on either side (two-step passes)
+  s->cur = key.cur_end;
   if (nuc_first) s->calls++;
   return 0;
 }

@@ -26,6 +26,7 @@
 // wait); an import into an arena block waits for the steps enqueued before
 // the latest removal, which may still read a freed block.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <deque>
@@ -57,6 +58,7 @@ struct RingEntry {
 
 struct BGraph {
   int len, parity, grid;
+  bool two;
   unsigned long long version;
   cudaGraphExec_t exec;
 };
@@ -71,12 +73,14 @@ struct Batch {
   int cur = 0;
   BatchGrid* d_grid = nullptr;
   int grid_cap = 0;
-  BatchUnit* d_unit = nullptr;
-  int unit_cap = 0;
-  int* d_counter = nullptr;  // counters of parity 0 / 1, unit count
-  int units = 0;
+  // unit tables of single steps [0] and of two steps in one pass [1]
+  BatchUnit* d_unit[2] = {};
+  int unit_cap[2] = {0, 0};
+  int units[2] = {0, 0};
+  int* d_counter = nullptr;  // counters of parity 0 / 1, unit counts of both tables
+  bool two = false;          // runs advance two steps per launch (refresh)
   bool dirty = true;
-  int rows = 64;         // rows per segment
+  int rows = 0;          // rows per segment (0: by auto_rows)
   int persistent = 1;    // persistent launch (else one warp per unit)
   int ctas = 0;          // CTAs of a persistent launch (0 = all resident)
   unsigned long long version = 1;  // bumps when the device tables move
@@ -165,11 +169,23 @@ void arena_free(Batch* b, size_t off, size_t bytes) {
   }
 }
 
+// Rows per segment until the caller tunes or sets them: the rules of the
+// single-grid kernels (segment_rows, segment_rows2) on the batch's rows of
+// strips per resident warp.
+int auto_rows(const Batch* b, bool two) {
+  double strip_rows = 0.0;
+  for (const Slot& s : b->slots)
+    if (s.live) strip_rows += double((s.Nx + batch_strip_cols(two) - 1) / batch_strip_cols(two)) * s.Ny;
+  const double load = strip_rows / (batch_resident_ctas(two) * batch_warps_per_cta());
+  if (!two) return load <= 1.0 ? 1 : (load <= 24.0 ? 6 : 32);
+  return 3 * std::max(2, int(std::sqrt(6.0 * load) / 3.0 + 0.5));
+}
+
 // The unit table for the current members and segment length: every grid's
 // rows are split into equal segments of at most `rows`; units are ordered by
 // decreasing length so that the counter hands out the long ones first.
-void make_units(const Batch* b, int rows, std::vector<BatchUnit>* out) {
-  const int cols = batch_strip_cols();
+void make_units(const Batch* b, int rows, bool two, std::vector<BatchUnit>* out) {
+  const int cols = batch_strip_cols(two);
   out->clear();
   for (int i = 0; i < int(b->slots.size()); i++) {
     const Slot& s = b->slots[i];
@@ -186,10 +202,13 @@ void make_units(const Batch* b, int rows, std::vector<BatchUnit>* out) {
 
 int upload_tables(Batch* b, int rows) {
   std::vector<BatchGrid> grids(b->slots.size());
+  double bytes = 0.0;
   for (size_t i = 0; i < b->slots.size(); i++)
-    if (b->slots[i].live) grids[i] = grid_entry(b, b->slots[i]);
-  std::vector<BatchUnit> units;
-  make_units(b, rows, &units);
+    if (b->slots[i].live) {
+      grids[i] = grid_entry(b, b->slots[i]);
+      bytes += double(b->slots[i].bytes);
+    }
+  b->two = two_steps_bytes(bytes);
   if (int(grids.size()) > b->grid_cap) {
     cudaStreamSynchronize(b->st);
     cudaFree(b->d_grid);
@@ -198,23 +217,29 @@ int upload_tables(Batch* b, int rows) {
     CKB(cudaMalloc(reinterpret_cast<void**>(&b->d_grid), sizeof(BatchGrid) * b->grid_cap));
     b->version++;
   }
-  if (int(units.size()) > b->unit_cap) {
-    cudaStreamSynchronize(b->st);
-    cudaFree(b->d_unit);
-    b->d_unit = nullptr;
-    b->unit_cap = std::max<int>(4096, int(units.size()) * 2);
-    CKB(cudaMalloc(reinterpret_cast<void**>(&b->d_unit), sizeof(BatchUnit) * b->unit_cap));
-    b->version++;
-  }
   // the copies are stream-ordered after every launch already enqueued
   if (!grids.empty())
     CKB(cudaMemcpyAsync(b->d_grid, grids.data(), sizeof(BatchGrid) * grids.size(),
                         cudaMemcpyHostToDevice, b->st));
-  if (!units.empty())
-    CKB(cudaMemcpyAsync(b->d_unit, units.data(), sizeof(BatchUnit) * units.size(),
-                        cudaMemcpyHostToDevice, b->st));
-  b->units = int(units.size());
-  const int counters[3] = {0, 0, b->units};
+  for (int t = 0; t < 2; t++) {
+    b->units[t] = 0;
+    if (t == 1 && !b->two) continue;  // not launched
+    std::vector<BatchUnit> units;
+    make_units(b, rows > 0 ? rows : auto_rows(b, t == 1), t == 1, &units);
+    if (int(units.size()) > b->unit_cap[t]) {
+      cudaStreamSynchronize(b->st);
+      cudaFree(b->d_unit[t]);
+      b->d_unit[t] = nullptr;
+      b->unit_cap[t] = std::max<int>(4096, int(units.size()) * 2);
+      CKB(cudaMalloc(reinterpret_cast<void**>(&b->d_unit[t]), sizeof(BatchUnit) * b->unit_cap[t]));
+      b->version++;
+    }
+    if (!units.empty())
+      CKB(cudaMemcpyAsync(b->d_unit[t], units.data(), sizeof(BatchUnit) * units.size(),
+                          cudaMemcpyHostToDevice, b->st));
+    b->units[t] = int(units.size());
+  }
+  const int counters[4] = {0, 0, b->units[0], b->units[1]};
   CKB(cudaMemcpyAsync(b->d_counter, counters, sizeof(counters), cudaMemcpyHostToDevice, b->st));
   // no host wait: copies from pageable host memory are staged before
   // cudaMemcpyAsync returns, and the launches that read the tables follow
@@ -229,41 +254,48 @@ int refresh(Batch* b) {
   return 0;
 }
 
-int persistent_ctas(const Batch* b) {
-  const int res = batch_resident_ctas();
-  const int need = (b->units + batch_warps_per_cta() - 1) / batch_warps_per_cta();
+int persistent_ctas(const Batch* b, bool two) {
+  const int res = batch_resident_ctas(two);
+  const int need = (b->units[two] + batch_warps_per_cta() - 1) / batch_warps_per_cta();
   const int c = b->ctas > 0 ? b->ctas : res;
   return std::max(1, std::min(c, need));
 }
 
-int launch(Batch* b, int parity) {
+// one pass (two: of two steps) from the records of `parity` to the other's
+int launch(Batch* b, int parity, bool two) {
   BatchArgs ba{};
   ba.grid = b->d_grid;
-  ba.unit = b->d_unit;
+  ba.unit = b->d_unit[two];
   ba.counter = b->d_counter;
-  ba.units = b->units;
+  ba.units = b->units[two];
   ba.parity = parity;
   ba.persistent = b->persistent;
-  CKB(launch_batch_f32(b->a, ba, persistent_ctas(b), b->st));
+  CKB(launch_batch_f32(b->a, ba, two, persistent_ctas(b, two), b->st));
   return 0;
 }
 
 int run(Batch* b, int nsteps) {
   if (int r = refresh(b)) return r;
-  if (b->units == 0) return 0;
+  if (b->units[0] == 0) return 0;
   while (nsteps > 0) {
-    if (nsteps == 1) {
-      if (int r = launch(b, b->cur)) return r;
+    bool two = b->two && nsteps >= 2;
+    const int per = two ? 2 : 1;
+    if (nsteps < 2 * per) {
+      if (int r = launch(b, b->cur, two)) return r;
       b->cur ^= 1;
-      return 0;
+      nsteps -= per;
+      continue;
     }
-    const int len = std::min(nsteps - nsteps % 2, 100);
+    // an even number of passes, so that the parity ends where it was
+    const int passes = std::min(nsteps / per - nsteps / per % 2, 100 / per);
+    const int len = passes * per;
     // a persistent launch reads the unit count from the device; the other
     // mode's grid size is the unit count
-    const int gsize = b->persistent ? persistent_ctas(b) : -b->units;
+    const int gsize = b->persistent ? persistent_ctas(b, two) : -b->units[two];
     cudaGraphExec_t exec = nullptr;
     for (auto& g : b->graphs)
-      if (g.len == len && g.parity == b->cur && g.grid == gsize && g.version == b->version)
+      if (g.len == len && g.parity == b->cur && g.grid == gsize && g.two == two &&
+          g.version == b->version)
         exec = g.exec;
     if (!exec) {
       // graphs of moved tables are not replayed again; keep at most 8
@@ -279,16 +311,16 @@ int run(Batch* b, int nsteps) {
       cudaGraph_t graph;
       CKB(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
       int r = 0;
-      for (int k = 0; k < len && !r; k++) r = launch(b, b->cur ^ (k & 1));
+      for (int k = 0; k < passes && !r; k++) r = launch(b, b->cur ^ (k & 1), two);
       const cudaError_t e = cudaStreamEndCapture(b->st, &graph);
       if (r) return r;
       if (e != cudaSuccess) return fail_cuda(e, "cudaStreamEndCapture");
       CKB(cudaGraphInstantiate(&exec, graph, 0));
       cudaGraphDestroy(graph);
-      b->graphs.push_back({len, b->cur, gsize, b->version, exec});
+      b->graphs.push_back({len, b->cur, gsize, two, b->version, exec});
     }
     CKB(cudaGraphLaunch(exec, b->st));
-    nsteps -= len;  // even: the parity is back where it was
+    nsteps -= len;  // even passes: the parity is back where it was
   }
   return 0;
 }
@@ -505,8 +537,8 @@ int pfa_batch_create(void** handle, const double* params, const double* dxy, siz
   CKB(cudaMalloc(reinterpret_cast<void**>(&b->ring), b->ring_cap));
   CKB(cudaMalloc(reinterpret_cast<void**>(&b->arena), b->cap));
   b->free_[0] = b->cap;
-  CKB(cudaMalloc(reinterpret_cast<void**>(&b->d_counter), 3 * sizeof(int)));
-  CKB(cudaMemsetAsync(b->d_counter, 0, 3 * sizeof(int), b->st));
+  CKB(cudaMalloc(reinterpret_cast<void**>(&b->d_counter), 4 * sizeof(int)));
+  CKB(cudaMemsetAsync(b->d_counter, 0, 4 * sizeof(int), b->st));
   CKB(cudaMalloc(reinterpret_cast<void**>(&b->sum_partial), sizeof(double) * kSumBlocks * 5));
   CKB(cudaMalloc(reinterpret_cast<void**>(&b->sum_out), sizeof(double) * 5));
   CKB(cudaStreamSynchronize(b->st));
@@ -651,10 +683,11 @@ int pfa_batch_get_launch(void* handle, int* rows, int* persistent, int* ctas, in
   Batch* b = get(handle);
   if (!b) return fail(PFA_ESTATE, "pfa_batch_get_launch: null handle");
   if (int r = refresh(b)) return r;
-  if (rows) *rows = b->rows;
+  const bool two = b->two;
+  if (rows) *rows = b->rows > 0 ? b->rows : auto_rows(b, two);
   if (persistent) *persistent = b->persistent;
-  if (ctas) *ctas = b->persistent ? persistent_ctas(b) : (b->units + batch_warps_per_cta() - 1) / batch_warps_per_cta();
-  if (units) *units = b->units;
+  if (ctas) *ctas = b->persistent ? persistent_ctas(b, two) : (b->units[two] + batch_warps_per_cta() - 1) / batch_warps_per_cta();
+  if (units) *units = b->units[two];
   return 0;
 }
 
@@ -662,28 +695,32 @@ int pfa_batch_tune(void* handle, int reps, float* best_ms) {
   Batch* b = get(handle);
   if (!b) return fail(PFA_ESTATE, "pfa_batch_tune: null handle");
   if (reps < 1) reps = 10;
-  static const int kRows[] = {16, 24, 32, 48, 64, 96, 128, 256, 1 << 30};
+  if (int r = refresh(b)) return r;
+  static const int kRows[2][9] = {{3, 6, 12, 24, 32, 48, 64, 128, 1 << 30},
+                                  {9, 15, 24, 30, 36, 48, 64, 96, 1 << 30}};
   float best = -1.f;
   int best_rows = b->rows, best_pers = b->persistent;
   cudaEvent_t e0, e1;
   CKB(cudaEventCreate(&e0));
   CKB(cudaEventCreate(&e1));
   for (int pers = 0; pers < 2; pers++) {
-    for (int rows : kRows) {
+    for (int i = 0; i < 9; i++) {
+      const bool two = b->two;  // the members decide, not the shape
+      const int rows = kRows[two][i];
       if (int r = upload_tables(b, rows)) return r;
-      if (b->units == 0) break;
+      if (b->units[0] == 0) break;
       b->persistent = pers;
       // cur -> cur ^ 1 every time: the grids' state does not advance
       for (int k = 0; k < reps + 2; k++) {
         if (k == 2) CKB(cudaEventRecord(e0, b->st));
         CKB(cudaMemsetAsync(b->d_counter, 0, 2 * sizeof(int), b->st));
-        if (int r = launch(b, b->cur)) return r;
+        if (int r = launch(b, b->cur, two)) return r;
       }
       CKB(cudaEventRecord(e1, b->st));
       CKB(cudaEventSynchronize(e1));
       float t = 0.f;
       CKB(cudaEventElapsedTime(&t, e0, e1));
-      t /= reps;
+      t /= two ? 2 * reps : reps;
       if (best < 0.f || t < best) {
         best = t;
         best_rows = rows;
@@ -754,7 +791,8 @@ int pfa_batch_destroy(void* handle) {
   cudaFree(b->ring);
   cudaFree(b->arena);
   cudaFree(b->d_grid);
-  cudaFree(b->d_unit);
+  cudaFree(b->d_unit[0]);
+  cudaFree(b->d_unit[1]);
   cudaFree(b->d_counter);
   cudaFree(b->sum_partial);
   cudaFree(b->sum_out);

@@ -87,20 +87,28 @@ struct BatchUnit {
 struct BatchArgs {
   const BatchGrid* grid;
   const BatchUnit* unit;
-  int* counter;   // unit counters of parity 0 / 1, then the unit count
+  int* counter;   // unit counters of parity 0 / 1, then the unit counts of
+                  // single and double passes
   int units;      // one-warp-per-unit mode: units of this launch
   int parity;     // records are read from parity, written to parity ^ 1
   int persistent;
 };
 
 cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s);
-cudaError_t launch_step2d_f32(const Step2DArgs& a, cudaStream_t s);
+// two: two steps in one pass (same bits as two launches)
+cudaError_t launch_step2d_f32(const Step2DArgs& a, bool two, cudaStream_t s);
+// whether two steps in one pass are the faster way for a grid, and for both
+// record sets of this many bytes (constant mobility)
+bool two_steps_f32(const Step2DArgs& a);
+bool two_steps_bytes(double bytes);
 cudaError_t prepare_step2d_f32();
-// ctas: CTAs of a persistent launch (b.persistent), else one warp per unit
-cudaError_t launch_batch_f32(const Step2DArgs& a, const BatchArgs& b, int ctas, cudaStream_t s);
-int batch_resident_ctas();   // CTAs of k_batch_f32 resident on the device at once
+// ctas: CTAs of a persistent launch (b.persistent), else one warp per unit;
+// two: two steps in one pass, on units of batch_strip_cols(true) columns
+cudaError_t launch_batch_f32(const Step2DArgs& a, const BatchArgs& b, bool two, int ctas,
+                             cudaStream_t s);
+int batch_resident_ctas(bool two);   // CTAs resident on the device at once
 int batch_warps_per_cta();
-int batch_strip_cols();
+int batch_strip_cols(bool two);
 cudaError_t launch_import_f32(const ConvArgs& a, cudaStream_t s);
 
 // initial conditions from a recipe (pfa_ic.cu): validation (message or

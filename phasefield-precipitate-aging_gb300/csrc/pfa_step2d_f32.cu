@@ -4,10 +4,11 @@
 // FP32 with every field Kahan-compensated (value = hi - c).  The gamma
 // solve is the equilibrium-referenced form (pfa_device.cuh, gamma_u32),
 // which keeps FP32 accurate inside precipitates where the plain num / den
-// form loses it to cancellation; rows whose phases are all below 1e-5 skip
-// the solve (x^gamma = X there).  At 48 bytes per cell the HBM budget leaves
-// ~250 instructions per cell, so the kernel is organised for instruction
-// economy:
+// form loses it to cancellation; cells whose phases are below 1e-5 skip the
+// solve (x^gamma = X there), and rows whose phases are all zero the
+// Allen-Cahn update.  Grids larger than the L2 take two steps per pass.  At
+// 48 bytes per cell and pass the HBM budget leaves ~250 instructions per
+// cell, so the kernels are organised for instruction economy:
 //  * each warp owns a strip of 30 output columns (lanes 1..30; lanes 0 and
 //    31 carry the neighbour columns) and streams down a segment of rows; the
 //    three rows a 5- or 9-point Laplacian needs live in registers, rotated by
@@ -25,6 +26,8 @@
 // Record layout: Ny rows of `pitch` records (pitch a multiple of 32), interior
 // cell (x, y) at record y * pitch + x, no ghost ring; zero-flux edges come
 // from clamped indexing (the mirror the reference's halo fill produces).
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -99,14 +102,6 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-template <bool PACK>
-__device__ __forceinline__ float4 comps(const CompT<PACK>& c) {
-  if constexpr (PACK)
-    return cq_unpack(c);
-  else
-    return c;
-}
-
 // the composition compensations only (what the gamma solve needs)
 template <bool PACK>
 __device__ __forceinline__ float2 comps_x(const CompT<PACK>& c) {
@@ -116,6 +111,22 @@ __device__ __forceinline__ float2 comps_x(const CompT<PACK>& c) {
   } else {
     return make_float2(c.x, c.y);
   }
+}
+
+// the phases' compensations, and the bits that are zero with them (signs of
+// FP32 zeros aside)
+template <bool PACK>
+__device__ __forceinline__ float2 comps_p(const CompT<PACK>& c) {
+  if constexpr (PACK) {
+    const float2 h = cq_halves(c.y);
+    return make_float2(h.x * kCqPi, h.y * kCqPi);
+  } else {
+    return make_float2(c.z, c.w);
+  }
+}
+__device__ __forceinline__ unsigned comp_bits(const uint2& c) { return c.y; }
+__device__ __forceinline__ unsigned comp_bits(const float4& c) {
+  return __float_as_uint(c.z) | __float_as_uint(c.w);
 }
 
 template <bool PACK, bool NINE, bool VM = false>
@@ -134,10 +145,21 @@ struct Stream {
     return Raw<PACK>{__ldg(A + off), __ldg(B + off)};
   }
 
-  // update row y from its window (up, c, dn); rc = raw centre record
-  __device__ __forceinline__ void update(int y, const NbT<NINE, VM>& up, const NbT<NINE, VM>& c,
-                                         const NbT<NINE, VM>& dn, const Raw<PACK>& rc) const {
-    float lapCr, lapNb, lapD, lapL;
+  __device__ __forceinline__ void store(int y, const Raw<PACK>& r) const {
+    if (out) {
+      const int i = y * P;
+      Ao[i] = r.a;
+      Bo[i] = r.c;
+    }
+  }
+
+  // The record of a row one step on, from its window (up, c, dn); rc = its
+  // raw record.  still: the phases and their compensations are zero in all
+  // three rows (Row::still): they stay zero.
+  __device__ __forceinline__ Raw<PACK> step(const NbT<NINE, VM>& up, const NbT<NINE, VM>& c,
+                                            const NbT<NINE, VM>& dn, const Raw<PACK>& rc,
+                                            bool still) const {
+    float lapCr, lapNb, lapD = 0.0f, lapL = 0.0f;
     if constexpr (VM) {
       // variable mobility: lapCr, lapNb hold dt times the divergence of
       // D grad u over the four faces, ((D_n + D_c)(u_n - u_c) summed), the
@@ -164,17 +186,19 @@ struct Stream {
               qy * (in(up, up.d00, up.d01, c.d00, c.d01) + in(dn, dn.d00, dn.d01, c.d00, c.d01));
       lapNb = (fNb - up1(fNb)) +
               qy * (in(up, up.d10, up.d11, c.d10, c.d11) + in(dn, dn.d10, dn.d11, c.d10, c.d11));
-      Nb w;
-      w.pd = up1(c.pd);
-      w.pl = up1(c.pl);
-      e.pd = dn1(c.pd);
-      e.pl = dn1(c.pl);
-      const float idx2 = a.idx2f[0], idy2 = a.idx2f[1];
-      auto lap = [&](float vw, float ve, float vn, float vs, float vc) {
-        return fmaf((vw - vc) + (ve - vc), idx2, ((vn - vc) + (vs - vc)) * idy2);
-      };
-      lapD = lap(w.pd, e.pd, up.pd, dn.pd, c.pd);
-      lapL = lap(w.pl, e.pl, up.pl, dn.pl, c.pl);
+      if (!still) {
+        Nb w;
+        w.pd = up1(c.pd);
+        w.pl = up1(c.pl);
+        e.pd = dn1(c.pd);
+        e.pl = dn1(c.pl);
+        const float idx2 = a.idx2f[0], idy2 = a.idx2f[1];
+        auto lap = [&](float vw, float ve, float vn, float vs, float vc) {
+          return fmaf((vw - vc) + (ve - vc), idx2, ((vn - vc) + (vs - vc)) * idy2);
+        };
+        lapD = lap(w.pd, e.pd, up.pd, dn.pd, c.pd);
+        lapL = lap(w.pl, e.pl, up.pl, dn.pl, c.pl);
+      }
     } else if constexpr (NINE) {
       // sum over the eight neighbours of w (v - v_c): with sy = (v_up - v_c)
       // + (v_dn - v_c) the corners add up to h_up + h_dn + 2 sy; then the
@@ -190,18 +214,16 @@ struct Stream {
       };
       lapCr = lap(up.h1, c.h1, dn.h1, up.u1, c.u1, dn.u1, a.lap9xe[0]);
       lapNb = lap(up.h2, c.h2, dn.h2, up.u2, c.u2, dn.u2, a.lap9xe[1]);
-      lapD = lap(up.hd, c.hd, dn.hd, up.pd, c.pd, dn.pd, 0.0f);
-      lapL = lap(up.hl, c.hl, dn.hl, up.pl, c.pl, dn.pl, 0.0f);
+      if (!still) {
+        lapD = lap(up.hd, c.hd, dn.hd, up.pd, c.pd, dn.pd, 0.0f);
+        lapL = lap(up.hl, c.hl, dn.hl, up.pl, c.pl, dn.pl, 0.0f);
+      }
     } else {
       Nb w, e;
       w.u1 = __shfl_up_sync(0xffffffffu, c.u1, 1);
       w.u2 = __shfl_up_sync(0xffffffffu, c.u2, 1);
-      w.pd = __shfl_up_sync(0xffffffffu, c.pd, 1);
-      w.pl = __shfl_up_sync(0xffffffffu, c.pl, 1);
       e.u1 = __shfl_down_sync(0xffffffffu, c.u1, 1);
       e.u2 = __shfl_down_sync(0xffffffffu, c.u2, 1);
-      e.pd = __shfl_down_sync(0xffffffffu, c.pd, 1);
-      e.pl = __shfl_down_sync(0xffffffffu, c.pl, 1);
       const float idx2 = a.idx2f[0], idy2 = a.idx2f[1];
       auto lap = [&](float vw, float ve, float vn, float vs, float vc) {
         const float sx = (vw - vc) + (ve - vc);
@@ -210,38 +232,90 @@ struct Stream {
       };
       lapCr = lap(w.u1, e.u1, up.u1, dn.u1, c.u1);
       lapNb = lap(w.u2, e.u2, up.u2, dn.u2, c.u2);
-      lapD = lap(w.pd, e.pd, up.pd, dn.pd, c.pd);
-      lapL = lap(w.pl, e.pl, up.pl, dn.pl, c.pl);
+      if (!still) {
+        w.pd = __shfl_up_sync(0xffffffffu, c.pd, 1);
+        w.pl = __shfl_up_sync(0xffffffffu, c.pl, 1);
+        e.pd = __shfl_down_sync(0xffffffffu, c.pd, 1);
+        e.pl = __shfl_down_sync(0xffffffffu, c.pl, 1);
+        lapD = lap(w.pd, e.pd, up.pd, dn.pd, c.pd);
+        lapL = lap(w.pl, e.pl, up.pl, dn.pl, c.pl);
+      }
     }
-    const float4 cc = comps<PACK>(rc.c);
+    const float2 cx = comps_x<PACK>(rc.c);
     // Cahn-Hilliard
     const float X = rc.a.x, Y = rc.a.y;
     float ycr, ynb;
     if constexpr (VM) {
-      ycr = lapCr - cc.x;
-      ynb = lapNb - cc.y;
+      ycr = lapCr - cx.x;
+      ynb = lapNb - cx.y;
     } else {
-      ycr = fmaf(a.dtD[0][0], lapCr, a.dtD[0][1] * lapNb) - cc.x;
-      ynb = fmaf(a.dtD[1][0], lapCr, a.dtD[1][1] * lapNb) - cc.y;
+      ycr = fmaf(a.dtD[0][0], lapCr, a.dtD[0][1] * lapNb) - cx.x;
+      ynb = fmaf(a.dtD[1][0], lapCr, a.dtD[1][1] * lapNb) - cx.y;
     }
     const float tcr = X + ycr, tnb = Y + ynb;
+    const float ox = (tcr - X) - ycr, oy = (tnb - Y) - ynb;
+    Raw<PACK> r;
+    if (still) {
+      r.a = make_float4(tcr, tnb, 0.0f, 0.0f);
+      if constexpr (PACK)
+        r.c = make_uint2(cq_pair(ox * kCqX, oy * kCqX), 0u);
+      else
+        r.c = make_float4(ox, oy, 0.0f, 0.0f);
+      return r;
+    }
     // Allen-Cahn
     const FastCoef& K = a.k;
+    const float2 cp = comps_p<PACK>(rc.c);
     const float phd = c.pd, phl = c.pl;
     const float dFd = fmaf(-a.kap[0], lapD, dF_local32(phd, phl, quad2(K.dP[0], c.u1, c.u2), a.om2[0], a.alpha2));
     const float dFl = fmaf(-a.kap[1], lapL, dF_local32(phl, phd, quad2(K.dP[1], c.u1, c.u2), a.om2[1], a.alpha2));
-    const float yd = fmaf(-a.dtL[0], dFd, -cc.z), td = phd + yd;
-    const float yl = fmaf(-a.dtL[1], dFl, -cc.w), tl = phl + yl;
-    if (out) {
-      const int i = y * P;
-      Ao[i] = make_float4(tcr, tnb, td, tl);
-      const float ox = (tcr - X) - ycr, oy = (tnb - Y) - ynb;
-      const float od = (td - phd) - yd, ol = (tl - phl) - yl;
-      if constexpr (PACK)
-        Bo[i] = cq_pack(ox, oy, od, ol);
-      else
-        Bo[i] = make_float4(ox, oy, od, ol);
+    const float yd = fmaf(-a.dtL[0], dFd, -cp.x), td = phd + yd;
+    const float yl = fmaf(-a.dtL[1], dFl, -cp.y), tl = phl + yl;
+    r.a = make_float4(tcr, tnb, td, tl);
+    const float od = (td - phd) - yd, ol = (tl - phl) - yl;
+    if constexpr (PACK)
+      r.c = cq_pack(ox, oy, od, ol);
+    else
+      r.c = make_float4(ox, oy, od, ol);
+    return r;
+  }
+
+  // What a step needs of a row's raw record: the gamma solve, and whether
+  // the whole warp's phases and their compensations are zero (compositions
+  // that are not finite make 0 x NaN in the Allen-Cahn terms and are not
+  // still).  Whole warp.
+  __device__ __forceinline__ NbT<NINE, VM> solve(const Raw<PACK>& r, bool& still) const {
+    const FastCoef& K = a.k;
+    const float2 cxy = comps_x<PACK>(r.c);
+    NbT<NINE, VM> n;
+    n.pd = r.a.z;
+    n.pl = r.a.w;
+    const unsigned cb = PACK ? comp_bits(r.c) : comp_bits(r.c) & 0x7fffffffu;
+    const unsigned z = __float_as_uint(fmaf(r.a.x, 0.0f, fmaf(r.a.y, 0.0f, fabsf(r.a.z)))) |
+                       __float_as_uint(fabsf(r.a.w)) | cb;
+    still = __all_sync(0xffffffffu, z == 0u);
+    // a cell of pure gamma needs no solve; each cell takes its own form,
+    // whatever its neighbours in the warp do, so that results do not depend
+    // on how a grid is cut into strips
+    if (fmaxf(fabsf(r.a.z), fabsf(r.a.w)) >= kBulkPhi)
+      gamma_u32(K, r.a.x, r.a.y, cxy.x, cxy.y, r.a.z, r.a.w, n.u1, n.u2);
+    else
+      gamma_bulk32(K, r.a.x, r.a.y, cxy.x, cxy.y, n.u1, n.u2);
+    if constexpr (VM) dmat32(a.vm_pre, r.a.x, r.a.y, n.d00, n.d01, n.d10, n.d11);
+    if constexpr (NINE) {
+      auto hx = [](float v) {
+        return (__shfl_up_sync(0xffffffffu, v, 1) - v) + (__shfl_down_sync(0xffffffffu, v, 1) - v);
+      };
+      n.h1 = hx(n.u1);
+      n.h2 = hx(n.u2);
+      if (still) {
+        n.hd = n.hl = 0.0f;
+      } else {
+        n.hd = hx(n.pd);
+        n.hl = hx(n.pl);
+      }
     }
+    return n;
   }
 };
 
@@ -262,54 +336,34 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
   static_assert(!(STAGED && NINE), "the staged (batched) form has the 5-point mask only");
   static_assert(!(STAGED && VM), "the staged (batched) form has the constant mobility only");
   static_assert(!(NINE && VM), "the variable-mobility form has the 5-point mask only");
-  const FastCoef& K = a.k;
   const Stream<PACK, NINE, VM> S{a, Ain + cx, Bin + cx, Aout + cx, Bout + cx,
                              Ny, P, lane >= 1 && lane <= kCols && gx < Nx};
-  auto solve_raw = [&](const Raw<PACK>& r) {
-    const float2 cxy = comps_x<PACK>(r.c);
-    NbT<NINE, VM> n;
-    n.pd = r.a.z;
-    n.pl = r.a.w;
-    // warp-uniform choice: a row of pure gamma needs no solve
-    if (__all_sync(0xffffffffu, fmaxf(fabsf(r.a.z), fabsf(r.a.w)) < kBulkPhi))
-      gamma_bulk32(K, r.a.x, r.a.y, cxy.x, cxy.y, n.u1, n.u2);
-    else
-      gamma_u32(K, r.a.x, r.a.y, cxy.x, cxy.y, r.a.z, r.a.w, n.u1, n.u2);
-    if constexpr (VM) dmat32(a.vm_pre, r.a.x, r.a.y, n.d00, n.d01, n.d10, n.d11);
-    if constexpr (NINE) {
-      auto hx = [](float v) {
-        return (__shfl_up_sync(0xffffffffu, v, 1) - v) + (__shfl_down_sync(0xffffffffu, v, 1) - v);
-      };
-      n.h1 = hx(n.u1);
-      n.h2 = hx(n.u2);
-      n.hd = hx(n.pd);
-      n.hl = hx(n.pl);
-    }
-    return n;
-  };
+  bool z0, z1, z2;  // rows y-1, y, y+1 are still
   if constexpr (!STAGED) {
     // window rows y-1, y, y+1 and raw records of rows y, y+1, y+2
     Raw<PACK> r0 = S.load(S.row(y0)), r1 = S.load(S.row(y0 + 1)), r2;
-    NbT<NINE, VM> n0 = solve_raw(S.load(S.row(y0 - 1))), n1 = solve_raw(r0), n2;
+    NbT<NINE, VM> n0 = S.solve(S.load(S.row(y0 - 1)), z0), n1 = S.solve(r0, z1), n2;
     // three rows per iteration with rotated roles: no register moves
     int y = y0;
     for (; y + 2 < y1; y += 3) {
       r2 = S.load(S.row(y + 2));
-      n2 = solve_raw(r1);
-      S.update(y, n0, n1, n2, r0);
+      n2 = S.solve(r1, z2);
+      S.store(y, S.step(n0, n1, n2, r0, z0 && z1 && z2));
       r0 = S.load(S.row(y + 3));
-      n0 = solve_raw(r2);
-      S.update(y + 1, n1, n2, n0, r1);
+      n0 = S.solve(r2, z0);
+      S.store(y + 1, S.step(n1, n2, n0, r1, z0 && z1 && z2));
       r1 = S.load(S.row(y + 4));
-      n1 = solve_raw(r0);
-      S.update(y + 2, n2, n0, n1, r2);
+      n1 = S.solve(r0, z1);
+      S.store(y + 2, S.step(n2, n0, n1, r2, z0 && z1 && z2));
     }
     for (; y < y1; y++) {
       r2 = S.load(S.row(y + 2));
-      n2 = solve_raw(r1);
-      S.update(y, n0, n1, n2, r0);
+      n2 = S.solve(r1, z2);
+      S.store(y, S.step(n0, n1, n2, r0, z0 && z1 && z2));
       n0 = n1;
       n1 = n2;
+      z0 = z1;
+      z1 = z2;
       r0 = r1;
       r1 = r2;
     }
@@ -334,29 +388,31 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
 #pragma unroll
     for (int k = 0; k < kDepth; k++) issue(y0 - 1 + k, k);
     cp_wait<kDepth - 2>();  // rows y0-1 and y0 have landed
-    Nb n0 = solve_raw(fetch(0)), n1 = solve_raw(fetch(1)), n2;
+    Nb n0 = S.solve(fetch(0), z0), n1 = S.solve(fetch(1), z1), n2;
     int s = 0;  // slot of row y-1
     // row y: refill the slot of row y-1 (read for row y-1's update) with row
     // y-1+kDepth, wait for row y+1 (kDepth-2 newer groups stay in flight),
     // solve it, update row y.  Rows up to y1 were all waited for by the last
     // row, so no copy into the ring is pending when the strip ends.
-    auto body = [&](int y, const Nb& up, const Nb& c, Nb& dn) {
+    auto body = [&](int y, const Nb& up, const Nb& c, Nb& dn, bool& zdn) {
       issue(y - 1 + kDepth, s);
       s = (s + 1) & (kDepth - 1);
       cp_wait<kDepth - 2>();
-      dn = solve_raw(fetch((s + 1) & (kDepth - 1)));
-      S.update(y, up, c, dn, fetch(s));
+      dn = S.solve(fetch((s + 1) & (kDepth - 1)), zdn);
+      S.store(y, S.step(up, c, dn, fetch(s), z0 && z1 && z2));
     };
     int y = y0;
     for (; y + 2 < y1; y += 3) {
-      body(y, n0, n1, n2);
-      body(y + 1, n1, n2, n0);
-      body(y + 2, n2, n0, n1);
+      body(y, n0, n1, n2, z2);
+      body(y + 1, n1, n2, n0, z0);
+      body(y + 2, n2, n0, n1, z1);
     }
     for (; y < y1; y++) {
-      body(y, n0, n1, n2);
+      body(y, n0, n1, n2, z2);
       n0 = n1;
       n1 = n2;
+      z0 = z1;
+      z1 = z2;
     }
   }
 }
@@ -378,21 +434,163 @@ __global__ void __launch_bounds__(32 * kWarps, VM ? 6 : (PACK && !NINE ? 9 : 8))
                             a.Nx, a.Ny, a.pitch, x0, y0, min(y0 + a.rows, a.Ny), nullptr);
 }
 
+// ---- two steps in one pass ----
+// The strip of output columns x0 .. x0+27 over rows y0 .. y1-1, two steps on:
+// row y+1 is advanced once (from rows y, y+1, y+2 as loaded), solved again,
+// and row y advanced the second time from its once-advanced neighbours, all
+// in registers, so a record crosses HBM once for two steps.  The values and
+// their order of operations are those of two single steps (the packed
+// compensations are rounded in between as the store would), so the result is
+// the same bits.  Lanes 0, 1 and 30, 31 are halo: the first step is right on
+// lanes 1 .. 30, the second on 2 .. 29.  A once-advanced record beyond the
+// domain mirrors the one at its edge.
+//
+// Bound: latency and issue (106 instructions a cell and step, 58 % of the
+// issue slots; HBM would allow 60 us a step at 4096^2).  Rows come through a
+// per-warp cp.async ring, which holds the row whose first step is due besides
+// the rows ahead and so leaves 80 registers without spills, 6 CTAs per SM
+// (rows in registers, one ahead: 89.8 us; 7 or 8 CTAs with spills: 118 and
+// 101).  4096^2: 129 us a step in single steps -> 76; FP32 compensations 176
+// -> 85, 9 points 131 -> 91; 2048^2 35.3 -> 22.8.
+constexpr int kCols2 = 28;
+constexpr int kDepth2 = 8;  // rows in the ring (a power of two)
+template <bool PACK>
+struct Ring2 {
+  float4 a[kDepth2][32];
+  CompT<PACK> c[kDepth2][32];
+};
+
+template <bool PACK, bool NINE>
+__device__ __forceinline__ void stream_strip2(const Step2DArgs& a, const float4* Ain,
+                                              const CompT<PACK>* Bin, float4* Aout,
+                                              CompT<PACK>* Bout, int Nx, int Ny, int P, int x0,
+                                              int y0, int y1, Ring2<PACK>* ring) {
+  const int lane = threadIdx.x & 31;
+  const int gx = x0 - 2 + lane;
+  const int cx = min(max(gx, 0), Nx - 1);
+  const Stream<PACK, NINE> S{a, Ain + cx, Bin + cx, Aout + cx, Bout + cx, Ny, P,
+                                 lane >= 2 && lane < 2 + kCols2 && gx < Nx};
+  const bool edge = x0 == 0 || x0 + kCols2 >= Nx;  // whole warp
+  const int mirror = cx - (x0 - 2);                // the lane holding column cx
+  using N = NbT<NINE>;
+  using R = Raw<PACK>;
+  // ring slot k holds rows y0-2+k, y0-2+k+kDepth2, ...; each lane copies and
+  // reads back only its own column's records, so the waits need no warp sync
+  const uint32_t sa = uint32_t(__cvta_generic_to_shared(&ring->a[0][lane]));
+  const uint32_t sc = uint32_t(__cvta_generic_to_shared(&ring->c[0][lane]));
+  constexpr uint32_t kSlotA = 32 * sizeof(float4), kSlotC = 32 * sizeof(CompT<PACK>);
+  auto issue = [&](int y, int slot) {
+    if (y <= y1 + 1) {  // rows past y1 + 1 are never read
+      const int off = S.row(y);
+      cp_async16(sa + slot * kSlotA, S.A + off);
+      if constexpr (PACK)
+        cp_async8(sc + slot * kSlotC, S.B + off);
+      else
+        cp_async16(sc + slot * kSlotC, S.B + off);
+    }
+    cp_commit();  // one group per row (empty past y1 + 1): the wait counts stay uniform
+  };
+  auto fetch = [&](int slot) { return R{ring->a[slot][lane], ring->c[slot][lane]}; };
+  // first step of a row
+  auto first = [&](const N& up, const N& c, const N& dn, const R& rc, bool still) {
+    R r = S.step(up, c, dn, rc, still);
+    if (edge) {
+      auto m = [&](float v) { return __shfl_sync(0xffffffffu, v, mirror); };
+      r.a = make_float4(m(r.a.x), m(r.a.y), m(r.a.z), m(r.a.w));
+      if constexpr (PACK)
+        r.c = make_uint2(__shfl_sync(0xffffffffu, r.c.x, mirror), __shfl_sync(0xffffffffu, r.c.y, mirror));
+      else
+        r.c = make_float4(m(r.c.x), m(r.c.y), m(r.c.z), m(r.c.w));
+    }
+    return r;
+  };
+#pragma unroll
+  for (int k = 0; k < kDepth2; k++) issue(y0 - 2 + k, k);
+  cp_wait<kDepth2 - 4>();  // rows y0-2 .. y0+1 have landed
+  // s: solves of the loaded rows y, y+1, y+2; u: solves of the once-advanced
+  // rows y-1, y, y+1; t: once-advanced records of rows y, y+1
+  N s0, s1, s2, u0, u1, u2;
+  R t1, t2, t0;
+  bool zs0, zs1, zs2, zu0, zu1, zu2;
+  {
+    bool za, zb;
+    const N sa_ = S.solve(fetch(0), za), sb_ = S.solve(fetch(1), zb);
+    s0 = S.solve(fetch(2), zs0);
+    s1 = S.solve(fetch(3), zs1);
+    t1 = first(sb_, s0, s1, fetch(2), zb && zs0 && zs1);
+    t0 = y0 == 0 ? t1 : first(sa_, sb_, s0, fetch(1), za && zb && zs0);
+    u0 = S.solve(t0, zu0);
+    u1 = S.solve(t1, zu1);
+  }
+  issue(y0 - 2 + kDepth2, 0);
+  issue(y0 - 1 + kDepth2, 1);
+  int s = 2;  // slot of row y
+  // one output row: row y's slot is refilled with row y+kDepth2, row y+2 waited
+  // for (kDepth2-2 newer groups stay in flight); window (sa, sb, sc), window
+  // (ua, ub, uc), records tb in, tc out
+  auto body = [&](int y, const N& sa, const N& sb, N& sc, bool za, bool zb, bool& zc, const N& ua,
+                  const N& ub, N& uc, bool wa, bool wb, bool& wc, const R& tb, R& tc) {
+    issue(y + kDepth2, s);
+    s = (s + 1) & (kDepth2 - 1);
+    cp_wait<kDepth2 - 2>();
+    sc = S.solve(fetch((s + 1) & (kDepth2 - 1)), zc);
+    tc = first(sa, sb, sc, fetch(s), za && zb && zc);
+    if (y + 1 >= Ny) tc = tb;
+    uc = S.solve(tc, wc);
+    S.store(y, S.step(ua, ub, uc, tb, wa && wb && wc));
+  };
+  int y = y0;
+  for (; y + 2 < y1; y += 3) {
+    body(y, s0, s1, s2, zs0, zs1, zs2, u0, u1, u2, zu0, zu1, zu2, t1, t2);
+    body(y + 1, s1, s2, s0, zs1, zs2, zs0, u1, u2, u0, zu1, zu2, zu0, t2, t0);
+    body(y + 2, s2, s0, s1, zs2, zs0, zs1, u2, u0, u1, zu2, zu0, zu1, t0, t1);
+  }
+  for (; y < y1; y++) {
+    body(y, s0, s1, s2, zs0, zs1, zs2, u0, u1, u2, zu0, zu1, zu2, t1, t2);
+    s0 = s1;
+    s1 = s2;
+    zs0 = zs1;
+    zs1 = zs2;
+    u0 = u1;
+    u1 = u2;
+    zu0 = zu1;
+    zu1 = zu2;
+    t1 = t2;
+  }
+  cp_wait<0>();  // only empty groups are left
+}
+
+template <bool PACK, bool NINE>
+__global__ void __launch_bounds__(32 * kWarps, PACK && !NINE ? 6 : 4) k_stream2_f32(Step2DArgs a) {
+  __shared__ Ring2<PACK> ring[kWarps];
+  const int strip = blockIdx.x * kWarps + (threadIdx.x >> 5);
+  const int x0 = strip * kCols2;
+  if (x0 >= a.Nx) return;
+  const int y0 = blockIdx.y * a.rows;
+  stream_strip2<PACK, NINE>(a, static_cast<const float4*>(a.in[0]),
+                                static_cast<const CompT<PACK>*>(a.in[1]),
+                                static_cast<float4*>(a.out[0]), static_cast<CompT<PACK>*>(a.out[1]),
+                                a.Nx, a.Ny, a.pitch, x0, y0, min(y0 + a.rows, a.Ny),
+                                &ring[threadIdx.x >> 5]);
+}
+
 // ---- many grids in one launch ----
 // Warps claim units (grid, strip, row segment) of the batch's unit table
 // through an atomic counter (counter[parity]) until the unit count in
-// counter[2] is reached, so a captured launch stays valid while the table's
+// counter[2] (TWO: counter[3]) is reached, so a captured launch stays valid while the table's
 // contents change.  The launch also zeroes the other parity's counter for the
-// next step, which stream order runs after this one.  A persistent launch
+// next launch, which stream order runs after this one.  A persistent launch
 // has one CTA per resident slot; the other shape has one warp per unit (and
-// leaves the balancing to the block scheduler).  Unit indices come only from
-// the counter: ptxas keeps this form within 64 registers without spills.
-// Rows are staged through a cp.async ring per warp (12 KB per CTA).
-__global__ void __launch_bounds__(32 * kWarps, 8) k_batch_f32(Step2DArgs a, BatchArgs b) {
+// leaves the balancing to the block scheduler).  TWO: two steps in one pass
+// (strips of 28 columns), else one (strips of 30).  Unit indices come only
+// from the counter.
+template <bool TWO>
+__global__ void __launch_bounds__(32 * kWarps, TWO ? 6 : 8) k_batch_f32(Step2DArgs a, BatchArgs b) {
   const int p = b.parity;
   if (blockIdx.x == 0 && threadIdx.x == 0) b.counter[p ^ 1] = 0;
-  const int units = b.counter[2];
-  __shared__ Ring<true> ring[kWarps];
+  const int units = b.counter[TWO ? 3 : 2];
+  using R = typename std::conditional<TWO, Ring2<true>, Ring<true>>::type;
+  __shared__ R ring[kWarps];
   for (;;) {
     int u = 0;
     if ((threadIdx.x & 31) == 0) u = atomicAdd(b.counter + p, 1);
@@ -400,8 +598,13 @@ __global__ void __launch_bounds__(32 * kWarps, 8) k_batch_f32(Step2DArgs a, Batc
     if (u >= units) return;
     const BatchUnit w = b.unit[u];
     const BatchGrid& g = b.grid[w.grid];
-    stream_strip<true, true>(a, g.A[p], g.B[p], g.A[p ^ 1], g.B[p ^ 1], g.Nx, g.Ny, g.pitch,
-                             w.x0, w.y0, w.y1, &ring[threadIdx.x >> 5]);
+    R* r = &ring[threadIdx.x >> 5];
+    if constexpr (TWO)
+      stream_strip2<true, false>(a, g.A[p], g.B[p], g.A[p ^ 1], g.B[p ^ 1], g.Nx, g.Ny, g.pitch,
+                                 w.x0, w.y0, w.y1, r);
+    else
+      stream_strip<true, true>(a, g.A[p], g.B[p], g.A[p ^ 1], g.B[p ^ 1], g.Nx, g.Ny, g.pitch,
+                               w.x0, w.y0, w.y1, r);
   }
 }
 
@@ -455,47 +658,27 @@ __global__ void k_export_records(ConvArgs a) {
   }
 }
 
-// Rows per warp segment.  Grids that give every resident CTA 24 rows or more:
-// the CTA count should fill whole waves of the resident CTAs (a partial last
-// wave idles SMs), while each segment pays two extra rows of gamma solves at
-// its ends.  Smaller grids leave SMs idle at that length and each row of a
-// segment is a serial load-solve-update chain (about 0.4 us when few warps
-// share an SM), so their segments are short: one row while the grid has no
-// more rows of CTAs than resident slots, else 3 (one pass of the unrolled
-// loop), and 6 once 3-row segments oversubscribe the slots.  Measured, us per
-// step, whole columns (the rule above with nothing to choose) -> these:
-// 256^2 87 -> 3.1 (3 rows 3.7), 512^2 165 -> 4.7 (1 row 5.4, 6 rows 5.7),
-// 1024^2 317 -> 10.0 (1 row 13.6, 12 rows 11.2), 1531 x 1021 432 -> 13.1
-// (3 rows 13.5, 12 rows 13.5); variable mobility 1531 x 1021 411 -> 17.0
-// (3 rows 18.5, 12 rows 17.9).
-int segment_rows(int Nx, int Ny, int resident) {
+// Rows per warp segment of a single step.  Each segment solves two extra
+// rows, but a row is a serial load-solve-update chain (about 0.4 us where few
+// warps share an SM), and the more segments there are the better they
+// balance: 3 rows, one pass of the unrolled loop, are the best or within 2 %
+// of it from 512^2 up (us a step at 3 / 6 / 24 / 96 rows: 512^2 4.2 / 5.3 /
+// 13.0 / 34.9, 1024^2 7.5 / 7.7 / 13.8 / 36, 2048^2 32.6 / 33.0 / 41 / 61,
+// 4096^2 119 / 120 / 130 / 159; FP32 compensations 4096^2 151 / 157 / 170 /
+// 186), and 1 row while a grid has no more rows of CTAs than resident slots
+// (256^2 3.0 against 3.6 at 3 rows).  The variable-mobility step, whose extra
+// rows cost three exponentials a cell, takes 6 and 9 from there (1531 x 1021
+// 18.5 at 3, 17.0 at 6; 4096^2 149 at 3, 139.9 at 6, 137.9 at 9).
+int segment_rows(int Nx, int Ny, int resident, bool varmob) {
   const int nbx = ((Nx + kCols - 1) / kCols + kWarps - 1) / kWarps;
-  const long long load = (long long)nbx * Ny;  // CTA rows
-  if (load < 24LL * resident) {
-    const int rows = load <= resident ? 1 : (load <= 6LL * resident ? 3 : 6);
-    return rows < Ny ? rows : Ny;
-  }
-  int best = Ny;
-  double best_score = 0.0;
-  for (int waves = 1; waves <= 256; waves++) {
-    const long long segs = (long long)waves * resident / nbx;
-    if (segs < 1) continue;
-    const int rows = int((Ny + segs - 1) / segs);
-    if (rows < 24 && segs > 1) break;
-    const long long used = (long long)nbx * ((Ny + rows - 1) / rows);
-    const long long slots = ((used + resident - 1) / resident) * (long long)resident;
-    const double score = double(used) / double(slots) / (1.0 + 2.0 / rows);
-    if (score > best_score) {
-      best_score = score;
-      best = rows;
-    }
-  }
-  return best;
+  const double load = double(nbx) * Ny / resident;  // CTA rows per resident CTA
+  const int rows = load <= 1.0 ? 1 : (!varmob || load <= 6.0 ? 3 : (load <= 24.0 ? 6 : 9));
+  return std::min(rows, Ny);
 }
 
 // resident CTAs: FP32 / packed variants, the batch kernel, the 9-point FP32 / packed
 // variants, the variable-mobility FP32 / packed variants
-int g_resident[7] = {0, 0, 0, 0, 0, 0, 0};
+int g_resident[12] = {};  // + 7: the two-step kernels (constant mobility), 11: the batch's
 
 template <typename K>
 cudaError_t query_resident(K kernel, int slot) {
@@ -512,20 +695,60 @@ template <bool PACK, bool NINE, bool VM = false>
 cudaError_t launch_stream(Step2DArgs a, cudaStream_t s) {
   const int slot = VM ? 5 + PACK : (NINE ? 3 + PACK : PACK);
   const int resident = g_resident[slot] > 0 ? g_resident[slot] : 152 * 8;
-  a.rows = segment_rows(a.Nx, a.Ny, resident);
+  a.rows = segment_rows(a.Nx, a.Ny, resident, VM);
   const int strips = (a.Nx + kCols - 1) / kCols;
   dim3 grid((strips + kWarps - 1) / kWarps, (a.Ny + a.rows - 1) / a.rows);
   k_stream_f32<PACK, NINE, VM><<<grid, 32 * kWarps, 0, s>>>(a);
   return cudaGetLastError();
 }
 
+// Rows per segment of a two-step pass: each segment solves six extra rows and
+// waits for its first four, fewer rows balance the CTAs better; the product
+// of (1 + c / rows) and (1 + d rows / load) is least at sqrt(c load / d),
+// with c / d = 6 from the sweeps (us a step at 6 / 9 / 15 / 24 / 36 / 96 rows:
+// 2048^2 26.2 / 24.1 / 22.8 / 24.1 / 27.1 / 35.8, 4096^2 94.2 / 86.1 / 79.5 /
+// 76.4 / 76.1 / 77.7); a multiple of the unrolled loop's three.
+int segment_rows2(int Nx, int Ny, int resident) {
+  const int nbx = ((Nx + kCols2 - 1) / kCols2 + kWarps - 1) / kWarps;
+  const double load = double(nbx) * Ny / resident;  // CTA rows per resident CTA
+  const int rows = 3 * std::max(2, int(std::sqrt(6.0 * load) / 3.0 + 0.5));
+  return std::min(rows, Ny);
+}
+
+template <bool PACK, bool NINE>
+cudaError_t launch_stream2(Step2DArgs a, cudaStream_t s) {
+  const int slot = 7 + 2 * NINE + PACK;
+  const int resident = g_resident[slot] > 0 ? g_resident[slot] : 152 * 4;
+  a.rows = segment_rows2(a.Nx, a.Ny, resident);
+  const int strips = (a.Nx + kCols2 - 1) / kCols2;
+  dim3 grid((strips + kWarps - 1) / kWarps, (a.Ny + a.rows - 1) / a.rows);
+  k_stream2_f32<PACK, NINE><<<grid, 32 * kWarps, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
-cudaError_t launch_step2d_f32(const Step2DArgs& a, cudaStream_t s) {
+// Two steps in one pass save HBM traffic, which binds once the two record
+// sets exceed the L2 (129 MB): at 1531 x 1021 (75 MB) single steps take 10.2
+// us and double ones 12.0, at 1536^2 (113 MB) 17.0 and 14.7.  Smaller grids
+// are bound by launches and latency, which a pass of twice the work does not
+// shorten (256^2 2.96 and 3.09 us).  The variable-mobility step is bound by
+// issue (4096^2 137.9 us, 133.8 in double passes): single steps.
+bool two_steps_bytes(double bytes) { return bytes > 96e6; }
+
+bool two_steps_f32(const Step2DArgs& a) {
+  return !a.varmob && two_steps_bytes(double(a.pitch) * a.Ny * (a.full_comp ? 64 : 48));
+}
+
+cudaError_t launch_step2d_f32(const Step2DArgs& a, bool two, cudaStream_t s) {
   if (a.varmob) {
-    if (a.nine) return cudaErrorInvalidValue;  // refused by the host before
+    if (a.nine || two) return cudaErrorInvalidValue;  // refused by the host before
     return a.full_comp ? launch_stream<false, false, true>(a, s)
                        : launch_stream<true, false, true>(a, s);
+  }
+  if (two) {
+    if (a.nine) return a.full_comp ? launch_stream2<false, true>(a, s) : launch_stream2<true, true>(a, s);
+    return a.full_comp ? launch_stream2<false, false>(a, s) : launch_stream2<true, false>(a, s);
   }
   if (a.nine) return a.full_comp ? launch_stream<false, true>(a, s) : launch_stream<true, true>(a, s);
   return a.full_comp ? launch_stream<false, false>(a, s) : launch_stream<true, false>(a, s);
@@ -535,24 +758,36 @@ cudaError_t launch_step2d_f32(const Step2DArgs& a, cudaStream_t s) {
 cudaError_t prepare_step2d_f32() {
   cudaError_t e = query_resident(k_stream_f32<false, false>, 0);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<true, false>, 1);
-  if (e == cudaSuccess) e = query_resident(k_batch_f32, 2);
+  if (e == cudaSuccess) e = query_resident(k_batch_f32<false>, 2);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<false, true>, 3);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<true, true>, 4);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<false, false, true>, 5);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<true, false, true>, 6);
+  if (e == cudaSuccess) e = query_resident(k_stream2_f32<false, false>, 7);
+  if (e == cudaSuccess) e = query_resident(k_stream2_f32<true, false>, 8);
+  if (e == cudaSuccess) e = query_resident(k_stream2_f32<false, true>, 9);
+  if (e == cudaSuccess) e = query_resident(k_stream2_f32<true, true>, 10);
+  if (e == cudaSuccess) e = query_resident(k_batch_f32<true>, 11);
   return e;
 }
 
-cudaError_t launch_batch_f32(const Step2DArgs& a, const BatchArgs& b, int ctas, cudaStream_t s) {
+cudaError_t launch_batch_f32(const Step2DArgs& a, const BatchArgs& b, bool two, int ctas,
+                             cudaStream_t s) {
   const int grid = b.persistent ? ctas : (b.units + kWarps - 1) / kWarps;
   if (grid <= 0) return cudaSuccess;
-  k_batch_f32<<<grid, 32 * kWarps, 0, s>>>(a, b);
+  if (two)
+    k_batch_f32<true><<<grid, 32 * kWarps, 0, s>>>(a, b);
+  else
+    k_batch_f32<false><<<grid, 32 * kWarps, 0, s>>>(a, b);
   return cudaGetLastError();
 }
 
-int batch_resident_ctas() { return g_resident[2] > 0 ? g_resident[2] : 152 * 8; }
+int batch_resident_ctas(bool two) {
+  const int n = g_resident[two ? 11 : 2];
+  return n > 0 ? n : 152 * (two ? 6 : 8);
+}
 int batch_warps_per_cta() { return kWarps; }
-int batch_strip_cols() { return kCols; }
+int batch_strip_cols(bool two) { return two ? kCols2 : kCols; }
 
 cudaError_t launch_import_f32(const ConvArgs& a, cudaStream_t s) {
   const int rows = (a.y1 > 0 ? a.y1 : a.Ny) - a.y0;

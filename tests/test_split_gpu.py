@@ -7,9 +7,9 @@ from pfa_gb300 import ic
 pytestmark = pytest.mark.gpu
 
 
-# sizes on both sides of the split rule's lines (152 SMs: one-row segments up
-# to 1368 CTA rows, three-row segments up to 8208, six-row ones above), one
-# strip and more, and row counts that leave remainders of the unrolled loop
+# sizes on both sides of the split rule's line (152 SMs: one-row segments up
+# to 1368 CTA rows, three-row segments above), one strip and more, and row
+# counts that leave remainders of the unrolled loop
 @pytest.mark.parametrize("nx,ny", [(1, 1), (30, 2), (31, 7), (120, 1368), (121, 685), (481, 275),
                                    (500, 1643), (361, 2741)])
 def test_rows_split_is_bit_neutral(pfa, nx, ny):
@@ -32,6 +32,27 @@ def test_rows_split_is_bit_neutral(pfa, nx, ny):
         assert np.array_equal(x[1:-1, 1:-1], y[1:-1, 1:-1])
 
 
+# strips of 28 and 30 columns (double and single passes) put the same cells in
+# different warps: tails that cross the bulk threshold of the gamma solve
+# everywhere must not notice
+def test_strip_width_is_bit_neutral(pfa):
+    nx, ny = 1500, 1500
+    f = ic.grid2d(nx, ny, seed=4, n_particles=0)
+    rng = np.random.default_rng(4)
+    for a in f[2:]:
+        a[1:-1, 1:-1] = 10.0 ** rng.uniform(-7, -3, (ny, nx))
+        ic.mirror_halo(a)
+    out = []
+    for single in (False, True):
+        g = pfa.Grid2D(f, pfa.model_params(), precision="fp32")
+        for n in ([1] * 12 if single else [12]):
+            g.run(n)
+        out.append(g.read())
+        g.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
 @pytest.mark.parametrize("n", [(20, 14, 3), (33, 27, 1), (40, 30, 35), (64, 26, 97)])
 def test_plane_split_3d(pfa, n):
     """Short z segments (small 3D grids): the FP32 form against FP64."""
@@ -47,3 +68,71 @@ def test_plane_split_3d(pfa, n):
         # the FP32 form's resolution is 2^-40 and its increments of a few
         # 1e-4 per step are rounded to 2^-24 of themselves
         assert np.max(np.abs(x - y)) <= 2e-8
+
+
+# record sets just above the line for double steps (96 MB): ragged columns
+# (the last strip of 28 one to three columns wide), one-strip and one-row
+# grids, row counts that leave remainders
+@pytest.mark.parametrize("precision,mask,nx,ny", [
+    ("fp32", 5, 1401, 1450), ("fp32", 5, 1430, 1403), ("fp32", 5, 29, 64000), ("fp32", 5, 1, 64001),
+    ("fp32", 5, 2000001, 1), ("fp32", 5, 1000002, 2), ("fp32k", 5, 1431, 1100),
+    ("fp32", 9, 1402, 1451), ("fp32k", 9, 1429, 1101)])
+def test_double_steps_are_bit_neutral(pfa, precision, mask, nx, ny):
+    """Runs of double passes (with single steps around the nucleation calls
+    and at odd ends) against the same steps one call at a time: the same
+    bits, events and counters."""
+    small = min(nx, ny) < 60
+    f = ic.grid2d(nx, ny, seed=nx + ny, stripe_width=max(1, min(64, nx // 4)),
+                  n_particles=0 if small else 6, radius=5.0)
+    if small:  # phases along the edges and across the strips
+        rng = np.random.default_rng(1)
+        for a in f[2:]:
+            a[1:-1, 1:-1] = 0.3 * (rng.random((ny, nx)) < 0.1)
+            ic.mirror_halo(a)
+    p = pfa.model_params()
+    m = (pfa.nine_point_mask if mask == 9 else pfa.five_point_mask)(p["dx"], p["dx"])
+    out = []
+    for single in (False, True):
+        g = pfa.Grid2D(f, p, precision=precision, mask=m)
+        g.set_nucleation(seed=7, interval=5)
+        for n in (11, 4, 7):
+            if single:
+                for _ in range(n):
+                    g.run(1)
+            else:
+                g.run(n)
+        out.append((g.read(), g.events()))
+        g.close()
+    for x, y in zip(out[0][0], out[1][0]):
+        assert np.array_equal(x[1:-1, 1:-1], y[1:-1, 1:-1])
+    assert out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("persistent,rows", [(True, 0), (False, 9), (True, 1 << 30)])
+def test_batch_double_steps_are_bit_neutral(pfa, persistent, rows):
+    """A batch above the line for double passes: runs of even and odd lengths,
+    with a member leaving in between, against each grid alone."""
+    p = pfa.model_params()
+    shapes = [(29, 3), (640, 1200), (1117, 900), (28, 28)]
+    fs = [ic.grid2d(nx, ny, seed=k, stripe_width=max(1, nx // 4),
+                    n_particles=3 if min(nx, ny) > 60 else 0) for k, (nx, ny) in enumerate(shapes)]
+    fs.append(ic.grid2d(500, 700, seed=9))
+    b = pfa.Batch(p, sum(pfa.Batch.footprint(f[0].shape) for f in fs))
+    slots = [b.add(f) for f in fs]
+    if rows:
+        b.set_launch(rows, persistent)
+    b.run(9)
+    b.run(4)
+    gone = b.read(slots[4])
+    b.remove(slots[4])
+    b.run(1)
+    b.run(6)
+    got = [b.read(k) for k in slots[:4]] + [gone]
+    b.close()
+    for f, x, n in zip(fs, got, (20, 20, 20, 20, 13)):
+        g = pfa.Grid2D(f, p, precision="fp32")
+        for _ in range(n):
+            g.run(1)
+        for u, v in zip(g.read(), x):
+            assert np.array_equal(u[1:-1, 1:-1], v[1:-1, 1:-1])
+        g.close()
