@@ -176,13 +176,15 @@ __device__ __forceinline__ double dlap64(double Dl, double Dm, double Dh, double
 //   kSolveHi: |phi| < 1e-7 in both phases.  p(phi) = 10 phi^3 < 1e-20, so the
 //     general solve returns X, Y themselves (p shifts them by less than half
 //     an ulp) and is skipped;
-//   kLinearHi: |phi| < 2^-60.  p' dP, the cubic terms of the double well and
-//     the coupling are below 2^-53 of 2 omega phi, so the Allen-Cahn update
-//     is phi + kl lap phi - kw phi.
+//   kLinearHi: |phi| < 2^-60.  p' dP and the cubic terms of the double well
+//     are below 2^-53 of 2 omega phi, and so is the coupling to the other
+//     phase where that is below 2^-27 (kLoneHi), so the Allen-Cahn update is
+//     phi + kl lap phi - kw phi.
 // Compositions that are not finite (or above kBigHi, 2^64) take the general
 // forms, whose NaN propagation is the reference's.
 constexpr int kSolveHi = 0x3e7ad7f2;   // high word of 1e-7
 constexpr int kLinearHi = 0x3c300000;  // 2^-60
+constexpr int kLoneHi = 0x3e400000;    // 2^-27
 constexpr int kBigHi = 0x43f00000;     // 2^64
 
 // high word without the sign: orders the magnitudes of doubles
@@ -191,6 +193,20 @@ __device__ __forceinline__ int mag_hi(double v) { return __double2hiint(v) & 0x7
 // neither phase nor composition needs the general forms of the given bound
 __device__ __forceinline__ bool below64(double X, double Y, double phd, double phl, int bound) {
   return max(mag_hi(phd), mag_hi(phl)) < bound && max(mag_hi(X), mag_hi(Y)) < kBigHi;
+}
+
+// x^gamma of a cell with one precipitate phase only (I: 1 delta, 2 laves; ph
+// its phase field): the forms of gamma64 with the other fraction zero, 30
+// FP64 operations for 56
+template <int I>
+__device__ __forceinline__ void gamma64_one(double X, double Y, double ph, double& g1, double& g2) {
+  constexpr int L = I == 1 ? 0 : 2, Q = I == 1 ? 0 : 5, M = I == 1 ? 1 : 4;  // p, p^2, p pG
+  constexpr double d0 = kDen[Q], d1 = kDen[M];
+  const double p = p64(ph), pG = 1.0 - p;
+  const double r = 1.0 / fma(p, fma(d0, p, d1 * pG), pG * pG);
+  constexpr FictRow a = kFict[0][0], b = kFict[0][1];
+  g1 = fma(p, fma(a.m[L], Y, fma(a.q[Q], p, a.q[M] * pG)), X * fma(a.l[L], p, pG)) * r;
+  g2 = fma(-p, fma(b.l[L], X, fma(b.m[L], Y, fma(b.q[Q], p, b.q[M] * pG))), Y * pG) * r;
 }
 
 // x^gamma of one cell (fict_gam_Cr / fict_gam_Nb, thermo/parabola625.c:245-261)
@@ -227,6 +243,25 @@ __device__ __forceinline__ void gamma64(double X, double Y, double phd, double p
   }
 }
 
+// The solve of a warp's cells that need one.  Next to a precipitate of one
+// kind the other phase is below 1e-7 and its p (below 1e-20) changes no bit of
+// the sums: the one-phase form, where it serves the whole warp (two forms in
+// one warp would cost more than the general one).  full: compositions above
+// kBigHi or not finite.  Whole warp.
+__device__ __forceinline__ void solve64(bool solved, bool full, double X, double Y, double phd,
+                                        double phl, double& g1, double& g2) {
+  const bool d = solved && (full || mag_hi(phd) >= kSolveHi);
+  const bool l = solved && (full || mag_hi(phl) >= kSolveHi);
+  const bool any_d = __any_sync(0xffffffffu, d), any_l = __any_sync(0xffffffffu, l);
+  if (!solved) return;
+  if (any_d && any_l)
+    gamma64(X, Y, phd, phl, g1, g2);
+  else if (any_d)
+    gamma64_one<1>(X, Y, phd, g1, g2);
+  else
+    gamma64_one<2>(X, Y, phl, g1, g2);
+}
+
 // Allen-Cahn update of phase I from its Laplacian (Coef64); u = x^gamma -
 // xe_gamma, e = phi_del phi_lav.  The increments are summed before they meet
 // phi, so phi' is rounded once at phi's own magnitude.
@@ -245,44 +280,31 @@ __device__ __forceinline__ double allen_cahn_linear64(const Coef64& K, double ph
   return ph + fma(K.kl[I], lap, -K.kw[I] * ph);
 }
 
-// both phases of one cell (gamma compositions g1, g2)
-__device__ __forceinline__ void phases64(const Coef64& K, double X, double Y, double g1, double g2,
-                                         double phd, double phl, double lapD, double lapL,
-                                         double& od, double& ol) {
-  if (below64(X, Y, phd, phl, kLinearHi)) {
-    od = allen_cahn_linear64<0>(K, phd, lapD);
-    ol = allen_cahn_linear64<1>(K, phl, lapL);
-  } else {
-    const double u1 = g1 - kXe[0][0], u2 = g2 - kXe[0][1], e = phd * phl;
-    od = allen_cahn64<0>(K, phd, phl, e, lapD, u1, u2);
-    ol = allen_cahn64<1>(K, phl, phd, e, lapL, u1, u2);
-  }
-}
-
-// ---- FP64 step: Cahn-Hilliard increments without FP64 operations ----
-// An explicit step adds D lap x^gamma, about 1e-3 of a composition or less,
-// to it, so the increment needs fewer bits than the composition.  Its parts:
-//  * the neighbour sum in 64-bit fixed point, units of 2^-58 (fix58): exact
-//    for compositions of 2^-6 and above (smaller ones lose bits below 2^-58,
-//    which D scales to 1e-20);
-//  * the product with D in FP32 pairs (inc58): 2^-48 of the increment;
-//  * the addition as one integer added to the composition's bits (add_inc),
-//    correctly rounded up to 2^-5 ulp of the increment's own rounding.
-// 266 FP64-pipe cycles per warp become about 60 of the FP32 and integer
-// pipes.  Valid for compositions in [2^-20, 1) (in_unit) and |x^gamma| below a
+// ---- FP64 step: Cahn-Hilliard without FP64 operations ----
+// An explicit step adds D lap x^gamma to a composition.  In fixed point:
+//  * the neighbour sum in units of 2^-58 (fix58): exact for compositions of
+//    2^-6 and above (smaller ones lose bits below 2^-58, which D < 2^-7 scales
+//    to 1e-20);
+//  * its product with D in units of 2^-64 (5e-20), the high halves of 64-bit
+//    products;
+//  * the addition as an integer number of the composition's last places added
+//    to its bits, so the sum is rounded once, like the FP64 addition (a
+//    result in another binade goes through FP64).
+// 14 FP64 operations (266 cycles of an SM per warp) become about 65 integer
+// ones.  Valid for compositions in [2^-11, 1) (in_unit) and |x^gamma| below a
 // few units (the neighbour sum must stay below 2^5); a tile with any other
 // value takes the FP64 forms.
 
-// v in [2^-20, 1)
+// v in [2^-11, 1)
 __device__ __forceinline__ bool in_unit(double v) {
-  return unsigned(__double2hiint(v)) - 0x3eb00000u < 0x01400000u;
+  return unsigned(__double2hiint(v)) - 0x3f400000u < 0x00b00000u;
 }
 
-// v 2^58 (toward zero), v in [2^-20, 1)
+// v 2^58 (toward zero), v in [2^-11, 1)
 __device__ __forceinline__ long long fix58(double v) {
   const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
   const unsigned th = __funnelshift_l(lo, hi, 11) | 0x80000000u, tl = lo << 11;  // 1.m at bit 63
-  const unsigned r = 1028u - (hi >> 20);                                       // 6 .. 25
+  const unsigned r = 1028u - (hi >> 20);                                       // 6 .. 16
   return (long long)(((unsigned long long)(th >> r) << 32) | __funnelshift_r(tl, th, r));
 }
 
@@ -297,45 +319,22 @@ __device__ __forceinline__ long long fix58_signed(double v) {
   return hi >> 31 ? -f : f;
 }
 
-// row K of D times the sums S1, S2 (2^-58): an unevaluated FP32 pair h + l
-__device__ __forceinline__ void split58(long long S, float& a, float& b) {
-  const int hi = int((S + 0x80000000ll) >> 32);
-  a = float(hi);
-  b = float(int(S));
-  if (hi > (1 << 24) || hi < -(1 << 24)) b += float(hi - int(a)) * 4294967296.0f;  // a was rounded
-}
-template <int K>
-__device__ __forceinline__ void inc58(const Coef64& c, float a1, float b1, float a2, float b2,
-                                      float& h, float& l) {
-  const float p1 = c.Dh[K][0] * a1, p2 = c.Dh[K][1] * a2;
-  float e = fmaf(c.Dh[K][0], a1, -p1) + fmaf(c.Dh[K][1], a2, -p2);
-  e = fmaf(c.Dl[K][0], a1, fmaf(c.Dl[K][1], a2, e));
-  e = fmaf(c.Dq[K][0], b1, fmaf(c.Dq[K][1], b2, e));
-  h = p1 + p2;  // the exact sum is h + (p1 - (h - t)) + (p2 - t)
-  const float t = h - p1;
-  l = e + ((p1 - (h - t)) + (p2 - t));
+// (a call: inlined, its FP64 operations were issued for every cell and the
+// result selected)
+static __device__ __noinline__ double advance64(double X, long long inc) {
+  return X + double(inc) * 0x1p-64;
 }
 
-// the FP64 form of add_inc (a call: inlined, its FP64 operations are issued
-// for every cell and the result selected)
-static __device__ __noinline__ double add_inc64(double X, float h, float l) {
-  return X + (double(h) + double(l));
-}
-
-// X + (h + l), X in [2^-20, 1): the increment in units of X's last place as
-// an integer, added to X's bits.  An increment above a quarter of X, or a
-// result in another binade, goes through FP64.
-__device__ __forceinline__ double add_inc(double X, float h, float l) {
-  const int E = __double2hiint(X) >> 20;
-  const float scale = __int_as_float((1202 - E) << 23);  // 2^(1075 - E)
-  const float hs = h * scale, ls = l * scale;
-  const int ai = __float2int_rn(hs * 0x1p-20f);
-  const int bi = __float2int_rn(fmaf(float(ai), -0x1p20f, hs) + ls);
+// X + D0 S1 + D1 S2, X in [2^-11, 1), S in units of 2^-58, D of 2^-70
+__device__ __forceinline__ double advance58(double X, long long D0, long long S1, long long D1,
+                                            long long S2) {
+  // + 1: the two high halves are rounded down
+  const long long inc = __mul64hi(D0, S1) + __mul64hi(D1, S2) + 1;
+  const int s = (__double2hiint(X) >> 20) - 1011;  // X's last place is 2^(s - 64)
   const long long old = __double_as_longlong(X);
-  const long long sum = old + ((long long)ai * (1 << 20) + bi);
-  if (fabsf(hs) < 0x1p50f && ((unsigned long long)(old ^ sum) >> 52) == 0)
-    return __longlong_as_double(sum);
-  return add_inc64(X, h, l);
+  const long long sum = old + ((inc + (1ll << (s - 1))) >> s);
+  if (((unsigned long long)(old ^ sum) >> 52) == 0) return __longlong_as_double(sum);
+  return advance64(X, inc);
 }
 
 // The diffusivities of dmatrix64 times the scale in `pre` (prefactors of Nb,

@@ -68,13 +68,12 @@ struct Coef64 {
   // neighbour weights: kMaskIso: faces equal, lap = weight (sum of the faces
   // + iso_c centre); kMaskIso9: faces four times the corners, lap = weight (4
   // faces + corners + iso_c centre); the weight is folded into D and kl.  Both
-  // need weights that sum to zero up to rounding.  Any other mask:
+  // need weights that sum to zero up to rounding, and |D| < 2^-7 (0.0078; an
+  // explicit step inside the KKS stability limit has 0.002).  Any other mask:
   // kMaskFive, kMaskNine.
   int mask;
   double iso_c;
-  // iso masks: D in FP32 parts for sums in units of 2^-58 (dev::inc58):
-  // 2^-26 D = Dh + Dl, Dq = 2^-58 D
-  float Dh[2][2], Dl[2][2], Dq[2][2];
+  long long Dfix[2][2];  // iso masks: D 2^70 (dev::advance58)
   double vm_pre[3];  // variable mobility: prefactors (Nb, Cr, Ni) times dt / (2 dx^2)
   double vm_qy;      // and the weight of the y faces, (1/dy^2) / (1/dx^2)
 };

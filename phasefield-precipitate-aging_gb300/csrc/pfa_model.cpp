@@ -122,6 +122,7 @@ void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
   double dP[2][6];
   model_dP(dP);
   double f = 1.0;  // the weight folded into D and kl
+  int general, iso = -1;
   if (mask9) {
     const double corner = mask9[0], face = mask9[1];
     double sum = 0.0;
@@ -129,30 +130,37 @@ void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
     const bool zero_sum = std::fabs(sum) <= 1e-15 * std::fabs(mask9[4]);
     const bool corners = mask9[2] == corner && mask9[6] == corner && mask9[8] == corner;
     const bool faces = mask9[3] == face && mask9[5] == face && mask9[7] == face && face != 0.0;
-    o->mask = corners && corner == 0.0 ? kMaskFive : kMaskNine;
+    general = corners && corner == 0.0 ? kMaskFive : kMaskNine;
     if (corners && faces && zero_sum) {
       if (corner == 0.0) {
-        o->mask = kMaskIso;
+        iso = kMaskIso;
         f = face;
       } else if (std::fabs(face - 4.0 * corner) <= 4e-16 * std::fabs(face)) {
-        o->mask = kMaskIso9;
+        iso = kMaskIso9;
         f = corner;
       }
-      o->iso_c = mask9[4] / f;
     }
+    o->iso_c = mask9[4] / f;
   } else {
-    const bool iso = m.idx2[1] == m.idx2[0] && m.idx2[2] == m.idx2[0];
-    o->mask = iso ? kMaskIso : kMaskFive;
+    general = kMaskFive;
+    if (m.idx2[1] == m.idx2[0] && m.idx2[2] == m.idx2[0]) {
+      iso = kMaskIso;
+      f = m.idx2[0];
+    }
     o->iso_c = -6.0;
-    if (iso) f = m.idx2[0];
   }
+  double most = 0.0;
+  for (int i = 0; i < 2; i++)
+    for (int j = 0; j < 2; j++) most = std::fmax(most, std::fabs(m.dt * m.D[i][j] * f));
+  if (iso < 0 || !(most < 0x1p-7)) {
+    iso = -1;
+    f = 1.0;
+  }
+  o->mask = iso < 0 ? general : iso;
   for (int i = 0; i < 2; i++) {
     for (int j = 0; j < 2; j++) {
       o->D[i][j] = m.dt * m.D[i][j] * f;
-      const double d = std::ldexp(o->D[i][j], -26);
-      o->Dh[i][j] = float(d);
-      o->Dl[i][j] = float(d - double(o->Dh[i][j]));
-      o->Dq[i][j] = float(std::ldexp(d, -32));
+      if (iso >= 0) o->Dfix[i][j] = std::llrint(std::ldexp(o->D[i][j], 70));
     }
     o->kl[i] = m.dt * m.L[i] * m.kappa[i] * f;
     o->kw[i] = 2.0 * m.dt * m.L[i] * m.omega[i];

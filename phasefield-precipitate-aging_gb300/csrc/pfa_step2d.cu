@@ -10,11 +10,12 @@
 // which is what the reference's halo fill produces.
 //
 // The FP64 pipe bounds it (19 cycles per warp instruction and SM), so the
-// arithmetic is in the reduced forms of pfa_device.cuh: 14 FP64 operations a
-// cell where both phases are exactly zero around it, 28 in the phases' far
-// tails, about 110 inside precipitates and their interfaces (the reference's
-// expressions: about 300 everywhere).  4096^2 with 4 particles: 7.78 -> 0.56
-// ms/step; 2048^2 1.95 -> 0.16 ms; 256^2 38.8 -> 14.5 us.
+// arithmetic is in the reduced forms of pfa_device.cuh: no FP64 operations in
+// a cell where both phases are exactly zero around it, 7 per phase in the
+// phases' far tails, about 65 next to a precipitate (the reference's
+// expressions: about 300 everywhere).  us a step: 4096^2 with 4 particles 7780
+// -> 277, 2048^2 1950 -> 73, 256^2 38.8 -> 9.8.  Without phases memory latency
+// binds it (2048^2 69 us at 41 % of HBM).
 //
 // Layout: the reference's, (Ny + 2) rows of pitch elements with a one-cell
 // ghost ring, interior cell (x, y) at (y + 1) * pitch + x + 1.  The FP32
@@ -23,17 +24,13 @@
 
 #include "pfa_device.cuh"
 #include "pfa_kernels.h"
+#include "pfa_tile64.cuh"
 
 namespace pfa {
 
 using namespace dev;
 
 namespace {
-
-constexpr int kTX = 32;   // tile width (one warp)
-constexpr int kEX = kTX + 2;
-
-__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 // The ghost cells that mirror interior cell (gx, gy) of the domain's edge
 // (corners take the diagonal value).
@@ -74,31 +71,6 @@ __device__ __forceinline__ void store_cell(const Step2DArgs& a, size_t i, int gx
 // Plain FP64 fused step.  MASK: the kind of Coef64::mask.  TY: rows of the tile, one row per warp; the warps
 // past them stage the tile's halo cells, so that a cell's solve and its
 // update are never behind another cell's in the same warp.
-constexpr int halo_warps(int ty) { return (2 * kEX + 2 * ty + 31) / 32; }
-constexpr int tile_threads(int ty) { return 32 * (ty + halo_warps(ty)); }
-
-// this thread's cell (ex, ey) of the (TY + 2) x 34 staged tile: its own
-// output cell in the first TY warps, a halo cell in the rest (false: none)
-template <int TY>
-__device__ __forceinline__ bool tile_cell(int& ex, int& ey) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (w < TY) {
-    ex = lane + 1;
-    ey = w + 1;
-    return true;
-  }
-  const int h = (w - TY) * 32 + lane;
-  if (h < 2 * kEX) {
-    ey = h < kEX ? 0 : TY + 1;
-    ex = h < kEX ? h : h - kEX;
-  } else {
-    const int k = h - 2 * kEX;
-    ey = 1 + (k < TY ? k : k - TY);
-    ex = k < TY ? 0 : kEX - 1;
-  }
-  return h < 2 * kEX + 2 * TY;
-}
-
 // Laplacian (iso masks: over the weight, which Coef64 folds into its factors)
 template <int MASK>
 __device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[kEX], int ex, int ey) {
@@ -137,38 +109,40 @@ __device__ __forceinline__ long long sum58(const long long (*s)[kEX], int ex, in
   return 4 * f + k - 20 * s[ey][ex];
 }
 
-// one staged cell: its values and x^gamma.  phase: the tile must look at the
-// phases at all (an all-zero phase field stays zero: its Laplacian, p' and
-// well vanish; compositions that are not finite make 0 x NaN, see kBigHi)
-struct Cell64 {
-  double X, Y, pd, pl, g1, g2;
-  size_t i;  // element of the fields
-  bool solved, phase;
-  bool unit;  // both compositions in [2^-20, 1)
-};
+// whether a staged phase is zero at a cell and all its neighbours
+template <int MASK>
+__device__ __forceinline__ bool none64(const double (*s)[kEX], int ex, int ey) {
+  auto b = [&](int y, int x) { return value_bits(s[y][x]); };
+  int m = b(ey, ex) | b(ey - 1, ex) | b(ey + 1, ex) | b(ey, ex - 1) | b(ey, ex + 1);
+  if constexpr (MASK == kMaskIso9 || MASK == kMaskNine)
+    m |= b(ey - 1, ex - 1) | b(ey - 1, ex + 1) | b(ey + 1, ex - 1) | b(ey + 1, ex + 1);
+  return m == 0;
+}
 
 __device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
-  Cell64 c;
-  c.i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
-  c.X = __ldg(static_cast<const double*>(a.in[0]) + c.i);
-  c.Y = __ldg(static_cast<const double*>(a.in[1]) + c.i);
-  c.pd = __ldg(static_cast<const double*>(a.in[2]) + c.i);
-  c.pl = __ldg(static_cast<const double*>(a.in[3]) + c.i);
-  c.g1 = c.X;
-  c.g2 = c.Y;
-  c.unit = in_unit(c.X) && in_unit(c.Y);
-  const bool big = !c.unit && max(mag_hi(c.X), mag_hi(c.Y)) >= kBigHi;
-  const int m = max(mag_hi(c.pd), mag_hi(c.pl));
-  c.phase = (m | __double2loint(c.pd) | __double2loint(c.pl)) != 0 || big;
-  c.solved = m >= kSolveHi || big;
-  if (c.solved) gamma64(c.X, c.Y, c.pd, c.pl, c.g1, c.g2);
+  const size_t i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
+  Cell64 c = cell64(__ldg(static_cast<const double*>(a.in[0]) + i),
+                    __ldg(static_cast<const double*>(a.in[1]) + i),
+                    __ldg(static_cast<const double*>(a.in[2]) + i),
+                    __ldg(static_cast<const double*>(a.in[3]) + i));
+  c.i = i;
   return c;
+}
+
+// Allen-Cahn of both phases, src/discretization.cu:888-980
+template <int MASK>
+__device__ __forceinline__ void phases64(const Step2DArgs& a, const Cell64& c, const double (*s_pd)[kEX],
+                                         const double (*s_pl)[kEX], int ex, int ey, double& od,
+                                         double& ol) {
+  od = phase64<0>(a.c, c, none64<MASK>(s_pd, ex, ey), [&] { return lap64<MASK>(a, s_pd, ex, ey); });
+  ol = phase64<1>(a.c, c, none64<MASK>(s_pl, ex, ey), [&] { return lap64<MASK>(a, s_pl, ex, ey); });
 }
 
 // MASK: Coef64::mask.  Bound by the FP64 pipe next to precipitates and by
 // memory elsewhere.
 template <int MASK, int TY>
-__global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_constant__ Step2DArgs a) {
+__global__ void __launch_bounds__(tile_threads(TY), TY == 8 ? 4 : (TY == 4 ? 6 : 8))
+    k_step2d_f64(const __grid_constant__ Step2DArgs a) {
   constexpr bool kFixed = MASK == kMaskIso || MASK == kMaskIso9;
   // |x^gamma| < 4 (5 points) or 1 (9 points): the neighbour sum stays below 2^5
   constexpr int kGammaHi = MASK == kMaskIso9 ? 0x3ff00000 : 0x40100000;
@@ -179,21 +153,14 @@ __global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_co
   int ex, ey;
   const bool staged = tile_cell<TY>(ex, ey);
   const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
-  Cell64 c;
-  c.phase = false;
-  bool wide = false;  // outside the fixed-point forms' range
+  const Cell64 c = stage64(a, gx, gy);
+  const bool wide = wide64(c, kGammaHi);  // outside the fixed-point forms' range
   if (staged) {
-    c = stage64(a, gx, gy);
-    wide = !c.unit || (c.solved && max(mag_hi(c.g1), mag_hi(c.g2)) >= kGammaHi);
     if (!kFixed || wide) {
       as_double(s_g1)[ey][ex] = c.g1;
       as_double(s_g2)[ey][ex] = c.g2;
-    } else if (c.solved) {
-      s_g1[ey][ex] = fix58_signed(c.g1);
-      s_g2[ey][ex] = fix58_signed(c.g2);
     } else {
-      s_g1[ey][ex] = fix58(c.X);
-      s_g2[ey][ex] = fix58(c.Y);
+      fix_cell(c, s_g1[ey][ex], s_g2[ey][ex]);
     }
     s_pd[ey][ex] = c.pd;
     s_pl[ey][ex] = c.pl;
@@ -212,24 +179,17 @@ __global__ void __launch_bounds__(tile_threads(TY)) k_step2d_f64(const __grid_co
   const Coef64& K = a.c;
   double ocr, onb;
   if (fixed) {
-    float a1, b1, a2, b2, h, l;
-    split58(sum58<MASK>(s_g1, ex, ey), a1, b1);
-    split58(sum58<MASK>(s_g2, ex, ey), a2, b2);
-    inc58<0>(K, a1, b1, a2, b2, h, l);
-    ocr = add_inc(c.X, h, l);
-    inc58<1>(K, a1, b1, a2, b2, h, l);
-    onb = add_inc(c.Y, h, l);
+    const long long S1 = sum58<MASK>(s_g1, ex, ey), S2 = sum58<MASK>(s_g2, ex, ey);
+    ocr = advance58(c.X, K.Dfix[0][0], S1, K.Dfix[0][1], S2);
+    onb = advance58(c.Y, K.Dfix[1][0], S1, K.Dfix[1][1], S2);
   } else {
     const double l1 = lap64<MASK>(a, as_double(s_g1), ex, ey);
     const double l2 = lap64<MASK>(a, as_double(s_g2), ex, ey);
     ocr = c.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
     onb = c.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
   }
-  // Allen-Cahn, src/discretization.cu:888-980
   double od = 0.0, ol = 0.0;
-  if (phases)
-    phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<MASK>(a, s_pd, ex, ey),
-             lap64<MASK>(a, s_pl, ex, ey), od, ol);
+  if (phases) phases64<MASK>(a, c, s_pd, s_pl, ex, ey, od, ol);
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
@@ -254,10 +214,8 @@ __global__ void __launch_bounds__(tile_threads(TY))
   int ex, ey;
   const bool staged = tile_cell<TY>(ex, ey);
   const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
-  Cell64 c;
-  c.phase = false;
+  const Cell64 c = stage64(a, gx, gy);
   if (staged) {
-    c = stage64(a, gx, gy);
     s_g1[ey][ex] = c.g1;
     s_g2[ey][ex] = c.g2;
     s_pd[ey][ex] = c.pd;
@@ -290,24 +248,22 @@ __global__ void __launch_bounds__(tile_threads(TY))
   const double onb = c.Y + fma(K.vm_qy, s_fy[1][ty + 1][tx] - s_fy[1][ty][tx],
                                s_fx[1][ty][tx + 1] - s_fx[1][ty][tx]);
   double od = 0.0, ol = 0.0;
-  if (phases)
-    phases64(K, c.X, c.Y, c.g1, c.g2, c.pd, c.pl, lap64<ISO ? kMaskIso : kMaskFive>(a, s_pd, ex, ey),
-             lap64<ISO ? kMaskIso : kMaskFive>(a, s_pl, ex, ey), od, ol);
+  if (phases) phases64<ISO ? kMaskIso : kMaskFive>(a, c, s_pd, s_pl, ex, ey, od, ol);
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
 // Rows per tile.  The tile's halo is staged (and, next to precipitates,
 // solved) again, so tall tiles do least; but a tile inside a precipitate takes
 // its SM's FP64 pipe for microseconds, so a small grid is cut finer to spread
-// such tiles over the SMs.  Measured, us per step at 1 / 2 / 4 / 8 rows:
-// 64 x 48 5.5 / 6.3 / 7.2 / 11.0, 256^2 27.3 / 14.8 / 14.5 / 16.4, 512^2 30.6
-// / 28.5 / 28.5 / 31.1, 1024^2 76 / 66.5 / 62.6 / 62.4; variable mobility
-// (every staged cell has its exponentials) 64 x 48 9.4 / 10.9 / 13.2 / 20.5,
-// 128^2 20.0 / 15.3 / 13.2 / 20.5, 256^2 61.6 / 45.1 / 38.3 / 35.6.
+// such tiles over the SMs.  Measured, us per step at 1 / 4 / 8 rows: 64 x 48
+// 6.3 / 7.8 / 12.1, 128^2 5.5 / 6.2 / 9.3, 256^2 13.9 / 9.8 / 13.7, 1024^2
+// 33.2 / 23.9 / 26.0, 2048^2 122 / 78 / 73, 4096^2 470 / 300 / 277; variable
+// mobility (every staged cell has its exponentials) 64 x 48 9.4 / 13.2 / 20.5,
+// 128^2 20.0 / 13.2 / 20.5, 256^2 61.6 / 38.3 / 35.6.
 int tile_rows(int Nx, int Ny, bool varmob) {
   const long long rows = (long long)((Nx + kTX - 1) / kTX) * Ny;  // tile rows of 32 cells
   if (varmob) return rows < 304 ? 1 : (rows < 1216 ? 4 : 8);
-  return rows < 1216 ? 1 : (rows < 9728 ? 4 : 8);
+  return rows < 1216 ? 1 : (rows < 65536 ? 4 : 8);
 }
 
 template <int TY>

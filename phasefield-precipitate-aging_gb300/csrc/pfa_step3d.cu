@@ -3,15 +3,9 @@
 // The reference supports 2D only (src/main.cpp:418-421); this extends its
 // equations unchanged to a 7-point stencil with six-face zero-flux ghost
 // fill.  Two kernels stream along z:
-//   k_stream3d_f64: plain FP64, the reference's formulas, ghost-ring layout
-//        ((Nz+2) planes of (Ny+2) rows of Nx+2 doubles, one array per field);
-//        a CTA of 16 warps covers 30 x-columns (lanes 1..30) by 14 y-rows
-//        (warps 1..14); lanes 0 / 31 and warps 0 / 15 carry the neighbour
-//        columns and rows.  x-neighbours come from shuffles, y-neighbours
-//        from planes published in shared memory, z-neighbours from a
-//        three-plane register window rotated by a 3x-unrolled loop, one
-//        barrier per plane; the reduced FP64 forms of pfa_device.cuh (128^3
-//        1.45 -> 0.34 ms, 256^3 9.3 -> 1.3 ms a step).
+//   k_stream3d_f64: plain FP64 in the reduced forms of pfa_device.cuh,
+//        ghost-ring layout ((Nz+2) planes of (Ny+2) rows of Nx+2 doubles, one
+//        array per field); tiles of 32 x 8 columns, described below.
 //   k_stream3d_f32: the precision form (FP32 arithmetic, every field
 //        Kahan-compensated, the equilibrium-referenced gamma solve) on
 //        interior-only records (pfa_step2d_f32.cu): A = float4 {x_Cr, x_Nb,
@@ -25,6 +19,7 @@
 
 #include "pfa_device.cuh"
 #include "pfa_kernels.h"
+#include "pfa_tile64.cuh"
 #include "pfa_tma.cuh"
 
 namespace pfa {
@@ -33,27 +28,21 @@ using namespace dev;
 
 namespace {
 
-constexpr int kW = 16;  // FP64: warps per CTA (y-rows including the 2 halo rows)
-constexpr int kRowsOut = kW - 2;
-constexpr int kCols = 30;  // FP64: output columns per warp
-
 template <class R>
 struct Nb3 {
-  R gcr, gnb, pd, pl;
+  R gcr, gnb, pd, pl;  // gcr, gnb: the deviations u = x^gamma - xe_gamma
 };
 
-// FP64: gcr / gnb are x^gamma; FP32: the deviations u = x^gamma - xe_gamma
 template <class R>
 struct Raw3 {
   R x, y, pd, pl;
-  uint2 cq;  // FP32: packed Kahan compensations
+  uint2 cq;  // packed Kahan compensations
 };
 
 // FP64 store of the interior cell (x, y, z) and of every ghost cell whose
 // nearest interior cell it is (the six-face fill; edges and corners take the
 // nearest interior cell).
-__device__ __forceinline__ void store64(double* f, const Step3DArgs& a, int x, int y, int z,
-                                        double v) {
+__device__ __noinline__ void store64(double* f, const Step3DArgs& a, int x, int y, int z, double v) {
   int xs[3] = {x, 0, 0}, ys[3] = {y, 0, 0}, zs[3] = {z, 0, 0};
   int nx = 1, ny = 1, nz = 1;
   if (x == 0) xs[nx++] = -1;
@@ -68,120 +57,140 @@ __device__ __forceinline__ void store64(double* f, const Step3DArgs& a, int x, i
         f[((long long)(zs[k] + 1) * (a.Ny + 2) + (ys[j] + 1)) * a.pitch + (xs[i] + 1)] = v;
 }
 
-// One thread's column of the FP64 kernel (ISO: equal spacings).
-template <bool ISO>
-struct S64 {
-  const Step3DArgs& a;
-  int cx, cy;  // clamped column / row of this thread
-  bool out;    // this thread owns an output column and row
+// ---- plain FP64 ----
+// Tiles of 32 x 8 columns (pfa_tile64.cuh) streaming along z: a thread keeps
+// its cell's last three planes (x^gamma, phases) and the records of the next
+// two, publishes x^gamma (fixed point, pfa_device.cuh) and the phases of
+// plane z in shared memory and passes one barrier per plane.  ISO: equal
+// spacings, which the fixed-point sum needs; other spacings, and planes with
+// a composition outside its range, take the FP64 sums.  Measured against the
+// kernel that formed the sums on the FP64 pipe (30 x 14 columns, halo lanes
+// and rows): 128^3 346 -> 184 us a step, 256^3 1444 -> 547.
+constexpr int kTY3 = 8;
+struct Plane64 {
+  long long g1[kTY3 + 2][kEX], g2[kTY3 + 2][kEX];
+  double pd[kTY3 + 2][kEX], pl[kTY3 + 2][kEX];
+};
 
-  __device__ __forceinline__ long long cell(int z) const {
-    const int zz = min(max(z, 0), a.Nz - 1);
-    return ((long long)(zz + 1) * (a.Ny + 2) + (cy + 1)) * a.pitch + (cx + 1);
-  }
-
-  __device__ __forceinline__ Raw3<double> load(int z) const {
-    const long long i = cell(z);
-    Raw3<double> r;
-    r.x = __ldg(static_cast<const double*>(a.in[0]) + i);
-    r.y = __ldg(static_cast<const double*>(a.in[1]) + i);
-    r.pd = __ldg(static_cast<const double*>(a.in[2]) + i);
-    r.pl = __ldg(static_cast<const double*>(a.in[3]) + i);
-    r.cq = make_uint2(0u, 0u);
-    return r;
-  }
-
-  // gamma solve of one cell (skipped where it returns X, Y themselves)
-  __device__ __forceinline__ Nb3<double> solve(const Raw3<double>& r) const {
-    Nb3<double> n{r.x, r.y, r.pd, r.pl};
-    if (!below64(r.x, r.y, r.pd, r.pl, kSolveHi)) gamma64(r.x, r.y, r.pd, r.pl, n.gcr, n.gnb);
-    return n;
-  }
-
-  // update plane z of this thread's column from the window (up, c, dn)
-  __device__ __forceinline__ void update(int z, const Nb3<double>& up, const Nb3<double>& c,
-                                         const Nb3<double>& dn, const Raw3<double>& rc,
-                                         Nb3<double> (*sh)[kW][32]) const {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    Nb3<double>(*b)[32] = sh[z & 1];
-    b[w][lane] = c;
-    __syncthreads();  // buffer z&1 was last read two planes ago, before the previous barrier
-    const Nb3<double> s = b[max(w - 1, 0)][lane], n = b[min(w + 1, kW - 1)][lane];
-    Nb3<double> wv, e;
-    wv.gcr = __shfl_up_sync(0xffffffffu, c.gcr, 1);
-    wv.gnb = __shfl_up_sync(0xffffffffu, c.gnb, 1);
-    e.gcr = __shfl_down_sync(0xffffffffu, c.gcr, 1);
-    e.gnb = __shfl_down_sync(0xffffffffu, c.gnb, 1);
-    // an all-zero phase neighbourhood stays zero (compositions that are not
-    // finite make 0 x NaN and go the general way)
-    auto bits = [](double v) { return mag_hi(v) | __double2loint(v); };
-    auto any = [&](const Nb3<double>& v) { return bits(v.pd) | bits(v.pl); };
-    const bool phases = __any_sync(0xffffffffu, (any(up) | any(c) | any(dn) | any(s) | any(n) |
-                                                 int(max(mag_hi(rc.x), mag_hi(rc.y)) >= kBigHi)) != 0);
-    if (phases) {  // the whole warp
-      wv.pd = __shfl_up_sync(0xffffffffu, c.pd, 1);
-      wv.pl = __shfl_up_sync(0xffffffffu, c.pl, 1);
-      e.pd = __shfl_down_sync(0xffffffffu, c.pd, 1);
-      e.pl = __shfl_down_sync(0xffffffffu, c.pl, 1);
-    }
-    if (!out) return;
-    const Coef64& K = a.c;
-    // 7-point Laplacian (ISO: over the weight, which Coef64 folds into its factors)
-    const double mx = a.m.idx2[0], my = a.m.idx2[1], mz = a.m.idx2[2];
-    auto lap = [&](double z0, double y0, double x0, double vc, double x1, double y1, double z1) {
-      if constexpr (ISO)
-        return fma(K.iso_c, vc, ((z0 + z1) + (y0 + y1)) + (x0 + x1));
-      else
-        return fma(mz, z0 + z1, fma(my, y0 + y1, fma(mx, x0 + x1, -2. * (mx + my + mz) * vc)));
-    };
-    const double l1 = lap(up.gcr, s.gcr, wv.gcr, c.gcr, e.gcr, n.gcr, dn.gcr);
-    const double l2 = lap(up.gnb, s.gnb, wv.gnb, c.gnb, e.gnb, n.gnb, dn.gnb);
-    store64(static_cast<double*>(a.out[0]), a, cx, cy, z,
-            rc.x + fma(K.D[0][0], l1, K.D[0][1] * l2));
-    store64(static_cast<double*>(a.out[1]), a, cx, cy, z,
-            rc.y + fma(K.D[1][0], l1, K.D[1][1] * l2));
-    double od = 0.0, ol = 0.0;
-    if (phases)
-      phases64(K, rc.x, rc.y, c.gcr, c.gnb, c.pd, c.pl,
-               lap(up.pd, s.pd, wv.pd, c.pd, e.pd, n.pd, dn.pd),
-               lap(up.pl, s.pl, wv.pl, c.pl, e.pl, n.pl, dn.pl), od, ol);
-    store64(static_cast<double*>(a.out[2]), a, cx, cy, z, od);
-    store64(static_cast<double*>(a.out[3]), a, cx, cy, z, ol);
-  }
+// one plane of a thread's column
+struct Col64 : Cell64 {
+  long long f1, f2;  // x^gamma in fixed point (unless wide)
+  bool wide;
 };
 
 template <bool ISO>
-__global__ void __launch_bounds__(32 * kW) k_stream3d_f64(Step3DArgs a) {
-  __shared__ Nb3<double> sh[2][kW][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = blockIdx.x * kCols - 1 + lane;
-  const int y = blockIdx.y * kRowsOut - 1 + w;
-  const int z0 = blockIdx.z * a.zrows;
-  const int z1 = min(z0 + a.zrows, a.Nz);
-  const S64<ISO> S{a, min(max(x, 0), a.Nx - 1), min(max(y, 0), a.Ny - 1),
-              lane >= 1 && lane <= kCols && w >= 1 && w <= kRowsOut && x < a.Nx && y < a.Ny};
-  Raw3<double> r0 = S.load(z0), r1 = S.load(z0 + 1), r2;
-  Nb3<double> n0 = S.solve(S.load(z0 - 1)), n1 = S.solve(r0), n2;
-  int z = z0;
-  for (; z + 2 < z1; z += 3) {
-    r2 = S.load(z + 2);
-    n2 = S.solve(r1);
-    S.update(z, n0, n1, n2, r0, sh);
-    r0 = S.load(z + 3);
-    n0 = S.solve(r2);
-    S.update(z + 1, n1, n2, n0, r1, sh);
-    r1 = S.load(z + 4);
-    n1 = S.solve(r0);
-    S.update(z + 2, n2, n0, n1, r2, sh);
-  }
-  for (; z < z1; z++) {
-    r2 = S.load(z + 2);
-    n2 = S.solve(r1);
-    S.update(z, n0, n1, n2, r0, sh);
-    n0 = n1;
-    n1 = n2;
-    r0 = r1;
-    r1 = r2;
+__global__ void __launch_bounds__(tile_threads(kTY3), 2)
+    k_stream3d_f64(const __grid_constant__ Step3DArgs a) {
+  __shared__ Plane64 sh[2];
+  __shared__ int s_wide[3];
+  int ex, ey;
+  const bool staged = tile_cell<kTY3>(ex, ey);
+  const int x = int(blockIdx.x) * kTX + ex - 1, y = int(blockIdx.y) * kTY3 + ey - 1;
+  const int cx = clampi(x, 0, a.Nx - 1), cy = clampi(y, 0, a.Ny - 1);
+  const bool own = threadIdx.x < 32 * kTY3 && x < a.Nx && y < a.Ny;
+  const int z0 = blockIdx.z * a.zrows, z1 = min(z0 + a.zrows, a.Nz);
+  const size_t plane = size_t(a.Ny + 2) * a.pitch, col = size_t(cy + 1) * a.pitch + cx + 1;
+  const Coef64& K = a.c;
+  const bool edge = cx == 0 || cx == a.Nx - 1 || cy == 0 || cy == a.Ny - 1;
+  if (threadIdx.x < 3) s_wide[threadIdx.x] = 0;
+
+  double rX, rY, rpd, rpl;  // the next plane's record
+  auto load = [&](int z) {
+    const size_t i = size_t(clampi(z, 0, a.Nz - 1) + 1) * plane + col;
+    rX = __ldg(static_cast<const double*>(a.in[0]) + i);
+    rY = __ldg(static_cast<const double*>(a.in[1]) + i);
+    rpd = __ldg(static_cast<const double*>(a.in[2]) + i);
+    rpl = __ldg(static_cast<const double*>(a.in[3]) + i);
+  };
+  // |x^gamma| < 2: the seven-point sum stays below 2^5
+  auto stage = [&]() {
+    Col64 c;
+    static_cast<Cell64&>(c) = cell64(rX, rY, rpd, rpl);
+    c.wide = wide64(c, 0x40000000);
+    if (ISO && !c.wide) fix_cell(c, c.f1, c.f2);
+    return c;
+  };
+  Col64 P, C, N;
+  load(z0 - 1);
+  P = stage();
+  load(z0);
+  C = stage();
+  load(z0 + 1);
+  __syncthreads();  // s_wide is set
+  int w = 0;  // slot of s_wide
+  for (int z = z0; z < z1; z++) {
+    N = stage();
+    if (z + 1 < z1) load(z + 2);
+    Plane64& S = sh[z & 1];
+    auto dg1 = reinterpret_cast<double (*)[kEX]>(S.g1), dg2 = reinterpret_cast<double (*)[kEX]>(S.g2);
+    if (staged) {
+      if (ISO && !C.wide) {
+        S.g1[ey][ex] = C.f1;
+        S.g2[ey][ex] = C.f2;
+      } else {
+        dg1[ey][ex] = C.g1;
+        dg2[ey][ex] = C.g2;
+      }
+      if (ISO && (P.wide || C.wide || N.wide)) s_wide[w] = 1;
+      S.pd[ey][ex] = C.pd;
+      S.pl[ey][ex] = C.pl;
+    }
+    // buffer z & 1 was last read before the previous barrier; slot w + 2 of
+    // s_wide was last read before this one
+    const bool phases = __syncthreads_or(staged && (P.phase || C.phase || N.phase));
+    const bool fixed = ISO && s_wide[w] == 0;
+    const int w2 = w == 0 ? 2 : w - 1;  // (w + 2) % 3
+    if (threadIdx.x == 0) s_wide[w2] = 0;
+    w = w == 2 ? 0 : w + 1;
+    if (ISO && !fixed) {  // the whole plane in FP64
+      if (staged) {
+        dg1[ey][ex] = C.g1;
+        dg2[ey][ex] = C.g2;
+      }
+      __syncthreads();
+    }
+    if (own) {
+      double ocr, onb, od = 0.0, ol = 0.0;
+      const double mx = a.m.idx2[0], my = a.m.idx2[1], mz = a.m.idx2[2];
+      auto lap = [&](double zm, double zp, const double (*s)[kEX], double c) {
+        const double sx = s[ey][ex - 1] + s[ey][ex + 1], sy = s[ey - 1][ex] + s[ey + 1][ex];
+        if constexpr (ISO)
+          return fma(K.iso_c, c, ((zm + zp) + sy) + sx);
+        else
+          return fma(mz, zm + zp, fma(my, sy, fma(mx, sx, -2. * (mx + my + mz) * c)));
+      };
+      if (fixed) {
+        auto sum = [&](long long zm, long long zp, const long long (*s)[kEX], long long c) {
+          return (zm + zp) + (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]) - 6 * c;
+        };
+        const long long S1 = sum(P.f1, N.f1, S.g1, C.f1), S2 = sum(P.f2, N.f2, S.g2, C.f2);
+        ocr = advance58(C.X, K.Dfix[0][0], S1, K.Dfix[0][1], S2);
+        onb = advance58(C.Y, K.Dfix[1][0], S1, K.Dfix[1][1], S2);
+      } else {
+        const double l1 = lap(P.g1, N.g1, dg1, C.g1), l2 = lap(P.g2, N.g2, dg2, C.g2);
+        ocr = C.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
+        onb = C.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
+      }
+      if (phases) {
+        auto none = [&](double zm, double zp, const double (*s)[kEX]) {
+          auto b = [&](int y, int x) { return value_bits(s[y][x]); };
+          return (value_bits(zm) | value_bits(zp) | b(ey, ex) | b(ey - 1, ex) | b(ey + 1, ex) |
+                  b(ey, ex - 1) | b(ey, ex + 1)) == 0;
+        };
+        od = phase64<0>(K, C, none(P.pd, N.pd, S.pd), [&] { return lap(P.pd, N.pd, S.pd, C.pd); });
+        ol = phase64<1>(K, C, none(P.pl, N.pl, S.pl), [&] { return lap(P.pl, N.pl, S.pl, C.pl); });
+      }
+      const double v[4] = {ocr, onb, od, ol};
+      const size_t i = size_t(z + 1) * plane + col;
+#pragma unroll
+      for (int k = 0; k < 4; k++) static_cast<double*>(a.out[k])[i] = v[k];
+      if (edge || z == 0 || z == a.Nz - 1) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) store64(static_cast<double*>(a.out[k]), a, cx, cy, z, v[k]);
+      }
+    }
+    P = C;
+    C = N;
   }
 }
 
@@ -491,12 +500,14 @@ int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
 
 // FP64: a column next to a precipitate costs several times one in the matrix,
 // so short segments that spread the precipitates over the SMs beat whole
-// waves of equal ones.  us per step at 3 / 12 / whole-wave planes: 128^3 336 /
-// 376 / 576, 200 x 100 x 60 213 / 284 / 513, 256^3 1371 / 1314 / 1415; 64^3
-// at 2 / 3 / 8: 117 / 123 / 151, 32^3 51 / 68 / 151.
+// waves of equal ones.  us per step at 1 / 2 / 3 / 8 / 16 planes: 32^3 26 / 36
+// / 47 / 97 / 178, 64^3 83 / 78 / 77 / 104 / 189, 128^3 215 / 189 / 184 / 208
+// / 282, 200 x 100 x 60 152 / 137 / 138 / 180 / 212, 256^3 907 / 697 / 622 /
+// 547 / 543, 384^3 2673 / 1980 / 1742 / 1470 / 1417.
 int segment_planes_f64(int Nx, int Ny, int Nz) {
-  const long long cols = (long long)((Nx + kCols - 1) / kCols) * ((Ny + kRowsOut - 1) / kRowsOut);
-  const int planes = cols * Nz <= 1216 ? 2 : (cols * Nz <= 12160 ? 3 : 12);
+  const long long cols = (long long)((Nx + kTX - 1) / kTX) * ((Ny + kTY3 - 1) / kTY3);
+  const long long n = cols * Nz;  // planes of tiles
+  const int planes = n <= 304 ? 1 : (n <= 12160 ? 3 : (n <= 97280 ? 8 : 16));
   return std::min(planes, Nz);
 }
 
@@ -509,7 +520,7 @@ cudaError_t query3() {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) {
     if (F64)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f64<true>, 32 * kW, 0);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f64<true>, tile_threads(kTY3), 0);
     else
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f32<false>, 32 * kW3, kSmem3);
   }
@@ -565,14 +576,14 @@ cudaError_t encode_step3d_maps(Tma3* t, const void* A, const void* B, int Nx, in
 
 cudaError_t launch_step3d(Step3DArgs a, bool f64, const Tma3* t, cudaStream_t s) {
   const int resident = g_resident3[f64] > 0 ? g_resident3[f64] : 152;
-  const int tx = f64 ? kCols : kCols3, ty = f64 ? kRowsOut : kRows3;
+  const int tx = f64 ? kTX : kCols3, ty = f64 ? kTY3 : kRows3;
   a.zrows = f64 ? segment_planes_f64(a.Nx, a.Ny, a.Nz) : segment_planes(a.Nx, a.Ny, a.Nz, resident, tx, ty);
   dim3 grid((a.Nx + tx - 1) / tx, (a.Ny + ty - 1) / ty, (a.Nz + a.zrows - 1) / a.zrows);
   if (f64) {
     if (a.c.mask == kMaskIso)
-      k_stream3d_f64<true><<<grid, 32 * kW, 0, s>>>(a);
+      k_stream3d_f64<true><<<grid, tile_threads(kTY3), 0, s>>>(a);
     else
-      k_stream3d_f64<false><<<grid, 32 * kW, 0, s>>>(a);
+      k_stream3d_f64<false><<<grid, tile_threads(kTY3), 0, s>>>(a);
   } else {
     if (!t) return cudaErrorInvalidValue;
     if (a.skip_plane >= 0)

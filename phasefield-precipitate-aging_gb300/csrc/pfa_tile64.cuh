@@ -1,0 +1,108 @@
+// pfa_tile64.cuh -- tiles of the FP64 step kernels (2D, and 3D plane by plane).
+// Included by .cu files only.
+#pragma once
+
+#include "pfa_device.cuh"
+
+namespace pfa {
+namespace {
+
+using namespace dev;
+
+constexpr int kTX = 32;       // tile width (one warp)
+constexpr int kEX = kTX + 2;  // staged width
+
+__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
+
+// A tile of 32 x TY cells: one row per warp; the warps past the TY rows stage
+// the tile's halo cells, so that a cell's solve and its update are never
+// behind another cell's in the same warp.
+constexpr int halo_warps(int ty) { return (2 * kEX + 2 * ty + 31) / 32; }
+constexpr int tile_threads(int ty) { return 32 * (ty + halo_warps(ty)); }
+
+// this thread's cell (ex, ey) of the (TY + 2) x 34 staged tile: its own
+// output cell in the first TY warps, a halo cell in the rest (false: none,
+// a duplicate of the last one)
+template <int TY>
+__device__ __forceinline__ bool tile_cell(int& ex, int& ey) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < TY) {
+    ex = lane + 1;
+    ey = w + 1;
+    return true;
+  }
+  constexpr int kHalo = 2 * kEX + 2 * TY;
+  const int i = (w - TY) * 32 + lane, h = i < kHalo ? i : kHalo - 1;
+  if (h < 2 * kEX) {
+    ey = h < kEX ? 0 : TY + 1;
+    ex = h < kEX ? h : h - kEX;
+  } else {
+    const int k = h - 2 * kEX;
+    ey = 1 + (k < TY ? k : k - TY);
+    ex = k < TY ? 0 : kEX - 1;
+  }
+  return i < kHalo;
+}
+
+// One staged cell: its values and x^gamma.  phase: the tile must look at the
+// phases at all (an all-zero phase field stays zero: its Laplacian, p' and
+// well vanish; compositions that are not finite make 0 x NaN, see kBigHi)
+struct Cell64 {
+  double X, Y, pd, pl, g1, g2;
+  size_t i;  // element of the fields
+  bool solved, phase, big;
+  bool unit;  // both compositions in [2^-11, 1)
+};
+
+// whole warp
+__device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double pl) {
+  Cell64 c;
+  c.X = X;
+  c.Y = Y;
+  c.pd = pd;
+  c.pl = pl;
+  c.g1 = X;
+  c.g2 = Y;
+  c.unit = in_unit(X) && in_unit(Y);
+  c.big = !c.unit && max(mag_hi(X), mag_hi(Y)) >= kBigHi;
+  const int m = max(mag_hi(pd), mag_hi(pl));
+  c.phase = (m | __double2loint(pd) | __double2loint(pl)) != 0 || c.big;
+  c.solved = m >= kSolveHi || c.big;
+  solve64(c.solved, c.big, X, Y, pd, pl, c.g1, c.g2);
+  return c;
+}
+
+// outside the fixed-point forms' range, with |x^gamma| bounded by the high
+// word `hi` (the neighbour sum has to stay below 2^5)
+__device__ __forceinline__ bool wide64(const Cell64& c, int hi) {
+  return !c.unit || (c.solved && max(mag_hi(c.g1), mag_hi(c.g2)) >= hi);
+}
+
+// x^gamma in fixed point (not wide)
+__device__ __forceinline__ void fix_cell(const Cell64& c, long long& f1, long long& f2) {
+  if (c.solved) {
+    f1 = fix58_signed(c.g1);
+    f2 = fix58_signed(c.g2);
+  } else {
+    f1 = fix58(c.X);
+    f2 = fix58(c.Y);
+  }
+}
+
+// the bits that are zero with a double (its sign aside)
+__device__ __forceinline__ int value_bits(double v) { return mag_hi(v) | __double2loint(v); }
+
+// Allen-Cahn of one phase of a cell.  none: the phase is zero at the cell and
+// its neighbours, and stays so; lap() forms its Laplacian.
+template <int I, class Lap>
+__device__ __forceinline__ double phase64(const Coef64& K, const Cell64& c, bool none, Lap lap) {
+  if (none && !c.big) return 0.0;
+  const double ph = I == 0 ? c.pd : c.pl, pj = I == 0 ? c.pl : c.pd;
+  if (mag_hi(ph) < kLinearHi && mag_hi(pj) < kLoneHi && !c.big)
+    return allen_cahn_linear64<I>(K, ph, lap());
+  constexpr double x1 = kXe[0][0], x2 = kXe[0][1];
+  return allen_cahn64<I>(K, ph, pj, ph * pj, lap(), c.g1 - x1, c.g2 - x2);
+}
+
+}  // namespace
+}  // namespace pfa

@@ -110,3 +110,32 @@ def test_not_a_number_spreads_as_in_the_plain_forms(pfa, orc):
     err = field_err([np.where(k, a, 0.0) for a, k in zip(got, ok)],
                     [np.where(k, b, 0.0) for b, k in zip(want, ok)])
     assert max(err) <= 1e-12
+
+
+# compositions a hair from the powers of two, so that half the cells change
+# their exponent in the step
+@pytest.mark.parametrize("dim", [2, 3])
+def test_exponent_changes(pfa, orc, dim):
+    shape = (60, 90) if dim == 2 else (20, 24, 40)
+    rng = np.random.default_rng(dim)
+    f = []
+    for k in range(2):
+        a = 2.0 ** -rng.integers(1, 8, shape) * (1.0 + rng.uniform(-2e-4, 2e-4, shape))
+        f.append(a)
+    f += [np.zeros(shape), np.zeros(shape)]
+    full = []
+    for a in f:
+        h = np.empty([n + 2 for n in shape])
+        h[(slice(1, -1),) * dim] = a
+        full.append(ic.mirror_halo(h))
+    p = pfa.model_params(dim=dim)
+    g = (pfa.Grid2D if dim == 2 else pfa.Grid3D)(full, p)
+    g.run(1)
+    got = g.read()
+    g.close()
+    want = (orc.run2d if dim == 2 else orc.run3d)(full, O.model_params(dim=dim), 1)
+    core = (slice(1, -1),) * dim
+    for a, b, o in zip(got[:2], want[:2], full[:2]):
+        # one rounding of the sum on each side, and the oracle's of its sums
+        # (four or six neighbours of up to 1/2, scaled by D < 1/400)
+        assert np.all(np.abs(a - b)[core] <= (np.spacing(np.maximum(a, b)) + 2.0 ** -60)[core])
