@@ -80,11 +80,11 @@ __global__ void __launch_bounds__(kThreads) k_energy_partial(EnergyArgs a) {
   if (threadIdx.x == 0) a.partial[blockIdx.x] = sh[0];
 }
 
-__global__ void k_energy_total(const double* partial, int n, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(32) k_energy_total(const double* partial, int n, double* out) {
   double s = 0.0;
-  for (int k = 0; k < n; k++) s += partial[k];
-  *out = s;
+  for (int k = threadIdx.x; k < n; k += 32) s += partial[k];
+  for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+  if (threadIdx.x == 0) *out = s;
 }
 
 }  // namespace

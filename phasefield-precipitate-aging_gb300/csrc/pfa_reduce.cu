@@ -70,16 +70,22 @@ __global__ void __launch_bounds__(kThreads) k_sum_partial(SumArgs a) {
   if (threadIdx.x < 5) a.partial[blockIdx.x * 5 + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-__global__ void k_sum_final(const double* partial, int nblocks, double inv_n, double* out) {
-  if (threadIdx.x >= 5) return;
+// One warp per sum: each lane adds its share of the partials (compensated),
+// then the lanes add up pairwise.  A single thread's chain over all of them
+// took 32 us (an FP64 operation's latency is 64 cycles).
+__global__ void __launch_bounds__(32 * 5) k_sum_final(const double* partial, int nblocks, double inv_n,
+                                                      double* out) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double s = 0.0, c = 0.0;
-  for (int b = 0; b < nblocks; b++) {
-    const double y = partial[b * 5 + threadIdx.x] - c;
+  for (int b = lane; b < nblocks; b += 32) {
+    const double y = partial[b * 5 + k] - c;
     const double t = s + y;
     c = (t - s) - y;
     s = t;
   }
-  out[threadIdx.x] = s * inv_n;
+  s -= c;
+  for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+  if (lane == 0) out[k] = s * inv_n;
 }
 
 }  // namespace
@@ -90,7 +96,7 @@ cudaError_t launch_summarize(const SumArgs& a, cudaStream_t s) {
   else
     k_sum_partial<double><<<kSumBlocks, kThreads, 0, s>>>(a);
   const double n = double(a.Nx) * double(a.Ny) * double(a.Nz);
-  k_sum_final<<<1, 32, 0, s>>>(a.partial, kSumBlocks, 1.0 / n, a.out);
+  k_sum_final<<<1, 32 * 5, 0, s>>>(a.partial, kSumBlocks, 1.0 / n, a.out);
   return cudaGetLastError();
 }
 

@@ -17,7 +17,7 @@ def mixed_fields(shape, seed):
     f = [rng.uniform(0.28, 0.33, shape), rng.uniform(0.02, 0.17, shape)]
     for _ in range(2):
         a = 10.0 ** rng.uniform(-40, -0.5, shape)
-        edges = 10.0 ** rng.choice([-18.1, -18.05, -7.01, -6.99], shape)
+        edges = 10.0 ** rng.choice([-18.1, -18.05, -11.45, -11.42, -7.01, -6.99], shape)
         a = np.where(rng.random(shape) < 0.2, edges, a)
         zero = rng.random([max(1, n // 16) + 1 for n in shape]) < 0.4
         for d in range(len(shape)):
