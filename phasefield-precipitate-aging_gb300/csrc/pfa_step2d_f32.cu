@@ -340,6 +340,22 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
                              Ny, P, lane >= 1 && lane <= kCols && gx < Nx};
   bool z0, z1, z2;  // rows y-1, y, y+1 are still
   if constexpr (!STAGED) {
+    if (y1 - y0 <= 3) {
+      // a short segment: all its rows are requested at once, so that a warp
+      // waits for memory once instead of row by row
+      const Raw<PACK> ra = S.load(S.row(y0 - 1)), rb = S.load(S.row(y0)), rc = S.load(S.row(y0 + 1)),
+                      rd = S.load(S.row(y0 + 2)), re = S.load(S.row(y0 + 3));
+      NbT<NINE, VM> na = S.solve(ra, z0), nb = S.solve(rb, z1);
+      const NbT<NINE, VM> nc = S.solve(rc, z2);
+      S.store(y0, S.step(na, nb, nc, rb, z0 && z1 && z2));
+      if (y0 + 1 >= y1) return;
+      na = S.solve(rd, z0);
+      S.store(y0 + 1, S.step(nb, nc, na, rc, z0 && z1 && z2));
+      if (y0 + 2 >= y1) return;
+      nb = S.solve(re, z1);
+      S.store(y0 + 2, S.step(nc, na, nb, rd, z0 && z1 && z2));
+      return;
+    }
     // window rows y-1, y, y+1 and raw records of rows y, y+1, y+2
     Raw<PACK> r0 = S.load(S.row(y0)), r1 = S.load(S.row(y0 + 1)), r2;
     NbT<NINE, VM> n0 = S.solve(S.load(S.row(y0 - 1)), z0), n1 = S.solve(r0, z1), n2;
@@ -659,20 +675,22 @@ __global__ void k_export_records(ConvArgs a) {
 }
 
 // Rows per warp segment of a single step.  Each segment solves two extra
-// rows, but a row is a serial load-solve-update chain (about 0.4 us where few
-// warps share an SM), and the more segments there are the better they
-// balance: 3 rows, one pass of the unrolled loop, are the best or within 2 %
-// of it from 512^2 up (us a step at 3 / 6 / 24 / 96 rows: 512^2 4.2 / 5.3 /
-// 13.0 / 34.9, 1024^2 7.5 / 7.7 / 13.8 / 36, 2048^2 32.6 / 33.0 / 41 / 61,
-// 4096^2 119 / 120 / 130 / 159; FP32 compensations 4096^2 151 / 157 / 170 /
-// 186), and 1 row while a grid has no more rows of CTAs than resident slots
-// (256^2 3.0 against 3.6 at 3 rows).  The variable-mobility step, whose extra
-// rows cost three exponentials a cell, takes 6 and 9 from there (1531 x 1021
-// 18.5 at 3, 17.0 at 6; 4096^2 149 at 3, 139.9 at 6, 137.9 at 9).
+// rows, but the more segments there are the better they balance, and a
+// segment of up to three rows waits for memory once (a longer one row by row,
+// about 0.4 us each where few warps share an SM).  us a step at 1 / 2 / 3 / 6
+// / 12 rows: 256^2 2.7 / 3.1 / 3.4 / 5.2 / 8.0, 384^2 3.3 / 3.3 / 3.7 / 5.2 /
+// 8.1, 700 x 433 4.5 / 4.1 / 4.4 / 5.7 / 8.4, 900 x 600 6.1 / 5.1 / 4.9 / 6.2
+// / 8.9, 1024^2 10.0 / 7.5 / 7.0 / 7.9 / 10.1, 2048^2 45.8 / 33.5 / 30.2 /
+// 33.0 / 36.3; the same order in the 9-point form.  The variable-mobility
+// step, whose extra rows cost three exponentials a cell, takes 6 and 9 from
+// there (1024^2 10.8 at 3, 11.3 at 6; 1531 x 1021 15.3 / 15.1; 2048^2 43.3 /
+// 41.0; 3000^2 87.8 / 81.6, 81.0 at 9).
 int segment_rows(int Nx, int Ny, int resident, bool varmob) {
   const int nbx = ((Nx + kCols - 1) / kCols + kWarps - 1) / kWarps;
   const double load = double(nbx) * Ny / resident;  // CTA rows per resident CTA
-  const int rows = load <= 1.0 ? 1 : (!varmob || load <= 6.0 ? 3 : (load <= 24.0 ? 6 : 9));
+  const int rows = load <= 1.0   ? 1
+                   : load <= 2.5 ? 2
+                                 : (!varmob || load <= 12.0 ? 3 : (load <= 24.0 ? 6 : 9));
   return std::min(rows, Ny);
 }
 
