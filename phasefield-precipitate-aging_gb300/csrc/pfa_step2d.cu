@@ -20,6 +20,7 @@
 // Layout: the reference's, (Ny + 2) rows of pitch elements with a one-cell
 // ghost ring, interior cell (x, y) at (y + 1) * pitch + x + 1.  The FP32
 // precision form has its own kernel and layout (pfa_step2d_f32.cu).
+#include <algorithm>
 #include <cstdint>
 
 #include "pfa_device.cuh"
@@ -138,6 +139,10 @@ __device__ __forceinline__ void phases64(const Step2DArgs& a, const Cell64& c, c
   ol = phase64<1>(a.c, c, none64<MASK>(s_pl, ex, ey), [&] { return lap64<MASK>(a, s_pl, ex, ey); });
 }
 
+// tile rows past what a grid's second dimension holds go on in the third
+// (tiles past the domain store nothing)
+__device__ __forceinline__ int tile_row() { return int(blockIdx.z * gridDim.y + blockIdx.y); }
+
 // MASK: Coef64::mask.  Bound by the FP64 pipe next to precipitates and by
 // memory elsewhere.
 template <int MASK, int TY>
@@ -152,7 +157,7 @@ __global__ void __launch_bounds__(tile_threads(TY), TY == 8 ? 4 : (TY == 4 ? 6 :
   auto as_double = [](long long (*s)[kEX]) { return reinterpret_cast<double (*)[kEX]>(s); };
   int ex, ey;
   const bool staged = tile_cell<TY>(ex, ey);
-  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
+  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = tile_row() * TY + ey - 1;
   const Cell64 c = stage64(a, gx, gy);
   const bool wide = wide64(c, kGammaHi);  // outside the fixed-point forms' range
   if (staged) {
@@ -213,7 +218,7 @@ __global__ void __launch_bounds__(tile_threads(TY))
   __shared__ double s_fx[2][TY][kTX + 1], s_fy[2][TY + 1][kTX];
   int ex, ey;
   const bool staged = tile_cell<TY>(ex, ey);
-  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = int(blockIdx.y) * TY + ey - 1;
+  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = tile_row() * TY + ey - 1;
   const Cell64 c = stage64(a, gx, gy);
   if (staged) {
     s_g1[ey][ex] = c.g1;
@@ -268,7 +273,8 @@ int tile_rows(int Nx, int Ny, bool varmob) {
 
 template <int TY>
 cudaError_t launch_rows(const Step2DArgs& a, cudaStream_t s) {
-  const dim3 grid((a.Nx + kTX - 1) / kTX, (a.Ny + TY - 1) / TY);
+  const int ny = (a.Ny + TY - 1) / TY;
+  const dim3 grid((a.Nx + kTX - 1) / kTX, std::min(ny, 65535), (ny + 65534) / 65535);
   constexpr int n = tile_threads(TY);
   if (a.varmob) {
     if (a.c.mask == kMaskIso)

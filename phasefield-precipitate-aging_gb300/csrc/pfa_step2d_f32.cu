@@ -674,6 +674,9 @@ __global__ void k_export_records(ConvArgs a) {
   }
 }
 
+// at most 65535 segments (the launch grid's second dimension), none past Ny
+int grid_rows(int rows, int Ny) { return std::min(std::max(rows, (Ny + 65534) / 65535), Ny); }
+
 // Rows per warp segment of a single step.  Each segment solves two extra
 // rows, but the more segments there are the better they balance, and a
 // segment of up to three rows waits for memory once (a longer one row by row,
@@ -691,7 +694,7 @@ int segment_rows(int Nx, int Ny, int resident, bool varmob) {
   const int rows = load <= 1.0   ? 1
                    : load <= 2.5 ? 2
                                  : (!varmob || load <= 12.0 ? 3 : (load <= 24.0 ? 6 : 9));
-  return std::min(rows, Ny);
+  return grid_rows(rows, Ny);
 }
 
 // resident CTAs: FP32 / packed variants, the batch kernel, the 9-point FP32 / packed
@@ -730,7 +733,7 @@ int segment_rows2(int Nx, int Ny, int resident) {
   const int nbx = ((Nx + kCols2 - 1) / kCols2 + kWarps - 1) / kWarps;
   const double load = double(nbx) * Ny / resident;  // CTA rows per resident CTA
   const int rows = 3 * std::max(2, int(std::sqrt(6.0 * load) / 3.0 + 0.5));
-  return std::min(rows, Ny);
+  return grid_rows(rows, Ny);
 }
 
 template <bool PACK, bool NINE>

@@ -32,6 +32,30 @@ def test_rows_split_is_bit_neutral(pfa, nx, ny):
         assert np.array_equal(x[1:-1, 1:-1], y[1:-1, 1:-1])
 
 
+# more segments of the usual height than a launch grid's second dimension holds
+@pytest.mark.parametrize("precision,nx,ny", [("fp32", 1, 196609), ("fp32", 2, 400001), ("fp64", 1, 530001)])
+def test_tall_grids(pfa, precision, nx, ny):
+    """A column without neighbours in x: the same values as in a 64-row piece
+    of it, away from the piece's ends."""
+    f = ic.grid2d(nx, ny, seed=ny, stripe_width=0, n_particles=0)
+    p = pfa.model_params()
+    out = []
+    for top in (0, ny - 64, ny):
+        part = [np.ascontiguousarray(a[top:top + 66]) for a in f] if top < ny else f
+        if top < ny:
+            for a in part:
+                ic.mirror_halo(a)
+        g = pfa.Grid2D(part, p, precision=precision)
+        for n in (1, 2):
+            g.run(n)
+        out.append(g.read())
+        g.close()
+    low, high, whole = out
+    for a, b, c in zip(low, high, whole):
+        assert np.array_equal(a[1:61, 1:-1], c[1:61, 1:-1])
+        assert np.array_equal(b[5:65, 1:-1], c[ny - 59:ny + 1, 1:-1])
+
+
 # strips of 28 and 30 columns (double and single passes) put the same cells in
 # different warps: tails that cross the bulk threshold of the gamma solve
 # everywhere must not notice
