@@ -14,8 +14,7 @@
 // a cell where both phases are exactly zero around it, 7 per phase in the
 // phases' far tails, about 65 next to a precipitate (the reference's
 // expressions: about 300 everywhere).  us a step: 4096^2 with 4 particles 7780
-// -> 277, 2048^2 1950 -> 73, 256^2 38.8 -> 9.8.  Without phases memory latency
-// binds it (2048^2 69 us at 41 % of HBM).
+// -> 277, 2048^2 1950 -> 67, 256^2 38.8 -> 6.5.
 //
 // Layout: the reference's, (Ny + 2) rows of pitch elements with a one-cell
 // ghost ring, interior cell (x, y) at (y + 1) * pitch + x + 1.  The FP32
@@ -69,12 +68,11 @@ __device__ __forceinline__ void store_cell(const Step2DArgs& a, size_t i, int gx
 }
 
 // ---------------------------------------------------------------------------
-// Plain FP64 fused step.  MASK: the kind of Coef64::mask.  TY: rows of the tile, one row per warp; the warps
-// past them stage the tile's halo cells, so that a cell's solve and its
-// update are never behind another cell's in the same warp.
+// Plain FP64 fused step over tiles of pfa_tile64.cuh.  MASK: the kind of
+// Coef64::mask.
 // Laplacian (iso masks: over the weight, which Coef64 folds into its factors)
-template <int MASK>
-__device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[kEX], int ex, int ey) {
+template <int MASK, int P>
+__device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[P], int ex, int ey) {
   if constexpr (MASK == kMaskIso) {
     return fma(a.c.iso_c, s[ey][ex],
                (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]));
@@ -102,8 +100,8 @@ __device__ __forceinline__ double lap64(const Step2DArgs& a, const double (*s)[k
 }
 
 // the same over a staged fixed-point array (iso masks; exact)
-template <int MASK>
-__device__ __forceinline__ long long sum58(const long long (*s)[kEX], int ex, int ey) {
+template <int MASK, int P>
+__device__ __forceinline__ long long sum58(const long long (*s)[P], int ex, int ey) {
   const long long f = (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]);
   if constexpr (MASK == kMaskIso) return f - 4 * s[ey][ex];
   const long long k = (s[ey - 1][ex - 1] + s[ey + 1][ex + 1]) + (s[ey - 1][ex + 1] + s[ey + 1][ex - 1]);
@@ -111,8 +109,8 @@ __device__ __forceinline__ long long sum58(const long long (*s)[kEX], int ex, in
 }
 
 // whether a staged phase is zero at a cell and all its neighbours
-template <int MASK>
-__device__ __forceinline__ bool none64(const double (*s)[kEX], int ex, int ey) {
+template <int MASK, int P>
+__device__ __forceinline__ bool none64(const double (*s)[P], int ex, int ey) {
   auto b = [&](int y, int x) { return value_bits(s[y][x]); };
   int m = b(ey, ex) | b(ey - 1, ex) | b(ey + 1, ex) | b(ey, ex - 1) | b(ey, ex + 1);
   if constexpr (MASK == kMaskIso9 || MASK == kMaskNine)
@@ -131,9 +129,9 @@ __device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
 }
 
 // Allen-Cahn of both phases, src/discretization.cu:888-980
-template <int MASK>
-__device__ __forceinline__ void phases64(const Step2DArgs& a, const Cell64& c, const double (*s_pd)[kEX],
-                                         const double (*s_pl)[kEX], int ex, int ey, double& od,
+template <int MASK, int P>
+__device__ __forceinline__ void phases64(const Step2DArgs& a, const Cell64& c, const double (*s_pd)[P],
+                                         const double (*s_pl)[P], int ex, int ey, double& od,
                                          double& ol) {
   od = phase64<0>(a.c, c, none64<MASK>(s_pd, ex, ey), [&] { return lap64<MASK>(a, s_pd, ex, ey); });
   ol = phase64<1>(a.c, c, none64<MASK>(s_pl, ex, ey), [&] { return lap64<MASK>(a, s_pl, ex, ey); });
@@ -143,21 +141,27 @@ __device__ __forceinline__ void phases64(const Step2DArgs& a, const Cell64& c, c
 // (tiles past the domain store nothing)
 __device__ __forceinline__ int tile_row() { return int(blockIdx.z * gridDim.y + blockIdx.y); }
 
+template <int MASK, int TX, int TY>
+using Tile2 = Tile<TX, TY, MASK == kMaskIso9 || MASK == kMaskNine>;
+// resident blocks asked for: 1408 threads per SM (46 registers)
+constexpr int blocks2(int threads) { return 1408 / threads; }
+
 // MASK: Coef64::mask.  Bound by the FP64 pipe next to precipitates and by
 // memory elsewhere.
-template <int MASK, int TY>
-__global__ void __launch_bounds__(tile_threads(TY), TY == 8 ? 4 : (TY == 4 ? 6 : 8))
+template <int MASK, int TX, int TY>
+__global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<MASK, TX, TY>::kThreads))
     k_step2d_f64(const __grid_constant__ Step2DArgs a) {
+  using T = Tile2<MASK, TX, TY>;
   constexpr bool kFixed = MASK == kMaskIso || MASK == kMaskIso9;
   // |x^gamma| < 4 (5 points) or 1 (9 points): the neighbour sum stays below 2^5
   constexpr int kGammaHi = MASK == kMaskIso9 ? 0x3ff00000 : 0x40100000;
   // x^gamma as doubles, or (kFixed) in fixed point
-  __shared__ long long s_g1[TY + 2][kEX], s_g2[TY + 2][kEX];
-  __shared__ double s_pd[TY + 2][kEX], s_pl[TY + 2][kEX];
-  auto as_double = [](long long (*s)[kEX]) { return reinterpret_cast<double (*)[kEX]>(s); };
+  __shared__ typename T::template Plane<long long> s_g1, s_g2;
+  __shared__ typename T::template Plane<double> s_pd, s_pl;
+  auto as_double = [](long long (*s)[T::kPitch]) { return reinterpret_cast<double (*)[T::kPitch]>(s); };
   int ex, ey;
-  const bool staged = tile_cell<TY>(ex, ey);
-  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = tile_row() * TY + ey - 1;
+  const bool staged = T::cell(ex, ey);
+  const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
   const Cell64 c = stage64(a, gx, gy);
   const bool wide = wide64(c, kGammaHi);  // outside the fixed-point forms' range
   if (staged) {
@@ -179,7 +183,7 @@ __global__ void __launch_bounds__(tile_threads(TY), TY == 8 ? 4 : (TY == 4 ? 6 :
     }
     __syncthreads();
   }
-  if (threadIdx.x >= 32 * TY || gx >= a.Nx || gy >= a.Ny) return;
+  if (threadIdx.x >= T::kOwn || gx >= a.Nx || gy >= a.Ny) return;
   // Cahn-Hilliard, composition_kernel src/discretization.cu:843-865
   const Coef64& K = a.c;
   double ocr, onb;
@@ -210,15 +214,15 @@ __global__ void __launch_bounds__(tile_threads(TY), TY == 8 ? 4 : (TY == 4 ? 6 :
 // exponentials), each face's flux is formed once: a thread forms its east and
 // lower faces, the halo warps the west faces of the first column and the
 // upper faces of the first row.
-template <bool ISO, int TY>
-__global__ void __launch_bounds__(tile_threads(TY))
+template <bool ISO, int TX, int TY>
+__global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, 768 / Tile<TX, TY, false>::kThreads)
     k_step2d_f64_varmob(const __grid_constant__ Step2DArgs a) {
-  __shared__ double s_g1[TY + 2][kEX], s_g2[TY + 2][kEX], s_pd[TY + 2][kEX], s_pl[TY + 2][kEX];
-  __shared__ double s_d[4][TY + 2][kEX];
-  __shared__ double s_fx[2][TY][kTX + 1], s_fy[2][TY + 1][kTX];
+  using T = Tile<TX, TY, false>;
+  __shared__ typename T::template Plane<double> s_g1, s_g2, s_pd, s_pl, s_d[4];
+  __shared__ double s_fx[2][TY][TX + 1], s_fy[2][TY + 1][TX];
   int ex, ey;
-  const bool staged = tile_cell<TY>(ex, ey);
-  const int gx = int(blockIdx.x) * kTX + ex - 1, gy = tile_row() * TY + ey - 1;
+  const bool staged = T::cell(ex, ey);
+  const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
   const Cell64 c = stage64(a, gx, gy);
   if (staged) {
     s_g1[ey][ex] = c.g1;
@@ -235,13 +239,13 @@ __global__ void __launch_bounds__(tile_threads(TY))
     f1 = fma(s_d[0][ny][nx] + s_d[0][y][x], u1, (s_d[1][ny][nx] + s_d[1][y][x]) * u2);
     f2 = fma(s_d[2][ny][nx] + s_d[2][y][x], u1, (s_d[3][ny][nx] + s_d[3][y][x]) * u2);
   };
-  const bool own = threadIdx.x < 32 * TY;
+  const bool own = threadIdx.x < T::kOwn;
   if (own) {
     flux(ex, ey, ex + 1, ey, s_fx[0][ey - 1][ex], s_fx[1][ey - 1][ex]);
     flux(ex, ey, ex, ey + 1, s_fy[0][ey][ex - 1], s_fy[1][ey][ex - 1]);
   } else if (staged && ex == 0 && ey >= 1 && ey <= TY) {
     flux(0, ey, 1, ey, s_fx[0][ey - 1][0], s_fx[1][ey - 1][0]);
-  } else if (staged && ey == 0 && ex >= 1 && ex <= kTX) {
+  } else if (staged && ey == 0 && ex >= 1 && ex <= TX) {
     flux(ex, 0, ex, 1, s_fy[0][0][ex - 1], s_fy[1][0][ex - 1]);
   }
   __syncthreads();
@@ -257,37 +261,29 @@ __global__ void __launch_bounds__(tile_threads(TY))
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
-// Rows per tile.  The tile's halo is staged (and, next to precipitates,
-// solved) again, so tall tiles do least; but a tile inside a precipitate takes
-// its SM's FP64 pipe for microseconds, so a small grid is cut finer to spread
-// such tiles over the SMs.  Measured, us per step at 1 / 4 / 8 rows: 64 x 48
-// 6.3 / 7.8 / 12.1, 128^2 5.5 / 6.2 / 9.3, 256^2 13.9 / 9.8 / 13.7, 1024^2
-// 33.2 / 23.9 / 26.0, 2048^2 122 / 78 / 73, 4096^2 470 / 300 / 277; variable
-// mobility (every staged cell has its exponentials) 64 x 48 9.4 / 13.2 / 20.5,
-// 128^2 20.0 / 13.2 / 20.5, 256^2 61.6 / 38.3 / 35.6.
-int tile_rows(int Nx, int Ny, bool varmob) {
-  const long long rows = (long long)((Nx + kTX - 1) / kTX) * Ny;  // tile rows of 32 cells
-  if (varmob) return rows < 304 ? 1 : (rows < 1216 ? 4 : 8);
-  return rows < 1216 ? 1 : (rows < 65536 ? 4 : 8);
+template <int TX, int TY>
+long long tiles(const Step2DArgs& a) {
+  return (long long)((a.Nx + TX - 1) / TX) * ((a.Ny + TY - 1) / TY);
 }
 
-template <int TY>
-cudaError_t launch_rows(const Step2DArgs& a, cudaStream_t s) {
+template <int TX, int TY, bool VM>
+cudaError_t launch_tiles(const Step2DArgs& a, cudaStream_t s) {
   const int ny = (a.Ny + TY - 1) / TY;
-  const dim3 grid((a.Nx + kTX - 1) / kTX, std::min(ny, 65535), (ny + 65534) / 65535);
-  constexpr int n = tile_threads(TY);
-  if (a.varmob) {
+  const dim3 grid((a.Nx + TX - 1) / TX, std::min(ny, 65535), (ny + 65534) / 65535);
+  if constexpr (VM) {
+    constexpr int n = Tile<TX, TY, false>::kThreads;
     if (a.c.mask == kMaskIso)
-      k_step2d_f64_varmob<true, TY><<<grid, n, 0, s>>>(a);
+      k_step2d_f64_varmob<true, TX, TY><<<grid, n, 0, s>>>(a);
     else
-      k_step2d_f64_varmob<false, TY><<<grid, n, 0, s>>>(a);
-    return cudaGetLastError();
-  }
-  switch (a.c.mask) {
-    case kMaskIso: k_step2d_f64<kMaskIso, TY><<<grid, n, 0, s>>>(a); break;
-    case kMaskIso9: k_step2d_f64<kMaskIso9, TY><<<grid, n, 0, s>>>(a); break;
-    case kMaskFive: k_step2d_f64<kMaskFive, TY><<<grid, n, 0, s>>>(a); break;
-    default: k_step2d_f64<kMaskNine, TY><<<grid, n, 0, s>>>(a);
+      k_step2d_f64_varmob<false, TX, TY><<<grid, n, 0, s>>>(a);
+  } else {
+    constexpr int n5 = Tile2<kMaskIso, TX, TY>::kThreads, n9 = Tile2<kMaskIso9, TX, TY>::kThreads;
+    switch (a.c.mask) {
+      case kMaskIso: k_step2d_f64<kMaskIso, TX, TY><<<grid, n5, 0, s>>>(a); break;
+      case kMaskIso9: k_step2d_f64<kMaskIso9, TX, TY><<<grid, n9, 0, s>>>(a); break;
+      case kMaskFive: k_step2d_f64<kMaskFive, TX, TY><<<grid, n5, 0, s>>>(a); break;
+      default: k_step2d_f64<kMaskNine, TX, TY><<<grid, n9, 0, s>>>(a);
+    }
   }
   return cudaGetLastError();
 }
@@ -297,11 +293,17 @@ cudaError_t launch_rows(const Step2DArgs& a, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s) {
   if (a.varmob && a.nine) return cudaErrorInvalidValue;  // refused by the host before
-  switch (tile_rows(a.Nx, a.Ny, a.varmob)) {
-    case 1: return launch_rows<1>(a, s);
-    case 4: return launch_rows<4>(a, s);
-    default: return launch_rows<8>(a, s);
-  }
+  // A tile next to a precipitate takes its SM's FP64 pipe for microseconds, and
+  // a step is as long as its most loaded SM: small tiles spread such work, and
+  // 8 x 8 has the least halo for its size.  us a step of 8 x 4 / 8 x 8 / 16 x 8
+  // / 16 x 16 / 32 x 8 cells: 64 x 48 5.1 / 5.8 / 6.3 / 9.4 / 9.9, 192^2 5.8 /
+  // 5.9 / 8.3 / 8.1 / 8.8, 256^2 6.8 / 6.5 / 8.0 / 9.9 / 10.1, 1024^2 27 / 19.6
+  // / 21 / 24 / 25, 2048^2 93 / 67 / 69 / 77 / 77 (32 x 8 in rows of 32: 76).
+  if (!a.varmob) return tiles<8, 4>(a) <= 1216 ? launch_tiles<8, 4, false>(a, s) : launch_tiles<8, 8, false>(a, s);
+  // every staged cell has its exponentials, so large grids take the tile with
+  // the smallest share of halo: 8 x 8 / 16 x 16 192^2 17.1 / 17.2, 256^2 27.7 /
+  // 29.2, 320^2 39.0 / 35.8, 512^2 86 / 74, 2048^2 1266 / 1050
+  return tiles<16, 16>(a) < 304 ? launch_tiles<8, 8, true>(a, s) : launch_tiles<16, 16, true>(a, s);
 }
 
 }  // namespace pfa

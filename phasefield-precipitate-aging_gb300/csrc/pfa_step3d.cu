@@ -5,7 +5,7 @@
 // fill.  Two kernels stream along z:
 //   k_stream3d_f64: plain FP64 in the reduced forms of pfa_device.cuh,
 //        ghost-ring layout ((Nz+2) planes of (Ny+2) rows of Nx+2 doubles, one
-//        array per field); tiles of 32 x 8 columns, described below.
+//        array per field); tiles of 8 x 8 columns, described below.
 //   k_stream3d_f32: the precision form (FP32 arithmetic, every field
 //        Kahan-compensated, the equilibrium-referenced gamma solve) on
 //        interior-only records (pfa_step2d_f32.cu): A = float4 {x_Cr, x_Nb,
@@ -58,18 +58,21 @@ __device__ __noinline__ void store64(double* f, const Step3DArgs& a, int x, int 
 }
 
 // ---- plain FP64 ----
-// Tiles of 32 x 8 columns (pfa_tile64.cuh) streaming along z: a thread keeps
+// Tiles of 8 x 8 columns (pfa_tile64.cuh) streaming along z: a thread keeps
 // its cell's last three planes (x^gamma, phases) and the records of the next
 // two, publishes x^gamma (fixed point, pfa_device.cuh) and the phases of
 // plane z in shared memory and passes one barrier per plane.  ISO: equal
 // spacings, which the fixed-point sum needs; other spacings, and planes with
-// a composition outside its range, take the FP64 sums.  Measured against the
-// kernel that formed the sums on the FP64 pipe (30 x 14 columns, halo lanes
-// and rows): 128^3 346 -> 184 us a step, 256^3 1444 -> 547.
-constexpr int kTY3 = 8;
+// a composition outside its range, take the FP64 sums.  Bound by the FP64
+// pipe next to precipitates, elsewhere by the latency of a plane's chain:
+// compact tiles put the fewest warps on a precipitate's surface, and three
+// warps per CTA wait least for one another.  us a step at the best split, 32
+// x 8 tiles in rows of 32 / 16 x 16 / 16 x 8 / 8 x 8 (eight CTAs per SM asked
+// for; six: 139, 506): 128^3 184 / 168 / 158 / 132, 256^3 543 / 569 / 557 / 470.
+using Tile3 = Tile<8, 8, false>;
 struct Plane64 {
-  long long g1[kTY3 + 2][kEX], g2[kTY3 + 2][kEX];
-  double pd[kTY3 + 2][kEX], pl[kTY3 + 2][kEX];
+  Tile3::Plane<long long> g1, g2;
+  Tile3::Plane<double> pd, pl;
 };
 
 // one plane of a thread's column
@@ -79,16 +82,17 @@ struct Col64 : Cell64 {
 };
 
 template <bool ISO>
-__global__ void __launch_bounds__(tile_threads(kTY3), 2)
+__global__ void __launch_bounds__(Tile3::kThreads, 8)
     k_stream3d_f64(const __grid_constant__ Step3DArgs a) {
   __shared__ Plane64 sh[2];
   __shared__ int s_wide[3];
   int ex, ey;
-  const bool staged = tile_cell<kTY3>(ex, ey);
-  const int x = int(blockIdx.x) * kTX + ex - 1, y = int(blockIdx.y) * kTY3 + ey - 1;
+  const bool staged = Tile3::cell(ex, ey);
+  const int xt = (a.Nx + Tile3::TX - 1) / Tile3::TX, by = int(blockIdx.x) / xt, bx = int(blockIdx.x) - by * xt;
+  const int x = bx * Tile3::TX + ex - 1, y = by * Tile3::TY + ey - 1;
   const int cx = clampi(x, 0, a.Nx - 1), cy = clampi(y, 0, a.Ny - 1);
-  const bool own = threadIdx.x < 32 * kTY3 && x < a.Nx && y < a.Ny;
-  const int z0 = blockIdx.z * a.zrows, z1 = min(z0 + a.zrows, a.Nz);
+  const bool own = threadIdx.x < Tile3::kOwn && x < a.Nx && y < a.Ny;
+  const int z0 = blockIdx.y * a.zrows, z1 = min(z0 + a.zrows, a.Nz);
   const size_t plane = size_t(a.Ny + 2) * a.pitch, col = size_t(cy + 1) * a.pitch + cx + 1;
   const Coef64& K = a.c;
   const bool edge = cx == 0 || cx == a.Nx - 1 || cy == 0 || cy == a.Ny - 1;
@@ -122,7 +126,7 @@ __global__ void __launch_bounds__(tile_threads(kTY3), 2)
     N = stage();
     if (z + 1 < z1) load(z + 2);
     Plane64& S = sh[z & 1];
-    auto dg1 = reinterpret_cast<double (*)[kEX]>(S.g1), dg2 = reinterpret_cast<double (*)[kEX]>(S.g2);
+    auto dg1 = reinterpret_cast<double (*)[Tile3::kPitch]>(S.g1), dg2 = reinterpret_cast<double (*)[Tile3::kPitch]>(S.g2);
     if (staged) {
       if (ISO && !C.wide) {
         S.g1[ey][ex] = C.f1;
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(tile_threads(kTY3), 2)
     if (own) {
       double ocr, onb, od = 0.0, ol = 0.0;
       const double mx = a.m.idx2[0], my = a.m.idx2[1], mz = a.m.idx2[2];
-      auto lap = [&](double zm, double zp, const double (*s)[kEX], double c) {
+      auto lap = [&](double zm, double zp, const double (*s)[Tile3::kPitch], double c) {
         const double sx = s[ey][ex - 1] + s[ey][ex + 1], sy = s[ey - 1][ex] + s[ey + 1][ex];
         if constexpr (ISO)
           return fma(K.iso_c, c, ((zm + zp) + sy) + sx);
@@ -160,7 +164,7 @@ __global__ void __launch_bounds__(tile_threads(kTY3), 2)
           return fma(mz, zm + zp, fma(my, sy, fma(mx, sx, -2. * (mx + my + mz) * c)));
       };
       if (fixed) {
-        auto sum = [&](long long zm, long long zp, const long long (*s)[kEX], long long c) {
+        auto sum = [&](long long zm, long long zp, const long long (*s)[Tile3::kPitch], long long c) {
           return (zm + zp) + (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]) - 6 * c;
         };
         const long long S1 = sum(P.f1, N.f1, S.g1, C.f1), S2 = sum(P.f2, N.f2, S.g2, C.f2);
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(tile_threads(kTY3), 2)
         onb = C.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
       }
       if (phases) {
-        auto none = [&](double zm, double zp, const double (*s)[kEX]) {
+        auto none = [&](double zm, double zp, const double (*s)[Tile3::kPitch]) {
           auto b = [&](int y, int x) { return value_bits(s[y][x]); };
           return (value_bits(zm) | value_bits(zp) | b(ey, ex) | b(ey - 1, ex) | b(ey + 1, ex) |
                   b(ey, ex - 1) | b(ey, ex + 1)) == 0;
@@ -500,33 +504,18 @@ int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
 
 // FP64: a column next to a precipitate costs several times one in the matrix,
 // so short segments that spread the precipitates over the SMs beat whole
-// waves of equal ones.  us per step at 1 / 2 / 3 / 8 / 16 planes: 32^3 26 / 36
-// / 47 / 97 / 178, 64^3 83 / 78 / 77 / 104 / 189, 128^3 215 / 189 / 184 / 208
-// / 282, 200 x 100 x 60 152 / 137 / 138 / 180 / 212, 256^3 907 / 697 / 622 /
-// 547 / 543, 384^3 2673 / 1980 / 1742 / 1470 / 1417.
-int segment_planes_f64(int Nx, int Ny, int Nz) {
-  const long long cols = (long long)((Nx + kTX - 1) / kTX) * ((Ny + kTY3 - 1) / kTY3);
-  const long long n = cols * Nz;  // planes of tiles
-  const int planes = n <= 304 ? 1 : (n <= 12160 ? 3 : (n <= 97280 ? 8 : 16));
-  return std::min(planes, Nz);
+// waves of equal ones.  us per step at 1 / 2 / 3 / 6 / 12 / 24 planes: 32^3 23
+// / 21 / 26 / 41 / 74 / 135, 64^3 61 / 56 / 60 / 57 / 80 / 128, 96^3 94 / 85 /
+// 86 / 94 / 118 / 151, 200 x 100 x 60 105 / 94 / 94 / 107 / 123 / 132, 128^3
+// 154 / 137 / 132 / 135 / 157 / 182, 192^3 368 / 290 / 268 / 255 / 254 / 280,
+// 256^3 783 / 602 / 541 / 488 / 471 / 471.
+int segment_planes_f64(long long columns, int Nz) {
+  const long long n = columns * Nz;  // planes of tiles
+  const int planes = n <= 16384 ? 2 : (n <= 65536 ? 3 : (n <= 180000 ? 6 : 16));
+  return std::min(std::max(planes, (Nz + 65534) / 65535), Nz);
 }
 
-int g_resident3[2] = {0, 0};
-
-template <bool F64>
-cudaError_t query3() {
-  int dev = 0, sms = 0, per = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) {
-    if (F64)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f64<true>, tile_threads(kTY3), 0);
-    else
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f32<false>, 32 * kW3, kSmem3);
-  }
-  g_resident3[F64] = sms * (per > 0 ? per : 1);
-  return e;
-}
+int g_resident3 = 0;  // resident CTAs of the FP32 kernel
 
 }  // namespace
 
@@ -536,8 +525,13 @@ cudaError_t prepare_step3d() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_stream3d_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(kSmem3));
-  if (e == cudaSuccess) e = query3<true>();
-  return e == cudaSuccess ? query3<false>() : e;
+  int dev = 0, sms = 0, per = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream3d_f32<false>, 32 * kW3, kSmem3);
+  g_resident3 = sms * (per > 0 ? per : 1);
+  return e;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the
@@ -575,17 +569,19 @@ cudaError_t encode_step3d_maps(Tma3* t, const void* A, const void* B, int Nx, in
 }
 
 cudaError_t launch_step3d(Step3DArgs a, bool f64, const Tma3* t, cudaStream_t s) {
-  const int resident = g_resident3[f64] > 0 ? g_resident3[f64] : 152;
-  const int tx = f64 ? kTX : kCols3, ty = f64 ? kTY3 : kRows3;
-  a.zrows = f64 ? segment_planes_f64(a.Nx, a.Ny, a.Nz) : segment_planes(a.Nx, a.Ny, a.Nz, resident, tx, ty);
-  dim3 grid((a.Nx + tx - 1) / tx, (a.Ny + ty - 1) / ty, (a.Nz + a.zrows - 1) / a.zrows);
   if (f64) {
+    const long long cols = (long long)((a.Nx + Tile3::TX - 1) / Tile3::TX) * ((a.Ny + Tile3::TY - 1) / Tile3::TY);
+    a.zrows = segment_planes_f64(cols, a.Nz);
+    const dim3 grid((unsigned)cols, (a.Nz + a.zrows - 1) / a.zrows);
     if (a.c.mask == kMaskIso)
-      k_stream3d_f64<true><<<grid, tile_threads(kTY3), 0, s>>>(a);
+      k_stream3d_f64<true><<<grid, Tile3::kThreads, 0, s>>>(a);
     else
-      k_stream3d_f64<false><<<grid, tile_threads(kTY3), 0, s>>>(a);
+      k_stream3d_f64<false><<<grid, Tile3::kThreads, 0, s>>>(a);
   } else {
     if (!t) return cudaErrorInvalidValue;
+    const int resident = g_resident3 > 0 ? g_resident3 : 152;
+    a.zrows = segment_planes(a.Nx, a.Ny, a.Nz, resident, kCols3, kRows3);
+    const dim3 grid((a.Nx + kCols3 - 1) / kCols3, (a.Ny + kRows3 - 1) / kRows3, (a.Nz + a.zrows - 1) / a.zrows);
     if (a.skip_plane >= 0)
       k_stream3d_f32<true><<<grid, 32 * kW3, kSmem3, s>>>(a, *t);
     else

@@ -9,40 +9,53 @@ namespace {
 
 using namespace dev;
 
-constexpr int kTX = 32;       // tile width (one warp)
-constexpr int kEX = kTX + 2;  // staged width
-
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// A tile of 32 x TY cells: one row per warp; the warps past the TY rows stage
-// the tile's halo cells, so that a cell's solve and its update are never
-// behind another cell's in the same warp.
-constexpr int halo_warps(int ty) { return (2 * kEX + 2 * ty + 31) / 32; }
-constexpr int tile_threads(int ty) { return 32 * (ty + halo_warps(ty)); }
+// A tile of TX x TY cells.  A warp owns a block of 8 x 4 of them: an FP64
+// operation costs a warp the same whatever its active lanes, and a precipitate
+// touches fewer compact blocks than rows of 32.  The warps past the tile's own
+// stage its halo, so that a cell's solve and its update are never behind
+// another cell's in the same warp; the corners only where the stencil reads
+// them (an 8 x 8 tile's halo without them is one warp).
+template <int TX_, int TY_, bool CORNERS>
+struct Tile {
+  static constexpr int TX = TX_, TY = TY_;
+  static constexpr int EX = TX + 2, EY = TY + 2;  // staged cells
+  // elements per staged row: 8 modulo 16, so that the two rows of 8 that a
+  // half warp reads fall into different banks
+  static constexpr int kPitch = (EX + 7) / 16 * 16 + 8;
+  static constexpr int kOwn = TX * TY, kHalo = 2 * (TX + TY) + 4 * CORNERS;
+  static constexpr int kThreads = kOwn + (kHalo + 31) / 32 * 32;
+  static_assert(TX % 8 == 0 && TY % 4 == 0 && kPitch >= EX, "whole warp blocks");
+  template <class T>
+  using Plane = T[EY][kPitch];
 
-// this thread's cell (ex, ey) of the (TY + 2) x 34 staged tile: its own
-// output cell in the first TY warps, a halo cell in the rest (false: none,
-// a duplicate of the last one)
-template <int TY>
-__device__ __forceinline__ bool tile_cell(int& ex, int& ey) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (w < TY) {
-    ex = lane + 1;
-    ey = w + 1;
-    return true;
+  // this thread's cell (ex, ey) of the staged tile: its own output cell in the
+  // first kOwn threads, a halo cell in the rest (false: none, a duplicate of
+  // the last one)
+  static __device__ __forceinline__ bool cell(int& ex, int& ey) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < kOwn / 32) {
+      ex = w % (TX / 8) * 8 + (lane & 7) + 1;
+      ey = w / (TX / 8) * 4 + (lane >> 3) + 1;
+      return true;
+    }
+    const int i = int(threadIdx.x) - kOwn, h = i < kHalo ? i : kHalo - 1;
+    if (h < 2 * TX) {
+      ey = h < TX ? 0 : TY + 1;
+      ex = 1 + (h < TX ? h : h - TX);
+    } else if (h < 2 * (TX + TY)) {
+      const int k = h - 2 * TX;
+      ey = 1 + (k < TY ? k : k - TY);
+      ex = k < TY ? 0 : TX + 1;
+    } else {
+      const int k = h - 2 * (TX + TY);
+      ey = k < 2 ? 0 : TY + 1;
+      ex = k & 1 ? TX + 1 : 0;
+    }
+    return i < kHalo;
   }
-  constexpr int kHalo = 2 * kEX + 2 * TY;
-  const int i = (w - TY) * 32 + lane, h = i < kHalo ? i : kHalo - 1;
-  if (h < 2 * kEX) {
-    ey = h < kEX ? 0 : TY + 1;
-    ex = h < kEX ? h : h - kEX;
-  } else {
-    const int k = h - 2 * kEX;
-    ey = 1 + (k < TY ? k : k - TY);
-    ex = k < TY ? 0 : kEX - 1;
-  }
-  return i < kHalo;
-}
+};
 
 // One staged cell: its values and x^gamma.  phase: the tile must look at the
 // phases at all (an all-zero phase field stays zero: its Laplacian, p' and

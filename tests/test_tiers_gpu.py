@@ -1,5 +1,5 @@
 """The FP64 step's cheaper forms (zero, far-tail and general phases; the
-skipped gamma solve) and its tile heights, against the oracle."""
+skipped gamma solve) and its tiles, against the oracle."""
 import numpy as np
 import pytest
 
@@ -50,8 +50,7 @@ def check_cells(got, want, rel):
         assert np.all((np.abs(a - b) <= rel * scale)[core])
 
 
-# tiles of 1, 4 and 8 rows (up to 1215, 9727 and more tile rows of 32 cells),
-# partial tiles on both axes
+# tiles of 8 x 4 (up to 1216 of them) and 8 x 8 cells, partial tiles on both axes
 @pytest.mark.parametrize("nx,ny", [(33, 9), (65, 405), (70, 406), (161, 1621), (191, 1622)])
 @pytest.mark.parametrize("mask", ["iso", "five", "nine"])
 def test_forms_2d(pfa, orc, nx, ny, mask):
@@ -71,7 +70,8 @@ def test_forms_2d(pfa, orc, nx, ny, mask):
     check_cells(got, want, 350 * 16 * 2.0 ** -53)
 
 
-@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 130), (40, 700)])
+# tiles of 8 x 8 and (from 304 of them) 16 x 16 cells
+@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 130), (40, 700), (330, 250)])
 def test_forms_varmob(pfa, orc, nx, ny):
     f = mixed_fields((ny, nx), nx + ny)
     g = pfa.Grid2D(f, pfa.model_params(), mobility="variable")
@@ -81,8 +81,8 @@ def test_forms_varmob(pfa, orc, nx, ny):
     check_cells(got, orc.run2d_varmob(f, O.model_params(), 1), 350 * 16 * 2.0 ** -53)
 
 
-# segments of 2, 3 and 12 planes; partial tiles on every axis
-@pytest.mark.parametrize("n", [(31, 15, 3), (64, 40, 131), (95, 61, 700)])
+# segments of 2, 3 and 6 planes; partial tiles on every axis
+@pytest.mark.parametrize("n", [(31, 15, 3), (64, 40, 131), (199, 93, 61), (95, 61, 700)])
 def test_forms_3d(pfa, orc, n):
     f = mixed_fields(n[::-1], sum(n))
     g = pfa.Grid3D(f, pfa.model_params(dim=3))
