@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 
+#include "pfa_exp64.cuh"
 #include "pfa_internal.h"
 #include "pfa_model.h"
 
@@ -337,19 +338,42 @@ __device__ __forceinline__ double advance58(double X, long long D0, long long S1
   return advance64(X, inc);
 }
 
-// The diffusivities of dmatrix64 times the scale in `pre` (prefactors of Nb,
-// Cr, Ni), regrouped: per column c the three weighted mobilities A = e_Nb
-// (s_c + h_Nb,c), B = e_Cr (s_c + h_Cr,c), C = e_Ni x_Ni s_c give W = X B + Y
-// A + C, D_Cr,c = X (B - W), D_Nb,c = Y (A - W): 22 operations for 60.
-__device__ __forceinline__ void dmatrix64_scaled(const double pre[3], double X, double Y,
+// v 2^64, v in [2^-11, 1) (exact)
+__device__ __forceinline__ uint64_t fix64(double v) {
+  const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
+  const uint64_t t = (uint64_t(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32) | (lo << 11);
+  return t >> ((1022u - (hi >> 20)) & 63u);
+}
+
+// e_Nb, e_Cr, e_Ni x_Ni of dmatrix64 times the prefactors, in FP64 (a call:
+// most cells take the integer forms of pfa_exp64.cuh)
+static __device__ __noinline__ void mobilities64(const Coef64& K, double X, double Y, double e[3]) {
+  const double xni = 1.0 - X - Y;
+  e[0] = K.vm_pre[0] * exp(Y * fma(-34.982563536715503, xni, 14.437947842988088));
+  e[1] = K.vm_pre[1] * exp(X * fma(-7.1543718172640256, xni, 3.3541967644499233));
+  e[2] = K.vm_pre[2] * xni *
+         exp(fma(X, fma(-8.5221193705645018, xni, 4.0036674816806448),
+                 -Y * fma(442.62877981749585, xni, 0.82164267100913768)));
+}
+
+// The diffusivities of dmatrix64 times dt / (2 dx^2), regrouped: per column c
+// the three weighted mobilities A = e_Nb (s_c + h_Nb,c), B = e_Cr (s_c +
+// h_Cr,c), C = e_Ni x_Ni s_c give W = X B + Y A + C, D_Cr,c = X (B - W), D_Nb,c
+// = Y (A - W): 26 operations and the mobilities for 60 and three exponentials.
+// unit: both compositions are in [2^-11, 1).
+__device__ __forceinline__ void dmatrix64_scaled(const Coef64& K, double X, double Y, bool unit,
                                                  double& d00, double& d01, double& d10,
                                                  double& d11) {
-  const double xni = 1.0 - X - Y;
-  const double eNb = pre[0] * exp(Y * fma(-34.982563536715503, xni, 14.437947842988088));
-  const double eCr = pre[1] * exp(X * fma(-7.1543718172640256, xni, 3.3541967644499233));
-  const double eNi = pre[2] * xni *
-                     exp(fma(X, fma(-8.5221193705645018, xni, 4.0036674816806448),
-                             -Y * fma(442.62877981749585, xni, 0.82164267100913768)));
+  double e[3];
+  const uint64_t x = fix64(X), y = fix64(Y);
+  if (unit && K.vm_fixed && uint64_t(x + y) > x) {  // x_Ni > 0
+    uint64_t b[3];
+    mobilities(K, x, y, b);
+    for (int k = 0; k < 3; k++) e[k] = __longlong_as_double((long long)b[k]);
+  } else {
+    mobilities64(K, X, Y, e);
+  }
+  const double eNb = e[0], eCr = e[1], eNi = e[2];
   {
     const double s = fma(-kHCrCr, X, -kHCrNb * Y);
     const double A = eNb * (s + kHCrNbAddA), B = eCr * (s + kHCrCrAdd);

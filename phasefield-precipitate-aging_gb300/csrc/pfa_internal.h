@@ -76,6 +76,9 @@ struct Coef64 {
   long long Dfix[2][2];  // iso masks: D 2^70 (dev::advance58)
   double vm_pre[3];  // variable mobility: prefactors (Nb, Cr, Ni) times dt / (2 dx^2)
   double vm_qy;      // and the weight of the y faces, (1/dy^2) / (1/dx^2)
+  unsigned long long vm_m[3];  // vm_pre = vm_m 2^(vm_e - 63), 2^63 <= vm_m
+  int vm_e[3];
+  int vm_fixed;  // vm_pre are positive and within 2^+-200: pfa_exp64.cuh applies
 };
 
 enum { kMaskIso = 0, kMaskFive = 1, kMaskNine = 2, kMaskIso9 = 3 };

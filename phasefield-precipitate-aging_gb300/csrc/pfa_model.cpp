@@ -172,6 +172,17 @@ void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
   o->vm_pre[1] = kMobPreCr * r2x;
   o->vm_pre[2] = kMobPreNi * r2x;
   o->vm_qy = m.idx2[0] > 0.0 ? m.idx2[1] / m.idx2[0] : 0.0;
+  o->vm_fixed = 1;
+  for (int k = 0; k < 3; k++) {
+    if (!(o->vm_pre[k] > 0x1p-200 && o->vm_pre[k] < 0x1p200)) {
+      o->vm_fixed = 0;
+      continue;
+    }
+    int e;
+    const double f = std::frexp(o->vm_pre[k], &e);  // [1/2, 1)
+    o->vm_m[k] = (unsigned long long)std::ldexp(f, 53) << 11;
+    o->vm_e[k] = e - 1;
+  }
 }
 
 void model_fast_coef(FastCoef* o) {

@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, 768 / Tile<TX, 
     s_g2[ey][ex] = c.g2;
     s_pd[ey][ex] = c.pd;
     s_pl[ey][ex] = c.pl;
-    dmatrix64_scaled(a.c.vm_pre, c.X, c.Y, s_d[0][ey][ex], s_d[1][ey][ex], s_d[2][ey][ex],
+    dmatrix64_scaled(a.c, c.X, c.Y, c.unit, s_d[0][ey][ex], s_d[1][ey][ex], s_d[2][ey][ex],
                      s_d[3][ey][ex]);
   }
   const bool phases = __syncthreads_or(c.phase);

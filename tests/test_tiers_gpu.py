@@ -81,6 +81,35 @@ def test_forms_varmob(pfa, orc, nx, ny):
     check_cells(got, orc.run2d_varmob(f, O.model_params(), 1), 350 * 16 * 2.0 ** -53)
 
 
+# compositions inside and outside the range of the integer mobilities: Nb below
+# 2^-11, Cr and Nb adding up to more than 1, both edges, in one grid and mixed
+# within a warp
+@pytest.mark.parametrize("nx,ny", [(37, 21), (330, 250)])
+def test_mobilities_out_of_range(pfa, orc, nx, ny):
+    rng = np.random.default_rng(nx)
+    kind = rng.integers(0, 5, (ny, nx))
+    kind[: ny // 3] = 0
+    x = rng.uniform(0.3, 0.6, (ny, nx))
+    y = rng.uniform(0.02, 0.12, (ny, nx))
+    x[kind == 1] = 0.95
+    y[kind == 1] = rng.uniform(0.049, 0.06, (ny, nx))[kind == 1]
+    y[kind == 2] = 10.0 ** rng.uniform(-6, -3, (ny, nx))[kind == 2]
+    y[kind == 3] = 2.0 ** -11 * (1 - 2.0 ** -53 * rng.integers(-1, 2, (ny, nx)))[kind == 3]
+    x[kind == 4], y[kind == 4] = 0.9375, 0.0625
+    f = []
+    for a in (x, y, np.zeros((ny, nx)), np.zeros((ny, nx))):
+        h = np.empty((ny + 2, nx + 2))
+        h[1:-1, 1:-1] = a
+        f.append(ic.mirror_halo(h))
+    g = pfa.Grid2D(f, pfa.model_params(), mobility="variable")
+    g.run(1)
+    got = g.read()
+    g.close()
+    # the oracle's exponents reach 50 (their rounding: 2^-47 of D), increments
+    # stay below the values around
+    check_cells(got, orc.run2d_varmob(f, O.model_params(), 1), 350 * 16 * 2.0 ** -53)
+
+
 # segments of 2, 3 and 6 planes; partial tiles on every axis
 @pytest.mark.parametrize("n", [(31, 15, 3), (64, 40, 131), (199, 93, 61), (95, 61, 700)])
 def test_forms_3d(pfa, orc, n):
