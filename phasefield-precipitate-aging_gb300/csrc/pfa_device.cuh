@@ -8,7 +8,7 @@
 
 #include <cuda_runtime.h>
 
-#include "pfa_exp64.cuh"
+#include "pfa_fixed64.cuh"
 #include "pfa_internal.h"
 #include "pfa_model.h"
 
@@ -345,8 +345,20 @@ __device__ __forceinline__ uint64_t fix64(double v) {
   return t >> ((1022u - (hi >> 20)) & 63u);
 }
 
+// v 2^63, v in [0, 1] (rounded down)
+__device__ __forceinline__ uint64_t fix63(double v) {
+  const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
+  const uint64_t t = (uint64_t(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32) | (lo << 11);
+  const unsigned r = 1023u - (hi >> 20);
+  return r < 64u ? t >> r : 0ull;
+}
+
+// h 2^-60, h 2^-58 as FP64
+__device__ __forceinline__ double value60(int64_t h) { return __longlong_as_double((long long)pack_signed(h, 60)); }
+__device__ __forceinline__ double value58(int64_t h) { return __longlong_as_double((long long)pack_signed(h, 58)); }
+
 // e_Nb, e_Cr, e_Ni x_Ni of dmatrix64 times the prefactors, in FP64 (a call:
-// most cells take the integer forms of pfa_exp64.cuh)
+// most cells take the integer forms of pfa_fixed64.cuh)
 static __device__ __noinline__ void mobilities64(const Coef64& K, double X, double Y, double e[3]) {
   const double xni = 1.0 - X - Y;
   e[0] = K.vm_pre[0] * exp(Y * fma(-34.982563536715503, xni, 14.437947842988088));

@@ -78,7 +78,7 @@ struct Coef64 {
   double vm_qy;      // and the weight of the y faces, (1/dy^2) / (1/dx^2)
   unsigned long long vm_m[3];  // vm_pre = vm_m 2^(vm_e - 63), 2^63 <= vm_m
   int vm_e[3];
-  int vm_fixed;  // vm_pre are positive and within 2^+-200: pfa_exp64.cuh applies
+  int vm_fixed;  // vm_pre are positive and within 2^+-200: dev::mobilities applies
 };
 
 enum { kMaskIso = 0, kMaskFive = 1, kMaskNine = 2, kMaskIso9 = 3 };

@@ -118,23 +118,24 @@ __device__ __forceinline__ bool none64(const double (*s)[P], int ex, int ey) {
   return m == 0;
 }
 
-__device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy) {
+template <bool FIXED, bool HOT>
+__device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy, int64_t most) {
   const size_t i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
-  Cell64 c = cell64(__ldg(static_cast<const double*>(a.in[0]) + i),
-                    __ldg(static_cast<const double*>(a.in[1]) + i),
-                    __ldg(static_cast<const double*>(a.in[2]) + i),
-                    __ldg(static_cast<const double*>(a.in[3]) + i));
+  Cell64 c = cell64<FIXED, HOT>(__ldg(static_cast<const double*>(a.in[0]) + i),
+                           __ldg(static_cast<const double*>(a.in[1]) + i),
+                           __ldg(static_cast<const double*>(a.in[2]) + i),
+                           __ldg(static_cast<const double*>(a.in[3]) + i), most);
   c.i = i;
   return c;
 }
 
 // Allen-Cahn of both phases, src/discretization.cu:888-980
-template <int MASK, int P>
-__device__ __forceinline__ void phases64(const Step2DArgs& a, const Cell64& c, const double (*s_pd)[P],
-                                         const double (*s_pl)[P], int ex, int ey, double& od,
-                                         double& ol) {
-  od = phase64<0>(a.c, c, none64<MASK>(s_pd, ex, ey), [&] { return lap64<MASK>(a, s_pd, ex, ey); });
-  ol = phase64<1>(a.c, c, none64<MASK>(s_pl, ex, ey), [&] { return lap64<MASK>(a, s_pl, ex, ey); });
+template <int MASK, int P, class Gam>
+__device__ __forceinline__ void update_phases(const Step2DArgs& a, const Cell64& c, const double (*s_pd)[P],
+                                              const double (*s_pl)[P], int ex, int ey, Gam gamma,
+                                              double& od, double& ol) {
+  od = phase64<0>(a.c, c, none64<MASK>(s_pd, ex, ey), [&] { return lap64<MASK>(a, s_pd, ex, ey); }, gamma);
+  ol = phase64<1>(a.c, c, none64<MASK>(s_pl, ex, ey), [&] { return lap64<MASK>(a, s_pl, ex, ey); }, gamma);
 }
 
 // tile rows past what a grid's second dimension holds go on in the third
@@ -143,18 +144,18 @@ __device__ __forceinline__ int tile_row() { return int(blockIdx.z * gridDim.y + 
 
 template <int MASK, int TX, int TY>
 using Tile2 = Tile<TX, TY, MASK == kMaskIso9 || MASK == kMaskNine>;
-// resident blocks asked for: 1408 threads per SM (46 registers)
-constexpr int blocks2(int threads) { return 1408 / threads; }
+// resident blocks asked for: 1152 threads per SM (56 registers), 1408 (46)
+constexpr int blocks2(int threads, bool hot) { return (hot ? 1152 : 1408) / threads; }
 
-// MASK: Coef64::mask.  Bound by the FP64 pipe next to precipitates and by
-// memory elsewhere.
-template <int MASK, int TX, int TY>
-__global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<MASK, TX, TY>::kThreads))
+// MASK: Coef64::mask.  HOT: see cell64.  Bound by the FP64 pipe next to
+// precipitates, by integer issue and memory latency elsewhere.
+template <int MASK, int TX, int TY, bool HOT>
+__global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<MASK, TX, TY>::kThreads, HOT))
     k_step2d_f64(const __grid_constant__ Step2DArgs a) {
   using T = Tile2<MASK, TX, TY>;
   constexpr bool kFixed = MASK == kMaskIso || MASK == kMaskIso9;
-  // |x^gamma| < 4 (5 points) or 1 (9 points): the neighbour sum stays below 2^5
-  constexpr int kGammaHi = MASK == kMaskIso9 ? 0x3ff00000 : 0x40100000;
+  // |x^gamma| < 2 (5 points) or 1 (9 points): the neighbour sum stays below 2^5
+  constexpr int64_t kMost = MASK == kMaskIso9 ? 1ll << 60 : 1ll << 61;
   // x^gamma as doubles, or (kFixed) in fixed point
   __shared__ typename T::template Plane<long long> s_g1, s_g2;
   __shared__ typename T::template Plane<double> s_pd, s_pl;
@@ -162,24 +163,20 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
   int ex, ey;
   const bool staged = T::cell(ex, ey);
   const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
-  const Cell64 c = stage64(a, gx, gy);
-  const bool wide = wide64(c, kGammaHi);  // outside the fixed-point forms' range
+  const Cell64 c = stage64<kFixed, HOT>(a, gx, gy, kMost);
   if (staged) {
-    if (!kFixed || wide) {
-      as_double(s_g1)[ey][ex] = c.g1;
-      as_double(s_g2)[ey][ex] = c.g2;
-    } else {
-      fix_cell(c, s_g1[ey][ex], s_g2[ey][ex]);
-    }
+    s_g1[ey][ex] = c.g1;
+    s_g2[ey][ex] = c.g2;
     s_pd[ey][ex] = c.pd;
     s_pl[ey][ex] = c.pl;
   }
   const bool phases = __syncthreads_or(c.phase);
-  const bool fixed = kFixed && !__syncthreads_or(wide);
+  const bool fixed = kFixed && !__syncthreads_or(c.wide);
   if (kFixed && !fixed) {  // the whole tile in FP64
-    if (staged) {
-      as_double(s_g1)[ey][ex] = c.g1;
-      as_double(s_g2)[ey][ex] = c.g2;
+    if (staged && !c.wide) {
+      const double2 g = gamma_values(c, s_g1[ey][ex], s_g2[ey][ex]);
+      as_double(s_g1)[ey][ex] = g.x;
+      as_double(s_g2)[ey][ex] = g.y;
     }
     __syncthreads();
   }
@@ -198,7 +195,14 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
     onb = c.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
   }
   double od = 0.0, ol = 0.0;
-  if (phases) phases64<MASK>(a, c, s_pd, s_pl, ex, ey, od, ol);
+  if (phases) {
+    auto gamma = [&] {
+      if constexpr (!HOT) return make_double2(c.v1, c.v2);
+      if (fixed) return gamma_values(c, s_g1[ey][ex], s_g2[ey][ex]);
+      return make_double2(as_double(s_g1)[ey][ex], as_double(s_g2)[ey][ex]);
+    };
+    update_phases<MASK>(a, c, s_pd, s_pl, ex, ey, gamma, od, ol);
+  }
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
@@ -223,13 +227,13 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, 768 / Tile<TX, 
   int ex, ey;
   const bool staged = T::cell(ex, ey);
   const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
-  const Cell64 c = stage64(a, gx, gy);
+  const Cell64 c = stage64<false, true>(a, gx, gy, 0);
   if (staged) {
-    s_g1[ey][ex] = c.g1;
-    s_g2[ey][ex] = c.g2;
+    s_g1[ey][ex] = __longlong_as_double(c.g1);
+    s_g2[ey][ex] = __longlong_as_double(c.g2);
     s_pd[ey][ex] = c.pd;
     s_pl[ey][ex] = c.pl;
-    dmatrix64_scaled(a.c, c.X, c.Y, c.unit, s_d[0][ey][ex], s_d[1][ey][ex], s_d[2][ey][ex],
+    dmatrix64_scaled(a.c, c.X, c.Y, in_unit(c.X) && in_unit(c.Y), s_d[0][ey][ex], s_d[1][ey][ex], s_d[2][ey][ex],
                      s_d[3][ey][ex]);
   }
   const bool phases = __syncthreads_or(c.phase);
@@ -257,16 +261,21 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, 768 / Tile<TX, 
   const double onb = c.Y + fma(K.vm_qy, s_fy[1][ty + 1][tx] - s_fy[1][ty][tx],
                                s_fx[1][ty][tx + 1] - s_fx[1][ty][tx]);
   double od = 0.0, ol = 0.0;
-  if (phases) phases64<ISO ? kMaskIso : kMaskFive>(a, c, s_pd, s_pl, ex, ey, od, ol);
+  if (phases) {
+    auto gamma = [&] { return make_double2(s_g1[ey][ex], s_g2[ey][ex]); };
+    update_phases<ISO ? kMaskIso : kMaskFive>(a, c, s_pd, s_pl, ex, ey, gamma, od, ol);
+  }
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
+
+constexpr long long kHotTiles = 12288;
 
 template <int TX, int TY>
 long long tiles(const Step2DArgs& a) {
   return (long long)((a.Nx + TX - 1) / TX) * ((a.Ny + TY - 1) / TY);
 }
 
-template <int TX, int TY, bool VM>
+template <int TX, int TY, bool VM, bool HOT>
 cudaError_t launch_tiles(const Step2DArgs& a, cudaStream_t s) {
   const int ny = (a.Ny + TY - 1) / TY;
   const dim3 grid((a.Nx + TX - 1) / TX, std::min(ny, 65535), (ny + 65534) / 65535);
@@ -279,10 +288,10 @@ cudaError_t launch_tiles(const Step2DArgs& a, cudaStream_t s) {
   } else {
     constexpr int n5 = Tile2<kMaskIso, TX, TY>::kThreads, n9 = Tile2<kMaskIso9, TX, TY>::kThreads;
     switch (a.c.mask) {
-      case kMaskIso: k_step2d_f64<kMaskIso, TX, TY><<<grid, n5, 0, s>>>(a); break;
-      case kMaskIso9: k_step2d_f64<kMaskIso9, TX, TY><<<grid, n9, 0, s>>>(a); break;
-      case kMaskFive: k_step2d_f64<kMaskFive, TX, TY><<<grid, n5, 0, s>>>(a); break;
-      default: k_step2d_f64<kMaskNine, TX, TY><<<grid, n9, 0, s>>>(a);
+      case kMaskIso: k_step2d_f64<kMaskIso, TX, TY, HOT><<<grid, n5, 0, s>>>(a); break;
+      case kMaskIso9: k_step2d_f64<kMaskIso9, TX, TY, HOT><<<grid, n9, 0, s>>>(a); break;
+      case kMaskFive: k_step2d_f64<kMaskFive, TX, TY, HOT><<<grid, n5, 0, s>>>(a); break;
+      default: k_step2d_f64<kMaskNine, TX, TY, HOT><<<grid, n9, 0, s>>>(a);
     }
   }
   return cudaGetLastError();
@@ -295,15 +304,26 @@ cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s) {
   if (a.varmob && a.nine) return cudaErrorInvalidValue;  // refused by the host before
   // A tile next to a precipitate takes its SM's FP64 pipe for microseconds, and
   // a step is as long as its most loaded SM: small tiles spread such work, and
-  // 8 x 8 has the least halo for its size.  us a step of 8 x 4 / 8 x 8 / 16 x 8
-  // / 16 x 16 / 32 x 8 cells: 64 x 48 5.1 / 5.8 / 6.3 / 9.4 / 9.9, 192^2 5.8 /
-  // 5.9 / 8.3 / 8.1 / 8.8, 256^2 6.8 / 6.5 / 8.0 / 9.9 / 10.1, 1024^2 27 / 19.6
-  // / 21 / 24 / 25, 2048^2 93 / 67 / 69 / 77 / 77 (32 x 8 in rows of 32: 76).
-  if (!a.varmob) return tiles<8, 4>(a) <= 1216 ? launch_tiles<8, 4, false>(a, s) : launch_tiles<8, 8, false>(a, s);
-  // every staged cell has its exponentials, so large grids take the tile with
-  // the smallest share of halo: 8 x 8 / 16 x 16 192^2 17.1 / 17.2, 256^2 27.7 /
-  // 29.2, 320^2 39.0 / 35.8, 512^2 86 / 74, 2048^2 1266 / 1050
-  return tiles<16, 16>(a) < 304 ? launch_tiles<8, 8, true>(a, s) : launch_tiles<16, 16, true>(a, s);
+  // 8 x 8 has the least halo for its size.  us a step (FP64 solves) of 8 x 4 /
+  // 8 x 8 / 16 x 8 / 16 x 16 / 32 x 8 cells: 64 x 48 5.1 / 5.8 / 6.3 / 9.4 /
+  // 9.9, 192^2 5.8 / 5.9 / 8.3 / 8.1 / 8.8, 256^2 6.8 / 6.5 / 8.0 / 9.9 / 10.1,
+  // 1024^2 27 / 19.6 / 21 / 24 / 25, 2048^2 93 / 67 / 69 / 77 / 77 (32 x 8 in
+  // rows of 32: 76).
+  if (!a.varmob) {
+    if (tiles<8, 4>(a) <= 1216) return launch_tiles<8, 4, false, true>(a, s);
+    // The solve in fixed point shortens tiles next to precipitates, but its
+    // call costs registers (56 for 40, fewer tiles in flight), which many
+    // waves of tiles without precipitate feel; fixed / FP64 with 8 particles,
+    // 5 points 256^2 6.6 / 7.5, 512^2 9.1 / 10.3, 1000 x 733 14.4 / 14.4,
+    // 1024^2 18.3 / 17.7, 2048^2 73.5 / 65.4; 9 points 7.7 / 9.8, 11.8 / 14.7,
+    // 18.1 / 19.3, 23.0 / 23.4, 91 / 85
+    return tiles<8, 8>(a) <= kHotTiles ? launch_tiles<8, 8, false, true>(a, s) : launch_tiles<8, 8, false, false>(a, s);
+  }
+  // every staged cell has its mobilities, so large grids take the tile with
+  // the smallest share of halo: 8 x 8 / 16 x 16 (before their exponentials
+  // were integers) 192^2 17.1 / 17.2, 256^2 27.7 / 29.2, 320^2 39.0 / 35.8,
+  // 512^2 86 / 74, 2048^2 1266 / 1050
+  return tiles<16, 16>(a) < 304 ? launch_tiles<8, 8, true, true>(a, s) : launch_tiles<16, 16, true, true>(a, s);
 }
 
 }  // namespace pfa

@@ -75,14 +75,8 @@ struct Plane64 {
   Tile3::Plane<double> pd, pl;
 };
 
-// one plane of a thread's column
-struct Col64 : Cell64 {
-  long long f1, f2;  // x^gamma in fixed point (unless wide)
-  bool wide;
-};
-
-template <bool ISO>
-__global__ void __launch_bounds__(Tile3::kThreads, 8)
+template <bool ISO, bool HOT>
+__global__ void __launch_bounds__(Tile3::kThreads, HOT ? 7 : 8)
     k_stream3d_f64(const __grid_constant__ Step3DArgs a) {
   __shared__ Plane64 sh[2];
   __shared__ int s_wide[3];
@@ -107,14 +101,8 @@ __global__ void __launch_bounds__(Tile3::kThreads, 8)
     rpl = __ldg(static_cast<const double*>(a.in[3]) + i);
   };
   // |x^gamma| < 2: the seven-point sum stays below 2^5
-  auto stage = [&]() {
-    Col64 c;
-    static_cast<Cell64&>(c) = cell64(rX, rY, rpd, rpl);
-    c.wide = wide64(c, 0x40000000);
-    if (ISO && !c.wide) fix_cell(c, c.f1, c.f2);
-    return c;
-  };
-  Col64 P, C, N;
+  auto stage = [&]() { return cell64<ISO, HOT>(rX, rY, rpd, rpl, 1ll << 61); };
+  Cell64 P, C, N;  // planes z - 1, z, z + 1 of the thread's column
   load(z0 - 1);
   P = stage();
   load(z0);
@@ -128,13 +116,8 @@ __global__ void __launch_bounds__(Tile3::kThreads, 8)
     Plane64& S = sh[z & 1];
     auto dg1 = reinterpret_cast<double (*)[Tile3::kPitch]>(S.g1), dg2 = reinterpret_cast<double (*)[Tile3::kPitch]>(S.g2);
     if (staged) {
-      if (ISO && !C.wide) {
-        S.g1[ey][ex] = C.f1;
-        S.g2[ey][ex] = C.f2;
-      } else {
-        dg1[ey][ex] = C.g1;
-        dg2[ey][ex] = C.g2;
-      }
+      S.g1[ey][ex] = C.g1;
+      S.g2[ey][ex] = C.g2;
       if (ISO && (P.wide || C.wide || N.wide)) s_wide[w] = 1;
       S.pd[ey][ex] = C.pd;
       S.pl[ey][ex] = C.pl;
@@ -147,9 +130,10 @@ __global__ void __launch_bounds__(Tile3::kThreads, 8)
     if (threadIdx.x == 0) s_wide[w2] = 0;
     w = w == 2 ? 0 : w + 1;
     if (ISO && !fixed) {  // the whole plane in FP64
-      if (staged) {
-        dg1[ey][ex] = C.g1;
-        dg2[ey][ex] = C.g2;
+      if (staged && !C.wide) {
+        const double2 g = gamma_values(C, C.g1, C.g2);
+        dg1[ey][ex] = g.x;
+        dg2[ey][ex] = g.y;
       }
       __syncthreads();
     }
@@ -167,11 +151,14 @@ __global__ void __launch_bounds__(Tile3::kThreads, 8)
         auto sum = [&](long long zm, long long zp, const long long (*s)[Tile3::kPitch], long long c) {
           return (zm + zp) + (s[ey - 1][ex] + s[ey + 1][ex]) + (s[ey][ex - 1] + s[ey][ex + 1]) - 6 * c;
         };
-        const long long S1 = sum(P.f1, N.f1, S.g1, C.f1), S2 = sum(P.f2, N.f2, S.g2, C.f2);
+        const long long S1 = sum(P.g1, N.g1, S.g1, C.g1), S2 = sum(P.g2, N.g2, S.g2, C.g2);
         ocr = advance58(C.X, K.Dfix[0][0], S1, K.Dfix[0][1], S2);
         onb = advance58(C.Y, K.Dfix[1][0], S1, K.Dfix[1][1], S2);
       } else {
-        const double l1 = lap(P.g1, N.g1, dg1, C.g1), l2 = lap(P.g2, N.g2, dg2, C.g2);
+        // (fixed: within 2^-58 of the plane's own values, 1e-20 in the sum)
+        auto value = [](const Cell64& c, long long g) { return ISO && !c.wide ? value58(g) : __longlong_as_double(g); };
+        const double l1 = lap(value(P, P.g1), value(N, N.g1), dg1, dg1[ey][ex]);
+        const double l2 = lap(value(P, P.g2), value(N, N.g2), dg2, dg2[ey][ex]);
         ocr = C.X + fma(K.D[0][0], l1, K.D[0][1] * l2);
         onb = C.Y + fma(K.D[1][0], l1, K.D[1][1] * l2);
       }
@@ -181,8 +168,9 @@ __global__ void __launch_bounds__(Tile3::kThreads, 8)
           return (value_bits(zm) | value_bits(zp) | b(ey, ex) | b(ey - 1, ex) | b(ey + 1, ex) |
                   b(ey, ex - 1) | b(ey, ex + 1)) == 0;
         };
-        od = phase64<0>(K, C, none(P.pd, N.pd, S.pd), [&] { return lap(P.pd, N.pd, S.pd, C.pd); });
-        ol = phase64<1>(K, C, none(P.pl, N.pl, S.pl), [&] { return lap(P.pl, N.pl, S.pl, C.pl); });
+        auto gamma = [&] { return gamma_values(C, C.g1, C.g2); };
+        od = phase64<0>(K, C, none(P.pd, N.pd, S.pd), [&] { return lap(P.pd, N.pd, S.pd, C.pd); }, gamma);
+        ol = phase64<1>(K, C, none(P.pl, N.pl, S.pl), [&] { return lap(P.pl, N.pl, S.pl, C.pl); }, gamma);
       }
       const double v[4] = {ocr, onb, od, ol};
       const size_t i = size_t(z + 1) * plane + col;
@@ -515,6 +503,11 @@ int segment_planes_f64(long long columns, int Nz) {
   return std::min(std::max(planes, (Nz + 65534) / 65535), Nz);
 }
 
+// up to here the solve in fixed point (cell64's HOT) pays for its registers
+// (pfa_step2d.cu), us a step fixed / FP64: 32^3 17.9 / 21.7, 64^3 39.6 / 56, 96^3
+// 71 / 86, 128^3 123 / 132, 192^3 265 / 251, 256^3 503 / 465
+constexpr long long kHotPlanes = 65536;
+
 int g_resident3 = 0;  // resident CTAs of the FP32 kernel
 
 }  // namespace
@@ -573,10 +566,12 @@ cudaError_t launch_step3d(Step3DArgs a, bool f64, const Tma3* t, cudaStream_t s)
     const long long cols = (long long)((a.Nx + Tile3::TX - 1) / Tile3::TX) * ((a.Ny + Tile3::TY - 1) / Tile3::TY);
     a.zrows = segment_planes_f64(cols, a.Nz);
     const dim3 grid((unsigned)cols, (a.Nz + a.zrows - 1) / a.zrows);
+    const bool hot = cols * a.Nz <= kHotPlanes;
+    auto launch = [&](auto kernel) { kernel<<<grid, Tile3::kThreads, 0, s>>>(a); };
     if (a.c.mask == kMaskIso)
-      k_stream3d_f64<true><<<grid, Tile3::kThreads, 0, s>>>(a);
+      launch(hot ? k_stream3d_f64<true, true> : k_stream3d_f64<true, false>);
     else
-      k_stream3d_f64<false><<<grid, Tile3::kThreads, 0, s>>>(a);
+      launch(hot ? k_stream3d_f64<false, true> : k_stream3d_f64<false, false>);
   } else {
     if (!t) return cudaErrorInvalidValue;
     const int resident = g_resident3 > 0 ? g_resident3 : 152;

@@ -59,62 +59,129 @@ struct Tile {
 
 // One staged cell: its values and x^gamma.  phase: the tile must look at the
 // phases at all (an all-zero phase field stays zero: its Laplacian, p' and
-// well vanish; compositions that are not finite make 0 x NaN, see kBigHi)
+// well vanish; compositions that are not finite make 0 x NaN, see kBigHi).
+// g1, g2: x^gamma, the bits of its FP64 values or (FIXED, not wide) 2^58 times
+// it.
 struct Cell64 {
-  double X, Y, pd, pl, g1, g2;
-  size_t i;  // element of the fields
+  double X, Y, pd, pl;
+  long long g1, g2;
+  double v1, v2;  // !HOT: x^gamma in FP64
+  size_t i;       // element of the fields
   bool solved, phase, big;
-  bool unit;  // both compositions in [2^-11, 1)
+  bool wide;  // FIXED: outside the range of the fixed-point sums
 };
 
-// whole warp
-__device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double pl) {
+// a phase that solve_fixed takes: in [0, 1], or too small for p to count
+__device__ __forceinline__ bool fraction(double v) {
+  const unsigned hi = unsigned(__double2hiint(v));
+  return mag_hi(v) < kSolveHi || hi < 0x3ff00000u || (hi == 0x3ff00000u && __double2loint(v) == 0);
+}
+
+// x^gamma of a cell next to a precipitate; take: in the range of solve_fixed;
+// kinds: the forms of it that the warp needs; most: the bound of 2^60
+// |x^gamma| for the fixed-point sums (the neighbour sum has to stay below
+// 2^5), 0: FP64 values are wanted.  (A call: its registers would weigh on the
+// cells that need none.)
+struct Gamma64 {
+  long long g1, g2;
+  bool wide;
+};
+static __device__ __noinline__ Gamma64 gamma_cell(double X, double Y, double pd, double pl, bool take, int kinds,
+                                                  int64_t most) {
+  Gamma64 g;
+  int64_t h1, h2;
+  const uint64_t x = fix64(X) >> 1, y = fix64(Y) >> 1;
+  const uint64_t fd = mag_hi(pd) < kSolveHi ? 0 : fix63(pd), fl = mag_hi(pl) < kSolveHi ? 0 : fix63(pl);
+  if (take && (kinds == 3   ? solve_fixed<3>(x, y, fd, fl, h1, h2)
+               : kinds == 1 ? solve_fixed<1>(x, y, fd, fl, h1, h2)
+                            : solve_fixed<2>(x, y, fd, fl, h1, h2))) {
+    g.wide = max(llabs(h1), llabs(h2)) >= most;
+    g.g1 = g.wide ? __double_as_longlong(value60(h1)) : (h1 + 2) >> 2;
+    g.g2 = g.wide ? __double_as_longlong(value60(h2)) : (h2 + 2) >> 2;
+  } else {
+    double g1, g2;
+    gamma64(X, Y, pd, pl, g1, g2);
+    g.wide = true;
+    g.g1 = __double_as_longlong(g1);
+    g.g2 = __double_as_longlong(g2);
+  }
+  return g;
+}
+
+// whole warp.  FIXED: x^gamma for the fixed-point sums; HOT: the solve in fixed
+// point (else in FP64, inline: no call, so that a kernel with many waves of
+// tiles without precipitate keeps its occupancy)
+template <bool FIXED, bool HOT>
+__device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double pl, int64_t most) {
   Cell64 c;
   c.X = X;
   c.Y = Y;
   c.pd = pd;
   c.pl = pl;
-  c.g1 = X;
-  c.g2 = Y;
-  c.unit = in_unit(X) && in_unit(Y);
-  c.big = !c.unit && max(mag_hi(X), mag_hi(Y)) >= kBigHi;
+  const bool unit = in_unit(X) && in_unit(Y);
+  c.big = !unit && max(mag_hi(X), mag_hi(Y)) >= kBigHi;
   const int m = max(mag_hi(pd), mag_hi(pl));
   c.phase = (m | __double2loint(pd) | __double2loint(pl)) != 0 || c.big;
   c.solved = m >= kSolveHi || c.big;
-  solve64(c.solved, c.big, X, Y, pd, pl, c.g1, c.g2);
+  c.wide = !FIXED || !unit;
+  if constexpr (HOT) {
+    c.g1 = c.wide ? __double_as_longlong(X) : fix58(X);
+    c.g2 = c.wide ? __double_as_longlong(Y) : fix58(Y);
+    if (__any_sync(0xffffffffu, c.solved)) {
+      // next to a precipitate of one kind the other's fraction is below 10
+      // 2^-70 and zero in fixed point
+      const bool take = c.solved && unit && fraction(pd) && fraction(pl);
+      const int kinds = int(__any_sync(0xffffffffu, take && mag_hi(pd) >= kSolveHi)) +
+                        2 * int(__any_sync(0xffffffffu, take && mag_hi(pl) >= kSolveHi));
+      if (c.solved) {
+        const Gamma64 g = gamma_cell(X, Y, pd, pl, take, kinds, FIXED ? most : 0);
+        c.g1 = g.g1;
+        c.g2 = g.g2;
+        c.wide = g.wide;
+      }
+    }
+  } else {
+    double g1 = X, g2 = Y;
+    solve64(c.solved, c.big, X, Y, pd, pl, g1, g2);
+    c.v1 = g1;
+    c.v2 = g2;
+    const double bound = double(most) * 0x1p-60;
+    if (c.solved && max(mag_hi(g1), mag_hi(g2)) >= __double2hiint(bound)) c.wide = true;
+    if (c.wide) {
+      c.g1 = __double_as_longlong(g1);
+      c.g2 = __double_as_longlong(g2);
+    } else if (c.solved) {
+      c.g1 = fix58_signed(g1);
+      c.g2 = fix58_signed(g2);
+    } else {
+      c.g1 = fix58(X);
+      c.g2 = fix58(Y);
+    }
+  }
   return c;
 }
 
-// outside the fixed-point forms' range, with |x^gamma| bounded by the high
-// word `hi` (the neighbour sum has to stay below 2^5)
-__device__ __forceinline__ bool wide64(const Cell64& c, int hi) {
-  return !c.unit || (c.solved && max(mag_hi(c.g1), mag_hi(c.g2)) >= hi);
-}
-
-// x^gamma in fixed point (not wide)
-__device__ __forceinline__ void fix_cell(const Cell64& c, long long& f1, long long& f2) {
-  if (c.solved) {
-    f1 = fix58_signed(c.g1);
-    f2 = fix58_signed(c.g2);
-  } else {
-    f1 = fix58(c.X);
-    f2 = fix58(c.Y);
-  }
+// x^gamma in FP64 from g1, g2 of its cell
+__device__ __forceinline__ double2 gamma_values(const Cell64& c, long long g1, long long g2) {
+  if (c.wide) return make_double2(__longlong_as_double(g1), __longlong_as_double(g2));
+  return c.solved ? make_double2(value58(g1), value58(g2)) : make_double2(c.X, c.Y);
 }
 
 // the bits that are zero with a double (its sign aside)
 __device__ __forceinline__ int value_bits(double v) { return mag_hi(v) | __double2loint(v); }
 
 // Allen-Cahn of one phase of a cell.  none: the phase is zero at the cell and
-// its neighbours, and stays so; lap() forms its Laplacian.
-template <int I, class Lap>
-__device__ __forceinline__ double phase64(const Coef64& K, const Cell64& c, bool none, Lap lap) {
+// its neighbours, and stays so; lap() forms its Laplacian, gamma() its
+// x^gamma.
+template <int I, class Lap, class Gam>
+__device__ __forceinline__ double phase64(const Coef64& K, const Cell64& c, bool none, Lap lap, Gam gamma) {
   if (none && !c.big) return 0.0;
   const double ph = I == 0 ? c.pd : c.pl, pj = I == 0 ? c.pl : c.pd;
   if (mag_hi(ph) < kLinearHi && mag_hi(pj) < kLoneHi && !c.big)
     return allen_cahn_linear64<I>(K, ph, lap());
   constexpr double x1 = kXe[0][0], x2 = kXe[0][1];
-  return allen_cahn64<I>(K, ph, pj, ph * pj, lap(), c.g1 - x1, c.g2 - x2);
+  const double2 g = gamma();
+  return allen_cahn64<I>(K, ph, pj, ph * pj, lap(), g.x - x1, g.y - x2);
 }
 
 }  // namespace

@@ -81,6 +81,48 @@ def test_forms_varmob(pfa, orc, nx, ny):
     check_cells(got, orc.run2d_varmob(f, O.model_params(), 1), 350 * 16 * 2.0 ** -53)
 
 
+# cells that the fixed-point gamma solve takes beside cells it refuses (a phase
+# below 0 or above 1, fractions that add up to more than 1, compositions out of
+# range, |x^gamma| of 2 and more), in the sizes that take it (2D up to 12288
+# tiles of 8 x 8, 3D up to 65536 planes of tiles)
+@pytest.mark.parametrize("mask", ["iso", "nine", "five", "variable", "3d"])
+def test_solve_out_of_range(pfa, orc, mask):
+    shape = (9, 40, 37) if mask == "3d" else (210, 190)
+    rng = np.random.default_rng(7)
+    kind = rng.integers(0, 7, shape)
+    x, y = rng.uniform(0.28, 0.33, shape), rng.uniform(0.02, 0.17, shape)
+    d, l = np.zeros(shape), np.zeros(shape)
+    near = kind >= 4  # the precipitates' compositions in half of their cells
+    x[near & (kind < 6)], y[near & (kind < 6)] = 0.03, 0.247
+    d[kind == 1], l[kind == 1] = 1.0, 0.0
+    d[kind == 2], l[kind == 2] = 1.0, 0.05
+    d[kind == 3] = -1e-3
+    d[kind == 4] = 1.0
+    d[kind == 5], l[kind == 5] = 0.5, 1e-9
+    l[kind == 6] = rng.choice([1.0 + 1e-12, 0.4, 1.0], shape)[kind == 6]
+    y[kind == 6] = rng.choice([1e-5, 0.2], shape)[kind == 6]
+    f = []
+    for a in (x, y, d, l):
+        h = np.empty([n + 2 for n in shape])
+        h[(slice(1, -1),) * len(shape)] = a
+        f.append(ic.mirror_halo(h))
+    p = pfa.model_params(dim=len(shape))
+    q = O.model_params(dim=len(shape))
+    if mask == "3d":
+        g, want = pfa.Grid3D(f, p), orc.run3d(f, q, 1)
+    elif mask == "variable":
+        g, want = pfa.Grid2D(f, p, mobility="variable"), orc.run2d_varmob(f, q, 1)
+    else:
+        q.dy = p["dx"] * (1.25 if mask == "five" else 1.0)
+        m = (pfa.nine_point_mask if mask == "nine" else pfa.five_point_mask)(p["dx"], q.dy)
+        g = pfa.Grid2D(f, dict(p, dy=q.dy), mask=m)
+        want = orc.run2d(f, q.with_mask(m) if mask == "nine" else q, 1)
+    g.run(1)
+    got = g.read()
+    g.close()
+    check_cells(got, want, 350 * 16 * 2.0 ** -53)
+
+
 # compositions inside and outside the range of the integer mobilities: Nb below
 # 2^-11, Cr and Nb adding up to more than 1, both edges, in one grid and mixed
 # within a warp
