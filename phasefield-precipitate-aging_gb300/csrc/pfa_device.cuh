@@ -326,16 +326,20 @@ static __device__ __noinline__ double advance64(double X, long long inc) {
   return X + double(inc) * 0x1p-64;
 }
 
-// X + D0 S1 + D1 S2, X in [2^-11, 1), S in units of 2^-58, D of 2^-70
-__device__ __forceinline__ double advance58(double X, long long D0, long long S1, long long D1,
-                                            long long S2) {
-  // + 1: the two high halves are rounded down
-  const long long inc = __mul64hi(D0, S1) + __mul64hi(D1, S2) + 1;
+// X + inc 2^-64, X in [2^-11, 1)
+__device__ __forceinline__ double advance_by(double X, long long inc) {
   const int s = (__double2hiint(X) >> 20) - 1011;  // X's last place is 2^(s - 64)
   const long long old = __double_as_longlong(X);
   const long long sum = old + ((inc + (1ll << (s - 1))) >> s);
   if (((unsigned long long)(old ^ sum) >> 52) == 0) return __longlong_as_double(sum);
   return advance64(X, inc);
+}
+
+// X + D0 S1 + D1 S2, S in units of 2^-58, D of 2^-70
+__device__ __forceinline__ double advance58(double X, long long D0, long long S1, long long D1,
+                                            long long S2) {
+  // + 1: the two high halves are rounded down
+  return advance_by(X, __mul64hi(D0, S1) + __mul64hi(D1, S2) + 1);
 }
 
 // v 2^64, v in [2^-11, 1) (exact)
@@ -379,9 +383,9 @@ __device__ __forceinline__ void dmatrix64_scaled(const Coef64& K, double X, doub
   double e[3];
   const uint64_t x = fix64(X), y = fix64(Y);
   if (unit && K.vm_fixed && uint64_t(x + y) > x) {  // x_Ni > 0
-    uint64_t b[3];
-    mobilities(K, x, y, b);
-    for (int k = 0; k < 3; k++) e[k] = __longlong_as_double((long long)b[k]);
+    Mobility v[3];
+    mobilities(K, x, y, v);
+    for (int k = 0; k < 3; k++) e[k] = __longlong_as_double((long long)mobility_bits(v[k]));
   } else {
     mobilities64(K, X, Y, e);
   }

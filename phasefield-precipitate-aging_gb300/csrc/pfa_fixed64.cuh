@@ -2,7 +2,7 @@
 //
 // An FP64 operation takes an SM 19 cycles per warp, the high half of a 64 x 64
 // bit product about three.  So for compositions in [2^-11, 1) and phase fields
-// in [0, 1] two parts of a cell are formed in fixed point (every other cell
+// in [0, 1] these parts of a cell are formed in fixed point (every other cell
 // takes the FP64 expressions):
 //   solve_fixed: x^gamma of a cell with precipitate, 30 to 56 FP64 operations.
 //     Error over the simplex (against 113 bits, units of 2^-53): at most 26,
@@ -11,6 +11,9 @@
 //   mobilities: the weighted mobilities of the variable-mobility step, 59
 //     operations with their three exponentials.  Error at most 1.6 (FP64: up
 //     to 30 and, near x_Ni = 0, 4e4); 512^2 73.9 -> 38.9 us a step.
+//   diffusivities: the matrix of that step, 26 operations.  Error in the usual
+//     range of compositions, units of 2^-60: at most 0.9, 0.06 on average (FP64:
+//     18 and 0.9); with the fluxes 512^2 38.9 -> 20.8 us a step.
 // Compiles as host code too.
 #pragma once
 
@@ -121,33 +124,77 @@ PFA_FIX_FN uint64_t pack64(uint64_t m, int e) {
 }
 
 // Weighted mobilities (e_Nb, e_Cr, e_Ni x_Ni of dmatrix64, times the
-// prefactors pm 2^(pe - 63)) as FP64 bits.  x, y: the compositions times 2^64,
-// 2^53 or more, x + y < 2^64.
-PFA_FIX_FN void mobilities(const Coef64& K, uint64_t x, uint64_t y, uint64_t e[3]) {
+// prefactors vm_pre): m 2^(e - 63), 2^63 <= m.  x, y: the compositions times
+// 2^64, 2^53 or more, x + y < 2^64.
+struct Mobility {
+  uint64_t m;
+  int e;
+};
+PFA_FIX_FN void mobilities(const Coef64& K, uint64_t x, uint64_t y, Mobility v[3]) {
   const uint64_t n = 0 - (x + y);  // x_Ni
-  auto weighted = [&](int64_t z, int q, int k, uint64_t w) {  // pre 2^(z 2^-q) w
-    const uint64_t m = mul_hi(exp2_mantissa(uint64_t(z) << (64 - q)), K.vm_m[k]);  // >= 2^62
-    const int lead = w ? lead_zeros(w) : 0;
-    const int ex = int(z >> q) + K.vm_e[k] + 1;
-    if (!w) return pack64(m, ex);
-    const uint64_t p = mul_hi(m << (m >> 63 ? 0 : 1), w << lead);
-    return pack64(p, ex - (m >> 63 ? 0 : 1) - lead);
+  auto normal = [](uint64_t m, int e) {  // m 2^(e - 62), 2^62 <= m
+    const int up = m >> 63 ? 0 : 1;
+    return Mobility{m << up, e + 1 - up};
+  };
+  auto weighted = [&](int64_t z, int q, int k) {  // vm_pre 2^(z 2^-q)
+    return normal(mul_hi(exp2_mantissa(uint64_t(z) << (64 - q)), K.vm_m[k]), int(z >> q) + K.vm_e[k]);
   };
   // exponents times log2(e): 2^-57, 2^-59, 2^-54
   const int64_t zn = mul_hi_su(0x29a8bb8820a29949ll - int64_t(mul_hi(0x64f0372c225e9378ull, n)), y);
   const int64_t zc = mul_hi_su(0x26b6712afedfd131ll - int64_t(mul_hi(0x529296d39d336238ull, n)), x);
   const int64_t zi = (mul_hi_su(0x2e3564d412fda0f2ll - int64_t(mul_hi(0x625bca3fd59b5547ull, n)), x) >> 5) -
                      int64_t(mul_hi(0x004bdd4343eff6b2ull + mul_hi(0x9fa5039d40b0facaull, n), y));
-  e[0] = weighted(zn, 57, 0, 0);
-  e[1] = weighted(zc, 59, 1, 0);
-  e[2] = weighted(zi, 54, 2, n);
+  v[0] = weighted(zn, 57, 0);
+  v[1] = weighted(zc, 59, 1);
+  const Mobility i = weighted(zi, 54, 2);
+  const int lead = lead_zeros(n);
+  v[2] = normal(mul_hi(i.m, n << lead), i.e - lead - 1);
+}
+
+// FP64 bits of a mobility
+PFA_FIX_FN uint64_t mobility_bits(const Mobility& v) { return pack64(v.m, v.e); }
+
+// ---- diffusivities ----
+PFA_FIX_FN constexpr uint64_t coef64(double c) { return uint64_t((c < 0 ? -c : c) * 0x1p64); }
+
+// D_CrCr, D_CrNb, D_NbCr, D_NbNb of dmatrix64_scaled times 2^67 (false: one of
+// them is 2^-5 or more).  The curvature weights are scaled by 2^-21 (to below
+// 1), the mobilities by the power of two that brings the largest to [1/16,
+// 1/8), so that no sum exceeds 1/2.
+PFA_FIX_FN bool diffusivities(const Coef64& K, uint64_t x, uint64_t y, long long d[4]) {
+  Mobility v[3];
+  mobilities(K, x, y, v);
+  const int top = v[0].e > v[1].e ? (v[0].e > v[2].e ? v[0].e : v[2].e) : (v[1].e > v[2].e ? v[1].e : v[2].e);
+  uint64_t e[3];  // 2^64 2^-(top + 4) times the mobilities
+  for (int k = 0; k < 3; k++) {
+    const int down = 3 + top - v[k].e;
+    e[k] = down < 64 ? v[k].m >> down : 0;
+  }
+  constexpr double q = 0x1p-21;
+  auto column = [&](uint64_t hx, uint64_t hy, uint64_t hn, uint64_t hc, long long& dc, long long& dn) {
+    const int64_t s = -int64_t((mul_hi(hx, x) + mul_hi(hy, y)) >> 1);  // 2^63, as all below
+    const int64_t A = mul_hi_su(s + int64_t(hn >> 1), e[0]), B = mul_hi_su(s + int64_t(hc >> 1), e[1]);
+    const int64_t W = mul_hi_su(B, x) + mul_hi_su(A, y) + mul_hi_su(s, e[2]);
+    dc = mul_hi_su((B - W) << 1, x);
+    dn = mul_hi_su((A - W) << 1, y);
+  };
+  column(coef64(kHCrCr * q), coef64(kHCrNb * q), coef64(kHCrNbAddA * q), coef64(kHCrCrAdd * q), d[0], d[2]);
+  column(coef64(kHCrNb * q), coef64(kHNbNb * q), coef64(kHNbNbAdd * q), coef64(kHCrNbAddB * q), d[1], d[3]);
+  const int up = top + 4 + 21 + 3;  // from 2^64 2^-(top + 25) to 2^67
+  if (up < -60 || up > 60) return false;
+  const uint64_t bound = up > 0 ? 1ull << 62 >> up : 1ull << 62;
+  bool ok = true;
+  for (int k = 0; k < 4; k++) {
+    ok = ok && uint64_t(d[k]) + bound < 2 * bound;
+    d[k] = up > 0 ? (long long)(uint64_t(d[k]) << up) : d[k] >> -up;
+  }
+  return ok;
 }
 
 // ---- x^gamma ----
 // All numbers are unsigned multiples of 2^-63 (1 is 2^63); signs are those of
 // the coefficients (kFict, kDen), known at compile time.
 constexpr uint64_t kOne63 = 1ull << 63;
-PFA_FIX_FN constexpr uint64_t coef64(double c) { return uint64_t((c < 0 ? -c : c) * 0x1p64); }
 
 PFA_FIX_FN uint64_t mul63(uint64_t a, uint64_t b) { return mul_hi(a, b) << 1; }
 PFA_FIX_FN uint64_t by(uint64_t coef, uint64_t v) { return mul_hi(coef, v); }

@@ -218,30 +218,84 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
 // exponentials), each face's flux is formed once: a thread forms its east and
 // lower faces, the halo warps the west faces of the first column and the
 // upper faces of the first row.
+//
+// ISO (equal spacings): all of it in fixed point where every cell of the tile
+// is in range: u in units of 2^-58, D of 2^-67 (pfa_fixed64.cuh), the fluxes of
+// 2^-65, whose differences are rounded once into the compositions; else, and
+// with other spacings, in FP64.  Bound by integer issue; with the matrix and
+// the fluxes in FP64, bound by that pipe, 512^2 took 38.9 us a step for 20.8,
+// 2048^2 521 for 237.
+struct Matrix64 {
+  double d[4];
+};
+static __device__ __noinline__ Matrix64 matrix64(const Coef64& K, double X, double Y, bool unit) {
+  Matrix64 m;
+  dmatrix64_scaled(K, X, Y, unit, m.d[0], m.d[1], m.d[2], m.d[3]);
+  return m;
+}
+
 template <bool ISO, int TX, int TY>
-__global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, 768 / Tile<TX, TY, false>::kThreads)
+__global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, TX == 16 ? 3 : 8)
     k_step2d_f64_varmob(const __grid_constant__ Step2DArgs a) {
   using T = Tile<TX, TY, false>;
-  __shared__ typename T::template Plane<double> s_g1, s_g2, s_pd, s_pl, s_d[4];
-  __shared__ double s_fx[2][TY][TX + 1], s_fy[2][TY + 1][TX];
+  // fixed point, or the bits of FP64 values
+  __shared__ typename T::template Plane<long long> s_g1, s_g2, s_d[4];
+  __shared__ typename T::template Plane<double> s_pd, s_pl;
+  __shared__ long long s_fx[2][TY][TX + 1], s_fy[2][TY + 1][TX];
+  const Coef64& K = a.c;
   int ex, ey;
   const bool staged = T::cell(ex, ey);
   const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
-  const Cell64 c = stage64<false, true>(a, gx, gy, 0);
+  const Cell64 c = stage64<ISO, true>(a, gx, gy, 1ll << 60);
+  const bool unit = in_unit(c.X) && in_unit(c.Y);
+  bool wide = true;
+  long long d[4];
+  if constexpr (ISO) {
+    const uint64_t x = fix64(c.X), y = fix64(c.Y);
+    wide = c.wide || !K.vm_fixed || uint64_t(x + y) <= x || !diffusivities(K, x, y, d);
+  }
+  auto stage_matrix = [&] {
+    const Matrix64 m = matrix64(K, c.X, c.Y, unit);
+#pragma unroll
+    for (int k = 0; k < 4; k++) s_d[k][ey][ex] = __double_as_longlong(m.d[k]);
+  };
   if (staged) {
-    s_g1[ey][ex] = __longlong_as_double(c.g1);
-    s_g2[ey][ex] = __longlong_as_double(c.g2);
+    s_g1[ey][ex] = c.g1;
+    s_g2[ey][ex] = c.g2;
     s_pd[ey][ex] = c.pd;
     s_pl[ey][ex] = c.pl;
-    dmatrix64_scaled(a.c, c.X, c.Y, in_unit(c.X) && in_unit(c.Y), s_d[0][ey][ex], s_d[1][ey][ex], s_d[2][ey][ex],
-                     s_d[3][ey][ex]);
+    if (wide) {
+      stage_matrix();
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) s_d[k][ey][ex] = d[k];
+    }
   }
   const bool phases = __syncthreads_or(c.phase);
+  const bool fixed = ISO && !__syncthreads_or(wide);
+  if (ISO && !fixed) {  // the whole tile in FP64
+    if (staged && !c.wide) {
+      const double2 g = gamma_values(c, c.g1, c.g2);
+      s_g1[ey][ex] = __double_as_longlong(g.x);
+      s_g2[ey][ex] = __double_as_longlong(g.y);
+    }
+    if (staged && !wide) stage_matrix();
+    __syncthreads();
+  }
   // flux into (ex, ey) from (nx, ny): component k is (D_n + D_c)_k . (u_n - u_c)
-  auto flux = [&](int x, int y, int nx, int ny, double& f1, double& f2) {
-    const double u1 = s_g1[ny][nx] - s_g1[y][x], u2 = s_g2[ny][nx] - s_g2[y][x];
-    f1 = fma(s_d[0][ny][nx] + s_d[0][y][x], u1, (s_d[1][ny][nx] + s_d[1][y][x]) * u2);
-    f2 = fma(s_d[2][ny][nx] + s_d[2][y][x], u1, (s_d[3][ny][nx] + s_d[3][y][x]) * u2);
+  auto flux = [&](int x, int y, int nx, int ny, long long& f1, long long& f2) {
+    if (fixed) {
+      const long long u1 = (s_g1[ny][nx] - s_g1[y][x]) << 4, u2 = (s_g2[ny][nx] - s_g2[y][x]) << 4;
+      f1 = __mul64hi(s_d[0][ny][nx] + s_d[0][y][x], u1) + __mul64hi(s_d[1][ny][nx] + s_d[1][y][x], u2);
+      f2 = __mul64hi(s_d[2][ny][nx] + s_d[2][y][x], u1) + __mul64hi(s_d[3][ny][nx] + s_d[3][y][x], u2);
+    } else {
+      auto v = [](const long long (*s)[T::kPitch], int y, int x) { return __longlong_as_double(s[y][x]); };
+      const double u1 = v(s_g1, ny, nx) - v(s_g1, y, x), u2 = v(s_g2, ny, nx) - v(s_g2, y, x);
+      const double m0 = v(s_d[0], ny, nx) + v(s_d[0], y, x), m1 = v(s_d[1], ny, nx) + v(s_d[1], y, x);
+      const double m2 = v(s_d[2], ny, nx) + v(s_d[2], y, x), m3 = v(s_d[3], ny, nx) + v(s_d[3], y, x);
+      f1 = __double_as_longlong(fma(m0, u1, m1 * u2));
+      f2 = __double_as_longlong(fma(m2, u1, m3 * u2));
+    }
   };
   const bool own = threadIdx.x < T::kOwn;
   if (own) {
@@ -254,15 +308,20 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, 768 / Tile<TX, 
   }
   __syncthreads();
   if (!own || gx >= a.Nx || gy >= a.Ny) return;
-  const Coef64& K = a.c;
   const int tx = ex - 1, ty = ey - 1;
-  const double ocr = c.X + fma(K.vm_qy, s_fy[0][ty + 1][tx] - s_fy[0][ty][tx],
-                               s_fx[0][ty][tx + 1] - s_fx[0][ty][tx]);
-  const double onb = c.Y + fma(K.vm_qy, s_fy[1][ty + 1][tx] - s_fy[1][ty][tx],
-                               s_fx[1][ty][tx + 1] - s_fx[1][ty][tx]);
+  auto sum = [&](int k, double X) {  // the faces' fluxes added to a composition
+    const long long n = s_fy[k][ty + 1][tx], s = s_fy[k][ty][tx], e = s_fx[k][ty][tx + 1], w = s_fx[k][ty][tx];
+    if (fixed) return advance_by(X, ((n - s) + (e - w) + 1) >> 1);
+    return X + fma(K.vm_qy, __longlong_as_double(n) - __longlong_as_double(s),
+                   __longlong_as_double(e) - __longlong_as_double(w));
+  };
+  const double ocr = sum(0, c.X), onb = sum(1, c.Y);
   double od = 0.0, ol = 0.0;
   if (phases) {
-    auto gamma = [&] { return make_double2(s_g1[ey][ex], s_g2[ey][ex]); };
+    auto gamma = [&] {
+      if (fixed) return gamma_values(c, c.g1, c.g2);
+      return make_double2(__longlong_as_double(s_g1[ey][ex]), __longlong_as_double(s_g2[ey][ex]));
+    };
     update_phases<ISO ? kMaskIso : kMaskFive>(a, c, s_pd, s_pl, ex, ey, gamma, od, ol);
   }
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
@@ -320,10 +379,10 @@ cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s) {
     return tiles<8, 8>(a) <= kHotTiles ? launch_tiles<8, 8, false, true>(a, s) : launch_tiles<8, 8, false, false>(a, s);
   }
   // every staged cell has its mobilities, so large grids take the tile with
-  // the smallest share of halo: 8 x 8 / 16 x 16 (before their exponentials
-  // were integers) 192^2 17.1 / 17.2, 256^2 27.7 / 29.2, 320^2 39.0 / 35.8,
-  // 512^2 86 / 74, 2048^2 1266 / 1050
-  return tiles<16, 16>(a) < 304 ? launch_tiles<8, 8, true, true>(a, s) : launch_tiles<16, 16, true, true>(a, s);
+  // the smallest share of halo: 8 x 8 / 16 x 16 64 x 48 6.5 / 9.9, 192^2 7.7 /
+  // 9.6, 320^2 11.2 / 12.5, 384^2 13.8 / 13.1, 512^2 21.5 / 20.8, 2048^2 279 /
+  // 237 (16 x 8: 271; 16 x 16 at two and four CTAs per SM: 272 and 243)
+  return tiles<16, 16>(a) < 576 ? launch_tiles<8, 8, true, true>(a, s) : launch_tiles<16, 16, true, true>(a, s);
 }
 
 }  // namespace pfa

@@ -70,8 +70,8 @@ def test_forms_2d(pfa, orc, nx, ny, mask):
     check_cells(got, want, 350 * 16 * 2.0 ** -53)
 
 
-# tiles of 8 x 8 and (from 304 of them) 16 x 16 cells
-@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 130), (40, 700), (330, 250)])
+# tiles of 8 x 8 and (from 576 of them) 16 x 16 cells
+@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 130), (40, 700), (330, 250), (401, 380)])
 def test_forms_varmob(pfa, orc, nx, ny):
     f = mixed_fields((ny, nx), nx + ny)
     g = pfa.Grid2D(f, pfa.model_params(), mobility="variable")
@@ -126,7 +126,7 @@ def test_solve_out_of_range(pfa, orc, mask):
 # compositions inside and outside the range of the integer mobilities: Nb below
 # 2^-11, Cr and Nb adding up to more than 1, both edges, in one grid and mixed
 # within a warp
-@pytest.mark.parametrize("nx,ny", [(37, 21), (330, 250)])
+@pytest.mark.parametrize("nx,ny", [(37, 21), (330, 250), (401, 380)])
 def test_mobilities_out_of_range(pfa, orc, nx, ny):
     rng = np.random.default_rng(nx)
     kind = rng.integers(0, 5, (ny, nx))
