@@ -731,8 +731,10 @@ static int read_core(CudaData* dev, double* cr, double* nb, double* pd, double* 
     if (int r = ensure_xfer(s)) return r;
     // at least two rows per band: the first band then holds the bottom ghost
     // row together with the interior row that writes it
-    const int rows = std::max(2, (ny + kXferBands - 1) / kXferBands);
-    for (int i = 0; i < kXferBands; i++) {
+    const size_t cells = size_t(nx) * ny;
+    const int bands = int(std::min<size_t>(std::max<size_t>(cells >> 20, 1), kXferBands));
+    const int rows = std::max(2, (ny + bands - 1) / bands);
+    for (int i = 0; i < bands; i++) {
       const int r0 = i * rows, r1 = r0 + rows < ny ? r0 + rows : ny;
       if (r0 >= r1) break;
       ConvArgs c = conv_args(dev, s);

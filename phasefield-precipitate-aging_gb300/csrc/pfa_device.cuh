@@ -574,7 +574,12 @@ __device__ __forceinline__ float dF_local32(float ph, float pj, float dP, float 
 // = -rem 2^(E-1075) is exact with |rem| <= 2^28, so rounding -rem to FP32
 // and scaling by the power of two gives the FP64 expression's result
 // bit-for-bit; zeros take hi = v, c = +0; every other double takes the FP64
-// expression itself.
+// expression itself, in a call (inlined, it was issued for every cell: 256^3
+// import 255 us, 196 so).
+static __device__ __noinline__ float2 split_call(double v) {
+  const float hi = float(v);
+  return make_float2(hi, float(double(hi) - v));
+}
 __device__ __forceinline__ void split_f64(double v, float& hi, float& c) {
   const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
   const int E = int((b >> 52) & 0x7ff);
@@ -585,8 +590,9 @@ __device__ __forceinline__ void split_f64(double v, float& hi, float& c) {
     return;
   }
   if (E < 950 || E > 1149) {
-    hi = float(v);
-    c = float(double(hi) - v);
+    const float2 r = split_call(v);
+    hi = r.x;
+    c = r.y;
     return;
   }
   const unsigned long long M = (b & 0xfffffffffffffull) | (1ull << 52);
@@ -602,6 +608,31 @@ __device__ __forceinline__ void split_f64(double v, float& hi, float& c) {
   // c = hi - v = -rem 2^(E-1075) for v > 0, +rem 2^(E-1075) for v < 0
   // (rem = 0 gives +0, as the FP64 subtraction does)
   c = __int2float_rn(sign ? rem : -rem) * scale;
+}
+
+// (a call, like advance64)
+static __device__ __noinline__ double merge_call(float v, float c) { return double(v) - double(c); }
+
+// double(v) - n 2^-(52 - up): the value of a packed record's field, n its
+// compensation's 16-bit count (up: 12 compositions, 13 phases).  For v = +0 and 2^-29 <= |v| < 2 both are
+// whole multiples of 2^-52 and the difference is below 2^53 of them, so the
+// integer difference is the FP64 one bit-for-bit; other v take FP64 (whose
+// three operations per field bound the export kernels: 256^3 411 us, 190 with
+// these; HBM's share is 140).
+__device__ __forceinline__ double merge_f64(float v, int n, int up) {
+  const unsigned b = __float_as_uint(v), E = (b >> 23) & 0xffu;
+  if (b != 0u && (E < 98u || E > 127u)) return merge_call(v, float(n) * (up == 12 ? kCqXi : kCqPi));
+  const int64_t m = int64_t((b & 0x7fffffu) | 0x800000u) << (E < 98u ? 0u : E - 98u);
+  const int64_t h = b == 0u ? 0 : (b >> 31 ? -m : m);
+  return __longlong_as_double((long long)pack_signed(h - (int64_t(n) << up), 52));
+}
+
+// the four fields of a packed record
+__device__ __forceinline__ void merge_record(float4 v, uint2 w, double out[4]) {
+  out[0] = merge_f64(v.x, short(w.x & 0xffffu), 12);
+  out[1] = merge_f64(v.y, short(w.x >> 16), 12);
+  out[2] = merge_f64(v.z, short(w.y & 0xffffu), 13);
+  out[3] = merge_f64(v.w, short(w.y >> 16), 13);
 }
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw: "Parallel random numbers: as

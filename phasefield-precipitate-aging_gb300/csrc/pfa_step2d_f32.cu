@@ -647,10 +647,16 @@ __global__ void k_export_records(ConvArgs a) {
   if (gx >= a.Nx || gy >= (a.y1 > 0 ? a.y1 : a.Ny)) return;
   const size_t r = size_t(gy) * a.pitch32 + gx;
   const float4 v = reinterpret_cast<const float4*>(a.A)[r];
-  const float4 c = a.pack ? cq_unpack(static_cast<const uint2*>(a.B)[r])
-                          : static_cast<const float4*>(a.B)[r];
-  const double val[4] = {double(v.x) - double(c.x), double(v.y) - double(c.y),
-                         double(v.z) - double(c.z), double(v.w) - double(c.w)};
+  double val[4];
+  if (a.pack) {
+    merge_record(v, static_cast<const uint2*>(a.B)[r], val);
+  } else {
+    const float4 c = static_cast<const float4*>(a.B)[r];
+    val[0] = double(v.x) - double(c.x);
+    val[1] = double(v.y) - double(c.y);
+    val[2] = double(v.z) - double(c.z);
+    val[3] = double(v.w) - double(c.w);
+  }
   const size_t row = size_t(gy + 1) * a.pitch64;
 #pragma unroll
   for (int k = 0; k < 4; k++) {

@@ -56,6 +56,41 @@ def test_tall_grids(pfa, precision, nx, ny):
         assert np.array_equal(b[5:65, 1:-1], c[ny - 59:ny + 1, 1:-1])
 
 
+@pytest.mark.parametrize("dim", [2, 3])
+def test_record_conversions(pfa, dim):
+    """Upload and read back without a step: FP32 value and 16-bit count of each
+    field, recombined exactly, for every range of the conversions."""
+    shape = (90, 71) if dim == 2 else (9, 21, 35)
+    rng = np.random.default_rng(dim)
+    f, want = [], []
+    for k in range(4):
+        v = 10.0 ** rng.uniform(-46, 1, shape) * rng.choice([-1.0, 1.0], shape)
+        edge = rng.choice([0.0, -0.0, 2.0 ** -29, 2.0 ** -29 * (1 - 2.0 ** -24), 1.0, 2.0, 2.0 * (1 - 2.0 ** -24),
+                           2.0 - 2.0 ** -26, 2.0 ** -75, 1e-40, 1e300], shape)
+        v = np.where(rng.random(shape) < 0.5, edge, v)
+        if k < 2:
+            v = np.where(rng.random(shape) < 0.5, rng.uniform(0.01, 0.6, shape), v)
+        h = np.empty([n + 2 for n in shape])
+        h[(slice(1, -1),) * dim] = v
+        f.append(ic.mirror_halo(h))
+        with np.errstate(over="ignore", under="ignore", invalid="ignore"):
+            hi = f[-1].astype(np.float32)
+            c = (hi.astype(np.float64) - f[-1]).astype(np.float32)
+            unit = 2.0 ** (40 if k < 2 else 39)
+            n = np.clip(np.rint(c.astype(np.float64) * unit), -32768, 32767)
+            want.append(hi.astype(np.float64) - n / unit)
+    g = (pfa.Grid2D if dim == 2 else pfa.Grid3D)(f, pfa.model_params(dim=dim), precision="fp32")
+    g.upload(f)
+    if dim == 3:  # (the FP64 fields stay in place until a step or a read of the records converts them)
+        raw = np.empty(int(g.L.pfa3d_f32_state_bytes(g.h)), dtype=np.uint8)
+        assert g.L.pfa3d_read_f32_state(g.h, raw.ctypes.data, raw.size) == 0
+    got = g.read()
+    g.close()
+    core = (slice(1, -1),) * dim
+    for a, b in zip(got, want):
+        assert np.array_equal(a[core], b[core])
+
+
 # strips of 28 and 30 columns (double and single passes) put the same cells in
 # different warps: tails that cross the bulk threshold of the gamma solve
 # everywhere must not notice
