@@ -1279,7 +1279,6 @@ int pfa_summarize(struct CudaData* dev, double* out) {
     for (int k = 0; k < 4; k++) a.f[k] = s->recA[s->cur] + k;
     a.comp = s->recB[s->cur];
     a.pack = s->precision == PFA_FP32;
-    a.stride = 4;
     a.is_f32 = 1;
     a.compact = 1;
     a.pitch = s->pitch32;
@@ -1290,7 +1289,6 @@ int pfa_summarize(struct CudaData* dev, double* out) {
     a.f[3] = dev->phi_lav_old;
     a.pitch = s->nx;
   }
-  if (a.stride == 0) a.stride = 1;
   a.Nx = s->Nx;
   a.Ny = s->Ny;
   a.Nz = 1;

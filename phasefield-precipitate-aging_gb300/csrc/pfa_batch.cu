@@ -748,7 +748,6 @@ int pfa_batch_summarize(void* handle, int slot, double* out) {
   for (int k = 0; k < 4; k++) a.f[k] = A + k;
   a.comp = g.B[b->cur];
   a.pack = 1;
-  a.stride = 4;
   a.is_f32 = 1;
   a.compact = 1;
   a.pitch = s->pitch;

@@ -12,6 +12,7 @@
 // fixed order and one block adds the partials, so the total is reproducible.
 #include "pfa_device.cuh"
 #include "pfa_reduce.h"
+#include "pfa_rows.cuh"
 
 namespace pfa {
 
@@ -19,65 +20,103 @@ using namespace dev;
 
 namespace {
 
-constexpr int kThreads = 256;
+// A phase below 2^-600 adds nothing: its square is below the least double.
+constexpr int kNoneHi = (1023 - 600) << 20;
 
-__global__ void __launch_bounds__(kThreads) k_energy_partial(EnergyArgs a) {
-  const size_t nx = size_t(a.Nx) + 2, ny = size_t(a.Ny) + 2;
-  const size_t plane = nx * ny;
-  const size_t cells = size_t(a.Nx) * a.Ny * (a.is3d ? a.Nz : 1);
+// omega phi^2 (1 - phi)^2
+__device__ __forceinline__ double well64(double omega, double ph, double sq) {
+  const double u = 1.0 - ph;
+  return omega * sq * (u * u);
+}
+
+// Chemical energy density of a phase PH (1 delta, 2 laves) below 1e-7 beside
+// gamma: p g_PH at the composition PH has in pure gamma (p shifts it by less
+// than half an ulp), where p counts, and the well
+template <int PH>
+__device__ __forceinline__ double trace64(double X, double Y, double omega, double ph) {
+  double g = well64(omega, ph, ph * ph);
+  if (mag_hi(ph) >= kLinearHi) {
+    constexpr FictRow r = kFict[PH][0], q = kFict[PH][1];
+    const double x = r.scale * fma(r.l[1], X, fma(r.m[1], Y, r.q[3]));
+    const double y = q.scale * fma(q.l[1], X, fma(q.m[1], Y, q.q[3]));
+    g = fma(p64(ph), g64<PH>(x, y), g);
+  }
+  return g;
+}
+
+// The FP64 pipe bounds the pass (19 cycles per warp instruction and SM), so a
+// cell takes the cheapest form of the same value: 9 operations where both
+// phases vanish around it (x^gamma is the composition itself), about 20 more
+// per phase in its tails (below 1e-7), about 150 next to a precipitate.
+// 1024^2: 423 us with the general form and 64-bit divisions everywhere, 61
+// with these; 256^2 33 -> 20.
+__global__ void __launch_bounds__(kSumThreads, 2) k_energy_partial(EnergyArgs a) {
+  const int lane = threadIdx.x & 31;
+  const size_t nx = size_t(a.Nx) + 2, plane = nx * (size_t(a.Ny) + 2);
   const double dV = a.dxyz[0] * a.dxyz[1] * (a.is3d ? a.dxyz[2] : 1.0);
   const double w[3] = {1.0 / (2.0 * a.dxyz[0]), 1.0 / (2.0 * a.dxyz[1]),
                        1.0 / (2.0 * a.dxyz[2])};
   double acc = 0.0;
-  for (size_t c = size_t(blockIdx.x) * kThreads + threadIdx.x; c < cells;
-       c += size_t(gridDim.x) * kThreads) {
-    const size_t x = c % a.Nx + 1;
-    const size_t rest = c / a.Nx;
-    const size_t y = rest % a.Ny + 1;
-    const size_t z = a.is3d ? rest / a.Ny + 1 : 0;
-    const size_t i = z * plane + y * nx + x;
+  RowWalk it(a.Nx, a.Ny, a.is3d ? a.Nz : 1, (threadIdx.x >> 5) * kSumBlocks + blockIdx.x,
+             kSumBlocks * (kSumThreads / 32));
+  for (; it.more(); it.next()) {
+    const int x = int(it.c) * 32 + lane;
+    if (x >= a.Nx) continue;
+    const size_t i = size_t(a.is3d ? it.z + 1 : 0) * plane + (size_t(it.y) + 1) * nx + (x + 1);
     const double X = a.f[0][i], Y = a.f[1][i];
     const double phi[2] = {a.f[2][i], a.f[3][i]};
-    const double pD = p64(phi[0]), pL = p64(phi[1]);
-    const double pG = 1.0 - pD - pL;
-    Poly64 m;
-    poly64(pD, pG, pL, m);
-    double g = pG * g64<0>(fict64<0, 0>(X, Y, m), fict64<0, 1>(X, Y, m));
-    g += pD * g64<1>(fict64<1, 0>(X, Y, m), fict64<1, 1>(X, Y, m));
-    g += pL * g64<2>(fict64<2, 0>(X, Y, m), fict64<2, 1>(X, Y, m));
-    const double sq[2] = {phi[0] * phi[0], phi[1] * phi[1]};
+    double g;
+    if (below64(X, Y, phi[0], phi[1], kSolveHi)) {
+      g = g64<0>(X, Y);
+      if (mag_hi(phi[0]) >= kNoneHi) g += trace64<1>(X, Y, a.omega[0], phi[0]);
+      if (mag_hi(phi[1]) >= kNoneHi) g += trace64<2>(X, Y, a.omega[1], phi[1]);
+      if (min(mag_hi(phi[0]), mag_hi(phi[1])) >= kLinearHi)
+        g += 2.0 * a.Omega * (phi[0] * phi[0]) * (phi[1] * phi[1]);
+    } else {
+      const double pD = p64(phi[0]), pL = p64(phi[1]);
+      const double pG = 1.0 - pD - pL;
+      Poly64 m;
+      poly64(pD, pG, pL, m);
+      g = pG * g64<0>(fict64<0, 0>(X, Y, m), fict64<0, 1>(X, Y, m));
+      g += pD * g64<1>(fict64<1, 0>(X, Y, m), fict64<1, 1>(X, Y, m));
+      g += pL * g64<2>(fict64<2, 0>(X, Y, m), fict64<2, 1>(X, Y, m));
+      const double sq[2] = {phi[0] * phi[0], phi[1] * phi[1]};
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const double u = 1.0 - phi[k];
-      g += a.omega[k] * sq[k] * (u * u);
+      for (int k = 0; k < 2; k++) g += well64(a.omega[k], phi[k], sq[k]);
+      g += 2.0 * a.Omega * sq[0] * sq[1];
     }
-    g += 2.0 * a.Omega * sq[0] * sq[1];
     double ge = 0.0;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      const double* p = a.f[2 + k];
-      const double gx = w[0] * (p[i + 1] - p[i - 1]);
-      const double gy = w[1] * (p[i + nx] - p[i - nx]);
-      double s = gx * gx + gy * gy;
+      const double* p = a.f[2 + k] + i;
+      const double e = p[1], we = p[-1], n = p[nx], s = p[-(long long)nx];
+      double u = 0.0, d = 0.0;
       if (a.is3d) {
-        const double gz = w[2] * (p[i + plane] - p[i - plane]);
-        s += gz * gz;
+        u = p[plane];
+        d = p[-(long long)plane];
       }
-      ge += a.kappa[k] * s;
+      const int most = max(max(max(mag_hi(e), mag_hi(we)), max(mag_hi(n), mag_hi(s))), max(mag_hi(u), mag_hi(d)));
+      if (most < kNoneHi) continue;
+      const double gx = w[0] * (e - we), gy = w[1] * (n - s);
+      double q = gx * gx + gy * gy;
+      if (a.is3d) {
+        const double gz = w[2] * (u - d);
+        q += gz * gz;
+      }
+      ge += a.kappa[k] * q;
     }
-    const double ce = g * dV, ee = ge * dV;
-    if (a.chem) a.chem[i] = ce;
-    if (a.grad) a.grad[i] = ee;
-    acc += ce + ee;
+    if (a.chem) a.chem[i] = g * dV;
+    if (a.grad) a.grad[i] = ge * dV;
+    acc += g + ge;
   }
-  __shared__ double sh[kThreads];
+  __shared__ double sh[kSumThreads];
   sh[threadIdx.x] = acc;
   __syncthreads();
-  for (int s = kThreads / 2; s > 0; s >>= 1) {
+  for (int s = kSumThreads / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
     __syncthreads();
   }
-  if (threadIdx.x == 0) a.partial[blockIdx.x] = sh[0];
+  if (threadIdx.x == 0) a.partial[blockIdx.x] = sh[0] * dV;
 }
 
 __global__ void __launch_bounds__(32) k_energy_total(const double* partial, int n, double* out) {
@@ -90,7 +129,7 @@ __global__ void __launch_bounds__(32) k_energy_total(const double* partial, int 
 }  // namespace
 
 cudaError_t launch_energy(const EnergyArgs& a, cudaStream_t s) {
-  k_energy_partial<<<kSumBlocks, kThreads, 0, s>>>(a);
+  k_energy_partial<<<kSumBlocks, kSumThreads, 0, s>>>(a);
   k_energy_total<<<1, 32, 0, s>>>(a.partial, kSumBlocks, a.out);
   return cudaGetLastError();
 }

@@ -5,15 +5,15 @@
 
 namespace pfa {
 
-constexpr int kSumBlocks = 256;  // fixed partial-sum count (deterministic order)
+constexpr int kSumBlocks = 304;  // fixed partial-sum count (deterministic order): two per SM
+constexpr int kSumThreads = 512;
 
 struct SumArgs {
-  const void* f[4];   // fields in the halo layout
+  const void* f[4];   // fields in the halo layout; FP32 form: f[0], the float4 records
   const void* comp;   // FP32 form: compensation records (value = f - c), or nullptr
   int pack;           // comp holds packed 16-bit counts (else float4)
   int is_f32, is3d;
   int compact;        // interior-only rows (FP32 form) instead of the ghost-ring layout
-  int stride;         // elements between consecutive cells of f (4 for FP32 records)
   int Nx, Ny, Nz, pitch;
   double* partial;    // scratch: kSumBlocks * 5 doubles
   double* out;        // 5 doubles (device)

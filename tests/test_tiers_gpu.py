@@ -1,5 +1,7 @@
 """The FP64 step's cheaper forms (zero, far-tail and general phases; the
 skipped gamma solve) and its tiles, against the oracle."""
+import math
+
 import numpy as np
 import pytest
 
@@ -161,6 +163,47 @@ def test_forms_3d(pfa, orc, n):
     got = g.read()
     g.close()
     check_cells(got, orc.run3d(f, O.model_params(dim=3), 1), 350 * 16 * 2.0 ** -53)
+
+
+# rows with and without a remainder of 32 cells, fewer and more pieces of 32
+# than the launch has warps (4864); phases of every range of the forms
+@pytest.mark.parametrize("nx,ny", [(33, 9), (5, 305), (700, 433)])
+def test_report_forms(pfa, orc, nx, ny):
+    f = mixed_fields((ny, nx), nx + ny)
+    core = (slice(1, -1), slice(1, -1))
+    rng = np.random.default_rng(nx)
+    for a in f[2:]:  # down to denormals, and values of the skipped forms
+        a[core] = np.where(rng.random((ny, nx)) < 0.3, 10.0 ** rng.uniform(-320, -100, (ny, nx)), a[core])
+    for a in f[:2]:  # outside the range of the exact sums
+        a[core] = np.where(rng.random((ny, nx)) < 0.02, rng.choice([-1e-3, 1e-5, 1.0], (ny, nx)), a[core])
+    for a in f:
+        ic.mirror_halo(a)
+    p = pfa.model_params()
+    for precision in ("fp64", "fp32"):
+        g = pfa.Grid2D(f, p, precision=precision)
+        g.upload(f)
+        e, chem, grad = g.energy(maps=True)
+        mean = g.summarize()
+        v = g.read()
+        g.close()
+        want = orc.energy2d(v, p["dx"], p["dx"], p["kappa"], p["omega"], p["alpha"], maps=True)
+        assert abs(e - want[0]) <= 1e-12 * abs(want[0])
+        for a, b in zip((chem, grad), want[1:]):
+            assert np.max(np.abs(a - b)[core]) <= 1e-12 * np.max(np.abs(b[core]))
+        X, Y, pd, pl = (a[core] for a in v)
+        # where both phases are below 1e-7: a few dozen roundings of gamma's
+        # paraboloid and the wells
+        tail = np.maximum(np.abs(pd), np.abs(pl)) < 1e-7
+        A, B, C, E = 2267132212.7620249, 15095482346.486225, 7913298631.5869827, 55193083240.685936
+        du, dv = X - 0.52421634830562147, Y - 0.01299272922003303
+        scale = p["dx"] ** 2 * (A * du ** 2 + (np.abs(B * X) + C) * np.abs(dv) + E * dv ** 2
+                                + p["omega"][0] * (pd ** 2 + pl ** 2))
+        assert np.all((np.abs(chem - want[1])[core] <= 32 * 2.0 ** -53 * scale)[tail])
+        P = [a ** 3 * (10 - 15 * a + 6 * a * a) for a in (pd, pl)]
+        # the additions of a fixed tree and a cell's own dozen roundings
+        for got, a in zip(mean, (X, Y, 1 - P[0] - P[1], *P)):
+            exact = math.fsum(a.ravel()) / a.size
+            assert abs(got - exact) <= 64 * 2.0 ** -53 * max(abs(exact), np.mean(np.abs(a)))
 
 
 def test_not_a_number_spreads_as_in_the_plain_forms(pfa, orc):
