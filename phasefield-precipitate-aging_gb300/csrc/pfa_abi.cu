@@ -238,8 +238,8 @@ static Step2DArgs step_args(State* s, double alpha, double dt) {
 }
 
 // One fused step: FP64 old -> new, or FP32 cur -> 1 - cur (*steps in: the most
-// steps it may take, out: the steps taken -- two in one pass where that is
-// the faster way).
+// steps it may take, out: the steps taken -- several in one pass where that
+// is the faster way).
 static int fused_step(CudaData* dev, State* s, double alpha, double dt, int* steps = nullptr) {
   Step2DArgs a = step_args(s, alpha, dt);
   const int most = steps ? *steps : 1;
@@ -271,9 +271,9 @@ static int fused_step(CudaData* dev, State* s, double alpha, double dt, int* ste
   // the 5-point FP32 kernel takes the centre weight as -2 (left + upper);
   // a mask whose weights do not sum to zero goes through the general form
   a.nine = !s->five_point || !s->zero_sum;
-  const bool two = most >= 2 && two_steps_f32(a);
-  if (two) *steps = 2;
-  CK(launch_step2d_f32(a, two, s->st));
+  const int taken = pass_steps_f32(a, most);
+  if (steps) *steps = taken;
+  CK(launch_step2d_f32(a, taken, s->st));
   s->cur = n;
   return 0;
 }

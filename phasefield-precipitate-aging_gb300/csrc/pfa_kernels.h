@@ -40,6 +40,7 @@ struct Step2DArgs {
                         // (Nb, Cr, Ni) times dt / (2 dx^2)
   float vm_qy;          // and the weight of the y faces, (1/dy^2) / (1/dx^2)
   int rows;             // FP32 form: rows per warp segment (set by the launcher)
+  int steps;            // FP32 form: steps of a launch of tiles (set by the launcher)
 };
 
 // Layout conversion between FP64 reference fields (ghost ring, pitch64) and
@@ -95,11 +96,13 @@ struct BatchArgs {
 };
 
 cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s);
-// two: two steps in one pass (same bits as two launches)
-cudaError_t launch_step2d_f32(const Step2DArgs& a, bool two, cudaStream_t s);
-// whether two steps in one pass are the faster way for a grid, and for both
-// record sets of this many bytes (constant mobility)
-bool two_steps_f32(const Step2DArgs& a);
+// steps: 1, or the steps of one pass (pass_steps_f32; the bits of as many
+// launches)
+cudaError_t launch_step2d_f32(const Step2DArgs& a, int steps, cudaStream_t s);
+// the steps to take in one pass where `most` are due
+int pass_steps_f32(const Step2DArgs& a, int most);
+// whether two steps in one pass over HBM are the faster way for both record
+// sets of this many bytes (constant mobility)
 bool two_steps_bytes(double bytes);
 cudaError_t prepare_step2d_f32();
 // ctas: CTAs of a persistent launch (b.persistent), else one warp per unit;

@@ -450,6 +450,19 @@ __global__ void __launch_bounds__(32 * kWarps, VM ? 6 : (PACK && !NINE ? 9 : 8))
                             a.Nx, a.Ny, a.pitch, x0, y0, min(y0 + a.rows, a.Ny), nullptr);
 }
 
+// the record of the lane that holds this lane's column
+template <bool PACK>
+__device__ __forceinline__ Raw<PACK> mirrored(const Raw<PACK>& r, int lane) {
+  auto m = [&](float v) { return __shfl_sync(0xffffffffu, v, lane); };
+  Raw<PACK> t;
+  t.a = make_float4(m(r.a.x), m(r.a.y), m(r.a.z), m(r.a.w));
+  if constexpr (PACK)
+    t.c = make_uint2(__shfl_sync(0xffffffffu, r.c.x, lane), __shfl_sync(0xffffffffu, r.c.y, lane));
+  else
+    t.c = make_float4(m(r.c.x), m(r.c.y), m(r.c.z), m(r.c.w));
+  return t;
+}
+
 // ---- two steps in one pass ----
 // The strip of output columns x0 .. x0+27 over rows y0 .. y1-1, two steps on:
 // row y+1 is advanced once (from rows y, y+1, y+2 as loaded), solved again,
@@ -509,16 +522,8 @@ __device__ __forceinline__ void stream_strip2(const Step2DArgs& a, const float4*
   auto fetch = [&](int slot) { return R{ring->a[slot][lane], ring->c[slot][lane]}; };
   // first step of a row
   auto first = [&](const N& up, const N& c, const N& dn, const R& rc, bool still) {
-    R r = S.step(up, c, dn, rc, still);
-    if (edge) {
-      auto m = [&](float v) { return __shfl_sync(0xffffffffu, v, mirror); };
-      r.a = make_float4(m(r.a.x), m(r.a.y), m(r.a.z), m(r.a.w));
-      if constexpr (PACK)
-        r.c = make_uint2(__shfl_sync(0xffffffffu, r.c.x, mirror), __shfl_sync(0xffffffffu, r.c.y, mirror));
-      else
-        r.c = make_float4(m(r.c.x), m(r.c.y), m(r.c.z), m(r.c.w));
-    }
-    return r;
+    const R r = S.step(up, c, dn, rc, still);
+    return edge ? mirrored(r, mirror) : r;
   };
 #pragma unroll
   for (int k = 0; k < kDepth2; k++) issue(y0 - 2 + k, k);
@@ -588,6 +593,67 @@ __global__ void __launch_bounds__(32 * kWarps, PACK && !NINE ? 6 : 4) k_stream2_
                                 static_cast<float4*>(a.out[0]), static_cast<CompT<PACK>*>(a.out[1]),
                                 a.Nx, a.Ny, a.pitch, x0, y0, min(y0 + a.rows, a.Ny),
                                 &ring[threadIdx.x >> 5]);
+}
+
+// ---- several steps in one launch of tiles ----
+// A CTA holds a region of 32 x kTileRows cells, a row per warp and a cell's
+// record per thread, and takes it a.steps steps S on: in each a warp solves
+// its row, publishes it for the rows above and below, and advances it; the
+// rows and columns that are right shrink by one a side and step, and the
+// region's middle (32 - 2 S) x (kTileRows - 2 S) cells are stored.  Records
+// beyond the domain mirror its edge: a warp's lanes by a copy after each
+// step, rows by reading the edge's own row.  The values and their order of
+// operations are those of single steps (the packed compensations are rounded
+// after each step as the store would), so the result is the same bits.
+//
+// What it saves is launches, 2.4 us each, of which a small grid's step itself
+// takes a quarter; it is bound by the latency of a step's chain (0.65 us where
+// an SM holds one CTA) and by issue.  Regions of 32 rows take 1.1 us a step:
+// 64 x 48 1.5 us a step against 1.0, 128^2 1.5 / 1.15, 256^2 1.74 / 1.76.
+constexpr int kTileRows = 16;
+template <bool NINE, bool VM>
+constexpr size_t tile_bytes() {
+  return 2 * kTileRows * (32 * sizeof(NbT<NINE, VM>) + sizeof(int));
+}
+
+template <bool PACK, bool NINE, bool VM>
+__global__ void __launch_bounds__(32 * kTileRows, 2) k_tile_f32(Step2DArgs a) {
+  using N = NbT<NINE, VM>;
+  extern __shared__ float4 s_tile[];
+  N* nb = reinterpret_cast<N*>(s_tile);                       // [2][kTileRows][32]
+  int* still = reinterpret_cast<int*>(nb + 2 * kTileRows * 32);  // [2][kTileRows]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, S = a.steps;
+  const int x0 = blockIdx.x * (32 - 2 * S), y0 = blockIdx.y * (kTileRows - 2 * S);
+  const int gx = x0 - S + lane, gy = y0 - S + w;
+  const int cx = min(max(gx, 0), a.Nx - 1);
+  using C = CompT<PACK>;
+  const Stream<PACK, NINE, VM> T{a, static_cast<const float4*>(a.in[0]) + cx, static_cast<const C*>(a.in[1]) + cx,
+                                 static_cast<float4*>(a.out[0]) + cx, static_cast<C*>(a.out[1]) + cx,
+                                 a.Ny, a.pitch, lane >= S && lane < 32 - S && gx < a.Nx};
+  Raw<PACK> r = T.load(T.row(gy));
+  const bool inside = gy >= 0 && gy < a.Ny;  // whole warp, as all below
+  const bool edge = x0 - S < 0 || x0 + 32 - S > a.Nx;
+  const int mirror = cx - (x0 - S);  // the lane holding column cx
+  const int up = gy <= 0 ? w : w - 1, dn = gy >= a.Ny - 1 ? w : w + 1;
+  for (int k = 0; k < S; k++) {
+    N* rows = nb + (k & 1) * kTileRows * 32;
+    int* z = still + (k & 1) * kTileRows;
+    const bool solves = inside && w >= k && w < kTileRows - k;
+    N n;
+    bool own = true;
+    if (solves) {
+      n = T.solve(r, own);
+      rows[w * 32 + lane] = n;
+      if (lane == 0) z[w] = own;
+    }
+    // this buffer was last read before the barrier of step k - 1
+    __syncthreads();
+    if (solves && w > k && w < kTileRows - 1 - k) {
+      r = T.step(rows[up * 32 + lane], n, rows[dn * 32 + lane], r, own && z[up] && z[dn]);
+      if (edge) r = mirrored(r, mirror);
+    }
+  }
+  if (inside && w >= S && w < kTileRows - S) T.store(gy, r);
 }
 
 // ---- many grids in one launch ----
@@ -705,6 +771,7 @@ int segment_rows(int Nx, int Ny, int resident, bool varmob) {
 
 // resident CTAs: FP32 / packed variants, the batch kernel, the 9-point FP32 / packed
 // variants, the variable-mobility FP32 / packed variants
+int g_sms = 0;
 int g_resident[12] = {};  // + 7: the two-step kernels (constant mobility), 11: the batch's
 
 template <typename K>
@@ -714,6 +781,7 @@ cudaError_t query_resident(K kernel, int slot) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 32 * kWarps, 0);
+  g_sms = sms;
   g_resident[slot] = sms * (per > 0 ? per : 1);
   return e;
 }
@@ -742,6 +810,15 @@ int segment_rows2(int Nx, int Ny, int resident) {
   return grid_rows(rows, Ny);
 }
 
+template <bool PACK, bool NINE, bool VM>
+cudaError_t launch_tile(Step2DArgs a, int steps, cudaStream_t s) {
+  a.steps = steps;
+  const int nx = 32 - 2 * steps, ny = kTileRows - 2 * steps;
+  const dim3 grid((a.Nx + nx - 1) / nx, (a.Ny + ny - 1) / ny);
+  k_tile_f32<PACK, NINE, VM><<<grid, 32 * kTileRows, tile_bytes<NINE, VM>(), s>>>(a);
+  return cudaGetLastError();
+}
+
 template <bool PACK, bool NINE>
 cudaError_t launch_stream2(Step2DArgs a, cudaStream_t s) {
   const int slot = 7 + 2 * NINE + PACK;
@@ -767,13 +844,51 @@ bool two_steps_f32(const Step2DArgs& a) {
   return !a.varmob && two_steps_bytes(double(a.pitch) * a.Ny * (a.full_comp ? 64 : 48));
 }
 
-cudaError_t launch_step2d_f32(const Step2DArgs& a, bool two, cudaStream_t s) {
-  if (a.varmob) {
-    if (a.nine || two) return cudaErrorInvalidValue;  // refused by the host before
-    return a.full_comp ? launch_stream<false, false, true>(a, s)
-                       : launch_stream<true, false, true>(a, s);
+// Steps per launch of tiles, 0: single steps are faster.  From the sweeps a
+// launch takes 2.4 us and, with m CTAs on the most loaded SM, a step 0.25 +
+// 0.4 m; past six CTAs per SM of three-step tiles single steps are (us a
+// step in tiles / singly: 64 x 48 1.0 / 2.4, 128^2 1.15 / 2.4, 256^2 1.76 /
+// 2.7, 384^2 2.7 / 3.3, 512^2 3.9 / 3.9, 700 x 433 4.1 / 4.1; 9 points 384^2
+// 3.1 / 3.7, 512^2 4.6 / 4.3; variable mobility 64 x 48 1.25 / 2.5, 256^2 2.2 /
+// 3.4, 384^2 3.6 / 4.3, 512^2 5.5 / 5.2).
+int tile_steps(int Nx, int Ny) {
+  const long long sms = g_sms > 0 ? g_sms : 152;
+  auto tiles = [&](int s) {
+    const int nx = 32 - 2 * s, ny = kTileRows - 2 * s;
+    return ((Nx + nx - 1) / nx) * (long long)((Ny + ny - 1) / ny);
+  };
+  if (tiles(3) > 6 * sms) return 0;
+  int best = 0;
+  double least = 1e30;
+  for (int s = 2; 2 * s < kTileRows; s++) {
+    const double us = 2.4 / s + 0.25 + 0.4 * double((tiles(s) + sms - 1) / sms);
+    if (us < least) {
+      least = us;
+      best = s;
+    }
   }
-  if (two) {
+  return best;
+}
+
+int pass_steps_f32(const Step2DArgs& a, int most) {
+  if (most < 2) return 1;
+  if (two_steps_f32(a)) return 2;
+  const int s = tile_steps(a.Nx, a.Ny);
+  if (s == 0) return 1;
+  const int passes = (most + s - 1) / s;  // as even as they go
+  return (most + passes - 1) / passes;
+}
+
+cudaError_t launch_step2d_f32(const Step2DArgs& a, int steps, cudaStream_t s) {
+  if (a.varmob && a.nine) return cudaErrorInvalidValue;  // refused by the host before
+  if (steps >= 2 && !two_steps_f32(a)) {
+    if (a.varmob) return a.full_comp ? launch_tile<false, false, true>(a, steps, s) : launch_tile<true, false, true>(a, steps, s);
+    if (a.nine) return a.full_comp ? launch_tile<false, true, false>(a, steps, s) : launch_tile<true, true, false>(a, steps, s);
+    return a.full_comp ? launch_tile<false, false, false>(a, steps, s) : launch_tile<true, false, false>(a, steps, s);
+  }
+  if (a.varmob)
+    return a.full_comp ? launch_stream<false, false, true>(a, s) : launch_stream<true, false, true>(a, s);
+  if (steps == 2) {
     if (a.nine) return a.full_comp ? launch_stream2<false, true>(a, s) : launch_stream2<true, true>(a, s);
     return a.full_comp ? launch_stream2<false, false>(a, s) : launch_stream2<true, false>(a, s);
   }
@@ -783,6 +898,17 @@ cudaError_t launch_step2d_f32(const Step2DArgs& a, bool two, cudaStream_t s) {
 
 // occupancy of the FP32 kernels on the current device (outside any capture)
 cudaError_t prepare_step2d_f32() {
+  cudaError_t et = cudaSuccess;
+  auto tile = [&](auto nine, auto vm) {
+    constexpr bool N = decltype(nine)::value, V = decltype(vm)::value;
+    for (auto k : {k_tile_f32<false, N, V>, k_tile_f32<true, N, V>})
+      if (et == cudaSuccess)
+        et = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_bytes<N, V>()));
+  };
+  tile(std::false_type{}, std::false_type{});
+  tile(std::true_type{}, std::false_type{});
+  tile(std::false_type{}, std::true_type{});
+  if (et != cudaSuccess) return et;
   cudaError_t e = query_resident(k_stream_f32<false, false>, 0);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<true, false>, 1);
   if (e == cudaSuccess) e = query_resident(k_batch_f32<false>, 2);

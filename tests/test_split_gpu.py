@@ -129,6 +129,32 @@ def test_plane_split_3d(pfa, n):
         assert np.max(np.abs(x - y)) <= 2e-8
 
 
+# launches of several steps on tiles (grids of up to 912 tiles of 26 x 10
+# cells): domains inside one tile, partial tiles, edges on every side; 13 steps
+# are passes of different lengths
+@pytest.mark.parametrize("kind", ["fp32", "fp32k", "nine", "variable"])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 35), (18, 2), (61, 5), (64, 48), (129, 131), (257, 255),
+                                   (1, 9000), (450, 448)])
+def test_tile_steps_are_bit_neutral(pfa, kind, nx, ny):
+    f = ic.grid2d(nx, ny, seed=nx + 7 * ny, stripe_width=max(1, nx // 4),
+                  n_particles=3 if min(nx, ny) > 40 else 0)
+    rng = np.random.default_rng(nx)
+    if min(nx, ny) <= 40:  # phases everywhere, some of them zero
+        for a in f[2:]:
+            a[1:-1, 1:-1] = rng.choice([0.0, 1e-9, 0.2, 0.5], (ny, nx))
+            ic.mirror_halo(a)
+    kw = {"nine": {"mask": pfa.nine_point_mask(5e-9, 5e-9)}, "variable": {"mobility": "variable"}}.get(kind, {})
+    out = []
+    for single in (False, True):
+        g = pfa.Grid2D(f, pfa.model_params(), precision="fp32k" if kind == "fp32k" else "fp32", **kw)
+        for n in ([1] * 13 if single else [13]):
+            g.run(n)
+        out.append(g.read())
+        g.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
 # record sets just above the line for double steps (96 MB): ragged columns
 # (the last strip of 28 one to three columns wide), one-strip and one-row
 # grids, row counts that leave remainders
