@@ -710,8 +710,9 @@ int pfa_batch_tune(void* handle, int reps, float* best_ms) {
       if (int r = upload_tables(b, rows)) return r;
       if (b->units[0] == 0) break;
       b->persistent = pers;
+      const int passes = two ? (reps + 1) / 2 : reps;  // of two steps or one
       // cur -> cur ^ 1 every time: the grids' state does not advance
-      for (int k = 0; k < reps + 2; k++) {
+      for (int k = 0; k < passes + 2; k++) {
         if (k == 2) CKB(cudaEventRecord(e0, b->st));
         CKB(cudaMemsetAsync(b->d_counter, 0, 2 * sizeof(int), b->st));
         if (int r = launch(b, b->cur, two)) return r;
@@ -720,7 +721,7 @@ int pfa_batch_tune(void* handle, int reps, float* best_ms) {
       CKB(cudaEventSynchronize(e1));
       float t = 0.f;
       CKB(cudaEventElapsedTime(&t, e0, e1));
-      t /= two ? 2 * reps : reps;
+      t /= two ? 2 * passes : passes;
       if (best < 0.f || t < best) {
         best = t;
         best_rows = rows;
