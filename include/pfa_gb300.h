@@ -81,7 +81,8 @@ int pfa_set_nucleation(struct CudaData* dev, uint64_t seed, int geometry);
  * mask.  The FP32 forms (pfa_set_precision, 5-point mask with zero weight
  * sum) take it too: with paraboloid energies the phases' fictitious
  * compositions share their diffusion potentials, so the flux is
- * div (D(x) grad x^gamma) with the same face sums, which they evaluate;
+ * div (D(x) grad x^gamma) with the same face sums, which the fused steps of
+ * both precisions evaluate;
  * within 1e-5 of the FP64 form after 1000 steps.  In compat mode (FP64)
  * device_mobilities / mobility_boundaries
  * (and device_laplacian, for a loop that does not call them) compute the
@@ -218,7 +219,7 @@ int pfa3d_test_skip_plane(void* handle, int plane);
 /* ---- batches of 2D grids (continuous batching) ----
  * No counterpart in the reference, which runs one grid per process
  * (src/main.cpp:285-321).  A batch owns a device arena of arena_bytes and
- * steps every member grid with one launch per time step (FP32 form,
+ * steps every member grid with one launch per one or two time steps (FP32 form,
  * packed compensations, 5-point Laplacian); all members share params (the 12
  * doubles of pfa3d_create) and dxy = dx, dy.  Grids join (pfa_batch_add:
  * fields in the reference layout, ny x nx doubles with the ghost ring;

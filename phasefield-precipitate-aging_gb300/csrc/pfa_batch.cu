@@ -3,8 +3,8 @@
 // The reference steps one grid per process (src/main.cpp:285-321).  A batch
 // holds any number of 2D grids of different sizes that share one parameter
 // set, in the FP32 precision form (packed compensations), and advances all of
-// them with one launch per time step: the grids' warp strips x row segments
-// form one table of units of work that a persistent kernel drains through an
+// them with one launch per one or two time steps: the grids' warp strips x row
+// segments form one table of units of work that a persistent kernel drains through an
 // atomic counter (or that a one-warp-per-unit launch covers).  Multi-step runs
 // replay captured CUDA graphs.  Grids join and leave between runs
 // (continuous batching): each owns one block of a fixed device arena (first

@@ -6,9 +6,10 @@
 // which keeps FP32 accurate inside precipitates where the plain num / den
 // form loses it to cancellation; cells whose phases are below 1e-5 skip the
 // solve (x^gamma = X there), and rows whose phases are all zero the
-// Allen-Cahn update.  Grids larger than the L2 take two steps per pass.  At
-// 48 bytes per cell and pass the HBM budget leaves ~250 instructions per
-// cell, so the kernels are organised for instruction economy:
+// Allen-Cahn update.  Grids larger than the L2 take two steps per pass, small
+// ones several steps per launch.  At 48 bytes per cell and pass the HBM budget
+// leaves ~250 instructions per cell, so the kernels are organised for
+// instruction economy:
 //  * each warp owns a strip of 30 output columns (lanes 1..30; lanes 0 and
 //    31 carry the neighbour columns) and streams down a segment of rows; the
 //    three rows a 5- or 9-point Laplacian needs live in registers, rotated by

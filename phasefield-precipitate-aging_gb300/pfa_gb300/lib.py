@@ -646,7 +646,7 @@ ENOMEM = 5
 
 
 class Batch:
-    """Many 2D grids (FP32 form) stepped together by one launch per step.
+    """Many 2D grids (FP32 form) stepped together, one launch per one or two steps.
 
     ``add`` returns a slot id, or None when the arena has no room for the grid
     (the admission refusal); ``remove`` frees the slot between runs."""

@@ -5,7 +5,7 @@ A request is one initial condition (four fields in the reference layout, 2D
 (ny, nx) or 3D (nz, ny, nx) with the ghost ring, or a recipe the device
 builds them from, pfa_ic_recipe) and a number of explicit steps.  Requests are admitted first-in first-out while their device
 footprint fits the budget; 2D requests join one ``Batch`` (all advance with
-one launch per time step), 3D requests get their own ``Grid3D`` handle on
+one launch per one or two time steps), 3D requests get their own ``Grid3D`` handle on
 their own stream, so 2D and 3D work overlap on the GPU.  Every tick advances
 each admitted request by up to ``tick_steps`` steps -- never past its own
 end -- then reads back and retires the finished ones and admits new ones.
@@ -139,7 +139,8 @@ class Server:
         self.done: List[Record] = []
         self.ticks = 0
         self.cell_updates = 0
-        self.step_launches = 0  # step kernels enqueued: one per batch step, one per 3D step
+        self.step_launches = 0  # least step kernels enqueued: one per two batch steps (a large batch's
+                                # launches advance two, a small one's one), one per 3D step
 
     def now(self):
         if self.t0 is None:
@@ -174,7 +175,7 @@ class Server:
         n2 = min([self.tick_steps] + [r.remaining for r in two]) if two else 0
         items3 = [(r.handle, min(self.tick_steps, r.remaining)) for r in three]
         self.backend.advance(n2, [r.handle for r in two], items3)
-        self.step_launches += n2 + sum(n for _, n in items3)
+        self.step_launches += (n2 + 1) // 2 + sum(n for _, n in items3)
         for r in two:
             r.done_steps += n2
             self.cell_updates += n2 * r.req.cells
