@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, TX == 16 ? 3 : 
   store_cell(a, c.i, gx, gy, ocr, onb, od, ol);
 }
 
-constexpr long long kHotTiles = 12288;
+constexpr long long kHotTiles = 12288, kWideTiles = 8192;
 
 template <int TX, int TY>
 long long tiles(const Step2DArgs& a) {
@@ -346,11 +346,15 @@ cudaError_t launch_tiles(const Step2DArgs& a, cudaStream_t s) {
       k_step2d_f64_varmob<false, TX, TY><<<grid, n, 0, s>>>(a);
   } else {
     constexpr int n5 = Tile2<kMaskIso, TX, TY>::kThreads, n9 = Tile2<kMaskIso9, TX, TY>::kThreads;
-    switch (a.c.mask) {
-      case kMaskIso: k_step2d_f64<kMaskIso, TX, TY, HOT><<<grid, n5, 0, s>>>(a); break;
-      case kMaskIso9: k_step2d_f64<kMaskIso9, TX, TY, HOT><<<grid, n9, 0, s>>>(a); break;
-      case kMaskFive: k_step2d_f64<kMaskFive, TX, TY, HOT><<<grid, n5, 0, s>>>(a); break;
-      default: k_step2d_f64<kMaskNine, TX, TY, HOT><<<grid, n9, 0, s>>>(a);
+    if (a.c.mask == kMaskIso9) {
+      k_step2d_f64<kMaskIso9, TX, TY, HOT><<<grid, n9, 0, s>>>(a);
+    } else if (a.c.mask == kMaskNine) {
+      k_step2d_f64<kMaskNine, TX, TY, HOT><<<grid, n9, 0, s>>>(a);
+    } else if constexpr (TX == 8) {  // (16 x 8: 9 points only)
+      if (a.c.mask == kMaskIso)
+        k_step2d_f64<kMaskIso, TX, TY, HOT><<<grid, n5, 0, s>>>(a);
+      else
+        k_step2d_f64<kMaskFive, TX, TY, HOT><<<grid, n5, 0, s>>>(a);
     }
   }
   return cudaGetLastError();
@@ -363,20 +367,22 @@ cudaError_t launch_step2d_f64(const Step2DArgs& a, cudaStream_t s) {
   if (a.varmob && a.nine) return cudaErrorInvalidValue;  // refused by the host before
   // A tile next to a precipitate takes its SM's FP64 pipe for microseconds, and
   // a step is as long as its most loaded SM: small tiles spread such work, and
-  // 8 x 8 has the least halo for its size.  us a step (FP64 solves) of 8 x 4 /
-  // 8 x 8 / 16 x 8 / 16 x 16 / 32 x 8 cells: 64 x 48 5.1 / 5.8 / 6.3 / 9.4 /
-  // 9.9, 192^2 5.8 / 5.9 / 8.3 / 8.1 / 8.8, 256^2 6.8 / 6.5 / 8.0 / 9.9 / 10.1,
-  // 1024^2 27 / 19.6 / 21 / 24 / 25, 2048^2 93 / 67 / 69 / 77 / 77 (32 x 8 in
-  // rows of 32: 76).
+  // 8 x 8 has the least halo for its size (with corners 36 cells, two warps: the
+  // 9-point form takes 16 x 8 from 8192 tiles of 8 x 8).  The solve in fixed
+  // point (HOT) shortens tiles next to precipitates, but its call costs
+  // registers (56 for 40, fewer tiles in flight), which many waves of tiles
+  // without precipitate feel.  us a step with 6 particles, HOT / FP64, 5
+  // points, 8 x 8: 64 x 48 5.1 / 5.8, 256^2 6.6 / 7.4, 512^2 9.0 / 9.8, 1000 x
+  // 733 14.2 / 14.3, 1024^2 17.4 / 16.6, 2048^2 73.6 / 64.8 (HOT 8 x 4: 5.3, 7.1,
+  // 10.9, 19.0, 24.6, 92; 16 x 8: 5.9, 7.5, 9.9, 15.1, 18.0, 78); 9 points 8 x 8
+  // 64 x 48 5.6 / 6.2, 512^2 11.0 / 13.4, 1000 x 733 17.6 / 18.9, 1024^2 21.8 /
+  // 21.6, 2048^2 91 / 84; 16 x 8 6.5 / 7.3, 12.0 / 14.5, 17.0 / 18.8, 19.5 / 19.5,
+  // 81 / 74.
   if (!a.varmob) {
-    if (tiles<8, 4>(a) <= 1216) return launch_tiles<8, 4, false, true>(a, s);
-    // The solve in fixed point shortens tiles next to precipitates, but its
-    // call costs registers (56 for 40, fewer tiles in flight), which many
-    // waves of tiles without precipitate feel; fixed / FP64 with 8 particles,
-    // 5 points 256^2 6.6 / 7.5, 512^2 9.1 / 10.3, 1000 x 733 14.4 / 14.4,
-    // 1024^2 18.3 / 17.7, 2048^2 73.5 / 65.4; 9 points 7.7 / 9.8, 11.8 / 14.7,
-    // 18.1 / 19.3, 23.0 / 23.4, 91 / 85
-    return tiles<8, 8>(a) <= kHotTiles ? launch_tiles<8, 8, false, true>(a, s) : launch_tiles<8, 8, false, false>(a, s);
+    const bool hot = tiles<8, 8>(a) <= kHotTiles, corners = a.c.mask == kMaskIso9 || a.c.mask == kMaskNine;
+    if (corners && tiles<8, 8>(a) > kWideTiles)
+      return hot ? launch_tiles<16, 8, false, true>(a, s) : launch_tiles<16, 8, false, false>(a, s);
+    return hot ? launch_tiles<8, 8, false, true>(a, s) : launch_tiles<8, 8, false, false>(a, s);
   }
   // every staged cell has its mobilities, so large grids take the tile with
   // the smallest share of halo: 8 x 8 / 16 x 16 64 x 48 6.5 / 9.9, 192^2 7.7 /

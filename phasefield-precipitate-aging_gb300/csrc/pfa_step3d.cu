@@ -491,19 +491,18 @@ int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
 
 // FP64: a column next to a precipitate costs several times one in the matrix,
 // so short segments that spread the precipitates over the SMs beat whole
-// waves of equal ones.  us per step at 1 / 2 / 3 / 6 / 12 / 24 planes: 32^3 23
-// / 21 / 26 / 41 / 74 / 135, 64^3 61 / 56 / 60 / 57 / 80 / 128, 96^3 94 / 85 /
-// 86 / 94 / 118 / 151, 200 x 100 x 60 105 / 94 / 94 / 107 / 123 / 132, 128^3
-// 154 / 137 / 132 / 135 / 157 / 182, 192^3 368 / 290 / 268 / 255 / 254 / 280,
-// 256^3 783 / 602 / 541 / 488 / 471 / 471.
+// waves of equal ones.  us per step at 1 / 2 / 3 / 6 / 12 planes: 32^3 15 / 18
+// / 22 / 38 / 70, 64^3 44 / 40 / 39 / 44 / 73, 96^3 79 / 71 / 71 / 80 / 94, 200
+// x 100 x 60 94 / 84 / 81 / 86 / 108, 128^3 146 / 130 / 123 / 124 / 133, 192^3
+// 362 / 285 / 263 / 250 / 252, 256^3 768 / 588 / 528 / 475 / 458.
 int segment_planes_f64(long long columns, int Nz) {
   const long long n = columns * Nz;  // planes of tiles
-  const int planes = n <= 16384 ? 2 : (n <= 65536 ? 3 : (n <= 180000 ? 6 : 16));
+  const int planes = n <= 1024 ? 1 : n <= 16384 ? 2 : (n <= 65536 ? 3 : (n <= 180000 ? 6 : 16));
   return std::min(std::max(planes, (Nz + 65534) / 65535), Nz);
 }
 
 // up to here the solve in fixed point (cell64's HOT) pays for its registers
-// (pfa_step2d.cu), us a step fixed / FP64: 32^3 17.9 / 21.7, 64^3 39.6 / 56, 96^3
+// (pfa_step2d.cu), us a step fixed / FP64: 32^3 15.1 / 21.7, 64^3 39.6 / 56, 96^3
 // 71 / 86, 128^3 123 / 132, 192^3 265 / 251, 256^3 503 / 465
 constexpr long long kHotPlanes = 65536;
 

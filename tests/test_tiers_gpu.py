@@ -52,8 +52,10 @@ def check_cells(got, want, rel):
         assert np.all((np.abs(a - b) <= rel * scale)[core])
 
 
-# tiles of 8 x 4 (up to 1216 of them) and 8 x 8 cells, partial tiles on both axes
-@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 405), (70, 406), (161, 1621), (191, 1622)])
+# tiles of 8 x 8 cells with the fixed-point solve (up to 12288 of them) and the
+# FP64 one, 16 x 8 from 8192 with the 9-point mask; partial tiles on both axes
+@pytest.mark.parametrize("nx,ny", [(33, 9), (65, 405), (70, 406), (161, 1621), (191, 1622), (650, 905),
+                                   (1001, 797)])
 @pytest.mark.parametrize("mask", ["iso", "five", "nine"])
 def test_forms_2d(pfa, orc, nx, ny, mask):
     f = mixed_fields((ny, nx), nx * ny)
@@ -154,8 +156,8 @@ def test_mobilities_out_of_range(pfa, orc, nx, ny):
     check_cells(got, orc.run2d_varmob(f, O.model_params(), 1), 350 * 16 * 2.0 ** -53)
 
 
-# segments of 2, 3 and 6 planes; partial tiles on every axis
-@pytest.mark.parametrize("n", [(31, 15, 3), (64, 40, 131), (199, 93, 61), (95, 61, 700)])
+# segments of 1, 2, 3 and 6 planes; partial tiles on every axis
+@pytest.mark.parametrize("n", [(31, 15, 3), (20, 14, 60), (64, 40, 131), (199, 93, 61), (95, 61, 700)])
 def test_forms_3d(pfa, orc, n):
     f = mixed_fields(n[::-1], sum(n))
     g = pfa.Grid3D(f, pfa.model_params(dim=3))
