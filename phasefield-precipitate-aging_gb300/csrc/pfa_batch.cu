@@ -81,7 +81,7 @@ struct Batch {
   bool two = false;          // runs advance two steps per launch (refresh)
   bool dirty = true;
   int rows = 0;          // rows per segment (0: by auto_rows)
-  int persistent = 1;    // persistent launch (else one warp per unit)
+  int persistent = -1;   // 1: persistent launch, 0: one warp per unit, -1: by size (is_persistent)
   int ctas = 0;          // CTAs of a persistent launch (0 = all resident)
   unsigned long long version = 1;  // bumps when the device tables move
   std::vector<BGraph> graphs;
@@ -177,7 +177,7 @@ int auto_rows(const Batch* b, bool two) {
   for (const Slot& s : b->slots)
     if (s.live) strip_rows += double((s.Nx + batch_strip_cols(two) - 1) / batch_strip_cols(two)) * s.Ny;
   const double load = strip_rows / (batch_resident_ctas(two) * batch_warps_per_cta());
-  if (!two) return load <= 1.0 ? 1 : (load <= 24.0 ? 6 : 32);
+  if (!two) return load <= 1.0 ? 1 : load <= 2.5 ? 2 : load <= 16.0 ? 3 : (load <= 24.0 ? 6 : 32);
   return 3 * std::max(2, int(std::sqrt(6.0 * load) / 3.0 + 0.5));
 }
 
@@ -254,6 +254,9 @@ int refresh(Batch* b) {
   return 0;
 }
 
+// small batches, in single steps, have one warp per unit
+int is_persistent(const Batch* b, bool two) { return b->persistent < 0 ? int(two) : b->persistent; }
+
 int persistent_ctas(const Batch* b, bool two) {
   const int res = batch_resident_ctas(two);
   const int need = (b->units[two] + batch_warps_per_cta() - 1) / batch_warps_per_cta();
@@ -269,7 +272,7 @@ int launch(Batch* b, int parity, bool two) {
   ba.counter = b->d_counter;
   ba.units = b->units[two];
   ba.parity = parity;
-  ba.persistent = b->persistent;
+  ba.persistent = is_persistent(b, two);
   CKB(launch_batch_f32(b->a, ba, two, persistent_ctas(b, two), b->st));
   return 0;
 }
@@ -291,7 +294,7 @@ int run(Batch* b, int nsteps) {
     const int len = passes * per;
     // a persistent launch reads the unit count from the device; the other
     // mode's grid size is the unit count
-    const int gsize = b->persistent ? persistent_ctas(b, two) : -b->units[two];
+    const int gsize = is_persistent(b, two) ? persistent_ctas(b, two) : -b->units[two];
     cudaGraphExec_t exec = nullptr;
     for (auto& g : b->graphs)
       if (g.len == len && g.parity == b->cur && g.grid == gsize && g.two == two &&
@@ -685,8 +688,8 @@ int pfa_batch_get_launch(void* handle, int* rows, int* persistent, int* ctas, in
   if (int r = refresh(b)) return r;
   const bool two = b->two;
   if (rows) *rows = b->rows > 0 ? b->rows : auto_rows(b, two);
-  if (persistent) *persistent = b->persistent;
-  if (ctas) *ctas = b->persistent ? persistent_ctas(b, two) : (b->units[two] + batch_warps_per_cta() - 1) / batch_warps_per_cta();
+  if (persistent) *persistent = is_persistent(b, two);
+  if (ctas) *ctas = is_persistent(b, two) ? persistent_ctas(b, two) : (b->units[two] + batch_warps_per_cta() - 1) / batch_warps_per_cta();
   if (units) *units = b->units[two];
   return 0;
 }
@@ -696,7 +699,7 @@ int pfa_batch_tune(void* handle, int reps, float* best_ms) {
   if (!b) return fail(PFA_ESTATE, "pfa_batch_tune: null handle");
   if (reps < 1) reps = 10;
   if (int r = refresh(b)) return r;
-  static const int kRows[2][9] = {{3, 6, 12, 24, 32, 48, 64, 128, 1 << 30},
+  static const int kRows[2][9] = {{1, 2, 3, 6, 9, 12, 16, 24, 48},
                                   {9, 15, 24, 30, 36, 48, 64, 96, 1 << 30}};
   float best = -1.f;
   int best_rows = b->rows, best_pers = b->persistent;

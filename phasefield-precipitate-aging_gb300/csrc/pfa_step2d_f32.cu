@@ -320,6 +320,25 @@ struct Stream {
   }
 };
 
+// Rows y0 .. y1-1 (three at most) of the warp's strip: all its rows are
+// requested at once, so that the warp waits for memory once instead of row by
+// row.
+template <bool PACK, bool NINE, bool VM>
+__device__ __forceinline__ void short_segment(const Stream<PACK, NINE, VM>& S, int y0, int y1) {
+  bool z0, z1, z2;
+  const Raw<PACK> ra = S.load(S.row(y0 - 1)), rb = S.load(S.row(y0)), rc = S.load(S.row(y0 + 1)),
+                  rd = S.load(S.row(y0 + 2)), re = S.load(S.row(y0 + 3));
+  NbT<NINE, VM> na = S.solve(ra, z0), nb = S.solve(rb, z1);
+  const NbT<NINE, VM> nc = S.solve(rc, z2);
+  S.store(y0, S.step(na, nb, nc, rb, z0 && z1 && z2));
+  if (y0 + 1 >= y1) return;
+  na = S.solve(rd, z0);
+  S.store(y0 + 1, S.step(nb, nc, na, rc, z0 && z1 && z2));
+  if (y0 + 2 >= y1) return;
+  nb = S.solve(re, z1);
+  S.store(y0 + 2, S.step(nc, na, nb, rd, z0 && z1 && z2));
+}
+
 // One warp updates the strip of output columns x0 .. x0+29 over rows
 // y0 .. y1-1 of one grid (the unit of work of both the single-grid and the
 // batched kernels).  Whole warp; x0 < Nx.  Rows reach the registers either
@@ -342,19 +361,7 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
   bool z0, z1, z2;  // rows y-1, y, y+1 are still
   if constexpr (!STAGED) {
     if (y1 - y0 <= 3) {
-      // a short segment: all its rows are requested at once, so that a warp
-      // waits for memory once instead of row by row
-      const Raw<PACK> ra = S.load(S.row(y0 - 1)), rb = S.load(S.row(y0)), rc = S.load(S.row(y0 + 1)),
-                      rd = S.load(S.row(y0 + 2)), re = S.load(S.row(y0 + 3));
-      NbT<NINE, VM> na = S.solve(ra, z0), nb = S.solve(rb, z1);
-      const NbT<NINE, VM> nc = S.solve(rc, z2);
-      S.store(y0, S.step(na, nb, nc, rb, z0 && z1 && z2));
-      if (y0 + 1 >= y1) return;
-      na = S.solve(rd, z0);
-      S.store(y0 + 1, S.step(nb, nc, na, rc, z0 && z1 && z2));
-      if (y0 + 2 >= y1) return;
-      nb = S.solve(re, z1);
-      S.store(y0 + 2, S.step(nc, na, nb, rd, z0 && z1 && z2));
+      short_segment(S, y0, y1);
       return;
     }
     // window rows y-1, y, y+1 and raw records of rows y, y+1, y+2
@@ -385,6 +392,10 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
       r1 = r2;
     }
   } else {
+    if (y1 - y0 <= 3) {
+      short_segment(S, y0, y1);
+      return;
+    }
     // ring slot k holds rows y0-1+k, y0-1+k+kDepth, ...; each lane copies and
     // reads back only its own column's records, so the wait needs no warp sync
     const uint32_t sa = uint32_t(__cvta_generic_to_shared(&ring->a[0][lane]));
@@ -658,15 +669,18 @@ __global__ void __launch_bounds__(32 * kTileRows, 2) k_tile_f32(Step2DArgs a) {
 }
 
 // ---- many grids in one launch ----
-// Warps claim units (grid, strip, row segment) of the batch's unit table
-// through an atomic counter (counter[parity]) until the unit count in
-// counter[2] (TWO: counter[3]) is reached, so a captured launch stays valid while the table's
-// contents change.  The launch also zeroes the other parity's counter for the
-// next launch, which stream order runs after this one.  A persistent launch
-// has one CTA per resident slot; the other shape has one warp per unit (and
-// leaves the balancing to the block scheduler).  TWO: two steps in one pass
-// (strips of 28 columns), else one (strips of 30).  Unit indices come only
-// from the counter.
+// The units (grid, strip, row segment) of the batch's unit table, their count
+// in counter[2] (TWO: counter[3]).  A persistent launch has one CTA per
+// resident slot, whose warps claim units through an atomic counter
+// (counter[parity]), so a captured launch stays valid while the table's
+// contents change; the launch also zeroes the other parity's counter for the
+// next launch, which stream order runs after this one.  The other shape has
+// one warp per unit and leaves the balancing to the block scheduler; single
+// steps then take the warp's own unit, with no claim to wait for, which small
+// batches of short segments feel (us a step, best of the persistent shapes
+// with segments of 6 and 12 rows -> segments of 3 rows, a warp each: 4 grids of
+// 64-512 9.1 -> 6.6, 24 of 64-512 19.4 -> 13.8).  TWO: two steps in one pass
+// (strips of 28 columns), else one (strips of 30).
 template <bool TWO>
 __global__ void __launch_bounds__(32 * kWarps, TWO ? 6 : 8) k_batch_f32(Step2DArgs a, BatchArgs b) {
   const int p = b.parity;
@@ -674,10 +688,12 @@ __global__ void __launch_bounds__(32 * kWarps, TWO ? 6 : 8) k_batch_f32(Step2DAr
   const int units = b.counter[TWO ? 3 : 2];
   using R = typename std::conditional<TWO, Ring2<true>, Ring<true>>::type;
   __shared__ R ring[kWarps];
-  for (;;) {
-    int u = 0;
-    if ((threadIdx.x & 31) == 0) u = atomicAdd(b.counter + p, 1);
-    u = __shfl_sync(0xffffffffu, u, 0);
+  const bool claims = TWO || b.persistent;
+  for (int u = blockIdx.x * kWarps + (threadIdx.x >> 5);; u = units) {
+    if (claims) {
+      if ((threadIdx.x & 31) == 0) u = atomicAdd(b.counter + p, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+    }
     if (u >= units) return;
     const BatchUnit w = b.unit[u];
     const BatchGrid& g = b.grid[w.grid];
