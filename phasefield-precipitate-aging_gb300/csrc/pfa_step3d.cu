@@ -92,27 +92,38 @@ __global__ void __launch_bounds__(Tile3::kThreads, HOT ? 7 : 8)
   const bool edge = cx == 0 || cx == a.Nx - 1 || cy == 0 || cy == a.Ny - 1;
   if (threadIdx.x < 3) s_wide[threadIdx.x] = 0;
 
-  double rX, rY, rpd, rpl;  // the next plane's record
+  struct Record {
+    double X, Y, pd, pl;
+  };
   auto load = [&](int z) {
     const size_t i = size_t(clampi(z, 0, a.Nz - 1) + 1) * plane + col;
-    rX = __ldg(static_cast<const double*>(a.in[0]) + i);
-    rY = __ldg(static_cast<const double*>(a.in[1]) + i);
-    rpd = __ldg(static_cast<const double*>(a.in[2]) + i);
-    rpl = __ldg(static_cast<const double*>(a.in[3]) + i);
+    return Record{__ldg(static_cast<const double*>(a.in[0]) + i), __ldg(static_cast<const double*>(a.in[1]) + i),
+                  __ldg(static_cast<const double*>(a.in[2]) + i), __ldg(static_cast<const double*>(a.in[3]) + i)};
   };
   // |x^gamma| < 2: the seven-point sum stays below 2^5
-  auto stage = [&]() { return cell64<ISO, HOT>(rX, rY, rpd, rpl, 1ll << 61); };
+  auto stage = [&](const Record& r) { return cell64<ISO, HOT>(r.X, r.Y, r.pd, r.pl, 1ll << 61); };
   Cell64 P, C, N;  // planes z - 1, z, z + 1 of the thread's column
-  load(z0 - 1);
-  P = stage();
-  load(z0);
-  C = stage();
-  load(z0 + 1);
+  Record next;     // the record of the plane after them
+  if constexpr (HOT) {
+    next = load(z0 - 1);
+    P = stage(next);
+    next = load(z0);
+    C = stage(next);
+    next = load(z0 + 1);
+  } else {
+    // the first three planes are requested together: one wait, not three (us a
+    // step 192^3 251 -> 241, 256^3 465 -> 455; with the solve's call the records
+    // do not fit the registers: 128^3 123 -> 128)
+    const Record r0 = load(z0 - 1), r1 = load(z0);
+    next = load(z0 + 1);
+    P = stage(r0);
+    C = stage(r1);
+  }
   __syncthreads();  // s_wide is set
   int w = 0;  // slot of s_wide
   for (int z = z0; z < z1; z++) {
-    N = stage();
-    if (z + 1 < z1) load(z + 2);
+    N = stage(next);
+    if (z + 1 < z1) next = load(z + 2);
     Plane64& S = sh[z & 1];
     auto dg1 = reinterpret_cast<double (*)[Tile3::kPitch]>(S.g1), dg2 = reinterpret_cast<double (*)[Tile3::kPitch]>(S.g2);
     if (staged) {
@@ -503,7 +514,7 @@ int segment_planes_f64(long long columns, int Nz) {
 
 // up to here the solve in fixed point (cell64's HOT) pays for its registers
 // (pfa_step2d.cu), us a step fixed / FP64: 32^3 15.1 / 21.7, 64^3 39.6 / 56, 96^3
-// 71 / 86, 128^3 123 / 132, 192^3 265 / 251, 256^3 503 / 465
+// 71 / 86, 128^3 123 / 132, 192^3 265 / 241, 256^3 503 / 455
 constexpr long long kHotPlanes = 65536;
 
 int g_resident3 = 0;  // resident CTAs of the FP32 kernel
