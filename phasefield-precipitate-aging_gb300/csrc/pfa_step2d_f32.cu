@@ -320,16 +320,19 @@ struct Stream {
   }
 };
 
-// Rows y0 .. y1-1 (three at most) of the warp's strip: all its rows are
+// Rows y0 .. y1-1 of the warp's strip, kShortRows at most: all its rows are
 // requested at once, so that the warp waits for memory once instead of row by
-// row.
+// row.  (The variable-mobility form has the registers for a fourth row.)
+template <bool VM>
+constexpr int kShortRows = VM ? 4 : 3;
 template <bool PACK, bool NINE, bool VM>
 __device__ __forceinline__ void short_segment(const Stream<PACK, NINE, VM>& S, int y0, int y1) {
   bool z0, z1, z2;
   const Raw<PACK> ra = S.load(S.row(y0 - 1)), rb = S.load(S.row(y0)), rc = S.load(S.row(y0 + 1)),
                   rd = S.load(S.row(y0 + 2)), re = S.load(S.row(y0 + 3));
-  NbT<NINE, VM> na = S.solve(ra, z0), nb = S.solve(rb, z1);
-  const NbT<NINE, VM> nc = S.solve(rc, z2);
+  Raw<PACK> rf;
+  if constexpr (VM) rf = S.load(S.row(y0 + 4));
+  NbT<NINE, VM> na = S.solve(ra, z0), nb = S.solve(rb, z1), nc = S.solve(rc, z2);
   S.store(y0, S.step(na, nb, nc, rb, z0 && z1 && z2));
   if (y0 + 1 >= y1) return;
   na = S.solve(rd, z0);
@@ -337,6 +340,11 @@ __device__ __forceinline__ void short_segment(const Stream<PACK, NINE, VM>& S, i
   if (y0 + 2 >= y1) return;
   nb = S.solve(re, z1);
   S.store(y0 + 2, S.step(nc, na, nb, rd, z0 && z1 && z2));
+  if constexpr (VM) {
+    if (y0 + 3 >= y1) return;
+    nc = S.solve(rf, z2);
+    S.store(y0 + 3, S.step(na, nb, nc, re, z0 && z1 && z2));
+  }
 }
 
 // One warp updates the strip of output columns x0 .. x0+29 over rows
@@ -360,7 +368,7 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
                              Ny, P, lane >= 1 && lane <= kCols && gx < Nx};
   bool z0, z1, z2;  // rows y-1, y, y+1 are still
   if constexpr (!STAGED) {
-    if (y1 - y0 <= 3) {
+    if (y1 - y0 <= kShortRows<VM>) {
       short_segment(S, y0, y1);
       return;
     }
@@ -392,7 +400,7 @@ __device__ __forceinline__ void stream_strip(const Step2DArgs& a, const float4* 
       r1 = r2;
     }
   } else {
-    if (y1 - y0 <= 3) {
+    if (y1 - y0 <= kShortRows<VM>) {
       short_segment(S, y0, y1);
       return;
     }
@@ -774,15 +782,14 @@ int grid_rows(int rows, int Ny) { return std::min(std::max(rows, (Ny + 65534) / 
 // 8.1, 700 x 433 4.5 / 4.1 / 4.4 / 5.7 / 8.4, 900 x 600 6.1 / 5.1 / 4.9 / 6.2
 // / 8.9, 1024^2 10.0 / 7.5 / 7.0 / 7.9 / 10.1, 2048^2 45.8 / 33.5 / 30.2 /
 // 33.0 / 36.3; the same order in the 9-point form.  The variable-mobility
-// step, whose extra rows cost three exponentials a cell, takes 6 and 9 from
-// there (1024^2 10.8 at 3, 11.3 at 6; 1531 x 1021 15.3 / 15.1; 2048^2 43.3 /
-// 41.0; 3000^2 87.8 / 81.6, 81.0 at 9).
+// step, whose extra rows cost three exponentials a cell, takes 4 from four CTA
+// rows per resident CTA on (us a step at 3 / 4 / 6 / 9 rows: 512^2 5.0 / 5.3 /
+// 6.3 / 7.4, 900 x 600 7.0 / 6.7 / 7.7 / 8.6, 1024^2 10.5 / 10.3 / 11.1 / 11.5,
+// 1531 x 1021 15.3 / 14.4 / 15.0 / 15.1, 4096^2 163 / 143 / 149 / 146).
 int segment_rows(int Nx, int Ny, int resident, bool varmob) {
   const int nbx = ((Nx + kCols - 1) / kCols + kWarps - 1) / kWarps;
   const double load = double(nbx) * Ny / resident;  // CTA rows per resident CTA
-  const int rows = load <= 1.0   ? 1
-                   : load <= 2.5 ? 2
-                                 : (!varmob || load <= 12.0 ? 3 : (load <= 24.0 ? 6 : 9));
+  const int rows = load <= 1.0 ? 1 : load <= 2.5 ? 2 : !varmob || load <= 4.0 ? 3 : 4;
   return grid_rows(rows, Ny);
 }
 

@@ -91,6 +91,27 @@ def test_record_conversions(pfa, dim):
         assert np.array_equal(a[core], b[core])
 
 
+# segments of four rows (variable mobility, from four CTA rows per resident
+# CTA on) with remainders of one to three rows, against a piece in shorter ones
+@pytest.mark.parametrize("precision", ["fp32", "fp32k"])
+@pytest.mark.parametrize("nx,ny", [(1001, 609), (1001, 610), (1001, 611)])
+def test_four_row_segments(pfa, precision, nx, ny):
+    f = ic.grid2d(nx, ny, seed=ny, stripe_width=300, n_particles=6)
+    out = []
+    for top in (ny - 64, ny):
+        part = [np.ascontiguousarray(a[top:top + 66]) for a in f] if top < ny else f
+        if top < ny:
+            for a in part:
+                ic.mirror_halo(a)
+        g = pfa.Grid2D(part, pfa.model_params(), precision=precision, mobility="variable")
+        for _ in range(3):
+            g.run(1)
+        out.append(g.read())
+        g.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a[5:65, 1:-1], b[ny - 59:ny + 1, 1:-1])
+
+
 # strips of 28 and 30 columns (double and single passes) put the same cells in
 # different warps: tails that cross the bulk threshold of the gamma solve
 # everywhere must not notice
