@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(32 * kWarps, PACK && !NINE ? 6 : 4) k_stream2_
 // 64 x 48 1.5 us a step against 1.0, 128^2 1.5 / 1.15, 256^2 1.74 / 1.76.
 constexpr int kTileRows = 16;
 template <bool NINE, bool VM>
-constexpr size_t tile_bytes() {
+constexpr size_t tile_bytes() {  // at most 33 KB
   return 2 * kTileRows * (32 * sizeof(NbT<NINE, VM>) + sizeof(int));
 }
 
@@ -922,17 +922,6 @@ cudaError_t launch_step2d_f32(const Step2DArgs& a, int steps, cudaStream_t s) {
 
 // occupancy of the FP32 kernels on the current device (outside any capture)
 cudaError_t prepare_step2d_f32() {
-  cudaError_t et = cudaSuccess;
-  auto tile = [&](auto nine, auto vm) {
-    constexpr bool N = decltype(nine)::value, V = decltype(vm)::value;
-    for (auto k : {k_tile_f32<false, N, V>, k_tile_f32<true, N, V>})
-      if (et == cudaSuccess)
-        et = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_bytes<N, V>()));
-  };
-  tile(std::false_type{}, std::false_type{});
-  tile(std::true_type{}, std::false_type{});
-  tile(std::false_type{}, std::true_type{});
-  if (et != cudaSuccess) return et;
   cudaError_t e = query_resident(k_stream_f32<false, false>, 0);
   if (e == cudaSuccess) e = query_resident(k_stream_f32<true, false>, 1);
   if (e == cudaSuccess) e = query_resident(k_batch_f32<false>, 2);
