@@ -47,7 +47,7 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 METRIC = "cell-updates/s FP32 vs plain FP64 on one GB300 at stated error; p50/p99 latency"
 N_SIDE = 4096
 STEPS_PER_BENCH_STEP = 100
-NUC_LAUNCHES = 3  # kernels per nucleation call: decide, FP64 decisions, paint
+NUC_LAUNCHES = 2  # kernels per nucleation call: decide; FP64 decisions and paint
 NUC = dict(sigma=(0.13, 0.13), unit_a=0.352e-9)
 FULL_RUN_STEPS = 10000  # the 4096^2 workload's step count
 WORKLOAD = (f"single 2D grid {N_SIDE}x{N_SIDE}, dx=5nm, 16 enriched stripes + 4 particles R=8 "

@@ -93,7 +93,7 @@ struct State {
   uint64_t step_counter = 0;
   // scratch (event buffer, counters, partial sums)
   NucEvent* ev = nullptr;
-  unsigned* ev_count = nullptr;  // [0] events, [1] listed cells
+  unsigned* ev_count = nullptr;  // kNucCounters (NucArgs::count)
   int* ev_status = nullptr;
   unsigned long long* call_dev = nullptr;
   long long* cand = nullptr;  // cells left to the FP64 nucleation decision
@@ -627,14 +627,14 @@ static int init_core(CudaData* dev, int nx, int ny, int nm, const double* mask,
   for (auto p : main_f)
     if (alloc_field(p, n)) return PFA_ECUDA;
   CK(cudaMalloc(reinterpret_cast<void**>(&s->ev), nucleation_event_bytes()));
-  CK(cudaMalloc(reinterpret_cast<void**>(&s->ev_count), 2 * sizeof(unsigned)));
+  CK(cudaMalloc(reinterpret_cast<void**>(&s->ev_count), kNucCounters * sizeof(unsigned)));
   s->cand_cap = nucleation_cand_cap(n);
   CK(cudaMalloc(reinterpret_cast<void**>(&s->cand), sizeof(long long) * size_t(s->cand_cap)));
   CK(cudaMalloc(reinterpret_cast<void**>(&s->ev_status), sizeof(int)));
   CK(cudaMalloc(reinterpret_cast<void**>(&s->call_dev), sizeof(unsigned long long)));
   CK(cudaMalloc(reinterpret_cast<void**>(&s->sum_partial), sizeof(double) * kSumBlocks * 5));
   CK(cudaMalloc(reinterpret_cast<void**>(&s->sum_out), sizeof(double) * 5));
-  CK(cudaMemsetAsync(s->ev_count, 0, 2 * sizeof(unsigned), s->st));
+  CK(cudaMemsetAsync(s->ev_count, 0, kNucCounters * sizeof(unsigned), s->st));
   CK(cudaMemsetAsync(s->ev_status, 0, sizeof(int), s->st));
   CK(cudaMemsetAsync(s->call_dev, 0, sizeof(unsigned long long), s->st));
   static bool nuc_ready = false;

@@ -47,7 +47,7 @@ struct Grid3D {
   double nuc_sigma[2] = {0.13, 0.13}, nuc_unit_a = 0.352e-9, nuc_d[3] = {}, nuc_dt = 0.0;
   uint64_t step_counter = 0;
   NucEvent* ev = nullptr;
-  unsigned* ev_count = nullptr;  // [0] events, [1] listed cells
+  unsigned* ev_count = nullptr;  // kNucCounters (NucArgs::count)
   int* ev_status = nullptr;
   unsigned long long* call_dev = nullptr;  // Philox call counter
   long long* cand = nullptr;               // cells left to the FP64 nucleation decision
@@ -368,12 +368,12 @@ static int create3d(void** handle, int nx, int ny, int nz, const double* params,
   CK3(cudaMalloc(reinterpret_cast<void**>(&g->sum_partial), sizeof(double) * kSumBlocks * 5));
   CK3(cudaMalloc(reinterpret_cast<void**>(&g->sum_out), sizeof(double) * 5));
   CK3(cudaMalloc(reinterpret_cast<void**>(&g->ev), nucleation_event_bytes()));
-  CK3(cudaMalloc(reinterpret_cast<void**>(&g->ev_count), 2 * sizeof(unsigned)));
+  CK3(cudaMalloc(reinterpret_cast<void**>(&g->ev_count), kNucCounters * sizeof(unsigned)));
   g->cand_cap = nucleation_cand_cap(size_t(g->Nx) * g->Ny * g->Nz);
   CK3(cudaMalloc(reinterpret_cast<void**>(&g->cand), sizeof(long long) * size_t(g->cand_cap)));
   CK3(cudaMalloc(reinterpret_cast<void**>(&g->ev_status), sizeof(int)));
   CK3(cudaMalloc(reinterpret_cast<void**>(&g->call_dev), sizeof(unsigned long long)));
-  CK3(cudaMemsetAsync(g->ev_count, 0, 2 * sizeof(unsigned), g->st));
+  CK3(cudaMemsetAsync(g->ev_count, 0, kNucCounters * sizeof(unsigned), g->st));
   CK3(cudaMemsetAsync(g->ev_status, 0, sizeof(int), g->st));
   CK3(cudaMemsetAsync(g->call_dev, 0, sizeof(unsigned long long), g->st));
   CK3(cudaStreamSynchronize(g->st));
@@ -425,7 +425,7 @@ int pfa3d_set_nucleation(void* handle, uint64_t seed, int interval, double sigma
   g->nuc_dt = dt_nuc;
   g->step_counter = 0;
   CK3(cudaMemsetAsync(g->call_dev, 0, sizeof(unsigned long long), g->st));
-  CK3(cudaMemsetAsync(g->ev_count, 0, 2 * sizeof(unsigned), g->st));
+  CK3(cudaMemsetAsync(g->ev_count, 0, kNucCounters * sizeof(unsigned), g->st));
   CK3(cudaStreamSynchronize(g->st));
   return 0;
 }

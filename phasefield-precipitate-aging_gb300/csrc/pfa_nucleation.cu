@@ -15,10 +15,10 @@
 //      u >= 2^-53 can fall below it, so skipping such cells changes no
 //      decision.  The cells the bound leaves open are listed (same atomic
 //      scheme) and
-//   1b. k_nuc_fp64 decides them in FP64, 32 listed cells per warp, with the
+//   1b. k_nuc_finish decides them in FP64, 32 listed cells per warp, with the
 //      same draws;
-//   2. k_nuc_apply: one CTA sorts the events by cell and paints them in that
-//      order, delta before laves (embed_OPC_kernel, :1046-1077).
+//   2. its last CTA sorts the events by cell and paints them in that order,
+//      delta before laves (embed_OPC_kernel, :1046-1077).
 // The event set does not depend on which kernel decided a cell, and the sort
 // fixes the painting order.
 #include <cmath>
@@ -129,31 +129,6 @@ __global__ void __launch_bounds__(256, 4) k_nuc_decide_own(NucArgs a) {
   }
 }
 
-// The FP64 decisions of the listed cells, 32 per warp.  Consecutive chunks
-// of 32 go to different CTAs (chunk c to CTA c mod gridDim.x): a short list
-// then spreads over the SMs instead of queueing on one SM's FP64 unit.
-template <class T>
-__global__ void __launch_bounds__(256) k_nuc_fp64(NucArgs a) {
-  const unsigned n = min(a.count[1], unsigned(a.cand_cap));
-  const int lane = threadIdx.x & 31;
-  const unsigned chunks = (n + 31) / 32;
-  const unsigned step = gridDim.x * (blockDim.x >> 5);
-  const long long nxr = a.Nx + 2, nyr = a.Ny + 2;
-  for (unsigned c = blockIdx.x + gridDim.x * (threadIdx.x >> 5); c < chunks; c += step) {
-    const unsigned i = 32 * c + lane;
-    bool ev = false;
-    NucEvent e;
-    if (i < n) {
-      const long long idx = a.cand[i];
-      const int x = int(idx % nxr);
-      const long long t = idx / nxr;
-      const int y = int(t % nyr), z = int(t / nyr);
-      ev = decide64<T>(a, idx, stor(a, x, y, z), nuc_draw(a, idx), e);
-    }
-    append_events(a, ev, e);
-  }
-}
-
 // store v at cell s of field k (and its compensation: value = hi - c)
 template <class T>
 __device__ __forceinline__ void put(const NucArgs& a, int k, size_t s, double v) {
@@ -254,12 +229,9 @@ __device__ void paint_own(const NucArgs& a, const NucEvent& e) {
     }
 }
 
+// The call's events painted by one block; n: their number
 template <class T>
-__global__ void __launch_bounds__(1024) k_nuc_apply(NucArgs a) {
-  const unsigned n = *a.count;
-  __syncthreads();
-  // the decision kernel of this call has read the counter: advance it
-  if (threadIdx.x == 0) *a.call_ptr += 1ull;
+__device__ void apply_events(const NucArgs& a, unsigned n) {
   if (n == 0) return;
   if (n > unsigned(a.cap)) {
     if (threadIdx.x == 0) *a.status = 1;  // overflow: nothing painted
@@ -311,11 +283,53 @@ __global__ void __launch_bounds__(1024) k_nuc_apply(NucArgs a) {
   }
 }
 
+// The FP64 decisions of the listed cells, 32 per warp, then the painting by
+// the last block to finish (each block a ticket; one launch, 2.9 us, less than
+// with a kernel of its own).  Consecutive chunks of 32 cells go to different
+// CTAs (chunk c to CTA c mod gridDim.x): a short list then spreads over the
+// SMs instead of queueing on one SM's FP64 unit.  The last block also
+// publishes the number of events and clears the counters for the next call
+// (instead of a memset before each).
+template <class T>
+__global__ void __launch_bounds__(512) k_nuc_finish(NucArgs a) {
+  const unsigned n = min(a.count[1], unsigned(a.cand_cap));
+  const int lane = threadIdx.x & 31;
+  const unsigned chunks = (n + 31) / 32;
+  const unsigned step = gridDim.x * (blockDim.x >> 5);
+  const long long nxr = a.Nx + 2, nyr = a.Ny + 2;
+  for (unsigned c = blockIdx.x + gridDim.x * (threadIdx.x >> 5); c < chunks; c += step) {
+    const unsigned i = 32 * c + lane;
+    bool ev = false;
+    NucEvent e;
+    if (i < n) {
+      const long long idx = a.cand[i];
+      const int x = int(idx % nxr);
+      const long long t = idx / nxr;
+      const int y = int(t % nyr), z = int(t / nyr);
+      ev = decide64<T>(a, idx, stor(a, x, y, z), nuc_draw(a, idx), e);
+    }
+    append_events(a, ev, e);
+  }
+  __shared__ bool s_last;
+  __threadfence();  // this thread's events, before its block's ticket
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(a.count + 3, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const unsigned events = __ldcg(a.count + 2);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.count[0] = events;
+    a.count[1] = a.count[2] = a.count[3] = 0;
+    *a.call_ptr += 1ull;  // every block of this call has read it
+  }
+  apply_events<T>(a, events);
+}
+
 }  // namespace
 
 cudaError_t launch_nucleation(const NucArgs& a, cudaStream_t s) {
-  cudaError_t err = cudaMemsetAsync(a.count, 0, 2 * sizeof(unsigned), s);
-  if (err != cudaSuccess) return err;
   dim3 grid((a.Nx + 31) / 32, (a.Ny + 7) / 8, a.is3d ? a.Nz : 1);
   const bool own = a.scan_lo == 0 && a.scan_hi == 1;  // the scan covers each cell alone
   // grid-stride over the FP64 list (its length is on the device): a CTA per SM
@@ -327,15 +341,13 @@ cudaError_t launch_nucleation(const NucArgs& a, cudaStream_t s) {
       k_nuc_decide_own<float><<<grid_own, 256, 0, s>>>(a);
     else
       k_nuc_decide<float><<<grid, 256, 0, s>>>(a);
-    k_nuc_fp64<float><<<fp64_blocks, 256, 0, s>>>(a);
-    k_nuc_apply<float><<<1, 1024, 0, s>>>(a);
+    k_nuc_finish<float><<<fp64_blocks, 512, 0, s>>>(a);
   } else {
     if (own)
       k_nuc_decide_own<double><<<grid_own, 256, 0, s>>>(a);
     else
       k_nuc_decide<double><<<grid, 256, 0, s>>>(a);
-    k_nuc_fp64<double><<<fp64_blocks, 256, 0, s>>>(a);
-    k_nuc_apply<double><<<1, 1024, 0, s>>>(a);
+    k_nuc_finish<double><<<fp64_blocks, 512, 0, s>>>(a);
   }
   return cudaGetLastError();
 }

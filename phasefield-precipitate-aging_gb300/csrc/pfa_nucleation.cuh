@@ -302,7 +302,7 @@ __device__ __forceinline__ void append_events(const NucArgs& a, bool ev, const N
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(bal) - 1;
   unsigned base = 0;
-  if (lane == leader) base = atomicAdd(a.count, unsigned(__popc(bal)));
+  if (lane == leader) base = atomicAdd(a.count + 2, unsigned(__popc(bal)));
   base = __shfl_sync(0xffffffffu, base, leader);
   if (ev) {
     const unsigned slot = base + __popc(bal & ((1u << lane) - 1u));
@@ -350,7 +350,7 @@ __device__ __forceinline__ bool nuc_screen(const NucArgs& a, float X, float Y, l
   return nuc_screen_rest(a, X, Y, idx, p, lnz[0], lnz[1], &w);
 }
 
-// Cells the screen cannot settle go to k_nuc_fp64 as a compact list: a warp
+// Cells the screen cannot settle go to k_nuc_finish as a compact list: a warp
 // issues the FP64 path if any of its lanes needs it, so in place a few such
 // cells would cost whole warps.  Cells past the list's capacity decide here,
 // from the stored values at storage index s.  Whole warp.

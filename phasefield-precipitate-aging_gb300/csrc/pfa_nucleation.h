@@ -8,6 +8,7 @@
 namespace pfa {
 
 constexpr int kNucCap = 1 << 14;  // events per nucleation call (scratch capacity)
+constexpr int kNucCounters = 4;   // NucArgs::count, zero before the first call
 constexpr int kNucIdxBits = 14;   // low key bits carrying the event index
 constexpr double kNucMaxScan = 64.0;    // largest neighbourhood scan radius (cells)
 constexpr double kNucMaxRadius = 256.0; // largest nucleus radius painted (cells)
@@ -47,7 +48,8 @@ struct NucArgs {
   unsigned long long* call_ptr;  // scratch: nucleation call counter (Philox counter word)
   NucEvent* events;    // scratch: kNucCap events, then kNucCap sort keys
   unsigned long long* keys;  // = (unsigned long long*)(events + kNucCap)
-  unsigned* count;     // scratch: [0] events, [1] cells listed for the FP64 decision
+  unsigned* count;     // [0] events of the last call; scratch, zero between calls: [1] cells listed
+                       // for the FP64 decision, [2] events so far, [3] blocks finished
   int* status;         // scratch: 1 = overflow
   int cap;
   long long* cand;     // scratch: cells the FP32 screen left to the FP64 decision
