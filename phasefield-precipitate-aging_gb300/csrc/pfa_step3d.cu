@@ -474,23 +474,30 @@ __global__ void k_export3d(Conv3DArgs a) {
   }
 }
 
-// z planes per segment: fill whole waves of resident CTAs, two extra planes
-// of gamma solves per segment; tiles of tx x ty output cells per plane.
-// Segments under 16 planes only where they fit one wave: a small grid's
-// columns leave SMs idle otherwise (FP32, us per step, whole columns ->
-// one wave of short segments: 32^3 29.4 -> 3.7, 64^3 47.5 -> 7.8, 96^3
-// 64.7 -> 13.0, 200 x 100 x 60 42.5 -> 17.4).
+// z planes per segment, tiles of tx x ty output cells per plane.  Large grids:
+// whole waves of resident CTAs, two extra planes of gamma solves per segment.
+// Small ones are bound by a segment's serial planes (0.85 us each), so the
+// segments are as short as fill the SMs once, then the resident slots once and
+// twice (us a step at that length, and in whole waves of at least 16 planes:
+// 32^3 3.5 and 16, 48^3 5.2 and 16, 64^3 6.9 and 16, 80^3 12.3 and 16, 47 x 191 x
+// 85 16.1 and 17.4, 110^3 21.0 and 23.7, 128^3 26.2 and 26.7, 178 x 47 x 202 23.4
+// and 25.8; from 150^3 on, 42 and 38, whole waves are the better way).
 int segment_planes(int Nx, int Ny, int Nz, int resident, int tx, int ty) {
   const long long cols = (long long)((Nx + tx - 1) / tx) * ((Ny + ty - 1) / ty);
+  const long long n = cols * Nz, r = resident;  // planes of tiles, CTAs
+  auto parts = [&](long long ctas) { return int(std::min<long long>((n + ctas - 1) / ctas, Nz)); };
+  if (2 * n <= 5 * r) return parts(std::max(1ll, r / 2));
+  if (n <= 10 * r) return parts(r);
+  if (n <= 20 * r) return parts(2 * r);
   int best = Nz;
   double best_score = 0.0;
   for (int waves = 1; waves <= 256; waves++) {
-    const long long segs = (long long)waves * resident / cols;
+    const long long segs = waves * r / cols;
     if (segs < 1) continue;
     const int planes = int((Nz + segs - 1) / segs);
-    if (planes < 16 && segs > 1 && waves > 1) break;
+    if (planes < 16 && segs > 1) break;
     const long long used = cols * ((Nz + planes - 1) / planes);
-    const long long slots = ((used + resident - 1) / resident) * (long long)resident;
+    const long long slots = ((used + r - 1) / r) * r;
     const double score = double(used) / double(slots) / (1.0 + 2.0 / planes);
     if (score > best_score) {
       best_score = score;
