@@ -229,7 +229,7 @@ template <int KIND>
 PFA_FIX_FN bool solve_fixed(uint64_t x, uint64_t y, uint64_t fd, uint64_t fl, int64_t& h1, int64_t& h2) {
   constexpr bool D = KIND & 1, L = KIND & 2;
   const uint64_t pD = D ? p63(fd) : 0, pL = L ? p63(fl) : 0;
-  if (pD + pL > kOne63) return false;
+  if (pD > kOne63 || pL > kOne63 - pD) return false;  // (their sum wraps where both are 1)
   const uint64_t pG = kOne63 - pD - pL;
   constexpr FictRow a = kFict[0][0], b = kFict[0][1];
   static_assert(a.l[0] > 0 && a.l[2] > 0 && a.m[0] < 0 && a.m[2] < 0 && a.q[0] > 0 && a.q[1] > 0 &&

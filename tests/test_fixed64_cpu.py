@@ -1,0 +1,95 @@
+"""The FP64 step's 64-bit fixed-point forms (csrc/pfa_fixed64.cuh), compiled for
+the host, against the expressions they stand for in extended precision."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import PKG_DIR
+
+SOURCE = r"""
+#include <cstdint>
+#include "pfa_fixed64.cuh"
+using namespace pfa;
+using namespace pfa::dev;
+
+static uint64_t f63(double v) { return uint64_t(v * 0x1p63); }  // v in [0, 1]: exact to 2^-63
+
+extern "C" int solve(int kind, double x, double y, double d, double l, double* g) {
+  int64_t h1 = 0, h2 = 0;
+  const bool ok = kind == 1   ? solve_fixed<1>(f63(x), f63(y), f63(d), f63(l), h1, h2)
+                  : kind == 2 ? solve_fixed<2>(f63(x), f63(y), f63(d), f63(l), h1, h2)
+                              : solve_fixed<3>(f63(x), f63(y), f63(d), f63(l), h1, h2);
+  g[0] = h1 * 0x1p-60;
+  g[1] = h2 * 0x1p-60;
+  return ok;
+}
+
+// x^gamma from the monomials, in long double
+extern "C" void exact(double x, double y, double d, double l, double* g) {
+  typedef long double T;
+  auto p = [](T v) { return v * v * v * (6 * v * v - 15 * v + 10); };
+  const T pD = p(d), pL = p(l), pG = 1 - pD - pL;
+  const T mono[6] = {pD * pD, pD * pG, pD * pL, pG * pG, pG * pL, pL * pL};
+  T den = 0;
+  for (int k = 0; k < 6; k++) den += T(kDen[k]) * mono[k];
+  for (int c = 0; c < 2; c++) {
+    const FictRow r = kFict[0][c];
+    T n = T(x) * (r.l[0] * pD + r.l[1] * pG + r.l[2] * pL) + T(y) * (r.m[0] * pD + r.m[1] * pG + r.m[2] * pL);
+    for (int k = 0; k < 6; k++) n += T(r.q[k]) * mono[k];
+    g[c] = double(T(r.scale) * n / den);
+  }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def fixed(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fixed64")
+    src, lib = d / "fixed64.cpp", d / "libfixed64.so"
+    src.write_text(SOURCE)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(os.environ.get("NVCC", "nvcc")))))
+    subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-I", os.path.join(PKG_DIR, "csrc"),
+                    "-I", os.path.join(cuda, "include"), str(src), "-o", str(lib)], check=True)
+    L = ctypes.CDLL(str(lib))
+    D = ctypes.c_double
+    L.solve.argtypes = [ctypes.c_int, D, D, D, D, ctypes.POINTER(D)]
+    L.exact.argtypes = [D, D, D, D, ctypes.POINTER(D)]
+    L.exact.restype = None
+    return L
+
+
+def _solve(L, kind, x, y, d, l):
+    g, e = (ctypes.c_double * 2)(), (ctypes.c_double * 2)()
+    ok = L.solve(kind, x, y, d, l, g)
+    L.exact(x, y, d, l, e)
+    return ok, np.array(g), np.array(e)
+
+
+def test_solve_refuses_fractions_that_add_up_to_more_than_one(fixed):
+    """Each phase up to exactly 1 (what nucleation paints), both of them too:
+    p = 2^63 twice, whose sum is 2^64."""
+    for d in (0.6, 0.95, 1.0 - 2.0 ** -53, 1.0):
+        for l in (0.6, 0.95, 1.0 - 2.0 ** -53, 1.0):
+            assert not _solve(fixed, 3, 0.3, 0.02, d, l)[0], (d, l)
+
+
+def test_solve_over_the_square_of_phases(fixed):
+    """Whatever solve_fixed accepts is x^gamma: within 64 units of 2^-53 (28 in
+    20 million random states), where the FP64 forms are off by thousands."""
+    phases = [0.0, 1e-7, 1e-3, 0.2, 0.5, 0.8, 0.999, 1.0 - 1e-9, 1.0 - 2.0 ** -53, 1.0]
+    comps = [2.0 ** -11, 0.01, 0.0229, 0.1, 0.3, 0.5, 0.9, 1.0 - 2.0 ** -53]
+    taken = 0
+    for kind, ds, ls in ((1, phases, [0.0]), (2, [0.0], phases), (3, phases, phases)):
+        for d in ds:
+            for l in ls:
+                for x in comps:
+                    for y in comps:
+                        ok, g, e = _solve(fixed, kind, x, y, d, l)
+                        if ok:
+                            taken += 1
+                            assert np.all(np.abs(g - e) <= 64 * 2.0 ** -53), (kind, x, y, d, l)
+    assert taken > 1000
