@@ -292,9 +292,9 @@ __device__ __forceinline__ double allen_cahn_linear64(const Coef64& K, double ph
 //    to its bits, so the sum is rounded once, like the FP64 addition (a
 //    result in another binade goes through FP64).
 // 14 FP64 operations (266 cycles of an SM per warp) become about 65 integer
-// ones.  Valid for compositions in [2^-11, 1) (in_unit) and |x^gamma| below a
-// few units (the neighbour sum must stay below 2^5); a tile with any other
-// value takes the FP64 forms.
+// ones.  Valid for compositions in [2^-11, 1) (in_unit) and x^gamma in the
+// range of the mask (Range60, pfa_fixed64.cuh); a tile with any other value
+// takes the FP64 forms.
 
 // v in [2^-11, 1)
 __device__ __forceinline__ bool in_unit(double v) {

@@ -282,6 +282,21 @@ PFA_FIX_FN bool solve_fixed(uint64_t x, uint64_t y, uint64_t fd, uint64_t fl, in
   return true;
 }
 
+// The x^gamma, in units of 2^-60, whose weighted neighbour sums stay in range:
+// low <= h < most.  A cell without a solve has x^gamma in [0, 1).
+struct Range60 {
+  int64_t low, most;
+};
+// The sums of 5 points (2D) and 7 (3D), weights 1 and -4 or -6, in units of
+// 2^-58: a 64-bit sum holds +-32, these reach 4 x 2 + 4 x 2 = 16 and 24.
+constexpr Range60 kRangeFaces = {-(1ll << 61), 1ll << 61};
+// 9 points, weights 4, 1 and -20: 20 (1 + 9/16) = 31.25.
+constexpr Range60 kRangeCorners = {-(9ll << 56), 1ll << 60};
+// A face's difference for the fluxes of the variable mobility, in units of
+// 2^-62: +-2 (the 2: h is rounded to units of 2^-58).
+constexpr Range60 kRangeFlux = {-(1ll << 60), (1ll << 60) - 2};
+constexpr Range60 kRangeNone = {0, 0};  // FP64 values are wanted
+
 // FP64 bits of v 2^-q
 PFA_FIX_FN uint64_t pack_signed(int64_t v, int q) {
   if (v == 0) return 0;

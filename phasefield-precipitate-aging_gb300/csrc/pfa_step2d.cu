@@ -119,12 +119,12 @@ __device__ __forceinline__ bool none64(const double (*s)[P], int ex, int ey) {
 }
 
 template <bool FIXED, bool HOT>
-__device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy, int64_t most) {
+__device__ __forceinline__ Cell64 stage64(const Step2DArgs& a, int gx, int gy, Range60 range) {
   const size_t i = size_t(clampi(gy, 0, a.Ny - 1) + 1) * a.pitch + clampi(gx, 0, a.Nx - 1) + 1;
   Cell64 c = cell64<FIXED, HOT>(__ldg(static_cast<const double*>(a.in[0]) + i),
                            __ldg(static_cast<const double*>(a.in[1]) + i),
                            __ldg(static_cast<const double*>(a.in[2]) + i),
-                           __ldg(static_cast<const double*>(a.in[3]) + i), most);
+                           __ldg(static_cast<const double*>(a.in[3]) + i), range);
   c.i = i;
   return c;
 }
@@ -154,8 +154,7 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
     k_step2d_f64(const __grid_constant__ Step2DArgs a) {
   using T = Tile2<MASK, TX, TY>;
   constexpr bool kFixed = MASK == kMaskIso || MASK == kMaskIso9;
-  // |x^gamma| < 2 (5 points) or 1 (9 points): the neighbour sum stays below 2^5
-  constexpr int64_t kMost = MASK == kMaskIso9 ? 1ll << 60 : 1ll << 61;
+  constexpr Range60 kRange = MASK == kMaskIso9 ? kRangeCorners : kRangeFaces;
   // x^gamma as doubles, or (kFixed) in fixed point
   __shared__ typename T::template Plane<long long> s_g1, s_g2;
   __shared__ typename T::template Plane<double> s_pd, s_pl;
@@ -163,7 +162,7 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
   int ex, ey;
   const bool staged = T::cell(ex, ey);
   const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
-  const Cell64 c = stage64<kFixed, HOT>(a, gx, gy, kMost);
+  const Cell64 c = stage64<kFixed, HOT>(a, gx, gy, kRange);
   if (staged) {
     s_g1[ey][ex] = c.g1;
     s_g2[ey][ex] = c.g2;
@@ -246,7 +245,7 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, TX == 16 ? 3 : 
   int ex, ey;
   const bool staged = T::cell(ex, ey);
   const int gx = int(blockIdx.x) * TX + ex - 1, gy = tile_row() * TY + ey - 1;
-  const Cell64 c = stage64<ISO, true>(a, gx, gy, 1ll << 60);
+  const Cell64 c = stage64<ISO, true>(a, gx, gy, kRangeFlux);
   const bool unit = in_unit(c.X) && in_unit(c.Y);
   bool wide = true;
   long long d[4];

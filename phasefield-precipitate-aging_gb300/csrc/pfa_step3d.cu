@@ -100,8 +100,7 @@ __global__ void __launch_bounds__(Tile3::kThreads, HOT ? 7 : 8)
     return Record{__ldg(static_cast<const double*>(a.in[0]) + i), __ldg(static_cast<const double*>(a.in[1]) + i),
                   __ldg(static_cast<const double*>(a.in[2]) + i), __ldg(static_cast<const double*>(a.in[3]) + i)};
   };
-  // |x^gamma| < 2: the seven-point sum stays below 2^5
-  auto stage = [&](const Record& r) { return cell64<ISO, HOT>(r.X, r.Y, r.pd, r.pl, 1ll << 61); };
+  auto stage = [&](const Record& r) { return cell64<ISO, HOT>(r.X, r.Y, r.pd, r.pl, kRangeFaces); };
   Cell64 P, C, N;  // planes z - 1, z, z + 1 of the thread's column
   Record next;     // the record of the plane after them
   if constexpr (HOT) {

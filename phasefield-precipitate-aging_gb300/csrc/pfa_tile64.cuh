@@ -78,16 +78,14 @@ __device__ __forceinline__ bool fraction(double v) {
 }
 
 // x^gamma of a cell next to a precipitate; take: in the range of solve_fixed;
-// kinds: the forms of it that the warp needs; most: the bound of 2^60
-// |x^gamma| for the fixed-point sums (the neighbour sum has to stay below
-// 2^5), 0: FP64 values are wanted.  (A call: its registers would weigh on the
-// cells that need none.)
+// kinds: the forms of it that the warp needs; range: of the fixed-point sums.
+// (A call: its registers would weigh on the cells that need none.)
 struct Gamma64 {
   long long g1, g2;
   bool wide;
 };
 static __device__ __noinline__ Gamma64 gamma_cell(double X, double Y, double pd, double pl, bool take, int kinds,
-                                                  int64_t most) {
+                                                  Range60 range) {
   Gamma64 g;
   int64_t h1, h2;
   const uint64_t x = fix64(X) >> 1, y = fix64(Y) >> 1;
@@ -95,7 +93,7 @@ static __device__ __noinline__ Gamma64 gamma_cell(double X, double Y, double pd,
   if (take && (kinds == 3   ? solve_fixed<3>(x, y, fd, fl, h1, h2)
                : kinds == 1 ? solve_fixed<1>(x, y, fd, fl, h1, h2)
                             : solve_fixed<2>(x, y, fd, fl, h1, h2))) {
-    g.wide = max(llabs(h1), llabs(h2)) >= most;
+    g.wide = min(h1, h2) < range.low || max(h1, h2) >= range.most;
     g.g1 = g.wide ? __double_as_longlong(value60(h1)) : (h1 + 2) >> 2;
     g.g2 = g.wide ? __double_as_longlong(value60(h2)) : (h2 + 2) >> 2;
   } else {
@@ -112,7 +110,7 @@ static __device__ __noinline__ Gamma64 gamma_cell(double X, double Y, double pd,
 // point (else in FP64, inline: no call, so that a kernel with many waves of
 // tiles without precipitate keeps its occupancy)
 template <bool FIXED, bool HOT>
-__device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double pl, int64_t most) {
+__device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double pl, Range60 range) {
   Cell64 c;
   c.X = X;
   c.Y = Y;
@@ -134,7 +132,7 @@ __device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double p
       const int kinds = int(__any_sync(0xffffffffu, take && mag_hi(pd) >= kSolveHi)) +
                         2 * int(__any_sync(0xffffffffu, take && mag_hi(pl) >= kSolveHi));
       if (c.solved) {
-        const Gamma64 g = gamma_cell(X, Y, pd, pl, take, kinds, FIXED ? most : 0);
+        const Gamma64 g = gamma_cell(X, Y, pd, pl, take, kinds, FIXED ? range : kRangeNone);
         c.g1 = g.g1;
         c.g2 = g.g2;
         c.wide = g.wide;
@@ -145,8 +143,10 @@ __device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double p
     solve64(c.solved, c.big, X, Y, pd, pl, g1, g2);
     c.v1 = g1;
     c.v2 = g2;
-    const double bound = double(most) * 0x1p-60;
-    if (c.solved && max(mag_hi(g1), mag_hi(g2)) >= __double2hiint(bound)) c.wide = true;
+    // (the bounds of the ranges used here have no low word)
+    const int low = __double2hiint(double(-range.low) * 0x1p-60), most = __double2hiint(double(range.most) * 0x1p-60);
+    auto out = [&](double g) { return mag_hi(g) >= (__double2hiint(g) < 0 ? low : most); };
+    if (c.solved && (out(g1) || out(g2))) c.wide = true;
     if (c.wide) {
       c.g1 = __double_as_longlong(g1);
       c.g2 = __double_as_longlong(g2);

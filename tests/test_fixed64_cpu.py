@@ -28,6 +28,14 @@ extern "C" int solve(int kind, double x, double y, double d, double l, double* g
   return ok;
 }
 
+extern "C" void ranges(int64_t* r) {
+  const Range60 v[3] = {kRangeFaces, kRangeCorners, kRangeFlux};
+  for (int k = 0; k < 3; k++) {
+    r[2 * k] = v[k].low;
+    r[2 * k + 1] = v[k].most;
+  }
+}
+
 // x^gamma from the monomials, in long double
 extern "C" void exact(double x, double y, double d, double l, double* g) {
   typedef long double T;
@@ -60,6 +68,35 @@ def fixed(tmp_path_factory):
     L.exact.argtypes = [D, D, D, D, ctypes.POINTER(D)]
     L.exact.restype = None
     return L
+
+
+def _extremes(fixed, which):
+    """Least and largest staged x^gamma, in units of 2^-58: a solved cell's,
+    rounded as gamma_cell does, or the composition of a cell without a solve."""
+    r = (ctypes.c_int64 * 6)()
+    fixed.ranges(r)
+    low, most = r[2 * which], r[2 * which + 1]
+    return (low + 2) >> 2, max((most - 1 + 2) >> 2, 2 ** 58 - 2 ** 5)
+
+
+@pytest.mark.parametrize("which,around,centre", [(0, 4, 4), (0, 6, 6), (1, 4 * 4 + 4, 20)])
+def test_neighbour_sums_stay_in_range(fixed, which, around, centre):
+    """The weighted sum of any cells in range fits 64 bits, and so does the
+    increment D0 S1 + D1 S2 with D below 2^-7, its rounding included."""
+    a, b = _extremes(fixed, which)
+    D = 2 ** 63 - 2 ** 10  # the largest D 2^70
+    for s in (around * b - centre * a, around * a - centre * b):
+        assert -2 ** 63 <= s < 2 ** 63
+        assert abs(2 * (D * s >> 64)) + 1 + 2 ** 10 < 2 ** 63
+
+
+def test_face_differences_stay_in_range(fixed):
+    """(u_n - u_c) 2^4, units of 2^-62, of the variable mobility's fluxes; each
+    flux (two products with sums of two D below 2^-5, in units of 2^-65)."""
+    a, b = _extremes(fixed, 2)
+    u = (b - a) << 4
+    assert u < 2 ** 63
+    assert 2 * ((2 ** 63 - 2) * u >> 64) + 2 < 2 ** 63
 
 
 def _solve(L, kind, x, y, d, l):

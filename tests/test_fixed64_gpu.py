@@ -85,3 +85,34 @@ def test_step_after_nuclei_of_both_kinds(pfa, orc):
     want, _, _ = orc.nucleation2d(f, nuc_struct(nuc), 99, 0)
     assert np.sum((want[2] == 1.0) & (want[3] == 1.0)) > 100
     check_cells(got, orc.run2d(want, O.model_params(), 1), TOL)
+
+
+# x^gamma of the two signs side by side: single cells of a delta domain whose
+# x_Nb lies 0.0045 to 0.006 above or below that of their neighbours (x^gamma_Cr
+# 0.8 and -0.8), single laves cells (-0.9) in a matrix of x_Cr 0.75.  The second
+# size of a mask as above.
+@pytest.mark.parametrize("mask", ["iso", "nine", "five", "variable", "3d"])
+@pytest.mark.parametrize("large", [False, True])
+def test_steep_gamma(pfa, orc, mask, large):
+    if mask == "3d":
+        shape = (70, 248, 248) if large else (9, 40, 37)
+    else:
+        shape = (905, 1000) if large else (210, 190)
+    rng = np.random.default_rng(11)
+    i = np.indices(shape)
+    single = np.all(i % 3 == 1, axis=0)
+    third = i[-1] * 3 // shape[-1]
+    x, y = np.full(shape, 0.02297), np.full(shape, 0.24905)
+    d, l = np.ones(shape), np.zeros(shape)
+    # (up to 0.0052 in half of the rows: |x^gamma| stays below 1 there)
+    step = rng.uniform(0.0045, np.where(i[-2] * 2 < shape[-2], 0.0052, 0.006))
+    y[(third == 0) & single] += step[(third == 0) & single]
+    y[third == 1] = 0.25385
+    y[(third == 1) & single] -= step[(third == 1) & single]
+    last = third == 2
+    x[last], y[last], d[last] = 0.75, 0.02, 0.0
+    last &= single
+    x[last] = rng.uniform(0.06, 0.12, shape)[last]
+    y[last], l[last] = 0.25, 1.0
+    got, want = step_and_oracle(pfa, orc, mask, [x, y, d, l])
+    check_cells(got, want, TOL)
