@@ -191,6 +191,18 @@ PFA_FIX_FN bool diffusivities(const Coef64& K, uint64_t x, uint64_t y, long long
   return ok;
 }
 
+// t = n - s + e - w, the fluxes through a cell's faces (units of 2^-65: each
+// below 1/4); false where a sum leaves 64 bits.  Diffusivities up to 2^-5 let
+// four faces reach 1/2 (found: 0.264 at 3.6 times the usual time step).  The
+// test costs the step 0.6 % (512^2); fluxes in units of 2^-63 would need none,
+// at two bits less.
+PFA_FIX_FN bool face_sum(int64_t n, int64_t s, int64_t e, int64_t w, int64_t& t) {
+  const uint64_t a = uint64_t(n) - uint64_t(s), b = uint64_t(e) - uint64_t(w), c = a + b;
+  const uint64_t un = uint64_t(n), ue = uint64_t(e);
+  t = int64_t(c);
+  return int64_t(((un ^ uint64_t(s)) & (un ^ a)) | ((ue ^ uint64_t(w)) & (ue ^ b)) | ((a ^ c) & (b ^ c))) >= 0;
+}
+
 // ---- x^gamma ----
 // All numbers are unsigned multiples of 2^-63 (1 is 2^63); signs are those of
 // the coefficients (kFict, kDen), known at compile time.

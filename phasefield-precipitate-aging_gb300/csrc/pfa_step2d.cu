@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
 //
 // ISO (equal spacings): all of it in fixed point where every cell of the tile
 // is in range: u in units of 2^-58, D of 2^-67 (pfa_fixed64.cuh), the fluxes of
-// 2^-65, whose differences are rounded once into the compositions; else, and
-// with other spacings, in FP64.  Bound by integer issue; with the matrix and
+// 2^-65, whose sum is rounded once into the composition (a sum that leaves 64
+// bits is formed in FP64); else, and with other spacings, in FP64.  Bound by integer issue; with the matrix and
 // the fluxes in FP64, bound by that pipe, 512^2 took 38.9 us a step for 20.8,
 // 2048^2 521 for 237.
 struct Matrix64 {
@@ -231,6 +231,11 @@ static __device__ __noinline__ Matrix64 matrix64(const Coef64& K, double X, doub
   Matrix64 m;
   dmatrix64_scaled(K, X, Y, unit, m.d[0], m.d[1], m.d[2], m.d[3]);
   return m;
+}
+
+// X and its faces' fluxes (units of 2^-65) where their sum leaves 64 bits
+static __device__ __noinline__ double advance_faces(double X, long long n, long long s, long long e, long long w) {
+  return X + ((double(n) - double(s)) + (double(e) - double(w))) * 0x1p-65;
 }
 
 template <bool ISO, int TX, int TY>
@@ -310,7 +315,10 @@ __global__ void __launch_bounds__(Tile<TX, TY, false>::kThreads, TX == 16 ? 3 : 
   const int tx = ex - 1, ty = ey - 1;
   auto sum = [&](int k, double X) {  // the faces' fluxes added to a composition
     const long long n = s_fy[k][ty + 1][tx], s = s_fy[k][ty][tx], e = s_fx[k][ty][tx + 1], w = s_fx[k][ty][tx];
-    if (fixed) return advance_by(X, ((n - s) + (e - w) + 1) >> 1);
+    if (fixed) {
+      int64_t t;
+      return face_sum(n, s, e, w, t) ? advance_by(X, (t >> 1) + (t & 1)) : advance_faces(X, n, s, e, w);
+    }
     return X + fma(K.vm_qy, __longlong_as_double(n) - __longlong_as_double(s),
                    __longlong_as_double(e) - __longlong_as_double(w));
   };

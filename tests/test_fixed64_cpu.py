@@ -28,6 +28,8 @@ extern "C" int solve(int kind, double x, double y, double d, double l, double* g
   return ok;
 }
 
+extern "C" int sum_of_faces(int64_t n, int64_t s, int64_t e, int64_t w, int64_t* t) { return face_sum(n, s, e, w, *t); }
+
 extern "C" void ranges(int64_t* r) {
   const Range60 v[3] = {kRangeFaces, kRangeCorners, kRangeFlux};
   for (int k = 0; k < 3; k++) {
@@ -97,6 +99,27 @@ def test_face_differences_stay_in_range(fixed):
     u = (b - a) << 4
     assert u < 2 ** 63
     assert 2 * ((2 ** 63 - 2) * u >> 64) + 2 < 2 ** 63
+
+
+def test_face_sum(fixed):
+    """The sum of four fluxes, or its refusal where it leaves 64 bits (or one
+    of its two differences does): never a wrapped one."""
+    I = ctypes.c_int64
+    fixed.sum_of_faces.argtypes = [I, I, I, I, ctypes.POINTER(I)]
+    top = 2 ** 63 - 1
+    values = [0, 1, -1, 2 ** 61, -2 ** 61, 2 ** 62 - 1, 2 ** 62, -2 ** 62, -2 ** 62 - 1, top, -top, -top - 1]
+    rng = np.random.default_rng(0)
+    cases = [[int(v) for v in rng.choice(len(values), 4)] for _ in range(4000)]
+    t = I()
+    refused = 0
+    for n, s, e, w in ([values[k] for k in c] for c in cases):
+        ok = fixed.sum_of_faces(n, s, e, w, ctypes.byref(t))
+        if all(-top - 1 <= v <= top for v in (n - s, e - w, n - s + e - w)):
+            assert ok and t.value == n - s + e - w
+        else:
+            assert not ok
+            refused += 1
+    assert 400 < refused < 3600
 
 
 def _solve(L, kind, x, y, d, l):

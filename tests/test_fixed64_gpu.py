@@ -116,3 +116,27 @@ def test_steep_gamma(pfa, orc, mask, large):
     y[last], l[last] = 0.25, 1.0
     got, want = step_and_oracle(pfa, orc, mask, [x, y, d, l])
     check_cells(got, want, TOL)
+
+
+# faces whose four fluxes add up to more than 1/4 (the integers' range) with
+# every diffusivity and x^gamma in the range of the fixed point, and of either
+# sign, at twelve times the usual time step (the constant mobilities, unused,
+# scaled down so that the mask keeps its fixed-point form)
+@pytest.mark.parametrize("nx,ny", [(60, 45), (400, 390)])
+def test_large_fluxes(pfa, orc, nx, ny):
+    shape = (ny, nx)
+    rng = np.random.default_rng(13)
+    i = np.indices(shape)
+    single = np.all(i % 3 == 1, axis=0)
+    flip = (i[0] // 16 + i[1] // 16) % 2 == 1
+    laves = (0.4089737663928951, 0.056577406168092814, 0.0, 1.0)
+    delta = (0.0093396110639775015, 0.51067932596175425, 0.590024, 0.0)
+    f = []
+    for k in range(4):
+        a = np.where(single != flip, laves[k], delta[k])
+        f.append(a * (1.0 - 0.01 * rng.random(shape)) if k < 2 else a)
+    p = pfa.model_params()
+    small = {k: [0.25 * v for v in p[k]] for k in ("D_Cr", "D_Nb")}
+    got, want = step_and_oracle(pfa, orc, "variable", f, dt=12 * p["dt"], **small)
+    assert np.max(np.abs(want[1][1:-1, 1:-1] - f[1])) > 0.27
+    check_cells(got, want, TOL)
