@@ -174,19 +174,18 @@ __device__ __forceinline__ double dlap64(double Dl, double Dm, double Dh, double
 // all cells are folded on the host (Coef64), tests are integer tests on the
 // high words, and a cell takes the cheapest form that rounds to the same
 // values:
-//   kSolveHi: |phi| < 1e-7 in both phases.  p(phi) = 10 phi^3 < 1e-20, so the
-//     general solve returns X, Y themselves (p shifts them by less than half
-//     an ulp) and is skipped;
-//   kLinearHi: |phi| < 2^-60.  p' dP and the cubic terms of the double well
-//     are below 2^-53 of 2 omega phi, and so is the coupling to the other
-//     phase where that is below 2^-27 (kLoneHi), so the Allen-Cahn update is
-//     phi + kl lap phi - kw phi.
-// Compositions that are not finite (or above kBigHi, 2^64) take the general
-// forms, whose NaN propagation is the reference's.
-constexpr int kSolveHi = 0x3e7ad7f2;   // high word of 1e-7
-constexpr int kLinearHi = 0x3c300000;  // 2^-60
-constexpr int kLoneHi = 0x3e400000;    // 2^-27
-constexpr int kBigHi = 0x43f00000;     // 2^64
+//   kSolveHi: |phi| < 1e-7 in both phases.  p(phi) = 10 phi^3 < 1e-20, which
+//     shifts x^gamma by less than p (x_Cr + x_Nb + 1/3): less than half a last
+//     place of compositions above 3e-4, below 2e-20 of smaller ones.  But for
+//     that the general solve returns X, Y and is skipped;
+//   Coef64::linear_hi, lone_hi: the Allen-Cahn update is phi + kl lap phi - kw
+//     phi; what p' dP, the cubic terms of the double well and the coupling to
+//     the other phase add is below 2^-54 of phi (bounds that depend on the
+//     time step, the mobilities and the wells are formed with them).
+// Compositions of 2 and more (kBigHi), or not finite, take the general forms,
+// whose NaN propagation is the reference's.
+constexpr int kSolveHi = 0x3e7ad7f2;  // high word of 1e-7
+constexpr int kBigHi = 0x40000000;    // 2
 
 // high word without the sign: orders the magnitudes of doubles
 __device__ __forceinline__ int mag_hi(double v) { return __double2hiint(v) & 0x7fffffff; }

@@ -177,7 +177,7 @@ template <int I, class Lap, class Gam>
 __device__ __forceinline__ double phase64(const Coef64& K, const Cell64& c, bool none, Lap lap, Gam gamma) {
   if (none && !c.big) return 0.0;
   const double ph = I == 0 ? c.pd : c.pl, pj = I == 0 ? c.pl : c.pd;
-  if (mag_hi(ph) < kLinearHi && mag_hi(pj) < kLoneHi && !c.big)
+  if (mag_hi(ph) < K.linear_hi && mag_hi(pj) < K.lone_hi && !c.big)
     return allen_cahn_linear64<I>(K, ph, lap());
   constexpr double x1 = kXe[0][0], x2 = kXe[0][1];
   const double2 g = gamma();

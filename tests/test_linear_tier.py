@@ -1,0 +1,126 @@
+"""The FP64 step's linear Allen-Cahn form: what it leaves out stays below the
+rounding of the phase for the caller's time step, mobilities and wells, not
+only for the workloads'."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import PKG_DIR
+from pfa_gb300 import ic
+from test_tiers_gpu import around
+
+SOURCE = r"""
+#include "pfa_model.cpp"
+using namespace pfa;
+// p: dt, then per phase L, kappa, omega, then alpha; out: the two bounds and,
+// per phase, kw, ka and the five P
+extern "C" void coef(const double* p, double* out) {
+  ModelConst m{};
+  m.dt = p[0];
+  for (int i = 0; i < 2; i++) {
+    m.L[i] = p[1 + 3 * i];
+    m.kappa[i] = p[2 + 3 * i];
+    m.omega[i] = p[3 + 3 * i];
+  }
+  m.alpha = p[7];
+  const double mask[9] = {0, 1, 0, 1, -4, 1, 0, 1, 0};
+  Coef64 c;
+  model_coef64(m, mask, &c);
+  const int hi[2] = {c.linear_hi, c.lone_hi};
+  for (int k = 0; k < 2; k++) {
+    const unsigned long long b = (unsigned long long)(unsigned)hi[k] << 32;
+    std::memcpy(out + k, &b, sizeof(b));
+  }
+  for (int i = 0; i < 2; i++) {
+    out[2 + 7 * i] = c.kw[i];
+    out[3 + 7 * i] = c.ka[i];
+    for (int j = 0; j < 5; j++) out[4 + 7 * i + j] = c.P[i][j];
+  }
+}
+"""
+
+
+def test_bounds_follow_the_coefficients(pfa, tmp_path):
+    src, lib = tmp_path / "coef.cpp", tmp_path / "libcoef.so"
+    src.write_text(SOURCE)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(os.environ.get("NVCC", "nvcc")))))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(PKG_DIR, "csrc"),
+                    "-I", os.path.join(cuda, "include"), str(src), "-o", str(lib)], check=True)
+    L = ctypes.CDLL(str(lib))
+    p = pfa.model_params()
+
+    def coef(dt=1.0, lmob=1.0, omega=1.0, alpha=1.0):
+        a = [p["dt"] * dt]
+        for i in range(2):
+            a += [p["Lmob"][i] * lmob, p["kappa"][i], p["omega"][i] * omega]
+        a.append(p["alpha"] * alpha)
+        out = np.zeros(16)
+        L.coef(np.array(a, dtype=np.float64).ctypes.data_as(ctypes.c_void_p),
+               out.ctypes.data_as(ctypes.c_void_p))
+        return out[0], out[1], out[2:].reshape(2, 7)
+
+    assert coef()[:2] == (2.0 ** -60, 2.0 ** -27)  # the workloads'
+    for kw in (dict(), dict(alpha=2.0 ** 20), dict(alpha=-1e9), dict(lmob=2.0 ** 20, omega=0.0), dict(dt=1e6),
+               dict(omega=1e12), dict(dt=1e-9), dict(alpha=0.0), dict(dt=1e200), dict(alpha=1e150, dt=1e20)):
+        linear, lone, c = coef(**kw)
+        assert 0.0 <= linear <= 2.0 ** -60 and 0.0 <= lone <= 2.0 ** -27
+        for kwell, ka, c1, c2, c11, c12, c22 in c:
+            for u1 in np.linspace(-2.6, 2.6, 9):
+                for u2 in np.linspace(-2.6, 2.6, 9):
+                    P = u1 * (c1 + c11 * u1 + c12 * u2) + u2 * (c2 + c22 * u2)
+                    assert linear * abs(P + 3 * kwell) <= 2.0 ** -54
+            assert abs(ka) * lone ** 2 <= 2.0 ** -54
+    for kw in (dict(dt=np.nan), dict(alpha=np.inf)):
+        assert 0.0 in coef(**kw)[:2]  # the form is not taken
+
+
+# one phase below 2^-60, the other below 2^-27, with a coupling 2^20 times the
+# workloads' (one step stays finite); a single phase without well and gradient
+# whose driving force is 2^20 times theirs; compositions far outside [0, 1]
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["coupling", "force", "compositions"])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_linear_form(pfa, orc, case, dim):
+    shape = (40, 51) if dim == 2 else (6, 20, 31)
+    rng = np.random.default_rng(dim)
+    tiny = lambda: 2.0 ** rng.uniform(-62, -59.8, shape)
+    f = [rng.uniform(0.28, 0.33, shape), rng.uniform(0.02, 0.17, shape), tiny(), tiny()]
+    p, q = pfa.model_params(dim=dim), O.model_params(dim=dim)
+    change = {}
+    if case == "coupling":
+        a = 2.0 ** rng.uniform(-28, -26.8, shape)
+        swap = rng.random(shape) < 0.5
+        f[2], f[3] = np.where(swap, a, f[2]), np.where(swap, f[3], a)
+        change = dict(alpha=p["alpha"] * 2.0 ** 20)
+    elif case == "force":
+        change = dict(Lmob=[v * 2.0 ** 20 for v in p["Lmob"]], omega=[0.0, 0.0], kappa=[0.0, 0.0])
+    else:
+        f[0] = rng.choice([-1e9, 0.3, 1e9, 1e12], shape)
+    full = []
+    for a in f:
+        h = np.empty([n + 2 for n in shape])
+        h[(slice(1, -1),) * dim] = a
+        full.append(ic.mirror_halo(h))
+    for k, v in change.items():
+        p[k] = v
+        if isinstance(v, list):
+            getattr(q, k)[:] = v
+        else:
+            setattr(q, k, v)
+    g = (pfa.Grid2D if dim == 2 else pfa.Grid3D)(full, p)
+    g.run(1)
+    got = g.read()
+    g.close()
+    want = (orc.run2d if dim == 2 else orc.run3d)(full, q, 1)
+    core = (slice(1, -1),) * dim
+    # the update's few operations in either form; where compositions are large
+    # the driving force's 40, on terms that cancel to 1e-2 of themselves
+    rel = (64 if case != "compositions" else 4096) * 2.0 ** -53
+    for a, b, o in zip(got[2:], want[2:], full[2:]):
+        scale = np.maximum(around(o), np.abs(b))
+        assert np.all((np.abs(a - b) <= rel * scale)[core])
