@@ -236,7 +236,8 @@ int pfa3d_test_skip_plane(void* handle, int plane);
  * bit-for-bit as it would alone.  pfa_batch_footprint gives the arena bytes a
  * grid takes.  pfa_batch_tune times the launch shapes (rows per segment,
  * persistent or one warp per unit) on the current members without advancing
- * them and keeps the fastest; pfa_batch_set_launch fixes one. */
+ * them and keeps the fastest for as long as the members take the same kind of
+ * pass (one or two steps); pfa_batch_set_launch fixes one for both kinds. */
 size_t pfa_batch_footprint(int nx, int ny);
 int pfa_batch_create(void** handle, const double* params, const double* dxy, size_t arena_bytes);
 int pfa_batch_add(void* handle, int nx, int ny, const double* conc_Cr, const double* conc_Nb,

@@ -80,8 +80,10 @@ struct Batch {
   int* d_counter = nullptr;  // counters of parity 0 / 1, unit counts of both tables
   bool two = false;          // runs advance two steps per launch (refresh)
   bool dirty = true;
-  int rows = 0;          // rows per segment (0: by auto_rows)
-  int persistent = -1;   // 1: persistent launch, 0: one warp per unit, -1: by size (is_persistent)
+  // launch shapes of single steps [0] and of two steps in one pass [1]: each is
+  // tuned by itself, and is the batch's only while its members take that pass
+  int rows[2] = {0, 0};          // rows per segment (0: by auto_rows)
+  int persistent[2] = {-1, -1};  // 1: persistent launch, 0: one warp per unit, -1: by pass (is_persistent)
   int ctas = 0;          // CTAs of a persistent launch (0 = all resident)
   unsigned long long version = 1;  // bumps when the device tables move
   std::vector<BGraph> graphs;
@@ -181,6 +183,8 @@ int auto_rows(const Batch* b, bool two) {
   return 3 * std::max(2, int(std::sqrt(6.0 * load) / 3.0 + 0.5));
 }
 
+int segment_rows(const Batch* b, bool two) { return b->rows[two] > 0 ? b->rows[two] : auto_rows(b, two); }
+
 // The unit table for the current members and segment length: every grid's
 // rows are split into equal segments of at most `rows`; units are ordered by
 // decreasing length so that the counter hands out the long ones first.
@@ -200,7 +204,7 @@ void make_units(const Batch* b, int rows, bool two, std::vector<BatchUnit>* out)
   });
 }
 
-int upload_tables(Batch* b, int rows) {
+int upload_tables(Batch* b) {
   std::vector<BatchGrid> grids(b->slots.size());
   double bytes = 0.0;
   for (size_t i = 0; i < b->slots.size(); i++)
@@ -225,7 +229,7 @@ int upload_tables(Batch* b, int rows) {
     b->units[t] = 0;
     if (t == 1 && !b->two) continue;  // not launched
     std::vector<BatchUnit> units;
-    make_units(b, rows > 0 ? rows : auto_rows(b, t == 1), t == 1, &units);
+    make_units(b, segment_rows(b, t == 1), t == 1, &units);
     if (int(units.size()) > b->unit_cap[t]) {
       cudaStreamSynchronize(b->st);
       cudaFree(b->d_unit[t]);
@@ -249,13 +253,13 @@ int upload_tables(Batch* b, int rows) {
 
 int refresh(Batch* b) {
   if (!b->dirty) return 0;
-  if (int r = upload_tables(b, b->rows)) return r;
+  if (int r = upload_tables(b)) return r;
   b->dirty = false;
   return 0;
 }
 
 // small batches, in single steps, have one warp per unit
-int is_persistent(const Batch* b, bool two) { return b->persistent < 0 ? int(two) : b->persistent; }
+int is_persistent(const Batch* b, bool two) { return b->persistent[two] < 0 ? int(two) : b->persistent[two]; }
 
 int persistent_ctas(const Batch* b, bool two) {
   const int res = batch_resident_ctas(two);
@@ -675,8 +679,8 @@ int pfa_batch_set_launch(void* handle, int rows, int persistent, int ctas) {
   Batch* b = get(handle);
   if (!b) return fail(PFA_ESTATE, "pfa_batch_set_launch: null handle");
   if (rows < 1 || ctas < 0) return fail(PFA_EINVAL, "pfa_batch_set_launch: rows >= 1, ctas >= 0");
-  b->rows = rows;
-  b->persistent = persistent ? 1 : 0;
+  b->rows[0] = b->rows[1] = rows;
+  b->persistent[0] = b->persistent[1] = persistent ? 1 : 0;
   b->ctas = ctas;
   b->dirty = true;
   return 0;
@@ -687,7 +691,7 @@ int pfa_batch_get_launch(void* handle, int* rows, int* persistent, int* ctas, in
   if (!b) return fail(PFA_ESTATE, "pfa_batch_get_launch: null handle");
   if (int r = refresh(b)) return r;
   const bool two = b->two;
-  if (rows) *rows = b->rows > 0 ? b->rows : auto_rows(b, two);
+  if (rows) *rows = segment_rows(b, two);
   if (persistent) *persistent = is_persistent(b, two);
   if (ctas) *ctas = is_persistent(b, two) ? persistent_ctas(b, two) : (b->units[two] + batch_warps_per_cta() - 1) / batch_warps_per_cta();
   if (units) *units = b->units[two];
@@ -702,17 +706,17 @@ int pfa_batch_tune(void* handle, int reps, float* best_ms) {
   static const int kRows[2][9] = {{1, 2, 3, 6, 9, 12, 16, 24, 48},
                                   {9, 15, 24, 30, 36, 48, 64, 96, 1 << 30}};
   float best = -1.f;
-  int best_rows = b->rows, best_pers = b->persistent;
+  const bool two = b->two;  // the members decide, not the shape
+  int best_rows = b->rows[two], best_pers = b->persistent[two];
   cudaEvent_t e0, e1;
   CKB(cudaEventCreate(&e0));
   CKB(cudaEventCreate(&e1));
   for (int pers = 0; pers < 2; pers++) {
     for (int i = 0; i < 9; i++) {
-      const bool two = b->two;  // the members decide, not the shape
-      const int rows = kRows[two][i];
-      if (int r = upload_tables(b, rows)) return r;
+      b->rows[two] = kRows[two][i];
+      b->persistent[two] = pers;
+      if (int r = upload_tables(b)) return r;
       if (b->units[0] == 0) break;
-      b->persistent = pers;
       const int passes = two ? (reps + 1) / 2 : reps;  // of two steps or one
       // cur -> cur ^ 1 every time: the grids' state does not advance
       for (int k = 0; k < passes + 2; k++) {
@@ -727,15 +731,15 @@ int pfa_batch_tune(void* handle, int reps, float* best_ms) {
       t /= two ? 2 * passes : passes;
       if (best < 0.f || t < best) {
         best = t;
-        best_rows = rows;
+        best_rows = b->rows[two];
         best_pers = pers;
       }
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  b->rows = best_rows;
-  b->persistent = best_pers;
+  b->rows[two] = best_rows;
+  b->persistent[two] = best_pers;
   b->dirty = true;
   if (int r = refresh(b)) return r;
   if (best_ms) *best_ms = best;
