@@ -254,6 +254,9 @@ int pfa_batch_summarize(void* handle, int slot, double* out);
 int pfa_batch_tune(void* handle, int reps, float* best_ms);
 int pfa_batch_set_launch(void* handle, int rows, int persistent, int ctas);
 int pfa_batch_get_launch(void* handle, int* rows, int* persistent, int* ctas, int* units);
+/* step kernels that the batch's runs have enqueued so far (one per one or two
+ * steps, by the members) */
+int pfa_batch_step_launches(void* handle, uint64_t* launches);
 int pfa_batch_info(void* handle, int* grids, size_t* used_bytes, size_t* arena_bytes);
 void* pfa_batch_stream(void* handle);
 int pfa_batch_destroy(void* handle);

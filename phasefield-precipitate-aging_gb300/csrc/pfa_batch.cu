@@ -86,6 +86,7 @@ struct Batch {
   int persistent[2] = {-1, -1};  // 1: persistent launch, 0: one warp per unit, -1: by pass (is_persistent)
   int ctas = 0;          // CTAs of a persistent launch (0 = all resident)
   unsigned long long version = 1;  // bumps when the device tables move
+  uint64_t launches = 0;           // step kernels enqueued by runs
   std::vector<BGraph> graphs;
   cudaStream_t up = nullptr, down = nullptr;  // host -> device / device -> host copies
   cudaStream_t cv = nullptr;                  // conversions (high priority)
@@ -290,6 +291,7 @@ int run(Batch* b, int nsteps) {
     if (nsteps < 2 * per) {
       if (int r = launch(b, b->cur, two)) return r;
       b->cur ^= 1;
+      b->launches++;
       nsteps -= per;
       continue;
     }
@@ -327,6 +329,7 @@ int run(Batch* b, int nsteps) {
       b->graphs.push_back({len, b->cur, gsize, two, b->version, exec});
     }
     CKB(cudaGraphLaunch(exec, b->st));
+    b->launches += uint64_t(passes);
     nsteps -= len;  // even passes: the parity is back where it was
   }
   return 0;
@@ -767,6 +770,13 @@ int pfa_batch_summarize(void* handle, int slot, double* out) {
   CKB(launch_summarize(a, b->st));
   CKB(cudaMemcpyAsync(out, b->sum_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, b->st));
   CKB(cudaStreamSynchronize(b->st));
+  return 0;
+}
+
+int pfa_batch_step_launches(void* handle, uint64_t* launches) {
+  Batch* b = get(handle);
+  if (!b) return fail(PFA_ESTATE, "pfa_batch_step_launches: null handle");
+  if (launches) *launches = b->launches;
   return 0;
 }
 

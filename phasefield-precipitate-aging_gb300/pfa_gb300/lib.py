@@ -193,6 +193,7 @@ def load():
         "pfa_batch_tune": (_i, [ctypes.c_void_p, _i, _fp]),
         "pfa_batch_set_launch": (_i, [ctypes.c_void_p, _i, _i, _i]),
         "pfa_batch_get_launch": (_i, [ctypes.c_void_p] + [ctypes.POINTER(_i)] * 4),
+        "pfa_batch_step_launches": (_i, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)]),
         "pfa_batch_info": (_i, [ctypes.c_void_p, ctypes.POINTER(_i),
                                 ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)]),
         "pfa_batch_stream": (ctypes.c_void_p, [ctypes.c_void_p]),
@@ -738,6 +739,12 @@ class Batch:
               "pfa_batch_get_launch")
         return {"rows": v[0].value, "persistent": bool(v[1].value), "ctas": v[2].value,
                 "units": v[3].value}
+
+    def step_launches(self):
+        """Step kernels that the runs have enqueued so far."""
+        n = ctypes.c_uint64()
+        check(self.L.pfa_batch_step_launches(self.h, ctypes.byref(n)), "pfa_batch_step_launches")
+        return n.value
 
     def info(self):
         n, used, cap = _i(), ctypes.c_size_t(), ctypes.c_size_t()

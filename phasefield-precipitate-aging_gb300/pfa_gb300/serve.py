@@ -103,7 +103,9 @@ class GpuBackend:
 
     def advance(self, steps_2d, handles_2d, items_3d):
         """Enqueue steps_2d steps of the batch (whose members are handles_2d)
-        and each (handle, steps) 3D run, then wait for all of them."""
+        and each (handle, steps) 3D run, then wait for all of them; returns
+        the step kernels enqueued."""
+        before = self.batch.step_launches()
         for h, n in items_3d:
             if n > 0:
                 h[1].run(n)
@@ -112,6 +114,7 @@ class GpuBackend:
         self.batch.sync()
         for h, _ in items_3d:
             h[1].sync()
+        return self.batch.step_launches() - before + sum(n for _, n in items_3d)
 
     def retire(self, handle):
         """Read the result back and free the request's device memory."""
@@ -139,8 +142,8 @@ class Server:
         self.done: List[Record] = []
         self.ticks = 0
         self.cell_updates = 0
-        self.step_launches = 0  # least step kernels enqueued: one per two batch steps (a large batch's
-                                # launches advance two, a small one's one), one per 3D step
+        self.step_launches = 0  # step kernels enqueued, as the backend counts them (one per step
+                                # where it does not)
 
     def now(self):
         if self.t0 is None:
@@ -174,8 +177,8 @@ class Server:
         # the batch advances its members together: stop at the first end
         n2 = min([self.tick_steps] + [r.remaining for r in two]) if two else 0
         items3 = [(r.handle, min(self.tick_steps, r.remaining)) for r in three]
-        self.backend.advance(n2, [r.handle for r in two], items3)
-        self.step_launches += (n2 + 1) // 2 + sum(n for _, n in items3)
+        launches = self.backend.advance(n2, [r.handle for r in two], items3)
+        self.step_launches += n2 + sum(n for _, n in items3) if launches is None else launches
         for r in two:
             r.done_steps += n2
             self.cell_updates += n2 * r.req.cells
