@@ -65,7 +65,7 @@ inline int nucleation_cand_cap(size_t cells) {
 
 // Device scratch of a nucleation handle: events, counters, status, list.
 inline size_t nucleation_scratch_bytes(size_t cells) {
-  return nucleation_event_bytes() + 2 * sizeof(unsigned) + sizeof(int) +
+  return nucleation_event_bytes() + kNucCounters * sizeof(unsigned) + sizeof(int) +
          sizeof(unsigned long long) + sizeof(long long) * size_t(nucleation_cand_cap(cells));
 }
 
