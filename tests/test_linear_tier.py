@@ -12,6 +12,7 @@ import pytest
 import oracle as O
 from conftest import PKG_DIR
 from pfa_gb300 import ic
+from test_fixed64_gpu import step_and_oracle
 from test_tiers_gpu import around
 
 SOURCE = r"""
@@ -43,6 +44,16 @@ extern "C" void coef(const double* p, double* out) {
   }
 }
 """
+
+
+def reach(a, corners):
+    """Largest magnitude a step reads around each cell."""
+    m = around(a)
+    if corners:
+        for s in (-1, 1):
+            for t in (-1, 1):
+                m = np.maximum(m, np.abs(np.roll(np.roll(a, s, axis=0), t, axis=1)))
+    return m
 
 
 def test_bounds_follow_the_coefficients(pfa, tmp_path):
@@ -124,3 +135,34 @@ def test_linear_form(pfa, orc, case, dim):
     for a, b, o in zip(got[2:], want[2:], full[2:]):
         scale = np.maximum(around(o), np.abs(b))
         assert np.all((np.abs(a - b) <= rel * scale)[core])
+
+
+# phases from 1e-40 to just below 1e-7, dense at the forms' lines, zero in
+# patches: no cell has a solve, so a step rounds each result once in either
+# form, and its increments (below 1/100 of the values around) a few times more:
+# four last halves of the largest value of the neighbourhood cover both sides
+@pytest.mark.gpu
+@pytest.mark.parametrize("mask", ["iso", "nine", "five", "variable", "3d"])
+@pytest.mark.parametrize("large", [False, True])
+def test_forms_without_a_solve(pfa, orc, mask, large):
+    if mask == "3d":
+        shape = (70, 248, 248) if large else (9, 40, 37)
+    else:
+        shape = (905, 1000) if large else (93, 130)
+    rng = np.random.default_rng(17)
+    f = [rng.uniform(0.28, 0.33, shape), rng.uniform(0.02, 0.17, shape)]
+    for _ in range(2):
+        a = 2.0 ** np.where(rng.random(shape) < 0.5, rng.uniform(-133, -23.5, shape),
+                            rng.choice([-60.0, -27.0], shape) + rng.uniform(-0.3, 0.3, shape))
+        a = np.minimum(a, 0.99e-7)
+        patch = tuple(np.arange(n) // 16 for n in shape)
+        zero = rng.random([n // 16 + 1 for n in shape]) < 0.4
+        a[zero[np.ix_(*patch)]] = 0.0
+        f.append(a)
+    got, want = step_and_oracle(pfa, orc, mask, f)
+    core = (slice(1, -1),) * len(shape)
+    for a, b, o in zip(got, want, f):
+        h = np.empty([n + 2 for n in shape])
+        h[core] = o
+        scale = np.maximum(reach(ic.mirror_halo(h), mask == "nine"), np.abs(b))
+        assert np.all((np.abs(a - b) <= 4 * 2.0 ** -53 * scale)[core])
