@@ -189,6 +189,9 @@ __device__ void paint(const NucArgs& a, const NucEvent& e, int ph) {
     }
     return;
   }
+  // A box wider than a row reaches a cell again from one row up (j - 1, i +
+  // nxr); in the reference's serial order, i then j ascending, the later visit
+  // counts.  Each visit leaves to it what it writes.
   const long long n = (long long)w * w;
   for (long long t = threadIdx.x; t < n; t += blockDim.x) {
     const int i = lo + int(t / w), j = lo + int(t % w);
@@ -199,7 +202,18 @@ __device__ void paint(const NucArgs& a, const NucEvent& e, int ph) {
     if (a.compact && (xx == 0 || yy == 0 || xx == nxr - 1 || yy == a.Ny + 1)) continue;
     const size_t s = stor(a, xx, yy);
     const double r = sqrt(double(i * i + j * j));
-    if (r <= R) {
+    if (w > nxr) {
+      bool inside = r <= R, cr = inside || r <= RdCr, nb = inside || r <= RdNb;
+      for (int u = i + nxr, v = j - 1; u < hi && v >= lo; u += nxr, v--) {
+        const double later = sqrt(double(u * u + v * v));
+        if (later <= R) inside = cr = nb = false;
+        if (later <= RdCr) cr = false;
+        if (later <= RdNb) nb = false;
+      }
+      if (cr) put<T>(a, 0, s, r <= R ? parCr : xgCr);
+      if (nb) put<T>(a, 1, s, r <= R ? parNb : xgNb);
+      if (inside) put<T>(a, 2 + ph, s, 1.0);
+    } else if (r <= R) {
       put<T>(a, 0, s, parCr);
       put<T>(a, 1, s, parNb);
       put<T>(a, 2 + ph, s, 1.0);
