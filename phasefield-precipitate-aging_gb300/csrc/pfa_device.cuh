@@ -178,14 +178,16 @@ __device__ __forceinline__ double dlap64(double Dl, double Dm, double Dh, double
 //     shifts x^gamma by less than p (x_Cr + x_Nb + 1/3): less than half a last
 //     place of compositions above 3e-4, below 2e-20 of smaller ones.  But for
 //     that the general solve returns X, Y and is skipped;
-//   Coef64::linear_hi, lone_hi: the Allen-Cahn update is phi + kl lap phi - kw
-//     phi; what p' dP, the cubic terms of the double well and the coupling to
-//     the other phase add is below 2^-54 of phi (bounds that depend on the
-//     time step, the mobilities and the wells are formed with them).
+//   kLinearHi: |phi| < 2^-60, the other phase below 2^-27 (kLoneHi).  The
+//     Allen-Cahn update is phi + kl lap phi - kw phi; what p' dP, the cubic
+//     terms of the double well and the coupling to the other phase add is below
+//     2^-54 of phi, or the form is not taken (Coef64::linear).
 // Compositions of 2 and more (kBigHi), or not finite, take the general forms,
 // whose NaN propagation is the reference's.
-constexpr int kSolveHi = 0x3e7ad7f2;  // high word of 1e-7
-constexpr int kBigHi = 0x40000000;    // 2
+constexpr int kSolveHi = 0x3e7ad7f2;   // high word of 1e-7
+constexpr int kLinearHi = 0x3c300000;  // 2^-60
+constexpr int kLoneHi = 0x3e400000;    // 2^-27
+constexpr int kBigHi = 0x40000000;     // 2
 
 // high word without the sign: orders the magnitudes of doubles
 __device__ __forceinline__ int mag_hi(double v) { return __double2hiint(v) & 0x7fffffff; }

@@ -22,10 +22,9 @@ namespace {
 
 // A phase below 2^-600 adds nothing: its square is below the least double.
 constexpr int kNoneHi = (1023 - 600) << 20;
-// Below 2^-60 a phase's p (2^-176) adds nothing to gamma's energy, and its
-// coupling to the other phase, 2 Omega / omega 2^-120 of the other's well, to
-// that.
-constexpr int kLinearHi = (1023 - 60) << 20;
+// Below 2^-60 (kLinearHi) a phase's p (2^-176) adds nothing to gamma's energy,
+// and its coupling to the other phase, 2 Omega / omega 2^-120 of the other's
+// well, nothing to that.
 
 // omega phi^2 (1 - phi)^2
 __device__ __forceinline__ double well64(double omega, double ph, double sq) {

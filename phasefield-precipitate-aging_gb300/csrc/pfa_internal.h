@@ -65,12 +65,11 @@ struct Coef64 {
   double D[2][2];
   double kl[2], kw[2], ka[2];
   double P[2][5];  // c1 c2 c11 c12 c22
-  // High words of the phase magnitudes below which a phase takes the linear
-  // update phi + kl lap phi - kw phi: its own, and the other phase's.  At most
-  // 2^-60 and 2^-27, and as much smaller as these coefficients need for the
-  // terms left out, phi^2 (P + 3 kw) and ka phi phi_j^2, to stay below 2^-54
-  // phi.
-  int linear_hi, lone_hi;
+  // Whether a phase below 2^-60 beside one below 2^-27 may take the linear
+  // update phi + kl lap phi - kw phi: the terms left out, phi^2 (P + 3 kw) and
+  // ka phi phi_j^2, are then below 2^-54 phi.  (Bounds that follow the
+  // coefficients would cost the 9-point step 3 % in registers.)
+  int linear;
   // neighbour weights: kMaskIso: faces equal, lap = weight (sum of the faces
   // + iso_c centre); kMaskIso9: faces four times the corners, lap = weight (4
   // faces + corners + iso_c centre); the weight is folded into D and kl.  Both

@@ -5,7 +5,6 @@
 // (set_diffusion_matrix, src/alloy625.cpp:80-109), kappa and omega
 // (src/parameters.h:42-48), the Allen-Cahn mobility and the time step, plus
 // the derived coefficients of the FP32 fast path.
-#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -118,15 +117,6 @@ static void model_dP(double dP[2][6]) {
   }
 }
 
-// High word of the largest power of two that is at most v and 2^most (0, which
-// no magnitude is below, where there is none)
-static int bound_hi(double v, int most) {
-  if (!(v > 0.0)) return 0;
-  int e;
-  std::frexp(std::fmin(v, 1.0), &e);  // 2^(e - 1) <= v
-  return std::max(std::min(e - 1, most) + 1023, 0) << 20;
-}
-
 void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
   std::memset(o, 0, sizeof(*o));
   double dP[2][6];
@@ -187,8 +177,7 @@ void model_coef64(const ModelConst& m, const double* mask9, Coef64* o) {
     cubic += P + 3.0 * std::fabs(o->kw[i]);
     coupling += std::fabs(o->ka[i]);
   }
-  o->linear_hi = bound_hi(0x1p-54 / cubic, -60);
-  o->lone_hi = bound_hi(std::sqrt(0x1p-54 / coupling), -27);
+  o->linear = cubic <= 0x1p6 && coupling <= 1.0;  // 2^-60 cubic, 2^-54 coupling: 2^-54 at most
   const double r2x = 0.5 * m.dt * m.idx2[0];
   o->vm_pre[0] = kMobPreNb * r2x;
   o->vm_pre[1] = kMobPreCr * r2x;

@@ -146,17 +146,16 @@ __device__ __forceinline__ Cell64 cell64(double X, double Y, double pd, double p
     // (the bounds of the ranges used here have no low word)
     const int low = __double2hiint(double(-range.low) * 0x1p-60), most = __double2hiint(double(range.most) * 0x1p-60);
     auto out = [&](double g) { return mag_hi(g) >= (__double2hiint(g) < 0 ? low : most); };
-    if (c.solved && (out(g1) || out(g2))) c.wide = true;
-    if (c.wide) {
-      c.g1 = __double_as_longlong(g1);
-      c.g2 = __double_as_longlong(g2);
-    } else if (c.solved) {
-      c.g1 = fix58_signed(g1);
-      c.g2 = fix58_signed(g2);
+    bool fixed = !c.wide;
+    if (c.solved) {
+      fixed = fixed && !out(g1) && !out(g2);
+      c.g1 = fixed ? fix58_signed(g1) : __double_as_longlong(g1);
+      c.g2 = fixed ? fix58_signed(g2) : __double_as_longlong(g2);
     } else {
-      c.g1 = fix58(X);
-      c.g2 = fix58(Y);
+      c.g1 = fixed ? fix58(X) : __double_as_longlong(X);
+      c.g2 = fixed ? fix58(Y) : __double_as_longlong(Y);
     }
+    c.wide = !fixed;
   }
   return c;
 }
@@ -177,7 +176,7 @@ template <int I, class Lap, class Gam>
 __device__ __forceinline__ double phase64(const Coef64& K, const Cell64& c, bool none, Lap lap, Gam gamma) {
   if (none && !c.big) return 0.0;
   const double ph = I == 0 ? c.pd : c.pl, pj = I == 0 ? c.pl : c.pd;
-  if (mag_hi(ph) < K.linear_hi && mag_hi(pj) < K.lone_hi && !c.big)
+  if (mag_hi(ph) < kLinearHi && mag_hi(pj) < kLoneHi && !c.big && K.linear)
     return allen_cahn_linear64<I>(K, ph, lap());
   constexpr double x1 = kXe[0][0], x2 = kXe[0][1];
   const double2 g = gamma();
