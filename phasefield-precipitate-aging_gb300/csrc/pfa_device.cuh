@@ -1,9 +1,11 @@
 // pfa_device.cuh -- device-side model functions of libpfa_gb300.
 //
-// FP64 functions follow the reference's generated formulas term by term
-// (thermo/parabola625.c; device copies src/parabola625.cu) so that the plain
-// FP64 step stays within 1e-12 of the reference.  FP32 helpers evaluate the
-// reduced forms whose coefficients pfa_model.cpp derives (pfa::FastCoef).
+// The first FP64 functions follow the reference's generated formulas term by
+// term (thermo/parabola625.c; device copies src/parabola625.cu): the compat
+// stages, the energy next to precipitates and the nucleation decisions use
+// them.  The fused FP64 steps take the reduced forms below ("FP64 step"), within
+// 1e-12 of the reference.  FP32 helpers evaluate the reduced forms whose
+// coefficients pfa_model.cpp derives (pfa::FastCoef).
 #pragma once
 
 #include <cuda_runtime.h>

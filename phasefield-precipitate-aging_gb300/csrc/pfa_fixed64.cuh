@@ -12,8 +12,8 @@
 //     operations with their three exponentials.  Error at most 1.6 (FP64: up
 //     to 30 and, near x_Ni = 0, 4e4); 512^2 73.9 -> 38.9 us a step.
 //   diffusivities: the matrix of that step, 26 operations.  Error in the usual
-//     range of compositions, units of 2^-60: at most 0.9, 0.06 on average (FP64:
-//     18 and 0.9); with the fluxes 512^2 38.9 -> 20.8 us a step.
+//     range of compositions, units of 2^-60: at most 1.6, 0.07 on average (FP64:
+//     22 and 1.1); with the fluxes 512^2 38.9 -> 20.9 us a step.
 // Compiles as host code too.
 #pragma once
 

@@ -13,8 +13,8 @@
 // arithmetic is in the reduced forms of pfa_device.cuh: no FP64 operations in
 // a cell where both phases are exactly zero around it, 7 per phase in the
 // phases' far tails, about 65 next to a precipitate (the reference's
-// expressions: about 300 everywhere).  us a step: 4096^2 with 4 particles 7780
-// -> 277, 2048^2 1950 -> 67, 256^2 38.8 -> 6.5.
+// expressions: about 300 everywhere).  us a step with 4 particles: 4096^2 7780
+// -> 248, 2048^2 1950 -> 65, 256^2 38.4 -> 6.1.
 //
 // Layout: the reference's, (Ny + 2) rows of pitch elements with a one-cell
 // ghost ring, interior cell (x, y) at (y + 1) * pitch + x + 1.  The FP32
@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(Tile2<MASK, TX, TY>::kThreads, blocks2(Tile2<M
 // is in range: u in units of 2^-58, D of 2^-67 (pfa_fixed64.cuh), the fluxes of
 // 2^-65, whose sum is rounded once into the composition (a sum that leaves 64
 // bits is formed in FP64); else, and with other spacings, in FP64.  Bound by integer issue; with the matrix and
-// the fluxes in FP64, bound by that pipe, 512^2 took 38.9 us a step for 20.8,
-// 2048^2 521 for 237.
+// the fluxes in FP64, bound by that pipe, 512^2 took 38.9 us a step for 20.9,
+// 2048^2 521 for 236.
 struct Matrix64 {
   double d[4];
 };

@@ -494,12 +494,12 @@ __device__ __forceinline__ Raw<PACK> mirrored(const Raw<PACK>& r, int lane) {
 // lanes 1 .. 30, the second on 2 .. 29.  A once-advanced record beyond the
 // domain mirrors the one at its edge.
 //
-// Bound: latency and issue (106 instructions a cell and step, 58 % of the
+// Bound: latency and issue (124 instructions a cell and step, 74 % of the
 // issue slots; HBM would allow 60 us a step at 4096^2).  Rows come through a
 // per-warp cp.async ring, which holds the row whose first step is due besides
 // the rows ahead and so leaves 80 registers without spills, 6 CTAs per SM
 // (rows in registers, one ahead: 89.8 us; 7 or 8 CTAs with spills: 118 and
-// 101).  4096^2: 129 us a step in single steps -> 76; FP32 compensations 176
+// 101).  4096^2: 129 us a step in single steps -> 71.7; FP32 compensations 176
 // -> 85, 9 points 131 -> 91; 2048^2 35.3 -> 22.8.
 constexpr int kCols2 = 28;
 constexpr int kDepth2 = 8;  // rows in the ring (a power of two)
